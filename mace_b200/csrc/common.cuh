@@ -139,6 +139,20 @@ static inline cudaError_t mb_launch_chained(mb_context *ctx, void (*kern)(KArgs.
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Division of a dividend below 2^31 by a divisor fixed at launch: with s = ceil(log2 d) and
+// m = ceil(2^(31 + s) / d) (which fits 32 bits), floor(n / d) = (n * m) >> (31 + s) for every
+// n < 2^31, because m * d - 2^(31 + s) < d <= 2^s.  d = 1 is encoded as m = 0.
+static inline void fast_div_make(uint32_t d, uint32_t *mul, uint32_t *shift) {
+  if (d <= 1) { *mul = 0; *shift = 0; return; }
+  uint32_t s = 0;
+  while ((1ull << s) < d) ++s;
+  *mul = static_cast<uint32_t>(((1ull << (31 + s)) + d - 1) / d);
+  *shift = s - 1;
+}
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t mul, uint32_t shift) {
+  return mul == 0 ? n : (__umulhi(n, mul) >> shift);
+}
+
 // ---- requantization arithmetic ---------------------------------------------
 // gemmlowp's output stage as MACE wires it (mace/ops/common/gemmlowp_util.h:
 // 37-74): SaturatingRoundingDoublingHighMul, RoundingDivideByPOT, + offset,

@@ -41,20 +41,6 @@ struct ConvParams {
   uint32_t wo_mul, wo_shift, ho_mul, ho_shift;
 };
 
-// Division of a dividend below 2^31 by a divisor fixed at launch: with s = ceil(log2 d) and
-// m = ceil(2^(31 + s) / d) (which fits 32 bits), floor(n / d) = (n * m) >> (31 + s) for every
-// n < 2^31, because m * d - 2^(31 + s) < d <= 2^s.  d = 1 is encoded as m = 0.
-static inline void fast_div_make(uint32_t d, uint32_t *mul, uint32_t *shift) {
-  if (d <= 1) { *mul = 0; *shift = 0; return; }
-  uint32_t s = 0;
-  while ((1ull << s) < d) ++s;
-  *mul = static_cast<uint32_t>(((1ull << (31 + s)) + d - 1) / d);
-  *shift = s - 1;
-}
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t mul, uint32_t shift) {
-  return mul == 0 ? n : (__umulhi(n, mul) >> shift);
-}
-
 // Direct convolution: thread = one output pixel, OT output channels at a time.
 // Filter (zero point removed, int16) lives in shared memory as [depth][O].
 template <int OT>

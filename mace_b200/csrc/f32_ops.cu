@@ -1,9 +1,8 @@
-// fp32 kernels of the path: batched GEMM, GEMV, general direct Conv2D and
-// depthwise conv in NCHW, with bias and activation fused into the epilogue.
+// fp32 kernels of the path: batched GEMM, GEMV and general Conv2D in NCHW, with bias and
+// activation fused into the epilogue (depthwise: dwconv_f32.cu).
 //
-// Reference behaviour: ref::Gemm / ref::Gemv / ref::Conv2d / ref::DepthwiseConv2d
-// (mace/ops/ref/gemm.cc:57-106, gemv.cc:45-81, conv_2d.cc:36-122,
-// depthwise_conv_2d.cc:36-125), ref::BiasAdd (bias_add.cc:74-103) and
+// Reference behaviour: ref::Gemm / ref::Gemv / ref::Conv2d (mace/ops/ref/gemm.cc:57-106,
+// gemv.cc:45-81, conv_2d.cc:36-122), ref::BiasAdd (bias_add.cc:74-103) and
 // ref::Activation (activation.cc:61-88).  The reference accumulates in fp32 in
 // index order; these kernels accumulate in fp32 in a tiled order, so results
 // agree to rounding (tests bound the difference at 1e-4 of the output range).
@@ -17,6 +16,11 @@ int mb_gemm_f32_tc_launch(mb_context *ctx, const float *X, const float *W, const
                           int64_t x_batch_stride, int64_t w_row_stride, int64_t w_batch_stride,
                           int64_t c_row_stride, int64_t c_batch_stride, int act, float max_limit,
                           float coef, const float *residual);
+
+int mb_dwconv_f32_launch(mb_context *ctx, const float *in, const float *filter, const float *bias, float *out,
+                         int64_t N, int64_t C, int64_t H, int64_t W, int64_t mult_ch, int64_t KH, int64_t KW,
+                         int stride_h, int stride_w, int dil_h, int dil_w, int pad_top, int pad_left, int64_t Ho,
+                         int64_t Wo, int activation, float max_limit, float coefficient);
 
 namespace {
 
@@ -105,11 +109,11 @@ gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs,
   }
 }
 
-// ---- direct convolutions ------------------------------------------------------------
+// ---- direct convolution ------------------------------------------------------------
 struct ConvF32Params {
   const float *in, *filter, *bias;
   float *out;
-  int N, C, H, W, O, KH, KW, sh, sw, dh, dw, pad_t, pad_l, Ho, Wo, mult_ch;
+  int N, C, H, W, O, KH, KW, sh, sw, dh, dw, pad_t, pad_l, Ho, Wo;
   int act;
   float max_limit, coef;
 };
@@ -137,34 +141,6 @@ __global__ void __launch_bounds__(256) conv2d_f32_direct_kernel(const ConvF32Par
         if (iw < 0 || iw >= p.W) continue;
         sum = fmaf(__ldg(ib + ih * p.W + iw), __ldg(fp + kh * p.KW + kw), sum);
       }
-    }
-  }
-  if (p.bias != nullptr) sum += p.bias[m];
-  p.out[tid] = mb_activate(sum, p.act, p.max_limit, p.coef);
-}
-
-__global__ void __launch_bounds__(256) dwconv_f32_kernel(const ConvF32Params p) {
-  const int OC = p.C * p.mult_ch;
-  const int64_t total = static_cast<int64_t>(p.N) * OC * p.Ho * p.Wo;
-  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (tid >= total) return;
-  const int w = static_cast<int>(tid % p.Wo);
-  int64_t r = tid / p.Wo;
-  const int h = static_cast<int>(r % p.Ho);
-  r /= p.Ho;
-  const int m = static_cast<int>(r % OC);
-  const int n = static_cast<int>(r / OC);
-  const int c = m / p.mult_ch, o = m % p.mult_ch;
-  const float *ib = p.in + (static_cast<int64_t>(n) * p.C + c) * p.H * p.W;
-  const float *fp = p.filter + (static_cast<int64_t>(o) * p.C + c) * p.KH * p.KW;
-  float sum = 0.f;
-  for (int kh = 0; kh < p.KH; ++kh) {
-    const int ih = -p.pad_t + h * p.sh + kh * p.dh;
-    if (ih < 0 || ih >= p.H) continue;
-    for (int kw = 0; kw < p.KW; ++kw) {
-      const int iw = -p.pad_l + w * p.sw + kw * p.dw;
-      if (iw < 0 || iw >= p.W) continue;
-      sum = fmaf(__ldg(ib + ih * p.W + iw), __ldg(fp + kh * p.KW + kw), sum);
     }
   }
   if (p.bias != nullptr) sum += p.bias[m];
@@ -497,7 +473,7 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
   p.N = static_cast<int>(N); p.C = static_cast<int>(C); p.H = static_cast<int>(H); p.W = static_cast<int>(W);
   p.O = static_cast<int>(O); p.KH = static_cast<int>(KH); p.KW = static_cast<int>(KW);
   p.sh = stride_h; p.sw = stride_w; p.dh = dil_h; p.dw = dil_w; p.pad_t = pad_top; p.pad_l = pad_left;
-  p.Ho = static_cast<int>(Ho); p.Wo = static_cast<int>(Wo); p.mult_ch = 1;
+  p.Ho = static_cast<int>(Ho); p.Wo = static_cast<int>(Wo);
   p.act = activation; p.max_limit = max_limit; p.coef = coefficient;
   const int64_t total = N * O * Ho * Wo;
   conv2d_f32_direct_kernel<<<static_cast<unsigned>(ceil_div64(total, 256)), 256, 0, ctx->stream>>>(p);
@@ -549,18 +525,8 @@ int mb_dwconv_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
                                     pad_left, Ho, Wo, activation, &empty));
   if (empty) return MB_SUCCESS;
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  ConvF32Params p;
-  p.in = in; p.filter = filter; p.bias = bias; p.out = out;
-  p.N = static_cast<int>(N); p.C = static_cast<int>(C); p.H = static_cast<int>(H); p.W = static_cast<int>(W);
-  p.O = static_cast<int>(C * mult_ch); p.KH = static_cast<int>(KH); p.KW = static_cast<int>(KW);
-  p.sh = stride_h; p.sw = stride_w; p.dh = dil_h; p.dw = dil_w; p.pad_t = pad_top; p.pad_l = pad_left;
-  p.Ho = static_cast<int>(Ho); p.Wo = static_cast<int>(Wo); p.mult_ch = static_cast<int>(mult_ch);
-  p.act = activation; p.max_limit = max_limit; p.coef = coefficient;
-  const int64_t total = N * C * mult_ch * Ho * Wo;
-  dwconv_f32_kernel<<<static_cast<unsigned>(ceil_div64(total, 256)), 256, 0, ctx->stream>>>(p);
-  MB_CUDA(ctx, cudaGetLastError());
-  ctx->launches++;
-  return MB_SUCCESS;
+  return mb_dwconv_f32_launch(ctx, in, filter, bias, out, N, C, H, W, mult_ch, KH, KW, stride_h, stride_w, dil_h,
+                              dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);
 }
 
 }  // extern "C"

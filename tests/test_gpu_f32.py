@@ -187,6 +187,27 @@ def test_winograd_f32(ctx, orc, case):
     assert np.array_equal(ctx.download(do, direct.shape, np.float32), got)
 
 
+@pytest.mark.parametrize("k", [3, 5])
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("shape", [(1, 3, 7, 9, 1), (2, 300, 33, 31, 1), (3, 5, 20, 65, 2), (4, 130, 57, 112, 1),
+                                   (8, 96, 56, 56, 1)])
+def test_dwconv_f32_rows(ctx, orc, k, stride, shape):
+    """The rows-per-thread kernel: every run length (the batch sizes make all of them reachable),
+    ragged last runs, narrow maps, a channel multiplier."""
+    N, C, H, W, mult = shape
+    rng = np.random.Generator(np.random.PCG64(C + k))
+    x = rng.standard_normal((N, C, H, W)).astype(np.float32)
+    f = rng.standard_normal((mult, C, k, k)).astype(np.float32)
+    bias = rng.standard_normal(C * mult).astype(np.float32)
+    ho, wo, ph, pw = orc.calc_padding_and_output_size(H, W, k, k, (1, 1), (stride, stride), 1)
+    ref = orc.dwconv_f32(x, f, bias, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
+    dx, df, db, do = ctx.upload(x), ctx.upload(f), ctx.upload(bias), ctx.alloc(ref.nbytes)
+    ctx.dwconv_f32(dx, df, db, do, N, C, H, W, mult, k, k, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
+    assert rel_err(ctx.download(do, ref.shape, np.float32), ref, 1e-5, "dwconv_f32") <= 1e-5
+    for b in (dx, df, db, do):
+        b.free()
+
+
 def test_dwconv_f32(ctx, orc, kats):
     k = kats["dwconv_f32_2x2_valid"]  # SimpleValidTest, depthwise_conv2d_test.cc:26-84
     x = np.transpose(np.array(k["input"], np.float32).reshape(1, 3, 3, 2), (0, 3, 1, 2)).copy()
