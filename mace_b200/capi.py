@@ -1,4 +1,5 @@
-"""ctypes binding of ``libmace_b200.so`` (the C ABI of include/mace_b200.h)."""
+"""Binding of ``libmace_b200.so`` (the C ABI of include/mace_b200.h): ctypes for everything, and the
+``_pycall`` extension module for the operators that Context calls (see csrc/pycall.cc)."""
 import ctypes as C
 import os
 import subprocess
@@ -107,6 +108,7 @@ PROTOTYPES = {
 }
 
 _lib = None
+_ops = None  # the _pycall module, loaded with the library
 
 
 def lib():
@@ -118,6 +120,9 @@ def lib():
                 "libmace_b200.so is missing: run `python -c 'import __graft_entry__ as g; "
                 "g.build()'` (or make -C mace_b200/csrc). There is no CPU fallback.")
         _lib = C.CDLL(_LIB)
+        from . import _pycall  # built with the library; raises ImportError when it is missing
+        global _ops
+        _ops = _pycall
         for name, (res, args) in PROTOTYPES.items():
             fn = getattr(_lib, name)
             fn.restype = res
@@ -149,6 +154,7 @@ class Context:
         st = lib().mb_init(int(device), C.byref(self.h))
         if st != 0:
             raise MaceB200Error(st, "mb_init failed (no sm_100a CUDA device?)")
+        self._p = self.h.value
         self._bufs = []
 
     def _check(self, st):
@@ -162,7 +168,7 @@ class Context:
             for p in getattr(self, "_pinned", []):
                 lib().mb_host_free(self.h, p)
             lib().mb_destroy(self.h)
-            self.h = None
+            self.h = self._p = None
 
     def __enter__(self):
         return self
@@ -195,7 +201,7 @@ class Context:
         return out
 
     def sync(self):
-        self._check(lib().mb_stream_sync(self.h))
+        self._check(_ops.mb_stream_sync(self._p))
 
     def event(self):
         e = _vp()
@@ -249,8 +255,7 @@ class Context:
     def gemm_u8(self, A, B, bias, Cout, batch, M, N, K, zp_a, zp_b, mult=1 << 30, shift=0,
                 zp_c=0, a_col_major=False, b_col_major=False, c_col_major=False,
                 a_batched=True, b_batched=True, out_int32=False, bias_per_row=False):
-        self._check(lib().mb_gemm_u8(
-            self.h, A.ptr, B.ptr, bias.ptr if bias is not None else None, Cout.ptr,
+        self._check(_ops.mb_gemm_u8(self._p, A.ptr, B.ptr, bias.ptr if bias is not None else None, Cout.ptr,
             int(out_int32), batch, M, N, K, int(a_col_major), int(b_col_major),
             int(c_col_major), int(a_batched), int(b_batched), zp_a, zp_b, mult, shift, zp_c,
             int(bias_per_row)))
@@ -258,15 +263,14 @@ class Context:
     def gemv_u8(self, lhs, rhs, bias, out, batch, rows, K, zp_l, zp_r, multiplier=0.0,
                 zp_out=0, add_zp_out=True, lhs_batched=False, rhs_batched=True,
                 out_int32=False):
-        self._check(lib().mb_gemv_u8(
-            self.h, lhs.ptr, rhs.ptr, bias.ptr if bias is not None else None, out.ptr,
+        self._check(_ops.mb_gemv_u8(self._p, lhs.ptr, rhs.ptr, bias.ptr if bias is not None else None, out.ptr,
             int(out_int32), batch, rows, K, int(lhs_batched), int(rhs_batched), zp_l, zp_r,
             float(multiplier), zp_out, int(add_zp_out)))
 
     def conv2d_u8(self, x, f, bias, out, N, H, W, Cc, O, KH, KW, strides, pad_tl, out_hw,
                   zp_in, zp_f, mult, shift, zp_out):
-        self._check(lib().mb_conv2d_u8_nhwc(
-            self.h, x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, H, W, Cc,
+        self._check(_ops.mb_conv2d_u8_nhwc(self._p,
+            x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, H, W, Cc,
             O, KH, KW, strides[0], strides[1], pad_tl[0], pad_tl[1], out_hw[0], out_hw[1],
             zp_in, zp_f, mult, shift, zp_out))
 
@@ -284,54 +288,53 @@ class Context:
                   zp_in, zp_f, mult=1 << 30, shift=0, zp_out=0, float_multiplier=None,
                   prepacked=None):
         if prepacked is not None:
-            self._check(lib().mb_dwconv_u8_nhwc_prepacked(
-                self.h, x.ptr, f.ptr, bias.ptr if bias is not None else None, prepacked.ptr,
+            self._check(_ops.mb_dwconv_u8_nhwc_prepacked(self._p,
+                x.ptr, f.ptr, bias.ptr if bias is not None else None, prepacked.ptr,
                 out.ptr, N, H, W, Cc, Mc, KH, KW, strides[0], strides[1], dil[0], dil[1],
                 pad_tl[0], pad_tl[1], out_hw[0], out_hw[1], zp_in, zp_f, mult, shift, zp_out,
                 int(float_multiplier is not None), float(float_multiplier or 0.0)))
             return
-        self._check(lib().mb_dwconv_u8_nhwc(
-            self.h, x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, H, W, Cc,
+        self._check(_ops.mb_dwconv_u8_nhwc(self._p,
+            x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, H, W, Cc,
             Mc, KH, KW, strides[0], strides[1], dil[0], dil[1], pad_tl[0], pad_tl[1],
             out_hw[0], out_hw[1], zp_in, zp_f, mult, shift, zp_out,
             int(float_multiplier is not None), float(float_multiplier or 0.0)))
 
     def gemm_f32(self, A, B, Cout, batch, M, N, K, a_col_major=False, b_col_major=False,
                  c_col_major=False, a_batched=True, b_batched=True):
-        self._check(lib().mb_gemm_f32(self.h, A.ptr, B.ptr, Cout.ptr, batch, M, N, K,
+        self._check(_ops.mb_gemm_f32(self._p, A.ptr, B.ptr, Cout.ptr, batch, M, N, K,
                                       int(a_col_major), int(b_col_major), int(c_col_major),
                                       int(a_batched), int(b_batched)))
 
     def gemv_f32(self, lhs, rhs, bias, out, batch, rows, K, lhs_batched=False, rhs_batched=True):
-        self._check(lib().mb_gemv_f32(self.h, lhs.ptr, rhs.ptr,
+        self._check(_ops.mb_gemv_f32(self._p, lhs.ptr, rhs.ptr,
                                       bias.ptr if bias is not None else None, out.ptr, batch,
                                       rows, K, int(lhs_batched), int(rhs_batched)))
 
     def conv2d_f32(self, x, f, bias, out, N, Cc, H, W, O, KH, KW, strides, dil, pad_tl, out_hw,
                    act=0, max_limit=0.0, coef=0.0):
-        self._check(lib().mb_conv2d_f32_nchw(
-            self.h, x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, Cc, H, W,
+        self._check(_ops.mb_conv2d_f32_nchw(self._p,
+            x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, Cc, H, W,
             O, KH, KW, strides[0], strides[1], dil[0], dil[1], pad_tl[0], pad_tl[1], out_hw[0],
             out_hw[1], act, max_limit, coef))
 
     def conv2d_f32_residual(self, x, f, bias, residual, out, N, Cc, H, W, O, KH, KW, strides, dil, pad_tl,
                             out_hw, act=0, max_limit=0.0, coef=0.0):
-        self._check(lib().mb_conv2d_f32_nchw_residual(
-            self.h, x.ptr, f.ptr, bias.ptr if bias is not None else None, residual.ptr, out.ptr, N, Cc, H,
+        self._check(_ops.mb_conv2d_f32_nchw_residual(self._p,
+            x.ptr, f.ptr, bias.ptr if bias is not None else None, residual.ptr, out.ptr, N, Cc, H,
             W, O, KH, KW, strides[0], strides[1], dil[0], dil[1], pad_tl[0], pad_tl[1], out_hw[0],
             out_hw[1], act, max_limit, coef))
 
     def dwconv_f32(self, x, f, bias, out, N, Cc, H, W, Mc, KH, KW, strides, dil, pad_tl, out_hw,
                    act=0, max_limit=0.0, coef=0.0):
-        self._check(lib().mb_dwconv_f32_nchw(
-            self.h, x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, Cc, H, W,
+        self._check(_ops.mb_dwconv_f32_nchw(self._p,
+            x.ptr, f.ptr, bias.ptr if bias is not None else None, out.ptr, N, Cc, H, W,
             Mc, KH, KW, strides[0], strides[1], dil[0], dil[1], pad_tl[0], pad_tl[1], out_hw[0],
             out_hw[1], act, max_limit, coef))
 
     def winograd_f32(self, x, f, bias, out, N, Cc, H, W, O, pad_tl, out_hw, act=0, max_limit=0.0,
                      coef=0.0, tile=0, transformed=None):
-        self._check(lib().mb_conv3x3_winograd_f32_nchw(
-            self.h, x.ptr, f.ptr if f is not None else None,
+        self._check(_ops.mb_conv3x3_winograd_f32_nchw(self._p, x.ptr, f.ptr if f is not None else None,
             transformed.ptr if transformed is not None else None,
             bias.ptr if bias is not None else None, out.ptr, N, Cc, H, W, O, pad_tl[0],
             pad_tl[1], out_hw[0], out_hw[1], act, max_limit, coef, tile))
@@ -340,29 +343,29 @@ class Context:
         self._check(lib().mb_winograd_transform_filter_f32(self.h, f.ptr, out.ptr, Cc, O, tile))
 
     def pooling_f32(self, x, out, N, Cc, H, W, kernel, strides, dil, pad_tl, out_hw, pooling_type):
-        self._check(lib().mb_pooling_f32_nchw(
-            self.h, x.ptr, out.ptr, N, Cc, H, W, kernel[0], kernel[1], strides[0], strides[1],
+        self._check(_ops.mb_pooling_f32_nchw(self._p,
+            x.ptr, out.ptr, N, Cc, H, W, kernel[0], kernel[1], strides[0], strides[1],
             dil[0], dil[1], pad_tl[0], pad_tl[1], out_hw[0], out_hw[1], pooling_type))
 
     def eltwise_f32(self, a, b, out, size, type_, coeff=None, swapped=False, scalar=1.0, act=0,
                     max_limit=0.0, coef=0.0):
         c = coeff if coeff else (0.0, 0.0)
-        self._check(lib().mb_eltwise_act_f32(
-            self.h, a.ptr, b.ptr if b is not None else None, out.ptr, size, type_, scalar,
+        self._check(_ops.mb_eltwise_act_f32(self._p,
+            a.ptr, b.ptr if b is not None else None, out.ptr, size, type_, scalar,
             1 if coeff else 0, c[0], c[1], 1 if swapped else 0, act, max_limit, coef))
 
     def activation_f32(self, x, out, size, act, max_limit=0.0, coef=0.0):
-        self._check(lib().mb_activation_f32(self.h, x.ptr, out.ptr, size, act, max_limit, coef))
+        self._check(_ops.mb_activation_f32(self._p, x.ptr, out.ptr, size, act, max_limit, coef))
 
     def softmax_f32(self, x, out, outer, classes, inner, use_log=False):
-        self._check(lib().mb_softmax_f32(self.h, x.ptr, out.ptr, outer, classes, inner,
+        self._check(_ops.mb_softmax_f32(self._p, x.ptr, out.ptr, outer, classes, inner,
                                          1 if use_log else 0))
 
     def quantize_f32_u8(self, x, out, size, scale, zero_point):
-        self._check(lib().mb_quantize_f32_u8(self.h, x.ptr, out.ptr, size, scale, zero_point))
+        self._check(_ops.mb_quantize_f32_u8(self._p, x.ptr, out.ptr, size, scale, zero_point))
 
     def dequantize_f32(self, q, out, size, scale, zero_point, int32=False):
-        self._check(lib().mb_dequantize_f32(self.h, q.ptr, 1 if int32 else 0, out.ptr, size, scale,
+        self._check(_ops.mb_dequantize_f32(self._p, q.ptr, 1 if int32 else 0, out.ptr, size, scale,
                                             zero_point))
 
     def minmax_f32(self, x, size):
@@ -372,13 +375,13 @@ class Context:
 
     def subsample_f32(self, x, out, planes, H, W, strides):
         """out[p][ho][wo] = x[p][ho * sh][wo * sw]."""
-        self._check(lib().mb_subsample_f32_nchw(self.h, x.ptr, out.ptr, planes, H, W, strides[0], strides[1]))
+        self._check(_ops.mb_subsample_f32_nchw(self._p, x.ptr, out.ptr, planes, H, W, strides[0], strides[1]))
 
     def transpose2d_batched(self, x, out, batch, rows, cols, elem_bytes):
         """out[b][c][r] = x[b][r][c]; NHWC -> NCHW is rows = H * W, cols = C."""
-        self._check(lib().mb_transpose2d_batched(self.h, x.ptr, out.ptr, batch, rows, cols, elem_bytes))
+        self._check(_ops.mb_transpose2d_batched(self._p, x.ptr, out.ptr, batch, rows, cols, elem_bytes))
 
     def avgpool_u8(self, x, out, N, H, W, Cc, kernel, strides, pad_tl, out_hw):
-        self._check(lib().mb_avgpool_u8_nhwc(
-            self.h, x.ptr, out.ptr, N, H, W, Cc, kernel[0], kernel[1], strides[0], strides[1],
+        self._check(_ops.mb_avgpool_u8_nhwc(self._p,
+            x.ptr, out.ptr, N, H, W, Cc, kernel[0], kernel[1], strides[0], strides[1],
             pad_tl[0], pad_tl[1], out_hw[0], out_hw[1]))
