@@ -135,8 +135,10 @@ uint64_t mb_launch_count_pair(const mb_context *ctx);
 /* How many such pairs the device holds at once (0 before the first pair launch). */
 int mb_pair_clusters(const mb_context *ctx);
 /* Options: "tensor_cores" (1 default; 0 forces the CUDA-core GEMM, for A/B
- * tests), "mn_major" (1 default; 0 transposes MN-major operands to K-major
- * in scratch instead of describing them to the tensor core directly),
+ * tests), "mn_major" (accepted, without effect: MN-major operands reach the
+ * tensor core as they lie), "cut_bn" / "cut_splits" / "cut_two" /
+ * "cut_aligned" (0 default: by rule; tile width, depth runs, CTAs per SM and
+ * use of the cluster-cut uint8 GEMM, for A/B tests),
  * "col_budget_mb" (1024 default: the fp32 general convolution gathers the
  * im2col columns of as many images at a time as fit into this many MiB of
  * scratch), "wino_plane" (1 default; 0 takes the one-thread-per-tile Winograd

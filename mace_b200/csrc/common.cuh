@@ -39,8 +39,8 @@ struct mb_context {
   int *dev_status = nullptr;   // device status word (bounded-wait failures)
   int *host_status = nullptr;  // pinned mirror read at sync
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
+  void *encode_im2col = nullptr; // cuTensorMapEncodeIm2col
   int use_tensor_cores = 1;      // cleared by mb_set_option for A/B tests
-  int use_mn_major = 1;
   uint64_t launches = 0;         // kernels launched through this context
   uint64_t launches_tc = 0;      // of which tcgen05 GEMM launches
   uint64_t launches_pair = 0;    // of which on CTA pairs (not adjusted for graph replays)
@@ -48,6 +48,12 @@ struct mb_context {
   long long *tc_timeline = nullptr;  // optional device buffer: per-role clock stamps of CTA 0
   uint64_t capture_launches0 = 0, capture_launches_tc0 = 0;
   uint64_t func_attr_mask = 0;   // kernels whose shared-memory limit was raised
+  int cut_aligned = 0;           // aligned u8 products on the cluster-cut kernel: 0 by rule, 1 never, 2 always
+  int cut_bn = 0, cut_splits = 0, cut_two = 0;  // cluster-cut GEMM: overrides of tile width, depth runs, CTAs per SM
+                                 // (1 / 2; 3: convolutions on the persistent kernel) (0: by rule)
+  int cut_clusters[4] = {0, 0, 0, 0};  // CTAs of clusters of 2 / 4 / 8 that are resident at once, one CTA per SM (0: not asked)
+  uint64_t cut_attr_mask = 0;    // kernels of gemm_u8_cut.cu / gemm_u8_gather.cu whose shared-memory limit was raised
+  uint64_t func_attr_mask_plain = 0;  // the same for the GEMM's plain-store instances
   uint64_t func_attr_mask2 = 0;  // the same for the thread-per-pixel convolution kernels
   int pdl_next_gemm = 0;         // the next tensor-core GEMM may start before its predecessor (the
                                  // operand-sum kernel) ends; it waits for it where it reads the sums

@@ -89,6 +89,12 @@ int mb_init(int device, mb_context **out) {
     fn = nullptr;
   }
   ctx->encode_tiled = fn;
+  fn = nullptr;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
+      qres != cudaDriverEntryPointSuccess) {
+    fn = nullptr;
+  }
+  ctx->encode_im2col = fn;
   *out = ctx;
   return MB_SUCCESS;
 }
@@ -422,7 +428,19 @@ int mb_set_option(mb_context *ctx, const char *name, int value) {
   if (strcmp(name, "tensor_cores") == 0) {
     ctx->use_tensor_cores = value;
   } else if (strcmp(name, "mn_major") == 0) {
-    ctx->use_mn_major = value;
+    // accepted and without effect: MN-major operands always reach the tensor core in place
+  } else if (strcmp(name, "cut_aligned") == 0) {
+    ctx->cut_aligned = value;
+  } else if (strcmp(name, "cut_bn") == 0) {
+    if (value != 0 && value != 64 && value != 128) return mb_fail(ctx, MB_INVALID_ARGS, "cut_bn must be 0, 64 or 128");
+    ctx->cut_bn = value;
+  } else if (strcmp(name, "cut_splits") == 0) {
+    if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8)
+      return mb_fail(ctx, MB_INVALID_ARGS, "cut_splits must be 0, 1, 2, 4 or 8");
+    ctx->cut_splits = value;
+  } else if (strcmp(name, "cut_two") == 0) {
+    if (value < 0 || value > 3) return mb_fail(ctx, MB_INVALID_ARGS, "cut_two must be 0 .. 3");
+    ctx->cut_two = value;
   } else if (strcmp(name, "host_alloc_wc") == 0) {
     ctx->host_alloc_wc = value;
   } else if (strcmp(name, "tc_rowsum") == 0) {

@@ -1,23 +1,17 @@
 // mb_gemm_u8: argument checks, operand preparation (row/column byte sums for
-// the zero-point correction, optional transposes) and the choice between the
-// tensor-core kernel (gemm_u8_tc.cu) and a CUDA-core kernel that takes any
-// layout, alignment and depth.
+// the zero-point correction, copies of rows that TMA cannot address) and the
+// choice between the tensor-core kernel (gemm_u8_tc.cu) and a CUDA-core kernel
+// that takes any depth and runs when the tensor cores are switched off.
 //
 // Reference behaviour: MatMulFixpointImpl (mace/ops/matmul.cc:228-394) and the
 // GEMM of the quantized Conv2D (mace/ops/conv_2d.cc:301-315).
 #include <algorithm>
 
 #include "common.cuh"
+#include "gemm_u8_cut.cuh"
 
-bool mb_gemm_u8_tc_supported(const mb_context *ctx, const void *A, const void *B, int64_t M,
-                             int64_t N, int64_t K, bool a_mn, bool b_mn, int a_batched,
-                             int b_batched);
-int mb_gemm_u8_tc_launch(mb_context *ctx, const uint8_t *A, const uint8_t *B,
-                         const uint32_t *sum_a, const uint32_t *sum_b, const int32_t *bias,
-                         void *C, int out_is_int32, int64_t batch, int64_t M, int64_t N,
-                         int64_t K, bool a_mn, bool b_mn, int a_batched, int b_batched,
-                         int32_t zp_a, int32_t zp_b, int32_t mult, int32_t shift, int32_t zp_c,
-                         int bias_per_row);
+bool mb_gemm_u8_tc_supported(const mb_context *ctx, const void *A, const void *B, int64_t M, int64_t N, int64_t K,
+                             int64_t lda, int64_t ldb);
 
 namespace {
 
@@ -45,6 +39,8 @@ struct GenericParams {
 __global__ void __launch_bounds__(256) gemm_u8_generic_kernel(const GenericParams p) {
   __shared__ int16_t As[GK][GT + 2];
   __shared__ int16_t Bs[GK][GT + 2];
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int b = blockIdx.z;
   const int64_t m0 = static_cast<int64_t>(blockIdx.y) * GT;
   const int64_t n0 = static_cast<int64_t>(blockIdx.x) * GT;
@@ -105,32 +101,59 @@ __global__ void __launch_bounds__(256) gemm_u8_generic_kernel(const GenericParam
   }
 }
 
-// ---- transpose [rows x cols] -> [cols x rows] bytes ------------------------------
-__global__ void __launch_bounds__(256) transpose_u8_kernel(const uint8_t *__restrict__ in,
-                                                           uint8_t *__restrict__ out,
-                                                           int64_t rows, int64_t cols) {
-  __shared__ uint8_t tile[64][65];
-  const int64_t batch_off = static_cast<int64_t>(blockIdx.z) * rows * cols;
-  const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 64, c0 = static_cast<int64_t>(blockIdx.x) * 64;
-  for (int i = threadIdx.x; i < 64 * 64; i += 256) {
-    const int r = i >> 6, c = i & 63;
-    tile[r][c] = (r0 + r < rows && c0 + c < cols) ? in[batch_off + (r0 + r) * cols + c0 + c] : 0;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 64 * 64; i += 256) {
-    const int c = i >> 6, r = i & 63;
-    if (r0 + r < rows && c0 + c < cols) out[batch_off + (c0 + c) * rows + r0 + r] = tile[r][c];
-  }
-}
+// ---- rows of any length -> rows of a 16-byte pitch ---------------------------------------
+// TMA addresses rows that start 16-byte aligned.  An operand whose rows do not (an odd depth, an odd
+// sequence length, a base inside another tensor) is copied once into scratch with its rows apart by
+// the next multiple of 16, the gap filled with one value; its major order stays.  Both operands in one
+// launch.  A thread writes one word per step: it reads the two aligned words that hold its four bytes
+// (neighbouring lanes read neighbouring words, whatever the alignment) and shifts.  Only words
+// that hold at least one byte of the row are read.  Bound by its launch for operands of a few
+// megabytes (they stay in L2): 333 x 1001 x 777, batch 4, both operands copied: 14 us in all, 195 us on the
+// CUDA-core kernel.
+struct RepackJob {
+  const uint8_t *src;
+  uint8_t *dst;
+  int64_t len, ld;          // bytes of a row; bytes from row to row in dst
+  uint32_t words;           // of dst
+  uint32_t fill;            // four times the byte of the gaps
+  uint32_t row_mul, row_shift;
+  int blocks;
+};
 
-int launch_transpose(mb_context *ctx, const uint8_t *in, uint8_t *out, int64_t nb, int64_t rows,
-                     int64_t cols) {
-  dim3 grid(static_cast<unsigned>(ceil_div64(cols, 64)), static_cast<unsigned>(ceil_div64(rows, 64)),
-            static_cast<unsigned>(nb));
-  transpose_u8_kernel<<<grid, 256, 0, ctx->stream>>>(in, out, rows, cols);
-  MB_CUDA(ctx, cudaGetLastError());
-  ctx->launches++;
-  return MB_SUCCESS;
+constexpr int REPACK_STEPS = 4;
+
+__global__ void __launch_bounds__(256) repack_rows_u8_kernel(const RepackJob a, const RepackJob b) {
+  mb_grid_dep_launch();
+  const bool first = static_cast<int>(blockIdx.x) < a.blocks;
+  const RepackJob &j = first ? a : b;
+  const uint32_t block = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const uint32_t row_words = static_cast<uint32_t>(j.ld >> 2);
+  mb_grid_dep_wait();
+  uint32_t lo[REPACK_STEPS], hi[REPACK_STEPS];
+  int sh[REPACK_STEPS], left[REPACK_STEPS];
+#pragma unroll
+  for (int s = 0; s < REPACK_STEPS; ++s) {
+    const uint32_t w = (block * REPACK_STEPS + s) * 256u + threadIdx.x;
+    const uint32_t row = fast_div(w, j.row_mul, j.row_shift);
+    const int64_t at = static_cast<int64_t>(w - row * row_words) * 4;
+    left[s] = w < j.words ? static_cast<int>(max(min(j.len - at, static_cast<int64_t>(4)), static_cast<int64_t>(0))) : 0;
+    const uint8_t *q = j.src + static_cast<int64_t>(row) * j.len + at;
+    const int off = static_cast<int>(reinterpret_cast<uintptr_t>(q) & 3u);
+    const uint32_t *aligned = reinterpret_cast<const uint32_t *>(q - off);
+    sh[s] = off * 8;
+    lo[s] = left[s] > 0 ? __ldg(aligned) : 0u;
+    hi[s] = left[s] + off > 4 ? __ldg(aligned + 1) : 0u;
+  }
+#pragma unroll
+  for (int s = 0; s < REPACK_STEPS; ++s) {
+    const uint32_t w = (block * REPACK_STEPS + s) * 256u + threadIdx.x;
+    uint32_t v = __funnelshift_r(lo[s], hi[s], sh[s]);
+    if (left[s] < 4) {
+      const uint32_t mask = (1u << (8 * left[s])) - 1u;
+      v = (v & mask) | (j.fill & ~mask);
+    }
+    if (w < j.words) reinterpret_cast<uint32_t *>(j.dst)[w] = v;
+  }
 }
 
 int launch_generic(mb_context *ctx, const uint8_t *A, const uint8_t *B, const int32_t *bias,
@@ -152,13 +175,34 @@ int launch_generic(mb_context *ctx, const uint8_t *A, const uint8_t *B, const in
   if (gy > 65535 || batch > 65535)
     return mb_fail(ctx, MB_UNSUPPORTED, "generic GEMM: M or batch too large for this path");
   dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(batch));
-  gemm_u8_generic_kernel<<<grid, 256, 0, ctx->stream>>>(p);
-  MB_CUDA(ctx, cudaGetLastError());
+  MB_CUDA(ctx, mb_launch_chained(ctx, gemm_u8_generic_kernel, grid, dim3(256), 0, p));
   ctx->launches++;
   return MB_SUCCESS;
 }
 
 }  // namespace
+
+// Rows of a_len bytes at A -> rows lda bytes apart at a_dst (lda a multiple of 16, fewer than 2^33 bytes in
+// all), the gap filled with fill_a; the same for B.  Either source may be null.
+int mb_repack_rows_u8(mb_context *ctx, const uint8_t *A, uint8_t *a_dst, int64_t a_rows, int64_t a_len, int64_t lda,
+                      int fill_a, const uint8_t *B, uint8_t *b_dst, int64_t b_rows, int64_t b_len, int64_t ldb,
+                      int fill_b) {
+  auto make = [](const uint8_t *src, uint8_t *dst, int64_t rows, int64_t len, int64_t ld, int fill) {
+    RepackJob j = {};
+    if (src == nullptr) return j;
+    j.src = src; j.dst = dst; j.len = len; j.ld = ld;
+    j.fill = static_cast<uint32_t>(fill & 255) * 0x01010101u;
+    j.words = static_cast<uint32_t>(rows * ld / 4);
+    fast_div_make(static_cast<uint32_t>(ld / 4), &j.row_mul, &j.row_shift);
+    j.blocks = static_cast<int>(ceil_div64(j.words, 256 * REPACK_STEPS));
+    return j;
+  };
+  const RepackJob ja = make(A, a_dst, a_rows, a_len, lda, fill_a), jb = make(B, b_dst, b_rows, b_len, ldb, fill_b);
+  MB_CUDA(ctx, mb_launch_chained(ctx, repack_rows_u8_kernel, dim3(static_cast<unsigned>(ja.blocks + jb.blocks)),
+                                 dim3(256), 0, ja, jb));
+  ctx->launches++;
+  return MB_SUCCESS;
+}
 
 bool mb_gemm_u8_skinny_supported(int64_t batch, int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn,
                                  const void *A, const void *B);
@@ -170,12 +214,12 @@ int mb_operand_sums_slices(const mb_context *ctx, bool mn, int64_t nb, int64_t K
 int mb_gemm_u8_tc_launch_sliced(mb_context *ctx, const uint8_t *A, const uint8_t *B,
                                 const uint32_t *sum_a, const uint32_t *sum_b, int sum_a_slices, int sum_b_slices,
                                 const int32_t *bias, void *C, int out_is_int32, int64_t batch, int64_t M, int64_t N,
-                                int64_t K, bool a_mn, bool b_mn, int a_batched, int b_batched,
+                                int64_t K, int64_t lda, int64_t ldb, bool a_mn, bool b_mn, int a_batched, int b_batched,
                                 int32_t zp_a, int32_t zp_b, int32_t mult, int32_t shift, int32_t zp_c,
                                 int bias_per_row);
 int mb_operand_sums_launch(mb_context *ctx, const uint8_t *A, bool a_mn, int64_t nb_a, int64_t M, uint32_t *sum_a,
                            const uint8_t *B, bool b_mn, int64_t nb_b, int64_t N, uint32_t *sum_b, int64_t K,
-                           int k_split);
+                           int k_split, int64_t lda, int64_t ldb);
 int mb_gemm_u8_tc_launch_splitk(mb_context *ctx, const uint8_t *A, const uint8_t *B,
                                 const uint32_t *sum_a, const uint32_t *sum_b, int sum_a_slices, int sum_b_slices,
                                 int32_t *parts, int k_split, int bn, int64_t M, int64_t N, int64_t K, bool a_mn,
@@ -253,6 +297,63 @@ int split_k_choice(const mb_context *ctx, int64_t batch, int64_t M, int64_t N, i
   return best >= 4 ? best : 1;
 }
 
+// ---- the choice between the tensor-core kernels ----------------------------------------
+// Estimated SM cycles of the persistent kernel (gemm_u8_tc.cu), from its times at 1024^3 (7.4 us), 512^3 (5.9 us),
+// 16 x 1024 x 1024 (7.3 us), 256 x 4096 x 4096 (17 us) and 4096^3 (58 us): about 4.4 us around the steps, a row-major
+// B whose column sums come from the tiles paces them; beyond a depth of 1024 (or with a column-major A) the sums
+// are a kernel of their own.
+int64_t persistent_cost(const mb_context *ctx, const mb_cut_gemm &g) {
+  const int64_t tiles_m = ceil_div64(g.M, 128), steps = ceil_div64(g.K, 128);
+  const bool fused = !g.a_mn && g.K <= 1024;
+  int64_t best = -1;
+  for (int w : {256, 128, 64}) {
+    if (w > 64 && g.N <= w / 2) continue;
+    const int64_t rounds = ceil_div64(g.batch * tiles_m * ceil_div64(g.N, w), ctx->num_sms);
+    const int64_t step = fused ? (g.b_mn ? (w == 256 ? 1400 : w == 128 ? 930 : 720) : (w == 256 ? 900 : 700)) : (w == 256 ? 900 : w == 128 ? 600 : 520);
+    const int64_t cost = rounds * std::max<int64_t>(steps * step, w == 256 ? 2600 : w == 128 ? 1500 : 900);
+    if (best < 0 || cost < best) best = cost;
+  }
+  return best + (fused ? 8300 : 13300);
+}
+
+// Runs the product on a cluster-cut kernel where that is estimated to be the fastest way: as it lies, or, with rows that
+// TMA cannot address, on copies that it can (2.4 us for the extra launch and the bytes at about 4 TB/s).
+bool try_cut(mb_context *ctx, const mb_cut_gemm &g, bool a_copy, bool b_copy, int *status) {
+  const mb_cut_plan direct = mb_gemm_u8_cut_plan(ctx, g);
+  int64_t other = persistent_cost(ctx, g);
+  if (!a_copy && !b_copy) {
+    if (direct.cost < 0 || (ctx->cut_aligned == 0 ? direct.cost >= other : ctx->cut_aligned == 1)) return false;
+    *status = mb_gemm_u8_cut_launch(ctx, g, direct);
+    return true;
+  }
+  const int64_t a_rows = (g.a_batched ? g.batch : 1) * (g.a_mn ? g.K : g.M), b_rows = (g.b_batched ? g.batch : 1) * (g.b_mn ? g.K : g.N);
+  const int64_t a_len = g.a_mn ? g.M : g.K, b_len = g.b_mn ? g.N : g.K;
+  const int64_t lda = static_cast<int64_t>(align_up(static_cast<size_t>(a_len), 16)), ldb = static_cast<int64_t>(align_up(static_cast<size_t>(b_len), 16));
+  const int64_t copy_cost = 4500 + ((a_copy ? 2 * a_rows * a_len : 0) + (b_copy ? 2 * b_rows * b_len : 0)) / 2000;
+  mb_cut_gemm c = g;
+  if (a_copy) { c.A = nullptr; c.lda = lda; }
+  if (b_copy) { c.B = nullptr; c.ldb = ldb; }
+  const mb_cut_plan copied = mb_gemm_u8_cut_plan(ctx, c);
+  other += copy_cost;
+  if (direct.cost >= 0 && direct.cost <= other && (copied.cost < 0 || direct.cost <= copied.cost + copy_cost)) {
+    *status = mb_gemm_u8_cut_launch(ctx, g, direct);
+    return true;
+  }
+  if (copied.cost < 0 || copied.cost + copy_cost >= other || (a_copy && a_rows * lda >= (1ll << 33)) || (b_copy && b_rows * ldb >= (1ll << 33)))
+    return false;
+  const size_t a_bytes = a_copy ? align_up(static_cast<size_t>(a_rows * lda), 256) : 0;
+  uint8_t *scratch = nullptr;
+  *status = mb_scratch(ctx, a_bytes + (b_copy ? static_cast<size_t>(b_rows * ldb) : 0), reinterpret_cast<void **>(&scratch));
+  if (*status != MB_SUCCESS) return true;
+  *status = mb_repack_rows_u8(ctx, a_copy ? g.A : nullptr, scratch, a_rows, a_len, lda, 0, b_copy ? g.B : nullptr,
+                              scratch + a_bytes, b_rows, b_len, ldb, 0);
+  if (*status != MB_SUCCESS) return true;
+  if (a_copy) c.A = scratch;
+  if (b_copy) c.B = scratch + a_bytes;
+  *status = mb_gemm_u8_cut_launch(ctx, c, copied);
+  return true;
+}
+
 }  // namespace
 
 // Row-major-C GEMM on device operands; a_mn / b_mn as in mb_gemm_u8_tc_launch.
@@ -261,29 +362,34 @@ int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, con
                         int64_t K, bool a_mn, bool b_mn, int a_batched, int b_batched,
                         int32_t zp_a, int32_t zp_b, int32_t mult, int32_t shift, int32_t zp_c,
                         int bias_per_row) {
-  const bool aligned16 =
-      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15u) == 0;
-  bool use_tc = ctx->use_tensor_cores && ctx->encode_tiled != nullptr && aligned16 &&
-                K % 16 == 0 && K <= 33000 && M >= 1 && N >= 1;
-  // A few rows against a large row-major B: stream B once over all SMs with CUDA cores.  From
-  // two rows on the tensor-core kernel over depth runs is faster where it applies (measured at
-  // K = N = 4096: 11.4 us against 12.4 at M = 2, 11.4 against 14.0 at M = 4, 11.7 against 28.8 at
-  // M = 16; a tie, 11.4 / 11.2, at M = 1).
+  bool use_tc = ctx->use_tensor_cores && ctx->encode_tiled != nullptr && K <= 33000 && M < (1ll << 31) && N < (1ll << 31);
+  // Each operand reaches the tensor core in its own major order, in place when its rows are 16-byte
+  // aligned, else through a copy with a 16-byte pitch.
+  const int64_t a_len = a_mn ? M : K, b_len = b_mn ? N : K;
+  const bool a_copy = a_len % 16 != 0 || (reinterpret_cast<uintptr_t>(A) & 15u) != 0;
+  const bool b_copy = b_len % 16 != 0 || (reinterpret_cast<uintptr_t>(B) & 15u) != 0;
+  // A ragged product of a few thousand multiplications per SM is not worth the copy: one launch of the
+  // CUDA-core kernel is over before the copy's successor could start.
+  if ((a_copy || b_copy) && batch * M * N * K <= (1 << 18)) use_tc = false;
+  if (use_tc && ctx->split_k && ctx->skinny_max_m > 0 && !ctx->pair_gemm && (ctx->force_bn == 0 || a_copy || b_copy)) {
+    mb_cut_gemm g;
+    g.A = A; g.B = B; g.bias = bias; g.C = C; g.out_is_int32 = out_is_int32; g.bias_per_row = bias_per_row;
+    g.batch = batch; g.M = M; g.N = N; g.K = K; g.a_mn = a_mn; g.b_mn = b_mn;
+    g.a_batched = a_batched; g.b_batched = b_batched; g.zp_a = zp_a; g.zp_b = zp_b;
+    g.rq = mb_make_requant(mult, shift, zp_c);
+    g.rq_variant = mb_requant_variant(shift, zp_c);
+    int st = MB_SUCCESS;
+    if (try_cut(ctx, g, a_copy, b_copy, &st)) return st;
+  }
+  // (With the cluster-cut kernels off -- split_k or skinny_max_m = 0 --: a few rows against a large row-major B
+  // on CUDA cores, or on the tensor cores with the depth cut into runs through global memory.)
   if (ctx->use_tensor_cores && M <= ctx->skinny_max_m && mb_gemm_u8_skinny_supported(batch, M, N, K, a_mn, b_mn, A, B)) {
     int bn_unused = 0;
-    const bool runs_apply = M >= ctx->runs_min_m && use_tc && !(a_mn && !(ctx->use_mn_major && M % 16 == 0)) &&
-                            !(b_mn && !(ctx->use_mn_major && N % 16 == 0)) &&
+    const bool runs_apply = M >= ctx->runs_min_m && use_tc && !a_copy && !b_copy &&
                             split_k_choice(ctx, batch, M, N, K, &bn_unused) > 1;
     if (!runs_apply)
       return mb_gemm_u8_skinny_launch(ctx, A, B, bias, C, out_is_int32, M, N, K, zp_a, zp_b, mult, shift,
                                       zp_c, bias_per_row);
-  }
-  // How each operand reaches the tensor core: natively in its own major, or
-  // through a K-major copy in scratch.
-  bool a_copy = false, b_copy = false;
-  if (use_tc) {
-    if (a_mn && !(ctx->use_mn_major && M % 16 == 0)) a_copy = true;
-    if (b_mn && !(ctx->use_mn_major && N % 16 == 0)) b_copy = true;
   }
   if (!use_tc) {
     return launch_generic(ctx, A, B, bias, C, out_is_int32, batch, M, N, K, a_mn, b_mn,
@@ -292,7 +398,7 @@ int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, con
   const int64_t nb_a = a_batched ? batch : 1, nb_b = b_batched ? batch : 1;
   int split_bn = 0;
   const int splits = (a_copy || b_copy) ? 1 : split_k_choice(ctx, batch, M, N, K, &split_bn);
-  if (splits > 1 && mb_gemm_u8_tc_supported(ctx, A, B, M, N, K / splits, a_mn, b_mn, 0, 0)) {
+  if (splits > 1 && mb_gemm_u8_tc_supported(ctx, A, B, M, N, K / splits, a_len, b_len)) {
     const int64_t Ks = K / splits;
     // runs no longer than 1024 with a K-major A: the kernel sums the bytes of its own tiles
     const bool fused = !a_mn && Ks <= 1024;
@@ -309,7 +415,7 @@ int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, con
     uint32_t *sum_a = want_a ? reinterpret_cast<uint32_t *>(scratch + off_sa) : nullptr;
     uint32_t *sum_b = want_b ? reinterpret_cast<uint32_t *>(scratch + off_sb) : nullptr;
     if (want_a || want_b)
-      MB_RETURN_IF_ERROR(mb_operand_sums_launch(ctx, A, a_mn, 1, M, sum_a, B, b_mn, 1, N, sum_b, K, splits));
+      MB_RETURN_IF_ERROR(mb_operand_sums_launch(ctx, A, a_mn, 1, M, sum_a, B, b_mn, 1, N, sum_b, K, splits, a_len, b_len));
     ctx->pdl_next_gemm = (want_a || want_b) ? 1 : 0;
     MB_RETURN_IF_ERROR(mb_gemm_u8_tc_launch_splitk(ctx, A, B, sum_a, sum_b, sl_a, sl_b, parts, splits, split_bn, M, N,
                                                    K, a_mn, b_mn, zp_a, zp_b));
@@ -332,48 +438,43 @@ int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, con
   // A K-major A with K <= 1024 (B in either order): the tensor-core kernel sums the operand
   // bytes itself from the tiles it has in shared memory.
   // (option pair = 2, the CTA-pair kernel wherever it can run, takes its sums from the sums kernel)
-  const bool fused_sums = !(a_mn && !a_copy) && K <= 1024 && ctx->pair_gemm != 2;
+  const bool fused_sums = !a_mn && K <= 1024 && ctx->pair_gemm != 2;
   const bool need_sum_a = zp_b != 0 && !fused_sums, need_sum_b = zp_a != 0 && !fused_sums;
+  const int64_t lda = a_copy ? static_cast<int64_t>(align_up(a_len, 16)) : a_len;
+  const int64_t ldb = b_copy ? static_cast<int64_t>(align_up(b_len, 16)) : b_len;
+  const int64_t a_rows = nb_a * (a_mn ? K : M), b_rows = nb_b * (b_mn ? K : N);
+  if (!mb_gemm_u8_tc_supported(ctx, nullptr, nullptr, M, N, K, lda, ldb) ||
+      (a_copy && a_rows * lda >= (1ll << 33)) || (b_copy && b_rows * ldb >= (1ll << 33))) {
+    return launch_generic(ctx, A, B, bias, C, out_is_int32, batch, M, N, K, a_mn, b_mn,
+                          a_batched, b_batched, zp_a, zp_b, mult, shift, zp_c, bias_per_row);
+  }
   size_t off = 0;
   // (an operand that reaches the tensor core MN-major gets its column sums as a few partial rows)
-  const int sl_a = need_sum_a ? mb_operand_sums_slices(ctx, a_mn && !a_copy, nb_a, K, M) : 1;
-  const int sl_b = need_sum_b ? mb_operand_sums_slices(ctx, b_mn && !b_copy, nb_b, K, N) : 1;
+  const int sl_a = need_sum_a ? mb_operand_sums_slices(ctx, a_mn, nb_a, K, M) : 1;
+  const int sl_b = need_sum_b ? mb_operand_sums_slices(ctx, b_mn, nb_b, K, N) : 1;
   const size_t off_sum_a = off; off += need_sum_a ? align_up(sizeof(uint32_t) * nb_a * M * sl_a, 256) : 0;
   const size_t off_sum_b = off; off += need_sum_b ? align_up(sizeof(uint32_t) * nb_b * N * sl_b, 256) : 0;
-  const size_t off_at = off; off += a_copy ? align_up(nb_a * M * K, 256) : 0;
-  const size_t off_bt = off; off += b_copy ? align_up(nb_b * N * K, 256) : 0;
+  const size_t off_at = off; off += a_copy ? align_up(a_rows * lda, 256) : 0;
+  const size_t off_bt = off; off += b_copy ? align_up(b_rows * ldb, 256) : 0;
 
   uint8_t *scratch = nullptr;
   if (off > 0) MB_RETURN_IF_ERROR(mb_scratch(ctx, off, reinterpret_cast<void **>(&scratch)));
   uint32_t *sum_a = need_sum_a ? reinterpret_cast<uint32_t *>(scratch + off_sum_a) : nullptr;
   uint32_t *sum_b = need_sum_b ? reinterpret_cast<uint32_t *>(scratch + off_sum_b) : nullptr;
-  const uint8_t *a_use = A, *b_use = B;
-  bool a_mn_use = a_mn, b_mn_use = b_mn;
-  if (a_copy) {
-    // MN-major A is [K x M]; its transpose [M x K] is K-major.
-    MB_RETURN_IF_ERROR(launch_transpose(ctx, A, scratch + off_at, nb_a, K, M));
-    a_use = scratch + off_at;
-    a_mn_use = false;
-  }
-  if (b_copy) {
-    MB_RETURN_IF_ERROR(launch_transpose(ctx, B, scratch + off_bt, nb_b, K, N));
-    b_use = scratch + off_bt;
-    b_mn_use = false;
-  }
+  const uint8_t *a_use = a_copy ? scratch + off_at : A, *b_use = b_copy ? scratch + off_bt : B;
+  if (a_copy || b_copy)
+    MB_RETURN_IF_ERROR(mb_repack_rows_u8(ctx, a_copy ? A : nullptr, scratch + off_at, a_rows, a_len, lda, 0,
+                                         b_copy ? B : nullptr, scratch + off_bt, b_rows, b_len, ldb, 0));
   // both operands' sums in one launch (see operand_sums.cu)
   if (need_sum_a || need_sum_b)
-    MB_RETURN_IF_ERROR(mb_operand_sums_launch(ctx, a_use, a_mn_use, nb_a, M, sum_a, b_use, b_mn_use, nb_b, N, sum_b, K, 1));
-  if (!mb_gemm_u8_tc_supported(ctx, a_use, b_use, M, N, K, a_mn_use, b_mn_use, a_batched,
-                               b_batched)) {
-    return launch_generic(ctx, A, B, bias, C, out_is_int32, batch, M, N, K, a_mn, b_mn,
-                          a_batched, b_batched, zp_a, zp_b, mult, shift, zp_c, bias_per_row);
-  }
+    MB_RETURN_IF_ERROR(mb_operand_sums_launch(ctx, a_use, a_mn, nb_a, M, sum_a, b_use, b_mn, nb_b, N, sum_b, K, 1,
+                                              lda, ldb));
   // The operand-sum kernel was the last launch: the GEMM may overlap it (programmatic
   // dependent launch); its operands were complete before that kernel started.
   ctx->pdl_next_gemm = (need_sum_a || need_sum_b) ? 1 : 0;
   return mb_gemm_u8_tc_launch_sliced(ctx, a_use, b_use, sum_a, sum_b, sl_a, sl_b, bias, C, out_is_int32, batch, M,
-                                     N, K, a_mn_use, b_mn_use, a_batched, b_batched, zp_a, zp_b, mult,
-                                     shift, zp_c, bias_per_row);
+                                     N, K, lda, ldb, a_mn, b_mn, a_batched, b_batched, zp_a, zp_b, mult, shift,
+                                     zp_c, bias_per_row);
 }
 
 extern "C" int mb_gemm_u8(mb_context *ctx, const uint8_t *A, const uint8_t *B,

@@ -20,9 +20,8 @@
 
 #include "common.cuh"
 
-bool mb_gemm_u8_tc_supported(const mb_context *ctx, const void *A, const void *B, int64_t M,
-                             int64_t N, int64_t K, bool a_mn, bool b_mn, int a_batched,
-                             int b_batched);
+bool mb_gemm_u8_tc_supported(const mb_context *ctx, const void *A, const void *B, int64_t M, int64_t N, int64_t K,
+                             int64_t lda, int64_t ldb);
 int mb_gemm_u8_tc_launch(mb_context *ctx, const uint8_t *A, const uint8_t *B,
                          const uint32_t *sum_a, const uint32_t *sum_b, const int32_t *bias,
                          void *C, int out_is_int32, int64_t batch, int64_t M, int64_t N,
@@ -191,7 +190,7 @@ extern "C" int mb_gemm_u8_static_scratch(void *stream, const uint8_t *A, const u
   }
 
   const bool a_mn = a_col_major != 0, b_mn = b_col_major == 0;
-  if (!mb_gemm_u8_tc_supported(&view, A, B, M, N, K, a_mn, b_mn, 0, 0) || K % 16 != 0) {
+  if (!mb_gemm_u8_tc_supported(&view, A, B, M, N, K, a_mn ? M : K, b_mn ? N : K) || K % 16 != 0) {
     snprintf(err, err_len,
              "operands must be 16-byte aligned with K and the contiguous dimension of each "
              "operand a multiple of 16 (and K <= 33000)");

@@ -24,7 +24,7 @@ struct SumJob {
   int kind;                  // 0: nothing, 1: row sums, 2: column sums
   int64_t nb;                // matrices
   int64_t rows, cols;        // kind 1: rows x cols(=K) per matrix; kind 2: K rows x cols
-  int64_t pitch, mat_stride; // kind 1: bytes from row to row and from matrix to matrix
+  int64_t pitch, mat_stride; // bytes from row to row and from matrix to matrix
   int num_blocks;
   // column sums: out is [nb][slices][cols]
   int col_blocks, slices;
@@ -35,7 +35,7 @@ template <int WARPS>
 __device__ __forceinline__ void row_sums(const SumJob &j, int block) {
   const int lane = threadIdx.x & 31;
   const int64_t total = j.nb * j.rows;
-  const int64_t nvec = j.cols >> 4;
+  const int64_t nvec = (j.cols + 15) >> 4;  // (a repacked row is padded with zeros)
   for (int64_t row = static_cast<int64_t>(block) * WARPS + (threadIdx.x >> 5); row < total;
        row += static_cast<int64_t>(j.num_blocks) * WARPS) {
     const uint4 *p = reinterpret_cast<const uint4 *>(j.x + (row / j.rows) * j.mat_stride + (row % j.rows) * j.pitch);
@@ -65,14 +65,14 @@ __device__ __forceinline__ void col_sums(const SumJob &j, int block, uint32_t (*
   const bool active = c16 * 16 < j.cols;
   const int64_t r0 = static_cast<int64_t>(sy) * j.rows_per_slice;
   const int64_t r1 = min(j.rows, r0 + j.rows_per_slice);
-  const uint8_t *base = j.x + b * j.rows * j.cols;
+  const uint8_t *base = j.x + b * j.mat_stride;
   uint32_t s[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) s[i] = 0;
   if (active) {
 #pragma unroll 8
     for (int64_t r = r0 + ty; r < r1; r += WARPS) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(base + r * j.cols) + c16);
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(base + r * j.pitch) + c16);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -101,7 +101,10 @@ __device__ __forceinline__ void col_sums(const SumJob &j, int block, uint32_t (*
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) operand_sums_kernel(const SumJob a, const SumJob b) {
   __shared__ uint32_t part[WARPS][32][17];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // The GEMM behind this kernel reads the operands without waiting for it: it may start only when
+  // whatever wrote them is complete.
+  mb_grid_dep_wait();
+  mb_grid_dep_launch();
   const int block = blockIdx.x;
   const SumJob &j = block < a.num_blocks ? a : b;
   const int local = block < a.num_blocks ? block : block - a.num_blocks;
@@ -130,28 +133,29 @@ int mb_operand_sums_slices(const mb_context *ctx, bool mn, int64_t nb, int64_t K
 // when a_mn) into sum_a and for B into sum_b; either output may be null (not needed).
 // k_split > 1: single matrices (nb_a = nb_b = 1) whose depth is cut into k_split equal runs, each
 // summed on its own as if it were a matrix of a batch (outputs [k_split][...]).
+// lda, ldb: bytes from row to row of the stored matrices.
 int mb_operand_sums_launch(mb_context *ctx, const uint8_t *A, bool a_mn, int64_t nb_a, int64_t M, uint32_t *sum_a,
                            const uint8_t *B, bool b_mn, int64_t nb_b, int64_t N, uint32_t *sum_b, int64_t K,
-                           int k_split) {
-  const int64_t k_full = K;
+                           int k_split, int64_t lda, int64_t ldb) {
   if (k_split > 1) {
     K /= k_split;
     nb_a = nb_b = k_split;
   }
-  auto make = [&](const uint8_t *x, bool mn, int64_t nb, int64_t extent, uint32_t *out) {
+  auto make = [&](const uint8_t *x, bool mn, int64_t nb, int64_t extent, int64_t ld, uint32_t *out) {
     SumJob j = {};
     if (out == nullptr) return j;
     j.x = x; j.out = out; j.nb = nb;
     if (!mn) {  // [extent x K], K contiguous
       j.kind = 1;
       j.rows = extent; j.cols = K;
-      j.pitch = k_full;
-      j.mat_stride = k_split > 1 ? K : extent * K;
+      j.pitch = ld;
+      j.mat_stride = k_split > 1 ? K : extent * ld;
       j.num_blocks = static_cast<int>(std::min<int64_t>(ceil_div64(nb * extent, SUM_WARPS),
                                                         static_cast<int64_t>(ctx->num_sms) * 2));
     } else {    // [K x extent] -> [slices][extent] partial rows
       j.kind = 2;
       j.rows = K; j.cols = extent;
+      j.pitch = ld; j.mat_stride = K * ld;
       j.col_blocks = static_cast<int>(ceil_div64(extent, 512));
       j.slices = mb_operand_sums_slices(ctx, true, nb, K, extent);
       j.rows_per_slice = ceil_div64(K, j.slices);
@@ -159,13 +163,13 @@ int mb_operand_sums_launch(mb_context *ctx, const uint8_t *A, bool a_mn, int64_t
     }
     return j;
   };
-  const SumJob ja = make(A, a_mn, nb_a, M, sum_a);
-  const SumJob jb = make(B, b_mn, nb_b, N, sum_b);
+  const SumJob ja = make(A, a_mn, nb_a, M, lda, sum_a);
+  const SumJob jb = make(B, b_mn, nb_b, N, ldb, sum_b);
   const int64_t blocks = static_cast<int64_t>(ja.num_blocks) + jb.num_blocks;
   if (blocks == 0) return MB_SUCCESS;
   if (blocks > 0x7fffffffll) return mb_fail(ctx, MB_UNSUPPORTED, "operand sums: too many blocks");
-  operand_sums_kernel<SUM_WARPS><<<static_cast<unsigned>(blocks), SUM_WARPS * 32, 0, ctx->stream>>>(ja, jb);
-  MB_CUDA(ctx, cudaGetLastError());
+  MB_CUDA(ctx, mb_launch_chained(ctx, operand_sums_kernel<SUM_WARPS>, dim3(static_cast<unsigned>(blocks)),
+                                 dim3(SUM_WARPS * 32), 0, ja, jb));
   ctx->launches++;
   return MB_SUCCESS;
 }

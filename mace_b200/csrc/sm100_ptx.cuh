@@ -175,8 +175,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap
       : "memory");
 }
 
-// Ask for the box of a 3-D tiled tensor to be brought into L2 (no shared memory, no completion
-// to wait for): lets a producer run further ahead of HBM than its shared-memory ring allows.
 // 4-D tiled load (for an NHWC tensor: c0 = channel byte, c1 = column, c2 = row, c3 = image).
 // c0 must keep the copy 16-byte aligned; the other coordinates may lie outside the tensor
 // (negative or too large): those elements arrive as the map's fill value, zero.
@@ -190,6 +188,22 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst_smem, const CUtensorMap
       : "memory");
 }
 
+// im2col load from an NHWC tensor: one channel run of consecutive output pixels' windows at one
+// filter tap.  (w, h, n) is the first window's top-left corner in the image (padding: negative), the
+// map's bounding box says where a row of windows ends; pixels outside the image arrive as zeros.
+__device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst_smem, const CUtensorMap *map, uint32_t bar, int c,
+                                                   int w, int h, int n, uint16_t tap_w, uint16_t tap_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+      :
+      : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(tap_w),
+        "h"(tap_h)
+      : "memory");
+}
+
+// Ask for the box of a 3-D tiled tensor to be brought into L2 (no shared memory, no completion
+// to wait for): lets a producer run further ahead of HBM than its shared-memory ring allows.
 __device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
                :

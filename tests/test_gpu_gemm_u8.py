@@ -162,6 +162,36 @@ def test_unaligned_generic_path(ctx, orc, a_cm, b_cm):
     assert np.array_equal(got, exp)
 
 
+@pytest.mark.parametrize("a_cm,b_cm", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("shape", [(1, 333, 1001, 777), (3, 129, 65, 1041), (2, 77, 128, 1023), (1, 1, 3467, 408),
+                                   (1, 17, 131, 2049), (2, 150, 99, 1040)])
+def test_ragged_rows_on_the_tensor_core(ctx, orc, shape, a_cm, b_cm):
+    """Rows that TMA cannot address (copied with a 16-byte pitch), outputs that it cannot store, with
+    the operand sums from the tiles (K <= 1024) and from the sums kernel, and operands at every
+    byte alignment."""
+    batch, M, N, K = shape
+    case = gemm_case(orc, M + K, batch, M, N, K, bias_len=N, a_col_major=a_cm, b_col_major=b_cm)
+    before = ctx.launches_tensor_core
+    got, exp = run_gemm(ctx, orc, case, batch, M, N, K, a_col_major=a_cm, b_col_major=b_cm)
+    assert ctx.launches_tensor_core == before + 1
+    assert np.array_equal(got, exp)
+    for off in (1, 2, 7):
+        pad = np.zeros(off, np.uint8)
+        dA = ctx.upload(np.concatenate([pad, case["A"].ravel()]))
+        dB = ctx.upload(np.concatenate([pad, case["B"].ravel()]))
+        dbias, out = ctx.upload(case["bias"]), ctx.alloc(batch * M * N + off)
+        pa, pb, po = dA.ptr, dB.ptr, out.ptr
+        try:
+            dA.ptr, dB.ptr, out.ptr = pa + off, pb + off, po + off
+            ctx.gemm_u8(dA, dB, dbias, out, batch, M, N, K, case["zp_a"], case["zp_b"], case["mult"], case["shift"],
+                        case["zp_c"], a_col_major=a_cm, b_col_major=b_cm)
+        finally:
+            dA.ptr, dB.ptr, out.ptr = pa, pb, po
+        assert np.array_equal(ctx.download(out, (batch * M * N + off,), np.uint8)[off:], exp.ravel()), off
+        for b in (dA, dB, dbias, out):
+            b.free()
+
+
 def test_one_side_batched_and_int32_and_colmajor_out(ctx, orc):
     M, N, K = 96, 160, 208
     case = gemm_case(orc, 7, 3, M, N, K, b_batched=False)
