@@ -18,6 +18,7 @@
 //   everything else   -> patch gather into scratch (rows padded to 16 bytes)
 //                        + tensor-core GEMM
 #include "common.cuh"
+#include "gemm_u8_cut.cuh"
 #include "sm100_ptx.cuh"
 
 int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, const int32_t *bias,
@@ -695,6 +696,36 @@ extern "C" int mb_conv2d_u8_nhwc(mb_context *ctx, const uint8_t *in, const uint8
     MB_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
     return MB_SUCCESS;
+  }
+  // k x k on the tensor cores, the windows fetched by TMA as the GEMM goes (gemm_u8_cut.cu).  Channel counts that are
+  // no multiple of 16 (or a misaligned input) are first copied to one that is: the added channels
+  // hold the input zero point and add nothing whatever the filter side holds.
+  if (ctx->use_tensor_cores && pixels * O * depth > (1 << 18)) {
+    const int64_t Cp = static_cast<int64_t>(align_up(static_cast<size_t>(C), 16));
+    const bool copy_in = Cp != C || (reinterpret_cast<uintptr_t>(in) & 15u) != 0;
+    const bool copy_f = Cp != C || (reinterpret_cast<uintptr_t>(filter) & 15u) != 0;
+    const size_t in_bytes = copy_in ? align_up(static_cast<size_t>(N * H * W * Cp), 256) : 0;
+    const size_t f_bytes = copy_f ? static_cast<size_t>(O * KH * KW * Cp) : 0;
+    mb_cut_gemm g;
+    g.A = copy_in ? nullptr : in; g.B = copy_f ? nullptr : filter; g.bias = bias; g.C = out;
+    g.M = pixels; g.N = O; g.K = KH * KW * Cp;
+    g.zp_a = zp_in; g.zp_b = zp_f;
+    g.rq = p.rq; g.rq_variant = p.rq_variant;
+    g.conv = true;
+    g.H = p.H; g.W = p.W; g.C_in = static_cast<int>(Cp); g.KH = p.KH; g.KW = p.KW; g.sh = p.stride_h; g.sw = p.stride_w;
+    g.pad_t = p.pad_top; g.pad_l = p.pad_left; g.Ho = p.Ho; g.Wo = p.Wo;
+    const mb_cut_plan plan = mb_gemm_u8_cut_plan(ctx, g);
+    if (plan.cost >= 0 && in_bytes < (1ull << 33) && f_bytes < (1ull << 33)) {
+      if (copy_in || copy_f) {
+        uint8_t *scratch = nullptr;
+        MB_RETURN_IF_ERROR(mb_scratch(ctx, in_bytes + f_bytes, reinterpret_cast<void **>(&scratch)));
+        MB_RETURN_IF_ERROR(mb_repack_rows_u8(ctx, copy_in ? in : nullptr, scratch, N * H * W, C, Cp, zp_in,
+                                             copy_f ? filter : nullptr, scratch + in_bytes, O * KH * KW, C, Cp, 0));
+        if (copy_in) g.A = scratch;
+        if (copy_f) g.B = scratch + in_bytes;
+      }
+      return mb_gemm_u8_cut_launch(ctx, g, plan);
+    }
   }
   const size_t direct_smem = static_cast<size_t>(depth) * O * sizeof(int16_t);
   if (direct_smem <= 32 * 1024 && depth <= 256) {

@@ -214,6 +214,41 @@ def test_conv2d_u8(ctx, orc, case):
     _conv_case(ctx, orc, *case)
 
 
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("splits", [1, 2, 8])
+@pytest.mark.parametrize("two", [1, 2, 3])
+@pytest.mark.parametrize("case", [
+    # N, H, W, C, O, k, stride, pads beyond SAME's: odd maps, every swizzle width (C 32 / 64 / 128 and
+    # beyond, C no multiple of 16), padded and unpadded, tails of pixels, channels and depth
+    (2, 9, 11, 32, 72, 3, 1, "SAME"), (1, 14, 13, 48, 130, 3, 2, "SAME"), (3, 7, 7, 64, 40, 5, 1, "SAME"),
+    (1, 17, 19, 144, 65, 3, 1, "VALID"), (2, 12, 12, 200, 96, 3, 2, "VALID"), (1, 23, 21, 18, 33, 5, 2, "SAME"),
+    (2, 8, 9, 67, 100, 1, 2, "VALID")])
+def test_conv2d_u8_cut_over_clusters(ctx, orc, case, bn, splits, two):
+    """Windows by TMA in im2col mode, outside pixels overwritten with the zero point, the depth cut over a
+    cluster (two = 3: the persistent kernel, uncut): every byte against the oracle."""
+    N, H, W, C, O, k, stride, pad = case
+    rng = np.random.Generator(np.random.PCG64(C * O + k))
+    ho, wo, ph, pw = orc.calc_padding_and_output_size(H, W, k, k, (1, 1), (stride, stride), {"VALID": 0, "SAME": 1}[pad])
+    x, f, zp_in, zp_f, mult, shift = conv_quant(orc, rng, (N, H, W, C), (O, k, k, C), C * k * k)
+    bias = np.rint(rng.normal(0, 1000, size=O)).astype(np.int32)
+    dx, df, db, out = ctx.upload(x), ctx.upload(f), ctx.upload(bias), ctx.alloc(N * ho * wo * O)
+    for zi in (zp_in, 0):
+        exp = orc.conv2d_u8(x, f, bias, (stride, stride), (ph, pw), (ho, wo), zi, zp_f, mult, shift, 127)
+        for name, v in (("cut_bn", bn), ("cut_splits", 0 if two == 3 else splits), ("cut_two", two)):
+            ctx.set_option(name, v)
+        try:
+            before = ctx.launches_tensor_core
+            ctx.conv2d_u8(dx, df, db, out, N, H, W, C, O, k, k, (stride, stride), (ph >> 1, pw >> 1), (ho, wo), zi, zp_f,
+                          mult, shift, 127)
+            assert ctx.launches_tensor_core == before + 1
+        finally:
+            for name in ("cut_bn", "cut_splits", "cut_two"):
+                ctx.set_option(name, 0)
+        assert np.array_equal(ctx.download(out, exp.shape, np.uint8), exp)
+    for b in (dx, df, db, out):
+        b.free()
+
+
 def test_conv2d_u8_pointwise_uses_tensor_core(ctx, orc):
     before = ctx.launches_tensor_core
     _conv_case(ctx, orc, 2, 28, 28, 256, 256, 1, 1, 1, "VALID")
