@@ -11,6 +11,7 @@
 // 128-bit loads and integer dot-product instructions.  When the matrix is shared by all
 // batch entries (the FullyConnected case) the warp keeps its row and loops over the vectors.
 #include "common.cuh"
+#include "gemm_u8_cut.cuh"
 #include "sm100_ptx.cuh"
 
 namespace {
@@ -281,9 +282,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32) gemv_u8_stream_kernel(const Gem
 
 }  // namespace
 
-bool mb_gemm_u8_tc_supported(const mb_context *ctx, const void *A, const void *B, int64_t M,
-                             int64_t N, int64_t K, bool a_mn, bool b_mn, int a_batched,
-                             int b_batched);
+bool mb_gemm_u8_tc_supported(const mb_context *ctx, const void *A, const void *B, int64_t M, int64_t N, int64_t K,
+                             int64_t lda, int64_t ldb);
 int mb_gemm_u8_tc_launch_float_rule(mb_context *ctx, const uint8_t *A, const uint8_t *B,
                                     const int32_t *bias, void *C, int out_is_int32, int64_t M,
                                     int64_t N, int64_t K, int32_t zp_a, int32_t zp_b, float mult_f,
@@ -307,7 +307,7 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
   // out[batch x rows] = rhs[batch x K] * lhs[rows x K]^T: the tensor-core kernel with the float
   // requantization rule in its epilogue reads the matrix once instead of once per vector.
   if (!lhs_batched && rhs_batched && batch >= 16 && K % 16 == 0 && K <= 1024 && ctx->use_tensor_cores &&
-      mb_gemm_u8_tc_supported(ctx, rhs, lhs, batch, rows, K, false, false, 0, 0)) {
+      mb_gemm_u8_tc_supported(ctx, rhs, lhs, batch, rows, K, K, K)) {
     ctx->gemm_b_const = ctx->gemv_lhs_const;  // the matrix is the GEMM's B
     const int st = mb_gemm_u8_tc_launch_float_rule(ctx, rhs, lhs, bias, out, out_is_int32, batch, rows, K, zp_rhs,
                                            zp_lhs, multiplier, zp_out, add_zp_out);
@@ -351,6 +351,17 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
     MB_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
     return MB_SUCCESS;
+  }
+  // Several vectors against one matrix, of any length: the GEMM that fetches its own operands (the matrix is
+  // read once, its depth cut over clusters where the rows do not fill the SMs).
+  if (!lhs_batched && (rhs_batched || batch == 1) && ctx->use_tensor_cores && (batch >= 2 || K % 16 != 0) &&
+      batch * rows * K > (1 << 18)) {
+    mb_cut_gemm g;
+    g.A = rhs; g.B = lhs; g.bias = bias; g.C = out; g.out_is_int32 = out_is_int32;
+    g.M = batch; g.N = rows; g.K = K; g.zp_a = zp_rhs; g.zp_b = zp_lhs;
+    g.rq_variant = 8; g.mult_f = multiplier; g.zp_f = add_zp_out ? static_cast<float>(zp_out) : 0.f;
+    const mb_cut_plan plan = mb_gemm_u8_cut_plan(ctx, g);
+    if (plan.cost >= 0) return mb_gemm_u8_cut_launch(ctx, g, plan);
   }
   GemvParams p;
   p.lhs = lhs; p.rhs = rhs; p.bias = bias; p.out = out;
