@@ -51,6 +51,9 @@ struct mb_context {
   int cut_aligned = 0;           // aligned u8 products on the cluster-cut kernel: 0 by rule, 1 never, 2 always
   int cut_bn = 0, cut_splits = 0, cut_two = 0;  // cluster-cut GEMM: overrides of tile width, depth runs, CTAs per SM
                                  // (1 / 2; 3: convolutions on the persistent kernel) (0: by rule)
+  int f32_bn = 0, f32_splits = 0;  // self-fetching fp32 GEMM: overrides of tile width and depth runs (0: by rule)
+  int f32_gather = 0;            // ... and of its use: 0 by rule, 1 never, 2 wherever it can run
+  uint64_t f32_gather_attr_mask = 0;
   int cut_clusters[4] = {0, 0, 0, 0};  // CTAs of clusters of 2 / 4 / 8 that are resident at once, one CTA per SM (0: not asked)
   uint64_t cut_attr_mask = 0;    // kernels of gemm_u8_cut.cu / gemm_u8_gather.cu whose shared-memory limit was raised
   uint64_t func_attr_mask_plain = 0;  // the same for the GEMM's plain-store instances
@@ -289,5 +292,21 @@ __device__ __forceinline__ float mb_activate(float x, int act, float max_limit, 
     case 2: return fmaxf(0.f, fminf(max_limit, x));
     case 6: return fmaxf(x, 0.f) + fminf(x, 0.f) * coef;
     default: return x;
+  }
+}
+
+// The activation of several values, one decision for all of them (a branch per value costs an epilogue more than the
+// arithmetic); the same results as mb_activate.
+template <int COUNT>
+__device__ __forceinline__ void mb_activate_n(float (&x)[COUNT], int act, float max_limit, float coef) {
+  if (act == 1) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) x[j] = fmaxf(0.f, x[j]);
+  } else if (act == 2) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) x[j] = fmaxf(0.f, fminf(max_limit, x[j]));
+  } else if (act == 6) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) x[j] = fmaxf(x[j], 0.f) + fminf(x[j], 0.f) * coef;
   }
 }

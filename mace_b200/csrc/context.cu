@@ -429,6 +429,15 @@ int mb_set_option(mb_context *ctx, const char *name, int value) {
     ctx->use_tensor_cores = value;
   } else if (strcmp(name, "mn_major") == 0) {
     // accepted and without effect: MN-major operands always reach the tensor core in place
+  } else if (strcmp(name, "f32_gather") == 0) {
+    ctx->f32_gather = value;
+  } else if (strcmp(name, "f32_bn") == 0) {
+    if (value != 0 && value != 64 && value != 128) return mb_fail(ctx, MB_INVALID_ARGS, "f32_bn must be 0, 64 or 128");
+    ctx->f32_bn = value;
+  } else if (strcmp(name, "f32_splits") == 0) {
+    if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8)
+      return mb_fail(ctx, MB_INVALID_ARGS, "f32_splits must be 0, 1, 2, 4 or 8");
+    ctx->f32_splits = value;
   } else if (strcmp(name, "cut_aligned") == 0) {
     ctx->cut_aligned = value;
   } else if (strcmp(name, "cut_bn") == 0) {

@@ -74,8 +74,11 @@ __global__ void __launch_bounds__(256) dwconv_f32_rows_kernel(const DwF32Params 
   }
   float *out = p.out + (static_cast<int64_t>(plane) * p.Ho + h0) * p.Wo + w;
 #pragma unroll
+  for (int r = 0; r < RH; ++r) acc[r] += bias;
+  mb_activate_n(acc, p.act, p.max_limit, p.coef);
+#pragma unroll
   for (int r = 0; r < RH; ++r) {
-    if (h0 + r < p.Ho) *out = mb_activate(acc[r] + bias, p.act, p.max_limit, p.coef);
+    if (h0 + r < p.Ho) *out = acc[r];
     out += p.Wo;
   }
 }

@@ -7,6 +7,7 @@
 // index order; these kernels accumulate in fp32 in a tiled order, so results
 // agree to rounding (tests bound the difference at 1e-4 of the output range).
 #include "common.cuh"
+#include "gemm_f32_gather.cuh"
 
 bool mb_gemm_f32_tc_supported(const mb_context *ctx, const float *X, const float *W, int64_t Mdim,
                               int64_t Ndim, int64_t K, int64_t x_row_stride, int64_t x_batch_stride,
@@ -40,6 +41,8 @@ struct GemmF32Params {
 };
 
 __global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmF32Params p) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   __shared__ float As[FK][FT + 4];
   __shared__ float Bs[FK][FT + 4];
   const int b = blockIdx.z;
@@ -88,24 +91,52 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmF32Params p) {
   }
 }
 
-// ---- GEMV: one warp per matrix row ------------------------------------------------
+// ---- GEMV: one warp per matrix row and up to VECS vectors -----------------------------------
+// Bound by the matrix's bytes: a row is read once for VECS vectors, 16 bytes per lane where the rows allow, with as
+// many rows in flight as warps fit.
+template <int VECS, bool VEC4>
 __global__ void __launch_bounds__(256)
-gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs,
-                const float *__restrict__ bias, float *__restrict__ out, int64_t batch,
-                int64_t rows, int64_t K, int lhs_batched, int rhs_batched, int batch_chunk) {
+gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs, const float *__restrict__ bias,
+                float *__restrict__ out, int64_t batch, int64_t rows, int64_t K, int lhs_batched, int rhs_batched) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
-  const int64_t b0 = static_cast<int64_t>(blockIdx.y) * batch_chunk;
-  const int64_t b1 = min(batch, b0 + batch_chunk);
-  for (int64_t b = b0; b < b1; ++b) {
-    const float *lp = lhs + (lhs_batched ? b * rows * K : 0) + row * K;
-    const float *rp = rhs + (rhs_batched ? b * K : 0);
-    float s = 0.f;
-    for (int64_t i = lane; i < K; i += 32) s = fmaf(__ldg(lp + i), __ldg(rp + i), s);
+  const int64_t b0 = static_cast<int64_t>(blockIdx.y) * VECS;
+  const float *lp = lhs + (lhs_batched ? b0 * rows * K : 0) + row * K;
+  const float *rp = rhs + (rhs_batched ? b0 * K : 0);
+  const int vecs = static_cast<int>(min(static_cast<int64_t>(VECS), batch - b0));
+  float s[VECS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[b * rows + row] = s + (bias != nullptr ? bias[row] : 0.f);
+  for (int v = 0; v < VECS; ++v) s[v] = 0.f;
+  if (VEC4) {
+#pragma unroll 4
+    for (int64_t i = lane * 4; i < K; i += 128) {
+      const float4 a = __ldg(reinterpret_cast<const float4 *>(lp + i));
+#pragma unroll
+      for (int v = 0; v < VECS; ++v) {
+        if (v < vecs) {
+          const float4 x = __ldg(reinterpret_cast<const float4 *>(rp + v * K + i));
+          s[v] = fmaf(a.x, x.x, s[v]); s[v] = fmaf(a.y, x.y, s[v]);
+          s[v] = fmaf(a.z, x.z, s[v]); s[v] = fmaf(a.w, x.w, s[v]);
+        }
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int64_t i = lane; i < K; i += 32) {
+      const float a = __ldg(lp + i);
+#pragma unroll
+      for (int v = 0; v < VECS; ++v)
+        if (v < vecs) s[v] = fmaf(a, __ldg(rp + v * K + i), s[v]);
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < VECS; ++v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[v] += __shfl_xor_sync(0xffffffffu, s[v], o);
+    if (lane == 0 && v < vecs) out[(b0 + v) * rows + row] = s[v] + (bias != nullptr ? __ldg(bias + row) : 0.f);
   }
 }
 
@@ -120,6 +151,8 @@ struct ConvF32Params {
 
 // One thread per output value; the loop order (c, kh, kw) is the reference's.
 __global__ void __launch_bounds__(256) conv2d_f32_direct_kernel(const ConvF32Params p) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t total = static_cast<int64_t>(p.N) * p.O * p.Ho * p.Wo;
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (tid >= total) return;
@@ -237,20 +270,44 @@ unmerge_f32_kernel(const float *__restrict__ src, float *__restrict__ dst, int64
   dst[i] = __ldg(src + o * src_rs + n * hw + pos);
 }
 
-// out[c][r] = in[r][c] for a [rows x cols] matrix, through a 32 x 33 shared-memory tile.
-__global__ void __launch_bounds__(256)
-transpose_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int rows, int cols) {
-  __shared__ float tile[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int i = ty; i < 32; i += 8)
-    if (r0 + i < rows && c0 + tx < cols) tile[i][tx] = __ldg(in + static_cast<int64_t>(r0 + i) * cols + c0 + tx);
-  __syncthreads();
-  for (int i = ty; i < 32; i += 8)
-    if (c0 + i < cols && r0 + tx < rows) out[static_cast<int64_t>(c0 + i) * rows + r0 + tx] = tile[tx][i];
+}  // namespace
+
+// Whether the kernel that fetches its own operands takes a product (see gemm_f32_gather.cu); by_tma: the TMA-fed one of
+// gemm_f32_tc.cu could.
+static bool take_gather(mb_context *ctx, const mb_f32_gemm &g, bool by_tma) {
+  if (ctx->f32_gather == 1 || !mb_gemm_f32_gather_supported(ctx, g)) return false;
+  if (ctx->f32_gather == 2 || !by_tma) return true;
+  // The TMA-fed kernel: tiles of 128 columns of one image (or matrix), 1200 cycles per step, 2.6 us for the results of 128
+  // channels (twice that with a residual), 4.4 us around them.
+  const int64_t images = g.conv ? g.M / (static_cast<int64_t>(g.Ho) * g.Wo) : g.batch;
+  const int64_t tiles_m = ceil_div64(g.M / (g.conv ? images : 1), 128), steps = ceil_div64(g.K, 32);
+  int64_t tma = -1;
+  for (int w : {128, 64}) {
+    if (w == 128 && g.N <= 64) continue;
+    const int64_t rounds = ceil_div64(images * tiles_m * ceil_div64(g.N, w), ctx->num_sms);
+    const int64_t results = (w == 128 ? 5000 : 3000) * (g.residual != nullptr ? 2 : 1);
+    const int64_t cost = 8300 + rounds * std::max<int64_t>(steps * 1200, results);
+    if (tma < 0 || cost < tma) tma = cost;
+  }
+  return mb_gemm_f32_gather_cost(ctx, g) < tma;
 }
 
-}  // namespace
+// The convolution as that kernel sees it.
+static mb_f32_gemm conv_gemm(const float *in, const float *filter, const float *bias, const float *residual, float *out,
+                             int64_t N, int64_t C, int64_t H, int64_t W, int64_t O, int64_t KH, int64_t KW, int sh,
+                             int sw, int dh, int dw, int pad_t, int pad_l, int64_t Ho, int64_t Wo, int act,
+                             float max_limit, float coef) {
+  mb_f32_gemm g;
+  g.X = in; g.W = filter; g.bias = bias; g.residual = residual; g.C = out;
+  g.M = N * Ho * Wo; g.N = O; g.K = C * KH * KW;
+  g.act = act; g.max_limit = max_limit; g.coef = coef;
+  g.conv = true;
+  g.C_in = static_cast<int>(C); g.H = static_cast<int>(H); g.Wd = static_cast<int>(W);
+  g.KH = static_cast<int>(KH); g.KW = static_cast<int>(KW);
+  g.sh = sh; g.sw = sw; g.dh = dh; g.dw = dw; g.pad_t = pad_t; g.pad_l = pad_l;
+  g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
+  return g;
+}
 
 // Strided batched fp32 GEMM with optional per-row bias and activation; the
 // building block of the 1x1 convolution and of the Winograd batched product.
@@ -259,10 +316,24 @@ int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *
                         int64_t a_rs, int64_t a_cs, int64_t a_bs, int64_t b_rs, int64_t b_cs,
                         int64_t b_bs, int64_t c_rs, int64_t c_cs, int64_t c_bs, int act,
                         float max_limit, float coef) {
+  mb_f32_gemm g;
+  if (c_cs == 1 || bias_per_row != nullptr) {  // the columns of C are the tensor core's M
+    g.X = B; g.x_ks = b_rs; g.x_ms = b_cs; g.x_bs = b_bs;
+    g.W = A; g.w_ns = a_rs; g.w_ks = a_cs; g.w_bs = a_bs;
+    g.M = N; g.N = M; g.c_ns = c_rs; g.c_ms = c_cs;
+  } else {
+    g.X = A; g.x_ks = a_cs; g.x_ms = a_rs; g.x_bs = a_bs;
+    g.W = B; g.w_ns = b_cs; g.w_ks = b_rs; g.w_bs = b_bs;
+    g.M = M; g.N = N; g.c_ns = c_cs; g.c_ms = c_rs;
+  }
+  g.batch = batch; g.K = K; g.C = C; g.c_bs = c_bs; g.bias = bias_per_row;
+  g.act = act; g.max_limit = max_limit; g.coef = coef;
+  const bool by_tma = a_cs == 1 && b_cs == 1 && c_cs == 1 &&
+                      mb_gemm_f32_tc_supported(ctx, B, A, N, M, K, b_rs, b_bs, a_rs, a_bs);
+  if (take_gather(ctx, g, by_tma)) return mb_gemm_f32_gather_launch(ctx, g);
   // C = A * B with A [M x K] k-contiguous, B [K x N] n-contiguous and C n-contiguous is the
   // tensor-core kernel's layout with the roles X = B (pixels x channels side), W = A.
-  if (a_cs == 1 && b_cs == 1 && c_cs == 1 &&
-      mb_gemm_f32_tc_supported(ctx, B, A, N, M, K, b_rs, b_bs, a_rs, a_bs)) {
+  if (by_tma) {
     return mb_gemm_f32_tc_launch(ctx, B, A, bias_per_row, C, batch, N, M, K, b_rs, b_bs, a_rs, a_bs,
                                  c_rs, c_bs, act, max_limit, coef, nullptr);
   }
@@ -276,7 +347,7 @@ int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *
   p.act = act; p.max_limit = max_limit; p.coef = coef;
   dim3 grid(static_cast<unsigned>(ceil_div64(N, FT)), static_cast<unsigned>(ceil_div64(M, FT)),
             static_cast<unsigned>(batch));
-  gemm_f32_kernel<<<grid, 256, 0, ctx->stream>>>(p);
+  MB_CUDA(ctx, mb_launch_chained(ctx, gemm_f32_kernel, dim3(grid), dim3(256), 0, p));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
@@ -385,37 +456,27 @@ int mb_gemv_f32(mb_context *ctx, const float *lhs, const float *rhs, const float
   if (lhs == nullptr || rhs == nullptr || out == nullptr)
     return mb_fail(ctx, MB_INVALID_ARGS, "mb_gemv_f32: null operand");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  // Many vectors against one matrix (FullyConnected on a batch) on the tensor cores: the
-  // vectors are transposed to [K x batch] (the kernel's activation operand has the long
-  // dimension contiguous), the product comes out as [rows x batch] and is transposed back.
-  if (!lhs_batched && rhs_batched && batch >= 32 && batch % 4 == 0 && K % 4 == 0 && rows >= 16 &&
-      batch < (1 << 30) && K < (1 << 30) && rows < (1 << 30)) {
-    float *scratch = nullptr;
-    const size_t xt_bytes = align_up(sizeof(float) * K * batch, 256);
-    MB_RETURN_IF_ERROR(mb_scratch(ctx, xt_bytes + sizeof(float) * rows * batch, reinterpret_cast<void **>(&scratch)));
-    float *xt = scratch, *ct = scratch + xt_bytes / sizeof(float);
-    if (mb_gemm_f32_tc_supported(ctx, xt, lhs, batch, rows, K, batch, 0, K, 0)) {
-      dim3 g1(static_cast<unsigned>(ceil_div64(K, 32)), static_cast<unsigned>(ceil_div64(batch, 32)));
-      transpose_f32_kernel<<<g1, 256, 0, ctx->stream>>>(rhs, xt, static_cast<int>(batch), static_cast<int>(K));
-      MB_CUDA(ctx, cudaGetLastError());
-      MB_RETURN_IF_ERROR(mb_gemm_f32_tc_launch(ctx, xt, lhs, bias, ct, 1, batch, rows, K, batch, 0, K, 0, batch, 0,
-                                               0, 0.f, 0.f, nullptr));
-      dim3 g2(static_cast<unsigned>(ceil_div64(batch, 32)), static_cast<unsigned>(ceil_div64(rows, 32)));
-      transpose_f32_kernel<<<g2, 256, 0, ctx->stream>>>(ct, out, static_cast<int>(rows), static_cast<int>(batch));
-      MB_CUDA(ctx, cudaGetLastError());
-      ctx->launches += 2;
-      return MB_SUCCESS;
-    }
+  if (!lhs_batched && rhs_batched && (batch > 8 || ctx->f32_gather == 2)) {
+    // the vectors are the tensor core's M, the matrix its N (up to eight vectors share a pass of the CUDA-core kernel)
+    mb_f32_gemm g;
+    g.X = rhs; g.x_ks = 1; g.x_ms = K;
+    g.W = lhs; g.w_ns = K; g.w_ks = 1;
+    g.bias = bias; g.C = out; g.c_ns = 1; g.c_ms = rows;
+    g.M = batch; g.N = rows; g.K = K;
+    if (take_gather(ctx, g, false)) return mb_gemm_f32_gather_launch(ctx, g);
   }
-  int64_t chunks = std::min<int64_t>(batch, 65535);
-  if (!lhs_batched)
-    chunks = std::min<int64_t>(chunks, std::max<int64_t>(1, (4ll * ctx->num_sms) / ceil_div64(rows, 8)));
-  const int batch_chunk = static_cast<int>(ceil_div64(batch, chunks));
-  dim3 grid(static_cast<unsigned>(ceil_div64(rows, 8)),
-            static_cast<unsigned>(ceil_div64(batch, batch_chunk)));
-  gemv_f32_kernel<<<grid, 256, 0, ctx->stream>>>(lhs, rhs, bias, out, batch, rows, K, lhs_batched,
-                                                 rhs_batched, batch_chunk);
-  MB_CUDA(ctx, cudaGetLastError());
+  const bool shared = !lhs_batched && rhs_batched;  // (one matrix, several vectors: up to eight per pass)
+  const int vecs = !shared || batch == 1 ? 1 : batch == 2 ? 2 : batch <= 4 ? 4 : 8;
+  if (ceil_div64(batch, vecs) > 65535) return mb_fail(ctx, MB_UNSUPPORTED, "mb_gemv_f32: batch too large");
+  const dim3 grid(static_cast<unsigned>(ceil_div64(rows, 8)), static_cast<unsigned>(ceil_div64(batch, vecs)));
+  const bool vec4 = K % 4 == 0 && ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) & 15u) == 0;
+#define MB_GEMV(V_)                                                                                                   \
+  MB_CUDA(ctx, vec4 ? mb_launch_chained(ctx, gemv_f32_kernel<V_, true>, grid, dim3(256), 0, lhs, rhs, bias, out, batch, \
+                                        rows, K, lhs_batched, rhs_batched)                                            \
+                    : mb_launch_chained(ctx, gemv_f32_kernel<V_, false>, grid, dim3(256), 0, lhs, rhs, bias, out, batch, \
+                                        rows, K, lhs_batched, rhs_batched));
+  if (vecs == 8) { MB_GEMV(8) } else if (vecs == 4) { MB_GEMV(4) } else if (vecs == 2) { MB_GEMV(2) } else { MB_GEMV(1) }
+#undef MB_GEMV
   ctx->launches++;
   return MB_SUCCESS;
 }
@@ -453,8 +514,16 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
                                     Wo, activation, &empty));
   if (empty) return MB_SUCCESS;
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  if (KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 &&
-      Ho == H && Wo == W && ((H * W) % 4 == 0 && H * W >= 128 || !ctx->use_tensor_cores)) {
+  const bool pointwise = KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 && Ho == H && Wo == W;
+  {
+    const mb_f32_gemm g = conv_gemm(in, filter, bias, nullptr, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h,
+                                    dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);
+    if (N * O * Ho * Wo * C * KH * KW >= (1ll << 16) &&
+        take_gather(ctx, g, pointwise && (H * W) % 4 == 0 && H * W >= 128 &&
+                                mb_gemm_f32_tc_supported(ctx, in, filter, H * W, O, C, H * W, C * H * W, C, 0)))
+      return mb_gemm_f32_gather_launch(ctx, g);
+  }
+  if (pointwise && ((H * W) % 4 == 0 && H * W >= 128 || !ctx->use_tensor_cores)) {
     // out_n[O x HW] = filter[O x C] * in_n[C x HW] for every image n
     // (arm::Conv2dK1x1, mace/ops/arm/base/conv_2d_1x1.cc:61-68)
     const int64_t hw = H * W;
@@ -476,8 +545,8 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
   p.Ho = static_cast<int>(Ho); p.Wo = static_cast<int>(Wo);
   p.act = activation; p.max_limit = max_limit; p.coef = coefficient;
   const int64_t total = N * O * Ho * Wo;
-  conv2d_f32_direct_kernel<<<static_cast<unsigned>(ceil_div64(total, 256)), 256, 0, ctx->stream>>>(p);
-  MB_CUDA(ctx, cudaGetLastError());
+  MB_CUDA(ctx, mb_launch_chained(ctx, conv2d_f32_direct_kernel, dim3(static_cast<unsigned>(ceil_div64(total, 256))),
+                                 dim3(256), 0, p));
   ctx->launches++;
   return MB_SUCCESS;
 }
@@ -498,6 +567,14 @@ int mb_conv2d_f32_nchw_residual(mb_context *ctx, const float *in, const float *f
   if (empty) return MB_SUCCESS;
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
   const int64_t hw = H * W;
+  {
+    const mb_f32_gemm g = conv_gemm(in, filter, bias, residual, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h,
+                                    dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);
+    if (take_gather(ctx, g, KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 && Ho == H &&
+                                Wo == W && hw % 4 == 0 && hw >= 128 &&
+                                mb_gemm_f32_tc_supported(ctx, in, filter, hw, O, C, hw, C * hw, C, 0)))
+      return mb_gemm_f32_gather_launch(ctx, g);
+  }
   // 1x1 stride 1 on the tensor cores: the sum and the activation ride in the GEMM's epilogue
   if (KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 && Ho == H &&
       Wo == W && hw % 4 == 0 && hw >= 128 &&

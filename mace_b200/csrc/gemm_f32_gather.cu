@@ -1,0 +1,638 @@
+// fp32 GEMM on tcgen05 (kind::tf32, split operands as in gemm_f32_tc.cu) whose warps fetch X from where it lies: no
+// column matrix for a convolution, no transposes, no 16-byte alignment.
+//
+// What it serves: the general Conv2D (mace/ops/arm/base/conv_2d_general.cc:26-197, ref/conv_2d.cc:36-122), the 3x3
+// Conv2D where a direct convolution beats Winograd (arm/base/conv_2d_3x3_winograd.cc:31-787), the 1x1 one of any stride
+// (conv_2d_1x1.cc:27-72), MatMul / Gemm of every transposition (arm/base/gemm.cc:520-683), FullyConnected on a batch.
+//
+// X (the MMA's A: 128 pixels = 128 TMEM lanes) never touches shared memory: lane i of a warp owns pixel i and loads its
+// 32 values of a depth step straight from the tensor (neighbouring lanes are neighbouring pixels of a row:
+// coalesced), splits them in registers and writes hi and lo to tensor memory, where the MMA takes A from.  Which
+// element a depth index k means -- channel, filter row, filter column -- is the same for all lanes: lane j works out
+// the offset and the row / column bits of k = 32 * step + j once per step and shares them through shared memory; a lane
+// holds its pixel's valid filter rows and columns as bit masks, so padding costs one logic instruction per value.
+// W comes by TMA where its rows are 16-byte aligned, else through registers, and is split in shared memory.
+//
+// Roles (22 warps): three groups of four load X, taking the steps in turn (three steps of loads in flight; fetching
+// with 4-byte asynchronous copies through shared memory instead took twice as long, 128 of them per step), four split
+// W, four store results, one thread issues the MMAs, one requests W.  Persistent over the tiles; where these do not fill
+// the SMs, one tile per cluster of 2 .. 8 CTAs with the depth cut between them, the partial tiles added up through
+// distributed shared memory.
+//
+// What bounds it: the tensor pipe at three tf32 MMAs per product for long depths (12 MMAs x 92 cycles per step of
+// 128 x 128 x 32; a convolution's loads bring the step to 1400), the launch, first loads and results for small shapes.
+// Measured, before -> now: 7x7 stride 2 of 3 -> 64 channels, 224 x 224, batch 256, 1360 us (column matrix) -> 732;
+// 5x5 stride 2 of 48 -> 32, 112 x 112, batch 24, 341 -> 116; 3x3 of 512 channels, 7 x 7, batch 1, 70 (Winograd) -> 20;
+// 384 x 384 x 64 times a transposed matrix, batch 12, 16.4 (CUDA cores) -> 7.9; 736 x 176 x 384, batch 24, 152 -> 29.
+#include <algorithm>
+
+#include "gemm_f32_gather.cuh"
+#include "gemm_u8_cut.cuh"  // mb_launch_clusters
+#include "sm100_ptx.cuh"
+
+int mb_make_map_w_f32(mb_context *ctx, CUtensorMap *map, const float *W, int64_t K, int64_t N, int64_t batch, int64_t w_ns,
+                      int64_t w_bs, int bn);
+
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128;         // pixels (m) per tile == TMEM lanes
+constexpr int KB = 32;          // depth per step
+constexpr int XGROUPS = 3;      // of four warps each, taking the steps in turn
+constexpr int FIRST_W = 4 * XGROUPS, FIRST_E = FIRST_W + 4, EWARPS = 4, MMA_WARP = FIRST_E + EWARPS, TMA_WARP = MMA_WARP + 1;
+constexpr int THREADS = (TMA_WARP + 1) * 32;
+constexpr int ACCS = 2;
+constexpr long long WAIT_BUDGET = 1ll << 31;        // ~1 s of SM clocks per wait
+enum { W_TMA = 0, W_ROWS = 1, W_COLS = 2 };         // k contiguous and 16-byte aligned; k contiguous; n contiguous
+enum { X_CONV = 0, X_ROWS = 1, X_COLS = 2 };        // convolution; m contiguous; k contiguous
+
+struct Params {
+  const float *X, *W, *bias, *residual;
+  float *C;
+  int M, N, K, batch;
+  int tiles_m, tiles_n, k_blocks, splits;
+  int step_m, step_n, step_b;  // gridDim.x in tile coordinates
+  int64_t x_ks, x_ms, x_bs, w_ns, w_ks, w_bs, c_ns, c_ms, c_bs;
+  int x_vec;                   // K-contiguous rows are 16-byte aligned
+  int act;
+  float max_limit, coef;
+  int H, Wd, KW, taps, sh, sw, dh, dw, pad_t, pad_l, Wo, hw, KH;
+  int64_t image;               // C_in * H * Wd
+  uint32_t taps_mul, taps_shift, kw_mul, kw_shift, hw_mul, hw_shift, wo_mul, wo_shift;
+  int *status;
+};
+
+template <int BN>
+struct Cfg {
+  static constexpr int W_BYTES = BN * KB * 4;            // hi (or lo) of a step
+  static constexpr int STAGE_BYTES = 2 * W_BYTES;
+  static constexpr int A_COL0 = ACCS * BN;               // TMEM: accumulators, then STAGES x 64 columns of A
+  static constexpr int STAGES = (512 - A_COL0) / (2 * KB);
+  static constexpr int RING = STAGES * STAGE_BYTES;
+  static constexpr int TABLE_BYTES = FIRST_W * KB * 8;
+  static constexpr int SMEM_BYTES = RING + 1024 /*align*/ + TABLE_BYTES + 256 /*barriers*/;
+  static_assert(BN * BM * 4 <= RING, "the partial tile reuses the ring");
+};
+
+struct TileIter {
+  int tm, tn, b;
+  __device__ __forceinline__ TileIter(const Params &p) {
+    const unsigned t = blockIdx.x / static_cast<unsigned>(p.splits);
+    tm = t % p.tiles_m;
+    const unsigned q = t / p.tiles_m;
+    tn = q % p.tiles_n;
+    b = q / p.tiles_n;
+  }
+  __device__ __forceinline__ bool valid(const Params &p) const { return b < p.batch; }
+  __device__ __forceinline__ void next(const Params &p) {
+    tm += p.step_m;
+    tn += p.step_n;
+    b += p.step_b;
+    if (tm >= p.tiles_m) { tm -= p.tiles_m; ++tn; }
+    if (tn >= p.tiles_n) { tn -= p.tiles_n; ++b; }
+  }
+};
+
+// (Rounding hi instead of cutting it off changed nothing: what error there is grows with the depth and comes from the
+// accumulator, which cuts off too.)
+__device__ __forceinline__ uint32_t tf32_hi(float v) { return __float_as_uint(v) & 0xffffe000u; }
+__device__ __forceinline__ uint32_t tf32_lo(float v) { return __float_as_uint(v - __uint_as_float(tf32_hi(v))); }
+
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
+// Rows of 32 k, 128 bytes, the 16-byte chunks of a row permuted by its low three bits (the tensor core's 128-byte swizzle).
+__device__ __forceinline__ uint32_t swz_at(int row, int chunk) { return static_cast<uint32_t>(row * 128 + ((chunk ^ (row & 7)) << 4)); }
+
+// Where pixel m of the result lies (channel 0).
+template <int XK>
+__device__ __forceinline__ int64_t out_offset(const Params &p, int m, int b) {
+  if (XK == X_CONV) {
+    const uint32_t img = fast_div(static_cast<uint32_t>(m), p.hw_mul, p.hw_shift);
+    return static_cast<int64_t>(img) * p.N * p.hw + (m - static_cast<int>(img) * p.hw);
+  }
+  return b * p.c_bs + m * p.c_ms;
+}
+
+template <int BN, int XK, int WK>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Params p) {
+  using C = Cfg<BN>;
+  constexpr int STAGES = C::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t bars = smem_base + C::RING + C::TABLE_BYTES;
+  const uint32_t full_bar = bars, empty_bar = bars + 8 * STAGES;          // [STAGES]
+  const uint32_t wfull_bar = empty_bar + 8 * STAGES;                      // [STAGES] W landed (by TMA)
+  const uint32_t tfull_bar = wfull_bar + 8 * STAGES, tempty_bar = tfull_bar + 8 * ACCS;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + C::RING + C::TABLE_BYTES + 24 * STAGES + 16 * ACCS);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  mb_grid_dep_launch();
+
+  if (threadIdx.x == MMA_WARP * 32) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full_bar + 8 * s, 8);  // four X warps and four W warps
+      mbar_init(empty_bar + 8 * s, 1);
+      mbar_init(wfull_bar + 8 * s, 1);
+    }
+    if (WK == W_TMA) prefetch_tensormap(&map_w);
+    for (int a = 0; a < ACCS; ++a) {
+      mbar_init(tfull_bar + 8 * a, 1);
+      mbar_init(tempty_bar + 8 * a, EWARPS);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == FIRST_E) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  const int rank = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int kb_begin = static_cast<int>(static_cast<int64_t>(p.k_blocks) * rank / p.splits);
+  const int steps = static_cast<int>(static_cast<int64_t>(p.k_blocks) * (rank + 1) / p.splits) - kb_begin;
+  auto fail = [&](int code) {
+    *abort_flag = 1;
+    atomicCAS(p.status, 0, code);
+  };
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  mb_grid_dep_wait();
+
+  if (warp < FIRST_W) {
+    // ---- X: tensor -> registers -> hi / lo in tensor memory ----
+    const int group = warp >> 2, quarter = warp & 3;
+    const uint32_t a_lane = static_cast<uint32_t>(quarter * 32) << 16;
+    int2 *table = reinterpret_cast<int2 *>(smem + C::RING) + warp * KB;
+    int it = 0;  // steps of this CTA so far, all tiles
+    bool ok = true;
+    for (TileIter t(p); ok && t.valid(p); t.next(p)) {
+      const int m = t.tm * BM + quarter * 32 + lane;
+      const float *base = p.X;
+      uint32_t valid = 0;  // filter rows (bits 0 ..) and columns (bits 16 ..) of this pixel that lie inside the image
+      if (XK == X_CONV) {
+        const uint32_t img = fast_div(static_cast<uint32_t>(m), p.hw_mul, p.hw_shift);
+        const int pix = m - static_cast<int>(img) * p.hw;
+        const int ho = static_cast<int>(fast_div(static_cast<uint32_t>(pix), p.wo_mul, p.wo_shift));
+        const int h0 = ho * p.sh - p.pad_t, w0 = (pix - ho * p.Wo) * p.sw - p.pad_l;
+        base += static_cast<int64_t>(img) * p.image + static_cast<int64_t>(h0) * p.Wd + w0;
+        if (m < p.M) {
+          for (int i = 0; i < p.KH; ++i) valid |= (h0 + i * p.dh >= 0 && h0 + i * p.dh < p.H ? 1u : 0u) << i;
+          for (int i = 0; i < p.KW; ++i) valid |= (w0 + i * p.dw >= 0 && w0 + i * p.dw < p.Wd ? 1u : 0u) << (16 + i);
+        }
+      } else {
+        base += t.b * p.x_bs + m * p.x_ms;
+        valid = m < p.M ? 1u : 0u;
+      }
+      for (int i = 0; i < steps; ++i, ++it) {
+        if (it % XGROUPS != group) continue;
+        const int stage = it % STAGES;
+        const int k0 = (kb_begin + i) * KB;
+        float v[KB];
+        if (XK == X_COLS) {
+          const float *row = base + k0;
+          if (p.x_vec) {
+#pragma unroll
+            for (int j = 0; j < KB; j += 4) {
+              const bool in = valid != 0 && k0 + j < p.K;
+              const float4 x = in ? __ldg(reinterpret_cast<const float4 *>(row + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < KB; ++j) v[j] = valid != 0 && k0 + j < p.K ? __ldg(row + j) : 0.f;
+          }
+        } else {
+          const int k = k0 + lane;
+          int2 e;
+          if (XK == X_CONV) {
+            const int c = static_cast<int>(fast_div(static_cast<uint32_t>(k), p.taps_mul, p.taps_shift));
+            const int tap = k - c * p.taps;
+            const int kh = static_cast<int>(fast_div(static_cast<uint32_t>(tap), p.kw_mul, p.kw_shift));
+            const int kw = tap - kh * p.KW;
+            e.x = (c * p.H + kh * p.dh) * p.Wd + kw * p.dw;
+            e.y = static_cast<int>((1u << kh) | (0x10000u << kw));
+          } else {
+            e.x = static_cast<int>(k * p.x_ks);
+            e.y = 1;
+          }
+          if (k >= p.K) e = make_int2(0, static_cast<int>(0x80000000u));  // (no pixel has bit 31)
+          __syncwarp();  // the table of the previous step has been read
+          table[lane] = e;
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < KB; j += 2) {
+            const int4 t2 = *reinterpret_cast<const int4 *>(table + j);
+            v[j] = (valid & t2.y) == static_cast<uint32_t>(t2.y) ? __ldg(base + t2.x) : 0.f;
+            v[j + 1] = (valid & t2.w) == static_cast<uint32_t>(t2.w) ? __ldg(base + t2.z) : 0.f;
+          }
+        }
+        if (it >= STAGES && !mbar_wait_warp(empty_bar + 8 * stage, ((it / STAGES) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
+          fail(MB_DEV_TIMEOUT_PRODUCER);
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t slot = tmem + a_lane + C::A_COL0 + stage * (2 * KB);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = tf32_hi(v[h * 16 + j]);
+          tmem_st_32x32b_x16(slot + h * 16, r);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = tf32_lo(v[h * 16 + j]);
+          tmem_st_32x32b_x16(slot + KB + h * 16, r);
+        }
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full_bar + 8 * stage);
+      }
+    }
+  } else if (warp < FIRST_E) {
+    // ---- W: (matrix -> registers ->) hi / lo in shared memory, rows of 32 k, 128-byte swizzle ----
+    const int w4 = warp - FIRST_W;
+    int it = 0;
+    bool ok = true;
+    for (TileIter t(p); ok && t.valid(p); t.next(p)) {
+      const int n0 = t.tn * BN;
+      const float *W = p.W + t.b * p.w_bs;
+      for (int i = 0; i < steps; ++i, ++it) {
+        const int stage = it % STAGES;
+        uint8_t *tile = smem + stage * C::STAGE_BYTES;
+        if (WK == W_TMA) {
+          if (!mbar_wait_warp(wfull_bar + 8 * stage, (it / STAGES) & 1, abort_flag, WAIT_BUDGET)) {
+            fail(MB_DEV_TIMEOUT_EPILOGUE);
+            ok = false;
+            break;
+          }
+#pragma unroll
+          for (int c = 0; c < C::W_BYTES / 2048; ++c) {
+            const int at = (c * 128 + w4 * 32 + lane) * 16;
+            const float4 v = *reinterpret_cast<const float4 *>(tile + at);
+            *reinterpret_cast<uint4 *>(tile + at) = make_uint4(tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w));
+            *reinterpret_cast<uint4 *>(tile + C::W_BYTES + at) = make_uint4(tf32_lo(v.x), tf32_lo(v.y), tf32_lo(v.z), tf32_lo(v.w));
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full_bar + 8 * stage);
+          continue;
+        }
+        const int k0 = (kb_begin + i) * KB;
+        constexpr int CH = BN / 16;  // 16-byte chunks per thread
+        float4 v[CH];
+        int row[CH], chunk[CH];
+        if (WK == W_COLS) {
+          // lane = row, a chunk is four depth rows of the matrix
+          constexpr int WARPS_N = BN / 32;  // warps along n; the others take other depth rows
+          const int n = (w4 % WARPS_N) * 32 + lane;
+          const bool in = n0 + n < p.N;
+#pragma unroll
+          for (int c = 0; c < CH; ++c) {
+            row[c] = n;
+            chunk[c] = (w4 / WARPS_N) * CH + c;
+            const int k = k0 + chunk[c] * 4;
+            const float *src = W + n0 + n + static_cast<int64_t>(k) * p.w_ks;
+            v[c].x = in && k < p.K ? __ldg(src) : 0.f;
+            v[c].y = in && k + 1 < p.K ? __ldg(src + p.w_ks) : 0.f;
+            v[c].z = in && k + 2 < p.K ? __ldg(src + 2 * p.w_ks) : 0.f;
+            v[c].w = in && k + 3 < p.K ? __ldg(src + 3 * p.w_ks) : 0.f;
+          }
+        } else {
+          const int c8 = lane & 7, k = k0 + c8 * 4;
+#pragma unroll
+          for (int c = 0; c < CH; ++c) {
+            row[c] = w4 * (BN / 4) + c * 4 + (lane >> 3);
+            chunk[c] = c8;
+            const float *src = W + static_cast<int64_t>(n0 + row[c]) * p.w_ns + k;
+            const bool in = n0 + row[c] < p.N;
+            v[c].x = in && k < p.K ? __ldg(src) : 0.f;
+            v[c].y = in && k + 1 < p.K ? __ldg(src + 1) : 0.f;
+            v[c].z = in && k + 2 < p.K ? __ldg(src + 2) : 0.f;
+            v[c].w = in && k + 3 < p.K ? __ldg(src + 3) : 0.f;
+          }
+        }
+        if (it >= STAGES && !mbar_wait_warp(empty_bar + 8 * stage, ((it / STAGES) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
+          fail(MB_DEV_TIMEOUT_PRODUCER);
+          ok = false;
+          break;
+        }
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          const uint32_t at = swz_at(row[c], chunk[c]);
+          *reinterpret_cast<uint4 *>(tile + at) = make_uint4(tf32_hi(v[c].x), tf32_hi(v[c].y), tf32_hi(v[c].z), tf32_hi(v[c].w));
+          *reinterpret_cast<uint4 *>(tile + C::W_BYTES + at) = make_uint4(tf32_lo(v[c].x), tf32_lo(v[c].y), tf32_lo(v[c].z), tf32_lo(v[c].w));
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full_bar + 8 * stage);
+      }
+    }
+  } else if (warp == TMA_WARP) {
+    if (WK == W_TMA && lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (TileIter t(p); ok && t.valid(p); t.next(p)) {
+        for (int i = 0; i < steps; ++i, ++it) {
+          const int stage = it % STAGES;
+          if (it >= STAGES && !mbar_wait(empty_bar + 8 * stage, ((it / STAGES) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
+            fail(MB_DEV_TIMEOUT_PRODUCER);
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(wfull_bar + 8 * stage, C::W_BYTES);
+          tma_load_3d(smem_base + stage * C::STAGE_BYTES, &map_w, wfull_bar + 8 * stage, (kb_begin + i) * KB, t.tn * BN,
+                      p.w_bs != 0 ? t.b : 0);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == MMA_WARP) {
+    // ---- MMA: one thread ----
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(/*c f32*/ 1, /*a tf32*/ 2, /*b tf32*/ 2, false, false, BM, BN);
+      const uint64_t wdesc = make_smem_desc(0, 16, 1024, 2);
+      int it = 0, local = 0;
+      bool ok = true;
+      for (TileIter t(p); ok && t.valid(p); t.next(p), ++local) {
+        const int acc = local % ACCS;
+        if (local >= ACCS && !mbar_wait(tempty_bar + 8 * acc, ((local / ACCS) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
+          fail(MB_DEV_TIMEOUT_MMA);
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t d = tmem + acc * BN;
+        for (int i = 0; i < steps; ++i, ++it) {
+          const int stage = it % STAGES;
+          if (!mbar_wait(full_bar + 8 * stage, (it / STAGES) & 1, abort_flag, WAIT_BUDGET)) {
+            fail(MB_DEV_TIMEOUT_MMA);
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t a_hi = tmem + C::A_COL0 + stage * (2 * KB), a_lo = a_hi + KB;
+          const uint32_t sw = smem_base + stage * C::STAGE_BYTES;
+          const uint64_t w_hi = wdesc | static_cast<uint64_t>((sw >> 4) & 0x3FFFu);
+          const uint64_t w_lo = wdesc | static_cast<uint64_t>(((sw + C::W_BYTES) >> 4) & 0x3FFFu);
+#pragma unroll
+          for (int j = 0; j < KB / 8; ++j) {
+            mma_tf32_ts(d, a_lo + j * 8, w_hi + 2 * j, idesc, (i > 0 || j > 0) ? 1u : 0u);
+            mma_tf32_ts(d, a_hi + j * 8, w_lo + 2 * j, idesc, 1u);
+            mma_tf32_ts(d, a_hi + j * 8, w_hi + 2 * j, idesc, 1u);
+          }
+          mma_commit(empty_bar + 8 * stage);
+        }
+        if (!ok) break;
+        mma_commit(tfull_bar + 8 * acc);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- results: a lane per pixel, one channel after the other, 32 adjacent pixels per store ----
+    const int quarter = warp & 3;
+    int local = 0;
+    for (TileIter t(p); t.valid(p); t.next(p), ++local) {
+      const int acc = local % ACCS;
+      if (!mbar_wait_warp(tfull_bar + 8 * acc, (local / ACCS) & 1, abort_flag, WAIT_BUDGET)) {
+        fail(MB_DEV_TIMEOUT_EPILOGUE);
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+      if (p.splits > 1) {
+        // this CTA's run of the depth: [n][128 m] into shared memory (the ring is idle: one tile per CTA)
+        float *part = reinterpret_cast<float *>(smem) + quarter * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < BN; c += 16) {
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(src + c, r);
+          tmem_ld_wait_x16(r);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) part[(c + j) * BM] = __uint_as_float(r[j]);
+        }
+        break;
+      }
+      const int m = t.tm * BM + quarter * 32 + lane;
+      const int64_t at = out_offset<XK>(p, m, t.b);
+      const int n0 = t.tn * BN;
+      uint32_t r[2][16];
+      tmem_ld_32x32b_x16(src, r[0]);
+#pragma unroll
+      for (int c = 0; c < BN; c += 16) {
+        uint32_t (&v)[16] = r[(c / 16) & 1];
+        tmem_ld_wait_x16(v);
+        if (c + 16 < BN) {
+          tmem_ld_32x32b_x16(src + c + 16, r[(c / 16 + 1) & 1]);
+        } else {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(tempty_bar + 8 * acc);
+        }
+        // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
+        // latency per channel made a 128 x 128 tile take 19 us)
+        float x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
+        if (p.bias != nullptr) {
+          const float mine = n0 + c + (lane & 15) < p.N ? __ldg(p.bias + n0 + c + (lane & 15)) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) x[j] += __shfl_sync(0xffffffffu, mine, j);
+        }
+        if (p.residual != nullptr && m < p.M) {
+          const float *src_r = p.residual + at + static_cast<int64_t>(n0 + c) * p.c_ns;
+          float res[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) res[j] = n0 + c + j < p.N ? __ldg(src_r + j * p.c_ns) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) x[j] += res[j];
+        }
+        mb_activate_n(x, p.act, p.max_limit, p.coef);
+        float *dst = p.C + at + static_cast<int64_t>(n0 + c) * p.c_ns;
+        if (n0 + c + 16 <= p.N) {
+          if (m < p.M) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[j * p.c_ns] = x[j];
+          }
+        } else if (m < p.M) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (n0 + c + j < p.N) dst[j * p.c_ns] = x[j];
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (*abort_flag != 0) {
+    // MMAs in flight must not outlive the memory they use (bounded: about 2 ms)
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+  if (p.splits > 1) {
+    cluster_sync_all();
+    // every CTA of the cluster adds up its share of the channels, all runs in the order of their rank
+    const TileIter t(p);
+    const int m = t.tm * BM + (threadIdx.x & 127);
+    const int64_t at = out_offset<XK>(p, m, t.b);
+    const int n0 = t.tn * BN;
+    const uint32_t mine = smem_base + (threadIdx.x & 127) * 4;
+    if (warp < 20 && m < p.M) {
+      // up to four channels per round, all loads before the first store (see above)
+      const int stride = 5 * p.splits;
+      for (int c0 = (warp >> 2) * p.splits + rank; c0 < BN; c0 += 4 * stride) {
+        float x[4], add[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int c = c0 + q * stride, n = n0 + c;
+          x[q] = add[q] = 0.f;
+          if (c < BN && n < p.N) {
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+              if (s < p.splits) x[q] += ld_cluster_f32(mapa_shared(mine + c * (BM * 4), s));
+            if (p.bias != nullptr) x[q] += __ldg(p.bias + n);
+            if (p.residual != nullptr) add[q] = __ldg(p.residual + at + static_cast<int64_t>(n) * p.c_ns);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] += add[q];
+        mb_activate_n(x, p.act, p.max_limit, p.coef);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int c = c0 + q * stride, n = n0 + c;
+          if (c < BN && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = x[q];
+        }
+      }
+    }
+    cluster_sync_all();  // no CTA may leave while another still reads its tile
+  }
+  if (warp == FIRST_E) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+template <int BN, int XK, int WK>
+int launch_cfg(mb_context *ctx, Params &p) {
+  using C = Cfg<BN>;
+  auto kern = gemm_f32_gather_kernel<BN, XK, WK>;
+  constexpr uint64_t bit = (BN == 128 ? 9 : 0) + XK * 3 + WK;
+  CUtensorMap map;
+  if (WK == W_TMA) MB_RETURN_IF_ERROR(mb_make_map_w_f32(ctx, &map, p.W, p.K, p.N, p.w_bs != 0 ? p.batch : 1, p.w_ns, p.w_bs, BN));
+  else memset(&map, 0, sizeof(map));
+  if (!(ctx->f32_gather_attr_mask & (1ull << bit))) {
+    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    ctx->f32_gather_attr_mask |= 1ull << bit;
+  }
+  const int64_t tiles = static_cast<int64_t>(p.batch) * p.tiles_m * p.tiles_n;
+  const int slots = p.splits > 1 ? static_cast<int>(tiles) : static_cast<int>(std::min<int64_t>(tiles, ctx->num_sms));
+  p.step_m = slots % p.tiles_m;
+  p.step_n = (slots / p.tiles_m) % p.tiles_n;
+  p.step_b = (slots / p.tiles_m) / p.tiles_n;
+  MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), THREADS, C::SMEM_BYTES, p.splits, map, p));
+  ctx->launches++;
+  ctx->launches_tc++;
+  return MB_SUCCESS;
+}
+
+struct Plan {
+  int bn = 64, splits = 1;
+  int64_t cost = -1;
+};
+
+// Tile width and depth runs with the smallest estimate, in SM cycles.  Measured: a step is bound by the MMAs, whose A
+// operand comes from tensor memory at the same rate for either width (0.6 us), or by a convolution's loads (0.72 us); a
+// tile's stores take 2.7 us per 64 channels, twice that with a residual; 5.5 us around the steps, 7.6 us with the
+// exchange between the CTAs of a cluster.
+Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
+  const int64_t tiles_m = ceil_div64(g.M, BM), k_blocks = ceil_div64(g.K, KB);
+  Plan best;
+  int asked = ctx->f32_splits;
+  while (asked > k_blocks) asked /= 2;
+  for (int w : {128, 64}) {
+    if (ctx->f32_bn != 0 ? w != ctx->f32_bn : (w == 128 && g.N <= 64)) continue;
+    const int64_t tiles = g.batch * tiles_m * ceil_div64(g.N, w);
+    for (int s : {1, 2, 4, 8}) {
+      if (asked != 0 ? s != asked : (s > 1 && s * 2 > k_blocks)) continue;
+      const int64_t rounds = ceil_div64(tiles * s, s == 1 ? ctx->num_sms : mb_resident_cluster_ctas(ctx, s));
+      if (s > 1 && rounds > 1 && asked == 0) continue;  // (one tile per CTA: a second round would start from nothing)
+      const int64_t steps = ceil_div64(k_blocks, s);
+      const int64_t step = g.conv ? (w == 128 ? 1450 : 1350) : (w == 128 ? 1250 : 1150);
+      const int64_t results = (w == 128 ? 10000 : 5000) * (g.residual != nullptr ? 2 : 1);
+      const int64_t cost = s == 1 ? 8500 + rounds * std::max<int64_t>(steps * step, results) + (w == 128 ? 4000 : 2000)
+                                  : w == 128 ? 17500 + steps * 1680 : 14500 + steps * 1370;
+      if (best.cost < 0 || cost < best.cost) {
+        best.bn = w; best.splits = s; best.cost = cost;
+      }
+    }
+  }
+  return best;
+}
+
+}  // namespace
+
+bool mb_gemm_f32_gather_supported(const mb_context *ctx, const mb_f32_gemm &g) {
+  if (!ctx->use_tensor_cores || g.M < 1 || g.N < 1 || g.K < 1 || g.batch < 1) return false;
+  if (g.M >= (1ll << 31) - 128 || g.N >= (1ll << 31) - 128 || g.K >= (1ll << 30) || g.batch >= (1ll << 31)) return false;
+  if (g.batch * ceil_div64(g.M, BM) * ceil_div64(g.N, 64) * 8 >= (1ll << 31)) return false;
+  if (g.conv)
+    return g.KH <= 16 && g.KW <= 15 && static_cast<int64_t>(g.C_in) * g.H * g.Wd < (1ll << 30) &&
+           g.C_in * static_cast<int64_t>(g.KH) * g.KW == g.K;
+  if ((g.x_ms != 1 && g.x_ks != 1) || (g.w_ns != 1 && g.w_ks != 1)) return false;
+  return g.x_ms != 1 || g.K * g.x_ks < (1ll << 31);
+}
+
+int64_t mb_gemm_f32_gather_cost(mb_context *ctx, const mb_f32_gemm &g) { return make_plan(ctx, g).cost; }
+
+int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
+  const Plan plan = make_plan(ctx, g);
+  Params p = {};
+  p.X = g.X; p.W = g.W; p.bias = g.bias; p.residual = g.residual; p.C = g.C;
+  p.M = static_cast<int>(g.M); p.N = static_cast<int>(g.N); p.K = static_cast<int>(g.K); p.batch = static_cast<int>(g.batch);
+  p.tiles_m = static_cast<int>(ceil_div64(g.M, BM));
+  p.tiles_n = static_cast<int>(ceil_div64(g.N, plan.bn));
+  p.k_blocks = static_cast<int>(ceil_div64(g.K, KB));
+  p.splits = plan.splits;
+  p.x_ks = g.x_ks; p.x_ms = g.x_ms; p.x_bs = g.x_bs;
+  p.w_ns = g.w_ns; p.w_ks = g.w_ks; p.w_bs = g.w_bs;
+  p.c_ns = g.c_ns; p.c_ms = g.c_ms; p.c_bs = g.c_bs;
+  p.act = g.act; p.max_limit = g.max_limit; p.coef = g.coef;
+  p.status = ctx->dev_status;
+  const bool w_nc = !g.conv && g.w_ks != 1;
+  const bool w_tma = !w_nc && ctx->encode_tiled != nullptr && (reinterpret_cast<uintptr_t>(g.W) & 15u) == 0 &&
+                     (g.conv ? g.K : g.w_ns) % 4 == 0 && g.w_bs % 4 == 0;
+  if (g.conv) {
+    p.H = g.H; p.Wd = g.Wd; p.KH = g.KH; p.KW = g.KW; p.taps = g.KH * g.KW;
+    p.sh = g.sh; p.sw = g.sw; p.dh = g.dh; p.dw = g.dw; p.pad_t = g.pad_t; p.pad_l = g.pad_l;
+    p.Wo = g.Wo; p.hw = g.Ho * g.Wo;
+    p.image = static_cast<int64_t>(g.C_in) * g.H * g.Wd;
+    p.w_ns = g.K; p.w_ks = 1;
+    p.c_ns = p.hw;
+    fast_div_make(static_cast<uint32_t>(p.taps), &p.taps_mul, &p.taps_shift);
+    fast_div_make(static_cast<uint32_t>(p.KW), &p.kw_mul, &p.kw_shift);
+    fast_div_make(static_cast<uint32_t>(p.hw), &p.hw_mul, &p.hw_shift);
+    fast_div_make(static_cast<uint32_t>(p.Wo), &p.wo_mul, &p.wo_shift);
+    if (plan.bn == 128) return w_tma ? launch_cfg<128, X_CONV, W_TMA>(ctx, p) : launch_cfg<128, X_CONV, W_ROWS>(ctx, p);
+    return w_tma ? launch_cfg<64, X_CONV, W_TMA>(ctx, p) : launch_cfg<64, X_CONV, W_ROWS>(ctx, p);
+  }
+  const bool cols = g.x_ms != 1;
+  p.x_vec = cols && (reinterpret_cast<uintptr_t>(g.X) & 15u) == 0 && g.x_ms % 4 == 0 && g.x_bs % 4 == 0 && g.K % 4 == 0;
+#define MB_F32_W(BN_, XK_)                                          \
+  if (w_nc) return launch_cfg<BN_, XK_, W_COLS>(ctx, p);            \
+  return w_tma ? launch_cfg<BN_, XK_, W_TMA>(ctx, p) : launch_cfg<BN_, XK_, W_ROWS>(ctx, p);
+#define MB_F32(BN_)                     \
+  if (cols) { MB_F32_W(BN_, X_COLS) }   \
+  MB_F32_W(BN_, X_ROWS)
+  if (plan.bn == 128) { MB_F32(128) }
+  MB_F32(64)
+#undef MB_F32
+#undef MB_F32_W
+}

@@ -608,6 +608,12 @@ int launch_f32(mb_context *ctx, const CUtensorMap &tx, const CUtensorMap &tw, co
 
 }  // namespace
 
+// The [BN x 32 k] boxes of a K-contiguous matrix, for gemm_f32_gather.cu.
+int mb_make_map_w_f32(mb_context *ctx, CUtensorMap *map, const float *W, int64_t K, int64_t N, int64_t batch, int64_t w_ns,
+                      int64_t w_bs, int bn) {
+  return make_map_f32(ctx, map, W, K, N, batch, w_ns, batch > 1 ? w_bs : w_ns * N, FKB, bn);
+}
+
 // Whether the tensor-core kernel can take C[b][n][m] = sum_k X[b][k][m] * W[b][n][k]: TMA needs
 // 16-byte aligned bases and strides, i.e. row lengths that are multiples of four floats.
 bool mb_gemm_f32_tc_supported(const mb_context *ctx, const float *X, const float *W, int64_t Mdim,

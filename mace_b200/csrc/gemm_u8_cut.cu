@@ -373,9 +373,11 @@ bool conv_map_possible(const mb_context *ctx, const mb_cut_gemm &g) {
          g.KW <= 256 && byte(upper_corner(g.H, g.Ho, g.sh, g.pad_t)) && byte(upper_corner(g.W, g.Wo, g.sw, g.pad_l));
 }
 
+}  // namespace
+
 // CTAs of clusters of `s` that the device holds at once with one CTA per SM (a cluster lies inside a
 // GPC, and not every GPC has a whole number of clusters' SMs).
-int64_t resident_ctas(mb_context *ctx, int s) {
+int64_t mb_resident_cluster_ctas(mb_context *ctx, int s) {
   if (s == 1) return ctx->num_sms;
   const int slot = s == 2 ? 1 : s == 4 ? 2 : 3;
   if (ctx->cut_clusters[slot] == 0) {
@@ -402,8 +404,6 @@ int64_t resident_ctas(mb_context *ctx, int s) {
   }
   return ctx->cut_clusters[slot];
 }
-
-}  // namespace
 
 mb_cut_plan mb_gemm_u8_cut_plan(mb_context *ctx, const mb_cut_gemm &g) {
   mb_cut_plan best;
@@ -439,7 +439,7 @@ mb_cut_plan mb_gemm_u8_cut_plan(mb_context *ctx, const mb_cut_gemm &g) {
     if (ctx->cut_two == 3 && g.conv) continue;
     for (int s : {1, 2, 4, 8}) {
       if (asked != 0 ? s != asked : (s > 1 && s * 2 > k_blocks)) continue;
-      const int64_t sms = resident_ctas(ctx, s);
+      const int64_t sms = mb_resident_cluster_ctas(ctx, s);
       const int64_t steps = ceil_div64(k_blocks, s);
       for (int two : {0, 1}) {
         if ((two && !g.conv) || ((ctx->cut_two == 1 || ctx->cut_two == 2) && by_tma && two != ctx->cut_two - 1)) continue;

@@ -38,6 +38,9 @@ mb_cut_plan mb_gemm_u8_cut_plan(mb_context *ctx, const mb_cut_gemm &g);
 int mb_gemm_u8_cut_launch(mb_context *ctx, const mb_cut_gemm &g, const mb_cut_plan &plan);
 int mb_gemm_u8_gather_launch(mb_context *ctx, const mb_cut_gemm &g, int bn, int splits);
 
+// CTAs of clusters of `s` that the device holds at once with one CTA per SM.
+int64_t mb_resident_cluster_ctas(mb_context *ctx, int s);
+
 // Rows of any length copied to a 16-byte pitch (gemm_u8.cu).
 int mb_repack_rows_u8(mb_context *ctx, const uint8_t *A, uint8_t *a_dst, int64_t a_rows, int64_t a_len, int64_t lda,
                       int fill_a, const uint8_t *B, uint8_t *b_dst, int64_t b_rows, int64_t b_len, int64_t ldb,

@@ -17,7 +17,10 @@
 //    the T products is ONE GEMM over all images (the CPU code runs T GEMMs per
 //    image);
 //  * the product runs as a strided-batched GEMM.
+#include <algorithm>
+
 #include "common.cuh"
+#include "gemm_f32_gather.cuh"
 
 int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *C,
                         const float *bias_per_row, int64_t batch, int64_t M, int64_t N, int64_t K,
@@ -368,6 +371,20 @@ int pick_tile(int64_t H, int64_t W, int tile_override) {
 
 }  // namespace
 
+// Estimated SM cycles of the three Winograd kernels, from their times at 56 x 56 x 64 (batch 1: 13 us, 32: 60, 256: 437),
+// 28 x 28 x 128 (8: 21, 256: 290), 14 x 14 x 256 (256: 299) and 7 x 7 x 512 (256: 230): about 12 us of launches, the
+// transforms' bytes (the intermediates written and read once each) at 9.5 TB/s (part of them stays in L2), the batched product at 1150 cycles per
+// step and tile or 2.4 us for a tile's stores.  An odd column count keeps the product off TMA (15 us at batch 1).
+static int64_t winograd_cost(const mb_context *ctx, int64_t N, int64_t C, int64_t H, int64_t W, int64_t O, int64_t Ho,
+                             int64_t Wo, int tile_override) {
+  const int tile = pick_tile(H, W, tile_override);
+  const int64_t T = static_cast<int64_t>(tile + 2) * (tile + 2);
+  const int64_t cols = N * ceil_div64(Ho, tile) * ceil_div64(Wo, tile);
+  const int64_t bytes = 4 * (N * C * H * W + 2 * T * C * cols + 2 * T * O * cols + N * O * Ho * Wo + T * O * C);
+  const int64_t rounds = ceil_div64(T * ceil_div64(cols, 128) * ceil_div64(O, O > 64 ? 128 : 64), ctx->num_sms);
+  return 23000 + bytes / 5000 + rounds * std::max<int64_t>(ceil_div64(C, 32) * 1150, 4500) + (cols % 4 != 0 ? 28000 : 0);
+}
+
 extern "C" {
 
 int mb_winograd_transform_filter_f32(mb_context *ctx, const float *filter, float *transformed,
@@ -406,6 +423,21 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
   if (Ho > H + 2 * 2 || Wo > W + 2 * 2)
     return mb_fail(ctx, MB_INVALID_ARGS, "mb_conv3x3_winograd_f32_nchw: output larger than a 3x3 stride-1 conv gives");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
+  // A direct convolution where the three launches cost more.  Only with both forms of the filter at hand: a call with one of
+  // them gives bit for bit what a call with the other does.
+  if (filter != nullptr && transformed_filter != nullptr && ctx->f32_gather != 1) {
+    mb_f32_gemm g;
+    g.X = in; g.W = filter; g.bias = bias; g.C = out;
+    g.M = N * Ho * Wo; g.N = O; g.K = C * 9;
+    g.act = activation; g.max_limit = max_limit; g.coef = coefficient;
+    g.conv = true;
+    g.C_in = static_cast<int>(C); g.H = static_cast<int>(H); g.Wd = static_cast<int>(W);
+    g.KH = 3; g.KW = 3; g.pad_t = pad_top; g.pad_l = pad_left;
+    g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
+    if (mb_gemm_f32_gather_supported(ctx, g) &&
+        (ctx->f32_gather == 2 || mb_gemm_f32_gather_cost(ctx, g) < winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override)))
+      return mb_gemm_f32_gather_launch(ctx, g);
+  }
   const int tile = pick_tile(H, W, tile_override);
   const int T = (tile + 2) * (tile + 2);
   const int64_t th = ceil_div64(Ho, tile), tw = ceil_div64(Wo, tile), tiles = th * tw;

@@ -187,6 +187,84 @@ def test_winograd_f32(ctx, orc, case):
     assert np.array_equal(ctx.download(do, direct.shape, np.float32), got)
 
 
+@pytest.fixture(params=[(0, 0), (64, 1), (64, 8), (128, 2)], ids=str)
+def gather(ctx, request):
+    """The self-fetching kernel wherever it can run, at a tile width and number of depth runs (0: by rule)."""
+    ctx.set_option("f32_gather", 2)
+    ctx.set_option("f32_bn", request.param[0])
+    ctx.set_option("f32_splits", request.param[1])
+    yield
+    for name in ("f32_gather", "f32_bn", "f32_splits"):
+        ctx.set_option(name, 0)
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, O, kernel, stride, dilation, padding: odd maps and channel counts, tails of pixels (also over
+    # several images), of channels and of the depth, every kind of window
+    (2, 35, 9, 11, 73, (5, 5), 1, 1, "SAME"), (3, 33, 7, 7, 130, (3, 3), 2, 1, "SAME"), (1, 3, 30, 31, 64, (7, 7), 2, 1, "SAME"),
+    (2, 64, 13, 14, 64, (1, 1), 1, 1, "SAME"), (2, 70, 15, 13, 40, (1, 1), 2, 1, "VALID"), (1, 20, 17, 19, 65, (3, 3), 1, 2, "SAME"),
+    (5, 16, 6, 5, 33, (1, 5), 1, 1, "SAME"), (1, 200, 8, 8, 129, (3, 3), 1, 1, "VALID")])
+@pytest.mark.parametrize("residual", [False, True])
+def test_conv2d_f32_without_column_matrix(ctx, orc, gather, case, residual):
+    N, C, H, W, O, k, s, d, pad = case
+    rng = np.random.Generator(np.random.PCG64(C + O))
+    x = rng.standard_normal((N, C, H, W)).astype(np.float32)
+    f = rng.standard_normal((O, C) + k).astype(np.float32)
+    bias = rng.standard_normal(O).astype(np.float32)
+    ho, wo, ph, pw = orc.calc_padding_and_output_size(H, W, k[0], k[1], (d, d), (s, s), PAD[pad])
+    dx, df, db = ctx.upload(x), ctx.upload(f), ctx.upload(bias)
+    do = ctx.alloc(N * O * ho * wo * 4)
+    before = ctx.launches_tensor_core
+    args = (N, C, H, W, O, k[0], k[1], (s, s), (d, d), (ph >> 1, pw >> 1), (ho, wo), 1)
+    if residual:
+        r = rng.standard_normal((N, O, ho, wo)).astype(np.float32)
+        dr = ctx.upload(r)
+        ctx.conv2d_f32_residual(dx, df, db, dr, do, *args)
+        ref = np.maximum(orc.conv2d_f32(x, f, bias, (s, s), (d, d), (ph >> 1, pw >> 1), (ho, wo), 0) + r, 0)
+        dr.free()
+    else:
+        ctx.conv2d_f32(dx, df, db, do, *args)
+        ref = orc.conv2d_f32(x, f, bias, (s, s), (d, d), (ph >> 1, pw >> 1), (ho, wo), 1)
+    assert ctx.launches_tensor_core == before + 1
+    assert rel_err(ctx.download(do, ref.shape, np.float32), ref, 1e-4, "conv2d_f32 without columns") <= 5e-5
+    for b in (dx, df, db, do):
+        b.free()
+
+
+@pytest.mark.parametrize("maj", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (1, 1, 0), (0, 0, 1), (0, 1, 1), (1, 1, 1)])
+@pytest.mark.parametrize("shape", [(1, 5, 5, 5), (2, 130, 61, 33), (3, 64, 128, 96), (1, 1, 300, 701), (2, 200, 67, 520)])
+def test_gemm_f32_of_any_layout_on_tensor_cores(ctx, orc, gather, maj, shape):
+    batch, M, N, K = shape
+    rng = np.random.Generator(np.random.PCG64(M + N))
+    A = rng.standard_normal((batch, M, K)).astype(np.float32)
+    B = rng.standard_normal((batch, K, N)).astype(np.float32)
+    A_st = np.ascontiguousarray(np.swapaxes(A, 1, 2)) if maj[0] else A
+    B_st = np.ascontiguousarray(np.swapaxes(B, 1, 2)) if maj[1] else B
+    dA, dB, dC = ctx.upload(A_st), ctx.upload(B_st), ctx.alloc(batch * M * N * 4)
+    before = ctx.launches_tensor_core
+    ctx.gemm_f32(dA, dB, dC, batch, M, N, K, bool(maj[0]), bool(maj[1]), bool(maj[2]))
+    assert ctx.launches_tensor_core == before + 1
+    ref = orc.gemm_f32(A_st, B_st, batch, M, N, K, bool(maj[0]), bool(maj[1]), bool(maj[2]))
+    assert rel_err(ctx.download(dC, (batch * M * N,), np.float32), ref, 1e-4, "gemm_f32 of any layout") <= 5e-5
+    for b in (dA, dB, dC):
+        b.free()
+
+
+@pytest.mark.parametrize("shape", [(1, 1000, 2048), (3, 77, 1023), (40, 130, 516)])
+def test_gemv_f32_on_tensor_cores(ctx, orc, gather, shape):
+    batch, rows, K = shape
+    rng = np.random.Generator(np.random.PCG64(rows))
+    w = rng.standard_normal((rows, K)).astype(np.float32)
+    x = rng.standard_normal((batch, K)).astype(np.float32)
+    bias = rng.standard_normal(rows).astype(np.float32)
+    dw, dx, db, do = ctx.upload(w), ctx.upload(x), ctx.upload(bias), ctx.alloc(batch * rows * 4)
+    ctx.gemv_f32(dw, dx, db, do, batch, rows, K)
+    ref = orc.gemv_f32(w, x, bias, batch, rows, K, False, True).reshape(batch, rows)
+    assert rel_err(ctx.download(do, ref.shape, np.float32), ref, 1e-4, "gemv_f32 on tensor cores") <= 5e-5
+    for b in (dw, dx, db, do):
+        b.free()
+
+
 @pytest.mark.parametrize("k", [3, 5])
 @pytest.mark.parametrize("stride", [1, 2])
 @pytest.mark.parametrize("shape", [(1, 3, 7, 9, 1), (2, 300, 33, 31, 1), (3, 5, 20, 65, 2), (4, 130, 57, 112, 1),
