@@ -27,6 +27,8 @@ struct PoolF32Params {
 // outputs fall into the same cache lines.
 template <bool IS_MAX>
 __global__ void __launch_bounds__(256) pooling_f32_kernel(const PoolF32Params p) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (tid >= p.total) return;
   const int w = static_cast<int>(tid % p.Wo);
@@ -53,11 +55,42 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(const PoolF32Params p)
   p.out[tid] = res;
 }
 
+// Global average pool: a warp per PLANES planes, whose loads are in flight together (a thread per plane read 49 values one
+// after the other, each from a line of its own: 2048 planes of 7 x 7 took 9.0 us, now 4).  Several planes per warp where
+// there are enough of them: 524288 planes one by one took 77 us.
+template <int PLANES>
+__global__ void __launch_bounds__(256) global_avgpool_f32_kernel(const float *__restrict__ in, float *__restrict__ out,
+                                                                 int64_t planes, int size) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
+  const int64_t plane = (static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * PLANES;
+  const int lane = threadIdx.x & 31;
+  if (plane >= planes) return;
+  const float *src = in + plane * size;
+  const int n = static_cast<int>(min(static_cast<int64_t>(PLANES), planes - plane));
+  float s[PLANES] = {};
+#pragma unroll 2
+  for (int i = lane; i < size; i += 32) {
+#pragma unroll
+    for (int q = 0; q < PLANES; ++q) s[q] += q < n ? __ldg(src + q * size + i) : 0.f;
+  }
+  float mine = 0.f;
+#pragma unroll
+  for (int q = 0; q < PLANES; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+    if (lane == q) mine = s[q];
+  }
+  if (lane < n) out[plane + lane] = mine / static_cast<float>(size);
+}
+
 // The same for the common "3x3 window, stride 2, no dilation" max pool on rows whose length is
 // a multiple of 4 with no left padding: a thread produces four neighbouring outputs of a row
 // from nine input columns, fetched per input row as two 128-bit loads and one scalar
 // (9 loads for 4 outputs instead of 36).  Taps right of the image are skipped as above.
 __global__ void __launch_bounds__(256) maxpool3x3s2_f32_kernel(const PoolF32Params p) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int wq = (p.Wo + 3) >> 2;
   if (tid >= p.total) return;  // total = planes * Ho * wq here
@@ -136,6 +169,8 @@ __device__ __forceinline__ float elt_apply(float a, float b, const EltParams &p)
 
 template <int TYPE>
 __global__ void __launch_bounds__(256) eltwise_f32_kernel(const EltParams p, int vec4) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (vec4) {
@@ -162,6 +197,8 @@ __global__ void __launch_bounds__(256) eltwise_f32_kernel(const EltParams p, int
 __global__ void __launch_bounds__(256)
 activation_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t size, int vec4,
                       int act, float max_limit, float coef) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   int64_t done = 0;
@@ -185,6 +222,8 @@ activation_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int
 __global__ void __launch_bounds__(256)
 softmax_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t positions,
                    int64_t classes, int64_t inner, int use_log) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int lane = threadIdx.x & 31;
   const int64_t pos = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (pos >= positions) return;
@@ -214,7 +253,8 @@ static unsigned stream_grid(const mb_context *ctx, int64_t work_items) {
 
 template <int TYPE>
 static void launch_eltwise(mb_context *ctx, const EltParams &p, int vec4) {
-  eltwise_f32_kernel<TYPE><<<stream_grid(ctx, vec4 ? p.size / 4 + 1 : p.size), 256, 0, ctx->stream>>>(p, vec4);
+  (void)mb_launch_chained(ctx, eltwise_f32_kernel<TYPE>, dim3(stream_grid(ctx, vec4 ? p.size / 4 + 1 : p.size)), dim3(256), 0,
+                          p, vec4);  // (the caller asks for the error)
 }
 
 // out[p][ho][wo] = in[p][ho * sh][wo * sw] over N * C planes: the pixels a 1x1 convolution with
@@ -224,6 +264,8 @@ static void launch_eltwise(mb_context *ctx, const EltParams &p, int vec4) {
 __global__ void __launch_bounds__(256)
 subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t total, int H, int W, int sh,
                      int sw, int Ho, int Wo) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t plane_out = static_cast<int64_t>(Ho) * Wo, plane_in = static_cast<int64_t>(H) * W;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -262,14 +304,25 @@ int mb_pooling_f32_nchw(mb_context *ctx, const float *in, float *out, int64_t N,
       pad_left == 0 && W % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0 &&
       (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
     p.total = N * C * Ho * ((Wo + 3) / 4);
-    maxpool3x3s2_f32_kernel<<<static_cast<unsigned>(ceil_div64(p.total, 256)), 256, 0, ctx->stream>>>(p);
+    MB_CUDA(ctx, mb_launch_chained(ctx, maxpool3x3s2_f32_kernel, dim3(static_cast<unsigned>(ceil_div64(p.total, 256))), dim3(256), 0, p));
     MB_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
     return MB_SUCCESS;
   }
+  if (pooling_type == 1 && KH == H && KW == W && Ho == 1 && Wo == 1 && dil_h == 1 && dil_w == 1 && pad_top == 0 && pad_left == 0) {
+    // eight planes per warp once that still leaves every SM 32 warps
+    if (N * C >= 256ll * ctx->num_sms && H * W < (1 << 27))
+      MB_CUDA(ctx, mb_launch_chained(ctx, global_avgpool_f32_kernel<8>, dim3(static_cast<unsigned>(ceil_div64(N * C, 64))),
+                                     dim3(256), 0, in, out, N * C, static_cast<int>(H * W)));
+    else
+      MB_CUDA(ctx, mb_launch_chained(ctx, global_avgpool_f32_kernel<1>, dim3(static_cast<unsigned>(ceil_div64(N * C, 8))),
+                                     dim3(256), 0, in, out, N * C, static_cast<int>(H * W)));
+    ctx->launches++;
+    return MB_SUCCESS;
+  }
   const unsigned grid = static_cast<unsigned>(ceil_div64(p.total, 256));
-  if (pooling_type == 2) pooling_f32_kernel<true><<<grid, 256, 0, ctx->stream>>>(p);
-  else pooling_f32_kernel<false><<<grid, 256, 0, ctx->stream>>>(p);
+  if (pooling_type == 2) MB_CUDA(ctx, mb_launch_chained(ctx, pooling_f32_kernel<true>, dim3(grid), dim3(256), 0, p));
+  else MB_CUDA(ctx, mb_launch_chained(ctx, pooling_f32_kernel<false>, dim3(grid), dim3(256), 0, p));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
@@ -332,8 +385,7 @@ int mb_activation_f32(mb_context *ctx, const float *in, float *out, int64_t size
   if (in == nullptr || out == nullptr) return mb_fail(ctx, MB_INVALID_ARGS, "mb_activation_f32: null operand");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
   const int vec4 = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
-  activation_f32_kernel<<<stream_grid(ctx, vec4 ? size / 4 + 1 : size), 256, 0, ctx->stream>>>(
-      in, out, size, vec4, activation, max_limit, coefficient);
+  MB_CUDA(ctx, mb_launch_chained(ctx, activation_f32_kernel, dim3(stream_grid(ctx, vec4 ? size / 4 + 1 : size)), dim3(256), 0, in, out, size, vec4, activation, max_limit, coefficient));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
@@ -348,8 +400,7 @@ int mb_softmax_f32(mb_context *ctx, const float *in, float *out, int64_t outer, 
   const int64_t positions = outer * inner;
   if (ceil_div64(positions, 8) >= (1ll << 31)) return mb_fail(ctx, MB_UNSUPPORTED, "mb_softmax_f32: tensor too large");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  softmax_f32_kernel<<<static_cast<unsigned>(ceil_div64(positions, 8)), 256, 0, ctx->stream>>>(
-      in, out, positions, classes, inner, use_log);
+  MB_CUDA(ctx, mb_launch_chained(ctx, softmax_f32_kernel, dim3(static_cast<unsigned>(ceil_div64(positions, 8))), dim3(256), 0, in, out, positions, classes, inner, use_log));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
@@ -366,9 +417,7 @@ int mb_subsample_f32_nchw(mb_context *ctx, const float *in, float *out, int64_t 
   if (in == nullptr || out == nullptr || in == out)
     return mb_fail(ctx, MB_INVALID_ARGS, "mb_subsample_f32_nchw: null or aliased buffers");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  subsample_f32_kernel<<<stream_grid(ctx, total), 256, 0, ctx->stream>>>(in, out, total, static_cast<int>(H),
-                                                                         static_cast<int>(W), stride_h, stride_w,
-                                                                         static_cast<int>(Ho), static_cast<int>(Wo));
+  MB_CUDA(ctx, mb_launch_chained(ctx, subsample_f32_kernel, dim3(stream_grid(ctx, total)), dim3(256), 0, in, out, total, static_cast<int>(H), static_cast<int>(W), stride_h, stride_w, static_cast<int>(Ho), static_cast<int>(Wo)));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
