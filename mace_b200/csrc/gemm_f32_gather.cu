@@ -67,7 +67,10 @@ template <int BN>
 struct Cfg {
   static constexpr int W_BYTES = BN * KB * 4;            // hi (or lo) of a step
   static constexpr int STAGE_BYTES = 2 * W_BYTES;
-  static constexpr int A_COL0 = ACCS * BN;               // TMEM: accumulators, then STAGES x 64 columns of A
+  // 64 channels: hi x [w_hi | w_lo] is one MMA of 128 columns (see the MMA role)
+  static constexpr bool WIDE = BN == 64;
+  static constexpr int ACC_COLS = WIDE ? 2 * BN : BN;
+  static constexpr int A_COL0 = ACCS * ACC_COLS;         // TMEM: accumulators, then STAGES x 64 columns of A
   static constexpr int STAGES = (512 - A_COL0) / (2 * KB);
   static constexpr int RING = STAGES * STAGE_BYTES;
   static constexpr int TABLE_BYTES = FIRST_W * KB * 8;
@@ -359,6 +362,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     // ---- MMA: one thread ----
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc(/*c f32*/ 1, /*a tf32*/ 2, /*b tf32*/ 2, false, false, BM, BN);
+      constexpr uint32_t idesc_wide = make_idesc(1, 2, 2, false, false, BM, C::WIDE ? 2 * BN : BN);
       const uint64_t wdesc = make_smem_desc(0, 16, 1024, 2);
       int it = 0, local = 0;
       bool ok = true;
@@ -369,7 +373,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           break;
         }
         tc_fence_after_sync();
-        const uint32_t d = tmem + acc * BN;
+        const uint32_t d = tmem + acc * C::ACC_COLS;
         for (int i = 0; i < steps; ++i, ++it) {
           const int stage = it % STAGES;
           if (!mbar_wait(full_bar + 8 * stage, (it / STAGES) & 1, abort_flag, WAIT_BUDGET)) {
@@ -382,8 +386,16 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           const uint32_t sw = smem_base + stage * C::STAGE_BYTES;
           const uint64_t w_hi = wdesc | static_cast<uint64_t>((sw >> 4) & 0x3FFFu);
           const uint64_t w_lo = wdesc | static_cast<uint64_t>(((sw + C::W_BYTES) >> 4) & 0x3FFFu);
+          // With A from tensor memory an MMA takes 92 cycles for 64 columns as for 128, so 64 channels take hi from there
+          // once for both halves of W, whose tiles lie one behind the other: 2 MMAs per 8 of k instead of 3, and hi * lo
+          // + lo * hi in columns of their own, which the epilogue adds.
 #pragma unroll
           for (int j = 0; j < KB / 8; ++j) {
+            if (C::WIDE) {
+              mma_tf32_ts(d, a_hi + j * 8, w_hi + 2 * j, idesc_wide, (i > 0 || j > 0) ? 1u : 0u);
+              mma_tf32_ts(d + BN, a_lo + j * 8, w_hi + 2 * j, idesc, 1u);
+              continue;
+            }
             mma_tf32_ts(d, a_lo + j * 8, w_hi + 2 * j, idesc, (i > 0 || j > 0) ? 1u : 0u);
             mma_tf32_ts(d, a_hi + j * 8, w_lo + 2 * j, idesc, 1u);
             mma_tf32_ts(d, a_hi + j * 8, w_hi + 2 * j, idesc, 1u);
@@ -406,41 +418,47 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         break;
       }
       tc_fence_after_sync();
-      const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+      const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * C::ACC_COLS;
       if (p.splits > 1) {
         // this CTA's run of the depth: [n][128 m] into shared memory (the ring is idle: one tile per CTA)
         float *part = reinterpret_cast<float *>(smem) + quarter * 32 + lane;
 #pragma unroll 1
         for (int c = 0; c < BN; c += 16) {
-          uint32_t r[16];
+          uint32_t r[16], r2[16];
           tmem_ld_32x32b_x16(src + c, r);
+          if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c, r2);
           tmem_ld_wait_x16(r);
+          if (C::WIDE) tmem_ld_wait_x16(r2);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) part[(c + j) * BM] = __uint_as_float(r[j]);
+          for (int j = 0; j < 16; ++j)
+            part[(c + j) * BM] = C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
         }
         break;
       }
       const int m = t.tm * BM + quarter * 32 + lane;
       const int64_t at = out_offset<XK>(p, m, t.b);
       const int n0 = t.tn * BN;
-      uint32_t r[2][16];
-      tmem_ld_32x32b_x16(src, r[0]);
+      // the next chunk's accumulators are on their way while this one is stored
+      uint32_t r[16], r2[16];
+      tmem_ld_32x32b_x16(src, r);
+      if (C::WIDE) tmem_ld_32x32b_x16(src + BN, r2);
 #pragma unroll
       for (int c = 0; c < BN; c += 16) {
-        uint32_t (&v)[16] = r[(c / 16) & 1];
-        tmem_ld_wait_x16(v);
+        tmem_ld_wait_x16(r);
+        if (C::WIDE) tmem_ld_wait_x16(r2);
+        // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
+        // latency per channel made a 128 x 128 tile take 19 us)
+        float x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
         if (c + 16 < BN) {
-          tmem_ld_32x32b_x16(src + c + 16, r[(c / 16 + 1) & 1]);
+          tmem_ld_32x32b_x16(src + c + 16, r);
+          if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c + 16, r2);
         } else {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(tempty_bar + 8 * acc);
         }
-        // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
-        // latency per channel made a 128 x 128 tile take 19 us)
-        float x[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
         if (p.bias != nullptr) {
           const float mine = n0 + c + (lane & 15) < p.N ? __ldg(p.bias + n0 + c + (lane & 15)) : 0.f;
 #pragma unroll

@@ -38,7 +38,7 @@
 //   warps 6..9    W split: hi/lo tiles in shared memory
 //   warps 10..17  epilogue: two sets of four warps (one per TMEM lane quarter), each on half
 //                 of the tile's columns: tcgen05.ld, bias, activation, TMA stores
-// TMEM columns: two accumulators of BN columns, then STAGES x 64 columns of A (hi 32, lo 32).
+// TMEM columns: two accumulators of 128 columns, then STAGES x 64 columns of A (hi 32, lo 32).
 // Every wait is bounded; on a timeout the kernel records a status word, lets outstanding
 // copies land, frees its TMEM and returns.
 #include "common.cuh"
@@ -106,7 +106,10 @@ struct F32Cfg {
   static constexpr int RING_BUDGET = 227 * 1024 - STAGING_BYTES - 1024 - BAR_BYTES;
   static constexpr int NUM_ACC = 2;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int A_COL0 = NUM_ACC * BN;     // first TMEM column of the A ring
+  // 64 channels: hi x [w_hi | w_lo] is one MMA of 128 columns (see the MMA issuer)
+  static constexpr bool WIDE = BN == 64;
+  static constexpr int ACC_COLS = WIDE ? 2 * BN : BN;
+  static constexpr int A_COL0 = NUM_ACC * ACC_COLS;  // first TMEM column of the A ring
   static constexpr int MAX_TMEM_STAGES = (TMEM_COLS - A_COL0) / F_A_COLS;
   static constexpr int SMEM_STAGES = RING_BUDGET / STAGE_BYTES;
   static constexpr int STAGES = SMEM_STAGES < MAX_TMEM_STAGES ? SMEM_STAGES : MAX_TMEM_STAGES;
@@ -242,6 +245,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc(/*c f32*/ 1, /*a tf32*/ 2, /*b tf32*/ 2, /*a mn*/ false,
                                             /*b mn*/ false, FBM, BN);
+      // 64 channels: with A from tensor memory an MMA takes 92 cycles for 64 columns as for 128, so hi comes from
+      // there once for both halves of W, whose tiles lie one behind the other: two MMAs per 8 of k instead of three, and
+      // hi * lo + lo * hi in columns of their own, which the epilogue adds (1x1 of 256 -> 64 channels, 56 x 56, batch 256:
+      // TIME_NOTE).
+      constexpr uint32_t idesc_wide = make_idesc(1, 2, 2, false, false, FBM, Cfg::WIDE ? 2 * BN : BN);
       // W (K-major): rows of 128 bytes (32 k), 8-row groups 1024 bytes apart; a K step of 8
       // moves 32 bytes inside the swizzled row (+2 in the descriptor's address field).
       const uint64_t wdesc = make_smem_desc(0, 16, 1024, 2);
@@ -261,7 +269,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
           break;
         }
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc_buf * BN;
+        const uint32_t d_tmem = tmem_base + acc_buf * Cfg::ACC_COLS;
         for (int kb = 0; kb < p.k_blocks; ++kb, ++kstep) {
           if (!mbar_wait(split_bar + 8 * stage, phase, abort_flag, F_WAIT_BUDGET)) {
             *abort_flag = 1;
@@ -281,12 +289,22 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
           if (kb + 1 < p.k_blocks || last_ksteps == FKB / FUMMA_K) {
 #pragma unroll
             for (int j = 0; j < FKB / FUMMA_K; ++j) {
+              if (Cfg::WIDE) {
+                mma_tf32_ts(d_tmem, a_hi + j * FUMMA_K, w_hi + 2 * j, idesc_wide, (kb > 0 || j > 0) ? 1u : 0u);
+                mma_tf32_ts(d_tmem + BN, a_lo + j * FUMMA_K, w_hi + 2 * j, idesc, 1u);
+                continue;
+              }
               mma_tf32_ts(d_tmem, a_lo + j * FUMMA_K, w_hi + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
               mma_tf32_ts(d_tmem, a_hi + j * FUMMA_K, w_lo + 2 * j, idesc, 1u);
               mma_tf32_ts(d_tmem, a_hi + j * FUMMA_K, w_hi + 2 * j, idesc, 1u);
             }
           } else {
             for (int j = 0; j < last_ksteps; ++j) {
+              if (Cfg::WIDE) {
+                mma_tf32_ts(d_tmem, a_hi + j * FUMMA_K, w_hi + 2 * j, idesc_wide, (kb > 0 || j > 0) ? 1u : 0u);
+                mma_tf32_ts(d_tmem + BN, a_lo + j * FUMMA_K, w_hi + 2 * j, idesc, 1u);
+                continue;
+              }
               mma_tf32_ts(d_tmem, a_lo + j * FUMMA_K, w_hi + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
               mma_tf32_ts(d_tmem, a_hi + j * FUMMA_K, w_lo + 2 * j, idesc, 1u);
               mma_tf32_ts(d_tmem, a_hi + j * FUMMA_K, w_hi + 2 * j, idesc, 1u);
@@ -430,11 +448,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int64_t m = static_cast<int64_t>(it.tm) * FBM + quarter * 32 + lane;
       const bool m_ok = m < p.Mdim;
       float *c = p.C + it.b * p.c_batch_stride + m;
-      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc_buf * BN +
+      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc_buf * Cfg::ACC_COLS +
                              set * (BN / 2);
       const int64_t n_first = static_cast<int64_t>(it.tn) * BN + set * (BN / 2);
-      uint32_t r[2][16];
-      tmem_ld_32x32b_x16(tbase, r[0]);
+      uint32_t r[16], r2[16];
+      tmem_ld_32x32b_x16(tbase, r);
+      if (Cfg::WIDE) tmem_ld_32x32b_x16(tbase + BN, r2);
       // Bias: lane j of a warp fetches the value of the chunk's channel j one chunk ahead and
       // the chunk broadcasts it with shuffles.  (A load per value needs a bounds branch per
       // value, and with eight warps nothing hides a branch: that form took 750 cycles a chunk.)
@@ -475,8 +494,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int m0 = it.tm * FBM;
 #pragma unroll
       for (int i = 0; i < CHUNKS; ++i) {
-        tmem_ld_wait_x16(r[i & 1]);
-        if (i + 1 < CHUNKS) tmem_ld_32x32b_x16(tbase + (i + 1) * 16, r[(i + 1) & 1]);
+        tmem_ld_wait_x16(r);
+        if (Cfg::WIDE) tmem_ld_wait_x16(r2);
+        float a[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a[j] = Cfg::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
+        if (i + 1 < CHUNKS) {
+          tmem_ld_32x32b_x16(tbase + (i + 1) * 16, r);
+          if (Cfg::WIDE) tmem_ld_32x32b_x16(tbase + BN + (i + 1) * 16, r2);
+        }
         if (i == CHUNKS - 1) {
           tc_fence_before_sync();
           __syncwarp();
@@ -495,12 +521,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
         float v[16];
         if constexpr (EPI == 1) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[i & 1][j]);
+          for (int j = 0; j < 16; ++j) v[j] = a[j];
         } else if constexpr (EPI == 2) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const float bj = __shfl_sync(0xffffffffu, b_cur, j);
-            const float x = (__uint_as_float(r[i & 1][j]) + bj) + r_cur[j];
+            const float x = (a[j] + bj) + r_cur[j];
             v[j] = fminf(fmaxf(x, act_lo), act_hi);
           }
         } else {
@@ -508,7 +534,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
           for (int j = 0; j < 16; ++j) {
             const float bj = __shfl_sync(0xffffffffu, b_cur, j);
             // (acc + bias) + residual: the rounding order of a convolution followed by a sum
-            const float x = (__uint_as_float(r[i & 1][j]) + bj) + r_cur[j];
+            const float x = (a[j] + bj) + r_cur[j];
             const float neg = leaky ? fminf(x, 0.f) * act_slope : 0.f;
             v[j] = fminf(fmaxf(x, act_lo), act_hi) + neg;
           }
