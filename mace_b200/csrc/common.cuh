@@ -36,7 +36,7 @@ struct mb_context {
   // call carves from the start; contents do not survive the call.
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
-  int *dev_status = nullptr;   // device status word (bounded-wait failures)
+  int *dev_status = nullptr;   // status word of bounded-wait failures: the device's address of host_status
   int *host_status = nullptr;  // pinned mirror read at sync
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
   void *encode_im2col = nullptr; // cuTensorMapEncodeIm2col

@@ -72,9 +72,9 @@ int mb_init(int device, mb_context **out) {
   ctx->max_smem_optin = static_cast<int>(prop.sharedMemPerBlockOptin);
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) !=
           cudaSuccess ||
-      cudaMalloc(&ctx->dev_status, sizeof(int)) != cudaSuccess ||
-      cudaMemset(ctx->dev_status, 0, sizeof(int)) != cudaSuccess ||
-      cudaMallocHost(&ctx->host_status, sizeof(int)) != cudaSuccess) {
+      // (in host memory, which a kernel writes only when it gives up a wait: mb_stream_sync then has no copy to wait for)
+      cudaHostAlloc(&ctx->host_status, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->dev_status), ctx->host_status, 0) != cudaSuccess) {
     delete ctx;
     return MB_RUNTIME_ERROR;
   }
@@ -115,7 +115,6 @@ int mb_destroy(mb_context *ctx) {
   }
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->skinny_ws) cudaFree(ctx->skinny_ws);
-  if (ctx->dev_status) cudaFree(ctx->dev_status);
   if (ctx->host_status) cudaFreeHost(ctx->host_status);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -297,13 +296,10 @@ int mb_memset(mb_context *ctx, void *dst, int value, size_t bytes) {
 
 int mb_stream_sync(mb_context *ctx) {
   if (ctx == nullptr) return MB_INVALID_ARGS;
-  MB_CUDA(ctx, cudaMemcpyAsync(ctx->host_status, ctx->dev_status, sizeof(int),
-                               cudaMemcpyDeviceToHost, ctx->stream));
   MB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (*ctx->host_status != 0) {
-    const int code = *ctx->host_status;
-    *ctx->host_status = 0;
-    cudaMemsetAsync(ctx->dev_status, 0, sizeof(int), ctx->stream);
+  const int code = *static_cast<volatile int *>(ctx->host_status);
+  if (code != 0) {
+    *static_cast<volatile int *>(ctx->host_status) = 0;
     return mb_fail(ctx, MB_RUNTIME_ERROR,
                    "a kernel gave up a bounded wait (device status %d)", code);
   }
