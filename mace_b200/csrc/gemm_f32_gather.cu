@@ -13,16 +13,16 @@
 // holds its pixel's valid filter rows and columns as bit masks, so padding costs one logic instruction per value.
 // W comes by TMA where its rows are 16-byte aligned, else through registers, and is split in shared memory.
 //
-// Roles (22 warps): three groups of four load X, taking the steps in turn (three steps of loads in flight; fetching
-// with 4-byte asynchronous copies through shared memory instead took twice as long, 128 of them per step), four split
-// W, four store results, one thread issues the MMAs, one requests W.  Persistent over the tiles; where these do not fill
+// Roles (18 warps): two groups of four load X, taking the steps in turn (two steps of loads in flight; a third group
+// gained nothing and cost 0.5 us per launch; fetching with 4-byte asynchronous copies through shared memory instead took
+// twice as long, 128 of them per step), four split W, four store results, one thread issues the MMAs, one requests W.  Persistent over the tiles; where these do not fill
 // the SMs, one tile per cluster of 2 .. 8 CTAs with the depth cut between them, the partial tiles added up through
 // distributed shared memory.
 //
 // What bounds it: the tensor pipe at three tf32 MMAs per product for long depths (12 MMAs x 92 cycles per step of
 // 128 x 128 x 32; a convolution's loads bring the step to 1400), the launch, first loads and results for small shapes.
-// Measured, before -> now: 7x7 stride 2 of 3 -> 64 channels, 224 x 224, batch 256, 1360 us (column matrix) -> 732;
-// 5x5 stride 2 of 48 -> 32, 112 x 112, batch 24, 341 -> 116; 3x3 of 512 channels, 7 x 7, batch 1, 70 (Winograd) -> 20;
+// Measured, before -> now: 7x7 stride 2 of 3 -> 64 channels, 224 x 224, batch 256, 1360 us (column matrix) -> 688;
+// 5x5 stride 2 of 48 -> 32, 112 x 112, batch 24, 341 -> 116; 3x3 of 512 channels, 7 x 7, batch 1, 70 (Winograd) -> 17;
 // 384 x 384 x 64 times a transposed matrix, batch 12, 16.4 (CUDA cores) -> 7.9; 736 x 176 x 384, batch 24, 152 -> 29.
 #include <algorithm>
 
@@ -39,7 +39,7 @@ using namespace sm100;
 
 constexpr int BM = 128;         // pixels (m) per tile == TMEM lanes
 constexpr int KB = 32;          // depth per step
-constexpr int XGROUPS = 3;      // of four warps each, taking the steps in turn
+constexpr int XGROUPS = 2;      // of four warps each, taking the steps in turn
 constexpr int FIRST_W = 4 * XGROUPS, FIRST_E = FIRST_W + 4, EWARPS = 4, MMA_WARP = FIRST_E + EWARPS, TMA_WARP = MMA_WARP + 1;
 constexpr int THREADS = (TMA_WARP + 1) * 32;
 constexpr int ACCS = 2;
@@ -74,8 +74,10 @@ struct Cfg {
   static constexpr int STAGES = (512 - A_COL0) / (2 * KB);
   static constexpr int RING = STAGES * STAGE_BYTES;
   static constexpr int TABLE_BYTES = FIRST_W * KB * 8;
+  static constexpr int PART_BYTES = BN * BM * 4;         // the runs' shares of this CTA's channels: [rank][channel][128 m]
+  // (PART_BYTES only where the depth is cut: what shared memory does not take is L1, which a convolution's windows live in)
   static constexpr int SMEM_BYTES = RING + 1024 /*align*/ + TABLE_BYTES + 256 /*barriers*/;
-  static_assert(BN * BM * 4 <= RING, "the partial tile reuses the ring");
+  static_assert(SMEM_BYTES + PART_BYTES <= 227 * 1024, "shared memory budget");
 };
 
 struct TileIter {
@@ -102,10 +104,8 @@ struct TileIter {
 __device__ __forceinline__ uint32_t tf32_hi(float v) { return __float_as_uint(v) & 0xffffe000u; }
 __device__ __forceinline__ uint32_t tf32_lo(float v) { return __float_as_uint(v - __uint_as_float(tf32_hi(v))); }
 
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
 // Rows of 32 k, 128 bytes, the 16-byte chunks of a row permuted by its low three bits (the tensor core's 128-byte swizzle).
@@ -165,9 +165,12 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   };
   tc_fence_before_sync();
   __syncthreads();
+  if (p.splits > 1) cluster_sync_all();  // every CTA of the cluster runs before one writes into another's memory
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  mb_grid_dep_wait();
+  // The X warps wait for the kernel in front only where they first read the tensor: tile coordinates and the first table
+  // are worked out while that kernel still runs.
+  const uint32_t part = bars + 256;
 
   if (warp < FIRST_W) {
     // ---- X: tensor -> registers -> hi / lo in tensor memory ----
@@ -175,7 +178,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const uint32_t a_lane = static_cast<uint32_t>(quarter * 32) << 16;
     int2 *table = reinterpret_cast<int2 *>(smem + C::RING) + warp * KB;
     int it = 0;  // steps of this CTA so far, all tiles
-    bool ok = true;
+    bool ok = true, waited = false;
     for (TileIter t(p); ok && t.valid(p); t.next(p)) {
       const int m = t.tm * BM + quarter * 32 + lane;
       const float *base = p.X;
@@ -200,6 +203,8 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         const int k0 = (kb_begin + i) * KB;
         float v[KB];
         if (XK == X_COLS) {
+          if (!waited) mb_grid_dep_wait();
+          waited = true;
           const float *row = base + k0;
           if (p.x_vec) {
 #pragma unroll
@@ -230,6 +235,8 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           __syncwarp();  // the table of the previous step has been read
           table[lane] = e;
           __syncwarp();
+          if (!waited) mb_grid_dep_wait();
+          waited = true;
 #pragma unroll
           for (int j = 0; j < KB; j += 2) {
             const int4 t2 = *reinterpret_cast<const int4 *>(table + j);
@@ -263,6 +270,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   } else if (warp < FIRST_E) {
     // ---- W: (matrix -> registers ->) hi / lo in shared memory, rows of 32 k, 128-byte swizzle ----
     const int w4 = warp - FIRST_W;
+    mb_grid_dep_wait();
     int it = 0;
     bool ok = true;
     for (TileIter t(p); ok && t.valid(p); t.next(p)) {
@@ -341,6 +349,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     }
   } else if (warp == TMA_WARP) {
     if (WK == W_TMA && lane == 0) {
+      mb_grid_dep_wait();
       int it = 0;
       bool ok = true;
       for (TileIter t(p); ok && t.valid(p); t.next(p)) {
@@ -360,6 +369,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     __syncwarp();
   } else if (warp == MMA_WARP) {
     // ---- MMA: one thread ----
+    mb_grid_dep_wait();  // (its waits below are bounded: they must not count the time of the kernel in front)
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc(/*c f32*/ 1, /*a tf32*/ 2, /*b tf32*/ 2, false, false, BM, BN);
       constexpr uint32_t idesc_wide = make_idesc(1, 2, 2, false, false, BM, C::WIDE ? 2 * BN : BN);
@@ -411,6 +421,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     // ---- results: a lane per pixel, one channel after the other, 32 adjacent pixels per store ----
     const int quarter = warp & 3;
     int local = 0;
+    mb_grid_dep_wait();
     for (TileIter t(p); t.valid(p); t.next(p), ++local) {
       const int acc = local % ACCS;
       if (!mbar_wait_warp(tfull_bar + 8 * acc, (local / ACCS) & 1, abort_flag, WAIT_BUDGET)) {
@@ -420,18 +431,21 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       tc_fence_after_sync();
       const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * C::ACC_COLS;
       if (p.splits > 1) {
-        // this CTA's run of the depth: [n][128 m] into shared memory (the ring is idle: one tile per CTA)
-        float *part = reinterpret_cast<float *>(smem) + quarter * 32 + lane;
+        // this CTA's run of the depth, each channel to the CTA that adds it up (writing it there takes nobody's time; read
+        // from there, one peer after the other, it took 2.1 us)
+        const int share = BN / p.splits;  // channels per CTA: 8 .. 64
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 16) {
-          uint32_t r[16], r2[16];
-          tmem_ld_32x32b_x16(src + c, r);
-          if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c, r2);
-          tmem_ld_wait_x16(r);
-          if (C::WIDE) tmem_ld_wait_x16(r2);
+        for (int c = 0; c < BN; c += 8) {
+          uint32_t r[8], r2[8];
+          tmem_ld_32x32b_x8(src + c, r);
+          if (C::WIDE) tmem_ld_32x32b_x8(src + BN + c, r2);
+          tmem_ld_wait_x8(r);
+          if (C::WIDE) tmem_ld_wait_x8(r2);
+          const int owner = c / share;
+          const uint32_t dst = mapa_shared(part, owner) + ((rank * share + c - owner * share) * BM + quarter * 32 + lane) * 4;
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            part[(c + j) * BM] = C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
+          for (int j = 0; j < 8; ++j)
+            st_cluster_f32(dst + j * (BM * 4), C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]));
         }
         break;
       }
@@ -497,27 +511,26 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   }
   if (p.splits > 1) {
     cluster_sync_all();
+    mb_grid_dep_wait();  // (some of these warps had nothing to wait for so far)
     // every CTA of the cluster adds up its share of the channels, all runs in the order of their rank
     const TileIter t(p);
     const int m = t.tm * BM + (threadIdx.x & 127);
     const int64_t at = out_offset<XK>(p, m, t.b);
-    const int n0 = t.tn * BN;
-    const uint32_t mine = smem_base + (threadIdx.x & 127) * 4;
-    if (warp < 20 && m < p.M) {
+    const int share = BN / p.splits, n0 = t.tn * BN + rank * share;
+    const float *mine = reinterpret_cast<const float *>(smem + C::RING + C::TABLE_BYTES + 256) + (threadIdx.x & 127);
+    if (warp < 16 && m < p.M) {
       // up to four channels per round, all loads before the first store (see above)
-      const int stride = 5 * p.splits;
-      for (int c0 = (warp >> 2) * p.splits + rank; c0 < BN; c0 += 4 * stride) {
+      for (int c0 = warp >> 2; c0 < share; c0 += 16) {
         float x[4], add[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int c = c0 + q * stride, n = n0 + c;
+          const int c = c0 + q * 4, n = n0 + c;
           x[q] = add[q] = 0.f;
-          if (c < BN && n < p.N) {
-#pragma unroll
-            for (int s = 0; s < 8; ++s)
-              if (s < p.splits) x[q] += ld_cluster_f32(mapa_shared(mine + c * (BM * 4), s));
-            if (p.bias != nullptr) x[q] += __ldg(p.bias + n);
+          if (c < share && n < p.N) {
             if (p.residual != nullptr) add[q] = __ldg(p.residual + at + static_cast<int64_t>(n) * p.c_ns);
+            const float b = p.bias != nullptr ? __ldg(p.bias + n) : 0.f;
+            for (int s = 0; s < p.splits; ++s) x[q] += mine[(s * share + c) * BM];
+            x[q] += b;
           }
         }
 #pragma unroll
@@ -525,12 +538,11 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         mb_activate_n(x, p.act, p.max_limit, p.coef);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int c = c0 + q * stride, n = n0 + c;
-          if (c < BN && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = x[q];
+          const int c = c0 + q * 4, n = n0 + c;
+          if (c < share && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = x[q];
         }
       }
     }
-    cluster_sync_all();  // no CTA may leave while another still reads its tile
   }
   if (warp == FIRST_E) {
     tc_fence_after_sync();
@@ -547,7 +559,7 @@ int launch_cfg(mb_context *ctx, Params &p) {
   if (WK == W_TMA) MB_RETURN_IF_ERROR(mb_make_map_w_f32(ctx, &map, p.W, p.K, p.N, p.w_bs != 0 ? p.batch : 1, p.w_ns, p.w_bs, BN));
   else memset(&map, 0, sizeof(map));
   if (!(ctx->f32_gather_attr_mask & (1ull << bit))) {
-    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES + C::PART_BYTES));
     ctx->f32_gather_attr_mask |= 1ull << bit;
   }
   const int64_t tiles = static_cast<int64_t>(p.batch) * p.tiles_m * p.tiles_n;
@@ -555,7 +567,8 @@ int launch_cfg(mb_context *ctx, Params &p) {
   p.step_m = slots % p.tiles_m;
   p.step_n = (slots / p.tiles_m) % p.tiles_n;
   p.step_b = (slots / p.tiles_m) / p.tiles_n;
-  MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), THREADS, C::SMEM_BYTES, p.splits, map, p));
+  MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), THREADS,
+                                  C::SMEM_BYTES + (p.splits > 1 ? C::PART_BYTES : 0), p.splits, map, p));
   ctx->launches++;
   ctx->launches_tc++;
   return MB_SUCCESS;
@@ -567,9 +580,9 @@ struct Plan {
 };
 
 // Tile width and depth runs with the smallest estimate, in SM cycles.  Measured: a step is bound by the MMAs, whose A
-// operand comes from tensor memory at the same rate for either width (0.6 us), or by a convolution's loads (0.72 us); a
-// tile's stores take 2.7 us per 64 channels, twice that with a residual; 5.5 us around the steps, 7.6 us with the
-// exchange between the CTAs of a cluster.
+// operand comes from tensor memory at the same rate for either width (0.6 us for the 12 of 128 channels), or by a
+// convolution's loads (0.72 us); a tile's stores take 2.7 us per 64 channels, twice that with a residual; 5.5 us around the
+// steps, 6.3 us with the exchange between the CTAs of a cluster.
 Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
   const int64_t tiles_m = ceil_div64(g.M, BM), k_blocks = ceil_div64(g.K, KB);
   Plan best;
@@ -579,14 +592,16 @@ Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
     if (ctx->f32_bn != 0 ? w != ctx->f32_bn : (w == 128 && g.N <= 64)) continue;
     const int64_t tiles = g.batch * tiles_m * ceil_div64(g.N, w);
     for (int s : {1, 2, 4, 8}) {
-      if (asked != 0 ? s != asked : (s > 1 && s * 2 > k_blocks)) continue;
+      if (asked != 0 ? s != asked : s > k_blocks) continue;
       const int64_t rounds = ceil_div64(tiles * s, s == 1 ? ctx->num_sms : mb_resident_cluster_ctas(ctx, s));
       if (s > 1 && rounds > 1 && asked == 0) continue;  // (one tile per CTA: a second round would start from nothing)
       const int64_t steps = ceil_div64(k_blocks, s);
-      const int64_t step = g.conv ? (w == 128 ? 1450 : 1350) : (w == 128 ? 1250 : 1150);
+      const int64_t step = g.conv ? (w == 128 ? 1450 : 1200) : (w == 128 ? 1250 : 1100);
       const int64_t results = (w == 128 ? 10000 : 5000) * (g.residual != nullptr ? 2 : 1);
-      const int64_t cost = s == 1 ? 8500 + rounds * std::max<int64_t>(steps * step, results) + (w == 128 ? 4000 : 2000)
-                                  : w == 128 ? 17500 + steps * 1680 : 14500 + steps * 1370;
+      const int64_t last = (w == 128 ? 4000 : 1500) + (g.residual != nullptr ? 2000 : 0);
+      const int64_t cost = s == 1 ? 8000 + (rounds - 1) * std::max<int64_t>(steps * step, results) + steps * step + last
+                           : w == 128 ? 10500 + steps * 1350 + last
+                                      : (s == 2 ? 11500 : s == 4 ? 10500 : 11000) + steps * (s == 2 ? 1150 : 1050) + last;
       if (best.cost < 0 || cost < best.cost) {
         best.bn = w; best.splits = s; best.cost = cost;
       }

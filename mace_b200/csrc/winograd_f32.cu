@@ -371,10 +371,11 @@ int pick_tile(int64_t H, int64_t W, int tile_override) {
 
 }  // namespace
 
-// Estimated SM cycles of the three Winograd kernels, from their times at 56 x 56 x 64 (batch 1: 13 us, 32: 60, 256: 437),
+// Estimated SM cycles of the three Winograd kernels, from their times at 56 x 56 x 64 (batch 1: 13 us, 32: 56, 256: 400),
 // 28 x 28 x 128 (8: 21, 256: 290), 14 x 14 x 256 (256: 299) and 7 x 7 x 512 (256: 230): about 12 us of launches, the
-// transforms' bytes (the intermediates written and read once each) at 9.5 TB/s (part of them stays in L2), the batched product at 1150 cycles per
-// step and tile or 2.4 us for a tile's stores.  An odd column count keeps the product off TMA (15 us at batch 1).
+// transforms' bytes (the intermediates written and read once each) at 9.5 TB/s (part of them stays in L2), the batched
+// product at 1150 cycles per step and tile or 2.4 us for a tile's stores.  An odd column count keeps the product off TMA
+// (15 us at batch 1).
 static int64_t winograd_cost(const mb_context *ctx, int64_t N, int64_t C, int64_t H, int64_t W, int64_t O, int64_t Ho,
                              int64_t Wo, int tile_override) {
   const int tile = pick_tile(H, W, tile_override);
