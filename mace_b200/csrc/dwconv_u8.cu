@@ -45,11 +45,9 @@ __device__ __forceinline__ uint32_t dw_requant(int32_t acc, const DwParams &p) {
 //   sum (in - zp_in) w = sum in * w - zp_in * sum w,
 // out-of-image taps read as zp_in (they then contribute zero).  dp4a multiplies four
 // unsigned input bytes with four SIGNED 8-bit weights, but w needs 9 bits.  It is split as
-// w = (f - 128) + k with k = 128 - zp_f the same for every tap of the tensor: a second dp4a with
-// k in every tap, which comes from two registers and is left out where zp_f == 128 (k = 128, of
-// zp_f == 0, does not fit a byte and takes two of 64).  (With w clamped to a byte and the few
-// taps' rests in words of their own, almost every warp had such a tap and loaded those words for
-// every output row: 56 x 56 x 128, batch 64, 23.9 us; now 22.4, 17.1 with zp_f == 128.)
+// w = w1 + w2 with w1 = clamp(w, -128, 127): w2 is zero except for the few taps at the far
+// end of the filter's range (none at all when zp_f == 128), and channel groups that have
+// such a tap run a second dp4a with w2.
 //
 // Layout of the work.  A thread owns 4 adjacent channels (one 32-bit word per pixel), 4
 // adjacent output columns and a run of output rows.  Per input row it loads the 6 (stride
@@ -63,10 +61,11 @@ __device__ __forceinline__ uint32_t dw_requant(int32_t acc, const DwParams &p) {
 // (or once per weight tensor through mb_dwconv_u8_prepack).
 
 // Per group of 4 channels, as structure of arrays [item][group] of 16-byte items:
-//   0..5   f - 128 [kh][align] : x,y,z,w = channels; bytes = [w0,w1,w2,0] (align 0) / [0,w0,w1,w2]
-//   6      start[c] = bias[c] - zp_in * sum_t w[t][c]
-//   7      x = the byte k (64 for 128) three times, y = how often it is added (0, 1, 2)
-constexpr int DW_PACK_ITEMS = 8;
+//   0..5   w1[kh][align] : x,y,z,w = channels; bytes = [w0,w1,w2,0] (align 0) / [0,w0,w1,w2]
+//   6..11  w2[kh][align]
+//   12     start[c] = bias[c] - zp_in * sum_t w[t][c]
+//   13     flags: x = group has a non-zero w2; y = bit kh set when filter row kh has one
+constexpr int DW_PACK_ITEMS = 14;
 #ifndef DW_THREADS
 #define DW_THREADS 256
 #define DW_BLOCKS_PER_SM 2
@@ -91,22 +90,28 @@ dwconv3x3_prepack_kernel(const uint8_t *__restrict__ filter, const int32_t *__re
 #pragma unroll
     for (int c = 0; c < 4; ++c) w[t][c] = static_cast<int32_t>((v >> (8 * c)) & 0xffu) - zp_f;
   }
-  uint32_t v[3][2][4];
+  int32_t any_w2 = 0;
+  uint32_t rows_w2 = 0;
+  uint32_t v1[3][2][4], v2[3][2][4];
   int32_t start[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     int32_t sum = 0;
 #pragma unroll
     for (int kh = 0; kh < 3; ++kh) {
-      uint32_t word = 0;
+      uint32_t p1 = 0, p2 = 0;
 #pragma unroll
       for (int kw = 0; kw < 3; ++kw) {
         const int32_t x = w[kh * 3 + kw][c];
+        const int32_t a = min(127, max(-128, x)), b = x - a;
         sum += x;
-        word |= (static_cast<uint32_t>(x + zp_f - 128) & 0xffu) << (8 * kw);
+        any_w2 |= b;
+        if (b != 0) rows_w2 |= 1u << kh;
+        p1 |= (static_cast<uint32_t>(a) & 0xffu) << (8 * kw);
+        p2 |= (static_cast<uint32_t>(b) & 0xffu) << (8 * kw);
       }
-      v[kh][0][c] = word;
-      v[kh][1][c] = word << 8;
+      v1[kh][0][c] = p1; v1[kh][1][c] = p1 << 8;
+      v2[kh][0][c] = p2; v2[kh][1][c] = p2 << 8;
     }
     const int32_t bv = bias != nullptr ? __ldg(bias + g * 4 + c) : 0;
     start[c] = bv - zp_in * sum;
@@ -114,11 +119,14 @@ dwconv3x3_prepack_kernel(const uint8_t *__restrict__ filter, const int32_t *__re
 #pragma unroll
   for (int kh = 0; kh < 3; ++kh)
 #pragma unroll
-    for (int al = 0; al < 2; ++al)
-      packed[(kh * 2 + al) * groups + g] = make_uint4(v[kh][al][0], v[kh][al][1], v[kh][al][2], v[kh][al][3]);
-  packed[6 * groups + g] = make_uint4(start[0], start[1], start[2], start[3]);
-  const int32_t k = 128 - zp_f;
-  packed[7 * groups + g] = make_uint4((static_cast<uint32_t>(k == 128 ? 64 : k) & 0xffu) * 0x010101u, k == 0 ? 0u : k == 128 ? 2u : 1u, 0u, 0u);
+    for (int al = 0; al < 2; ++al) {
+      packed[(kh * 2 + al) * groups + g] =
+          make_uint4(v1[kh][al][0], v1[kh][al][1], v1[kh][al][2], v1[kh][al][3]);
+      packed[(6 + kh * 2 + al) * groups + g] =
+          make_uint4(v2[kh][al][0], v2[kh][al][1], v2[kh][al][2], v2[kh][al][3]);
+    }
+  packed[12 * groups + g] = make_uint4(start[0], start[1], start[2], start[3]);
+  packed[13 * groups + g] = make_uint4(any_w2 != 0 ? 1u : 0u, rows_w2, 0u, 0u);
 }
 
 // Windows of one input row: win[j][c] holds, for channel c, the 4 horizontally adjacent
@@ -209,16 +217,6 @@ __device__ __forceinline__ void dw_mac(int32_t (&acc)[4][4], const DwRow<STRIDE>
   }
 }
 
-// acc[j][c] += the same weight for all nine taps (w = [k,k,k,0]).
-template <int STRIDE>
-__device__ __forceinline__ void dw_mac_same(int32_t (&acc)[4][4], const DwRow<STRIDE> &r0, const DwRow<STRIDE> &r1,
-                                            const DwRow<STRIDE> &r2, uint32_t w) {
-  const uint4 wa = make_uint4(w, w, w, w), wb = make_uint4(w << 8, w << 8, w << 8, w << 8);
-  dw_mac<STRIDE>(acc, r0, wa, wb);
-  dw_mac<STRIDE>(acc, r1, wa, wb);
-  dw_mac<STRIDE>(acc, r2, wa, wb);
-}
-
 // VAR: requantization variant (mb_requant_variant): 0..3 = mb_requant_t, 4 / 5 = packed form.
 template <int STRIDE, int VAR>
 __global__ void __launch_bounds__(DW_THREADS, DW_BLOCKS_PER_SM)
@@ -255,11 +253,12 @@ dwconv3x3_u8_kernel(const DwParams p, const uint4 *__restrict__ packed, int rows
     if (STRIDE == 1) w1[kh][1] = __ldg(packed + (kh * 2 + 1) * groups + g);
     else w1[kh][1] = w1[kh][0];
   }
-  const uint4 st4 = __ldg(packed + 6 * groups + g);
-  const uint4 extra = __ldg(packed + 7 * groups + g);
-  const uint32_t k_first = extra.x, k_times = extra.y;
+  const uint4 st4 = __ldg(packed + 12 * groups + g);
+  const uint4 flags = __ldg(packed + 13 * groups + g);
   const int32_t start[4] = {static_cast<int32_t>(st4.x), static_cast<int32_t>(st4.y),
                             static_cast<int32_t>(st4.z), static_cast<int32_t>(st4.w)};
+  const bool has_w2 = flags.x != 0;
+  const uint32_t rows_w2 = flags.y;  // the filter rows that have a 9-bit tap (rare: most warps skip most rows)
   if (weights_cached) mb_grid_dep_wait();
 
   // columns: byte offsets inside a row and validity bits, fixed for the thread
@@ -293,7 +292,11 @@ dwconv3x3_u8_kernel(const DwParams p, const uint4 *__restrict__ packed, int rows
     dw_mac<STRIDE>(acc, r0, w1[0][0], w1[0][1]);
     dw_mac<STRIDE>(acc, r1, w1[1][0], w1[1][1]);
     dw_mac<STRIDE>(acc, r2, w1[2][0], w1[2][1]);
-    for (uint32_t i = 0; i < k_times; ++i) dw_mac_same<STRIDE>(acc, r0, r1, r2, k_first);
+    if (has_w2) {
+      if (rows_w2 & 1u) dw_mac<STRIDE>(acc, r0, __ldg(packed + 6 * groups + g), __ldg(packed + 7 * groups + g));
+      if (rows_w2 & 2u) dw_mac<STRIDE>(acc, r1, __ldg(packed + 8 * groups + g), __ldg(packed + 9 * groups + g));
+      if (rows_w2 & 4u) dw_mac<STRIDE>(acc, r2, __ldg(packed + 10 * groups + g), __ldg(packed + 11 * groups + g));
+    }
     uint32_t o = out_off + static_cast<uint32_t>(y) * out_row_stride;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -430,11 +433,14 @@ dwconv3x3_u8_tma_kernel(const __grid_constant__ CUtensorMap tmap_in, const DwPar
     if (STRIDE == 1) w1[kh][1] = __ldg(packed + (kh * 2 + 1) * groups + gg);
     else w1[kh][1] = w1[kh][0];
   }
-  const uint4 st4 = __ldg(packed + 6 * groups + gg);
-  const uint4 extra = __ldg(packed + 7 * groups + gg);
-  const uint32_t k_first = extra.x, k_times = extra.y;
+  const uint4 st4 = __ldg(packed + 12 * groups + gg);
+  const uint4 flags = __ldg(packed + 13 * groups + gg);
   const int32_t start[4] = {static_cast<int32_t>(st4.x), static_cast<int32_t>(st4.y),
                             static_cast<int32_t>(st4.z), static_cast<int32_t>(st4.w)};
+  // the filter rows that have a 9-bit tap in ANY lane's channel group (rare: most warps skip most
+  // rows); the same for all lanes, so that the tests below do not diverge -- groups without such a
+  // tap hold zeros in those weight words
+  const uint32_t rows_w2 = __reduce_or_sync(0xffffffffu, flags.x != 0 ? flags.y : 0u);
   if (weights_cached) mb_grid_dep_wait();
   if (threadIdx.x < t.setup_lanes) {
     const int xi0 = ct * t.OWT * STRIDE - p.pad_left;
@@ -476,7 +482,9 @@ dwconv3x3_u8_tma_kernel(const __grid_constant__ CUtensorMap tmap_in, const DwPar
     dw_mac<STRIDE>(acc, r0, w1[0][0], w1[0][1]);
     dw_mac<STRIDE>(acc, r1, w1[1][0], w1[1][1]);
     dw_mac<STRIDE>(acc, r2, w1[2][0], w1[2][1]);
-    for (uint32_t i = 0; i < k_times; ++i) dw_mac_same<STRIDE>(acc, r0, r1, r2, k_first);
+    if (rows_w2 & 1u) dw_mac<STRIDE>(acc, r0, __ldg(packed + 6 * groups + gg), __ldg(packed + 7 * groups + gg));
+    if (rows_w2 & 2u) dw_mac<STRIDE>(acc, r1, __ldg(packed + 8 * groups + gg), __ldg(packed + 9 * groups + gg));
+    if (rows_w2 & 4u) dw_mac<STRIDE>(acc, r2, __ldg(packed + 10 * groups + gg), __ldg(packed + 11 * groups + gg));
     uint32_t o = out_off + static_cast<uint32_t>(y) * out_row_stride;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
