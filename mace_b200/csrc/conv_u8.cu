@@ -46,6 +46,8 @@ struct ConvParams {
 // Filter (zero point removed, int16) lives in shared memory as [depth][O].
 template <int OT>
 __global__ void __launch_bounds__(128) conv_u8_direct_kernel(const ConvParams p) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   extern __shared__ int16_t fsm[];  // [depth][O]
   for (int i = threadIdx.x; i < p.depth * p.O; i += blockDim.x) {
     const int d = i / p.O, o = i % p.O;
@@ -730,8 +732,8 @@ extern "C" int mb_conv2d_u8_nhwc(mb_context *ctx, const uint8_t *in, const uint8
   const size_t direct_smem = static_cast<size_t>(depth) * O * sizeof(int16_t);
   if (direct_smem <= 32 * 1024 && depth <= 256) {
     const unsigned blocks = static_cast<unsigned>(ceil_div64(pixels, 128));
-    if (O % 32 == 0 || O > 16) conv_u8_direct_kernel<32><<<blocks, 128, direct_smem, ctx->stream>>>(p);
-    else conv_u8_direct_kernel<8><<<blocks, 128, direct_smem, ctx->stream>>>(p);
+    if (O % 32 == 0 || O > 16) MB_CUDA(ctx, mb_launch_chained(ctx, conv_u8_direct_kernel<32>, dim3(blocks), dim3(128), direct_smem, p));
+    else MB_CUDA(ctx, mb_launch_chained(ctx, conv_u8_direct_kernel<8>, dim3(blocks), dim3(128), direct_smem, p));
     MB_CUDA(ctx, cudaGetLastError());
     ctx->launches++;
     return MB_SUCCESS;

@@ -33,6 +33,8 @@ struct GemvParams {
 // batch entry.  A matrix shared by the batch is loaded once and kept in registers.
 template <bool VEC>
 __global__ void __launch_bounds__(256) gemv_u8_kernel(const GemvParams p) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   extern __shared__ uint4 xs[];  // VEC: the vector, K / 16 words
   __shared__ uint32_t sum_r_sm;
   const int lane = threadIdx.x & 31;
@@ -381,8 +383,8 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
   dim3 grid(static_cast<unsigned>(ceil_div64(rows, 8)),
             lhs_batched ? static_cast<unsigned>(batch)
                         : static_cast<unsigned>(ceil_div64(batch, p.batch_chunk)));
-  if (vec) gemv_u8_kernel<true><<<grid, 256, static_cast<size_t>(K), ctx->stream>>>(p);
-  else gemv_u8_kernel<false><<<grid, 256, 0, ctx->stream>>>(p);
+  if (vec) MB_CUDA(ctx, mb_launch_chained(ctx, gemv_u8_kernel<true>, dim3(grid), dim3(256), static_cast<size_t>(K), p));
+  else MB_CUDA(ctx, mb_launch_chained(ctx, gemv_u8_kernel<false>, dim3(grid), dim3(256), 0, p));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;

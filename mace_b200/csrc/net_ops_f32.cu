@@ -257,23 +257,40 @@ static void launch_eltwise(mb_context *ctx, const EltParams &p, int vec4) {
                           p, vec4);  // (the caller asks for the error)
 }
 
-// out[p][ho][wo] = in[p][ho * sh][wo * sw] over N * C planes: the pixels a 1x1 convolution with
-// strides (sh, sw) reads, gathered once so that several such convolutions of one tensor (a
-// residual block's shortcut and its first convolution) can run as plain 1x1 convolutions on
-// the compact copy.  One thread per output value, grid-stride; writes are contiguous.
+// out[p][ho][wo] = in[p][ho * sh][wo * sw] over N * C planes: the pixels a 1x1 convolution with strides (sh, sw) reads,
+// gathered once so that several such convolutions of one tensor (a residual block's shortcut and its first convolution) can
+// run as plain 1x1 convolutions on the compact copy.  Bound by memory, which reads the kept rows
+// whole: a thread takes four neighbouring outputs of a row, with two 16-byte loads where the column stride is 2 and rows
+// are aligned (one output per thread and 64-bit divisions: 56 x 56 x 256, batch 256, 187 us; now SUBS_NOTE).
 __global__ void __launch_bounds__(256)
-subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t total, int H, int W, int sh,
-                     int sw, int Ho, int Wo) {
+subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t quads, int H, int W, int sh, int sw,
+                     int Ho, int Wo, int vec) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int64_t plane_out = static_cast<int64_t>(Ho) * Wo, plane_in = static_cast<int64_t>(H) * W;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int64_t pl = i / plane_out;
-    const int rem = static_cast<int>(i - pl * plane_out);
-    const int ho = rem / Wo, wo = rem - ho * Wo;
-    out[i] = __ldg(in + pl * plane_in + static_cast<int64_t>(ho) * sh * W + wo * sw);
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= quads) return;
+  const unsigned wq = (static_cast<unsigned>(Wo) + 3u) >> 2;
+  const int64_t row = quads <= UINT32_MAX ? static_cast<int64_t>(static_cast<uint32_t>(i) / wq) : i / wq;  // of the output, all planes
+  const int wo = static_cast<int>(i - row * wq) * 4;
+  const int64_t pl = quads <= UINT32_MAX ? static_cast<int64_t>(static_cast<uint32_t>(row) / static_cast<unsigned>(Ho)) : row / Ho;
+  const int ho = static_cast<int>(row - pl * Ho);
+  const float *src = in + (pl * H + static_cast<int64_t>(ho) * sh) * W + static_cast<int64_t>(wo) * sw;
+  float *dst = out + (pl * Ho + ho) * Wo + wo;
+  if (vec && wo * 2 + 8 <= W) {
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(src)), b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+    if ((Wo & 3) == 0) {
+      *reinterpret_cast<float4 *>(dst) = make_float4(a.x, a.z, b.x, b.z);
+    } else {  // (eight columns of the input are there: so are four of the output)
+      dst[0] = a.x; dst[1] = a.z; dst[2] = b.x; dst[3] = b.z;
+    }
+    return;
   }
+  float v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = wo + j < Wo ? __ldg(src + static_cast<int64_t>(j) * sw) : 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (wo + j < Wo) dst[j] = v[j];
 }
 
 }  // namespace
@@ -417,7 +434,11 @@ int mb_subsample_f32_nchw(mb_context *ctx, const float *in, float *out, int64_t 
   if (in == nullptr || out == nullptr || in == out)
     return mb_fail(ctx, MB_INVALID_ARGS, "mb_subsample_f32_nchw: null or aliased buffers");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  MB_CUDA(ctx, mb_launch_chained(ctx, subsample_f32_kernel, dim3(stream_grid(ctx, total)), dim3(256), 0, in, out, total, static_cast<int>(H), static_cast<int>(W), stride_h, stride_w, static_cast<int>(Ho), static_cast<int>(Wo)));
+  const int64_t quads = planes * Ho * ((Wo + 3) / 4);
+  const int vec = stride_w == 2 && W % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+  MB_CUDA(ctx, mb_launch_chained(ctx, subsample_f32_kernel, dim3(static_cast<unsigned>(ceil_div64(quads, 256))), dim3(256), 0, in,
+                                 out, quads, static_cast<int>(H), static_cast<int>(W), stride_h, stride_w, static_cast<int>(Ho),
+                                 static_cast<int>(Wo), vec));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;

@@ -12,6 +12,8 @@ namespace {
 __global__ void __launch_bounds__(256)
 avgpool_u8_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int N, int H, int W,
                   int C, int KH, int KW, int sh, int sw, int pad_top, int pad_left, int Ho, int Wo) {
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
   const int64_t total = static_cast<int64_t>(N) * Ho * Wo * C;
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (tid >= total) return;
@@ -119,10 +121,10 @@ extern "C" int mb_avgpool_u8_nhwc(mb_context *ctx, const uint8_t *in, uint8_t *o
     ctx->launches++;
     return MB_SUCCESS;
   }
-  avgpool_u8_kernel<<<static_cast<unsigned>(ceil_div64(total, 256)), 256, 0, ctx->stream>>>(
-      in, out, static_cast<int>(N), static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
-      static_cast<int>(KH), static_cast<int>(KW), stride_h, stride_w, pad_top, pad_left,
-      static_cast<int>(Ho), static_cast<int>(Wo));
+  MB_CUDA(ctx, mb_launch_chained(ctx, avgpool_u8_kernel, dim3(static_cast<unsigned>(ceil_div64(total, 256))), dim3(256), 0, in,
+                                 out, static_cast<int>(N), static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
+                                 static_cast<int>(KH), static_cast<int>(KW), stride_h, stride_w, pad_top, pad_left,
+                                 static_cast<int>(Ho), static_cast<int>(Wo)));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
