@@ -261,7 +261,7 @@ static void launch_eltwise(mb_context *ctx, const EltParams &p, int vec4) {
 // gathered once so that several such convolutions of one tensor (a residual block's shortcut and its first convolution) can
 // run as plain 1x1 convolutions on the compact copy.  Bound by memory, which reads the kept rows
 // whole: a thread takes four neighbouring outputs of a row, with two 16-byte loads where the column stride is 2 and rows
-// are aligned (one output per thread and 64-bit divisions: 56 x 56 x 256, batch 256, 187 us; now SUBS_NOTE).
+// are aligned (one output per thread and 64-bit divisions: 56 x 56 x 256, batch 256, 187 us; now 111).
 __global__ void __launch_bounds__(256)
 subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t quads, int H, int W, int sh, int sw,
                      int Ho, int Wo, int vec) {
