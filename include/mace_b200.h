@@ -172,9 +172,8 @@ int mb_pair_clusters(const mb_context *ctx);
  * "dw_fixed_groups" (1 default: the TMA-fed 3x3 depthwise kernel takes a
  * variant that knows the number of channel groups per CTA at compile time;
  * 0 keeps the generic one, for A/B tests),
- * "dw_tma_fill" (4 default: that kernel's row runs are halved until the grid
- * has this many quarter-CTAs per SM, i.e. one CTA per SM; 8 = two per SM was
- * the earlier rule and 2.4 % slower on MobileNet-v1),
+ * "dw_tma_fill" (4 default: half this many CTAs per SM count as one round when
+ * that kernel's rows are cut into runs),
  * "dw_lane_setup" (1 default: a lane per input row requests that kernel's
  * row copies; 0: one thread does, for A/B tests),
  * "conv_filter_const" (0 default; 1 promises that filter and bias of the

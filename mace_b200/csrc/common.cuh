@@ -72,7 +72,7 @@ struct mb_context {
   int skinny_max_m = 16;         // row counts up to this take the streaming few-row GEMM
   int max_pair_clusters = 0;     // co-resident clusters of the pair GEMM (0: not asked yet)
   int stem_tc = 1;               // 3x3x3 first-layer convolution: the products on the tensor core
-  int dw_tma_fill = 4;           // TMA-fed depthwise: row runs are halved until the grid has this many quarter-CTAs per SM
+  int dw_tma_fill = 4;           // TMA-fed depthwise: half this many CTAs per SM count as a round when rows are cut into runs
   int gemm_b_const = 0;          // set around a GEMM whose B operand is a weight (see conv_filter_const)
   int b_prefetch = 1;            // such a GEMM asks for its first B tiles before it waits for its predecessor (0: A/B tests)
   int conv_filter_const = 0;     // promise: filter and bias of the following mb_conv2d_u8_nhwc calls are weights

@@ -673,13 +673,26 @@ static int dwconv_u8_impl(mb_context *ctx, const uint8_t *in, const uint8_t *fil
         t.chan_chunks = static_cast<int>(C / t.CB);
         const int row_bytes = t.TWB * t.CB;
         t.row_pitch = static_cast<int>(align_up(static_cast<size_t>(row_bytes), 128));
-        // output rows per CTA: what ~72 KB of input rows allow (two CTAs per SM), fewer when
-        // that would leave SMs without a CTA
-        const int max_rows_in = std::max(3, (72 * 1024) / t.row_pitch);
-        int rows_out = std::max(1, (max_rows_in - 3) / stride_h + 1);
-        rows_out = static_cast<int>(std::min<int64_t>(rows_out, Ho));
-        const int64_t per_seg = N * t.col_tiles * t.chan_chunks;
-        while (rows_out > 2 && per_seg * ceil_div64(Ho, rows_out) < static_cast<int64_t>(ctx->dw_tma_fill) * ctx->num_sms / 4) rows_out = (rows_out + 1) / 2;
+        // output rows per CTA: the number with the fewest rows in sequence, counted as rounds of CTAs (two fit an SM with
+        // up to 108 KB of input rows) x (rows + 4 for the start of a CTA).  Measured on MobileNet, against halving a run
+        // of 72 KB down to 2 rows until every SM had a CTA: batch 1, one row, 117 -> 107 us a pass; batch 96, 14 -> 19
+        // rows at 56 x 56, 372 -> 360.
+        const int64_t per_seg = N * t.col_tiles * t.chan_chunks, resident = std::max<int64_t>(1, static_cast<int64_t>(ctx->dw_tma_fill) * ctx->num_sms / 2);
+        const int max_rows_in = std::max(3, (108 * 1024) / t.row_pitch);
+        const int max_rows = static_cast<int>(std::min<int64_t>((max_rows_in - 3) / stride_h + 1, Ho));
+        int rows_out = per_seg * Ho <= resident ? 1 : max_rows;
+        if (rows_out > 1) {
+          int64_t best = -1;
+          for (int64_t segs = ceil_div64(Ho, max_rows); segs <= Ho; ++segs) {
+            const int64_t rows = ceil_div64(Ho, segs), rounds = ceil_div64(per_seg * ceil_div64(Ho, rows), resident);
+            const int64_t cost = rounds * (rows + 4);
+            if (best < 0 || cost < best) {
+              best = cost;
+              rows_out = static_cast<int>(rows);
+            }
+            if (rounds * 5 >= best && segs > 1) break;  // (more segments, no fewer rounds)
+          }
+        }
         t.rows_out = rows_out;
         t.segments = static_cast<int>(ceil_div64(Ho, rows_out));
         const int rows_in = (rows_out - 1) * stride_h + 3;
@@ -688,7 +701,7 @@ static int dwconv_u8_impl(mb_context *ctx, const uint8_t *in, const uint8_t *fil
         t.setup_lanes = ctx->dw_lane_setup ? 32 : 1;
         const size_t smem = static_cast<size_t>(t.ring_bytes) + sizeof(uint64_t) * rows_in + 128 /* alignment */;
         const int64_t grid64 = per_seg * t.segments;
-        if (smem <= 100 * 1024 && grid64 < (1ll << 31) && row_bytes % 16 == 0) {
+        if (smem <= 110 * 1024 && grid64 < (1ll << 31) && row_bytes % 16 == 0) {
           CUtensorMap tmap;
           const cuuint64_t dims[4] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(W),
                                       static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(N)};
@@ -712,7 +725,7 @@ static int dwconv_u8_impl(mb_context *ctx, const uint8_t *in, const uint8_t *fil
     auto kern = dwconv3x3_u8_tma_kernel<S, V, GT>;                                                          \
     const uint64_t bit = 1ull << (SLOT);                                                                    \
     if (!(ctx->dw_attr_mask & bit)) {                                                                       \
-      MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 101 * 1024));    \
+      MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 111 * 1024));    \
       ctx->dw_attr_mask |= bit;                                                                             \
     }                                                                                                       \
     MB_CUDA(ctx, mb_launch_chained(ctx, kern, dim3(static_cast<unsigned>(grid64)), dim3(DW_THREADS), smem,  \
