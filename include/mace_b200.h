@@ -57,6 +57,9 @@ int mb_host_free(mb_context *ctx, void *hptr);
 /* Asynchronous copies on the context's stream. */
 int mb_memcpy_h2d(mb_context *ctx, void *dst_dev, const void *src_host, size_t bytes);
 int mb_memcpy_d2h(mb_context *ctx, void *dst_host, const void *src_dev, size_t bytes);
+/* The same for a result that kernels further up the stream are still computing: small ones into
+ * page-locked memory are written by a kernel instead of the copy engine. */
+int mb_result_d2h(mb_context *ctx, void *dst, const void *src, size_t bytes);
 int mb_memset(mb_context *ctx, void *dst_dev, int value, size_t bytes);
 int mb_memcpy_d2d(mb_context *ctx, void *dst_dev, const void *src_dev, size_t bytes);
 /* Uploads that overlap the compute stream's work (double-buffered inputs): the

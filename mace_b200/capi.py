@@ -46,6 +46,7 @@ PROTOTYPES = {
     "mb_host_free": (_int, [_vp, _vp]),
     "mb_memcpy_h2d": (_int, [_vp, _vp, _vp, _sz]),
     "mb_memcpy_d2h": (_int, [_vp, _vp, _vp, _sz]),
+    "mb_result_d2h": (_int, [_vp, _vp, _vp, _sz]),
     "mb_memset": (_int, [_vp, _vp, _int, _sz]),
     "mb_memcpy_d2d": (_int, [_vp, _vp, _vp, _sz]),
     "mb_upload_h2d": (_int, [_vp, _vp, _vp, _sz]),

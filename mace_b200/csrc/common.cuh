@@ -51,6 +51,7 @@ struct mb_context {
   int cut_aligned = 0;           // aligned u8 products on the cluster-cut kernel: 0 by rule, 1 never, 2 always
   int cut_bn = 0, cut_splits = 0, cut_two = 0;  // cluster-cut GEMM: overrides of tile width, depth runs, CTAs per SM
                                  // (1 / 2; 3: convolutions on the persistent kernel) (0: by rule)
+  void *pointer_attributes = nullptr;  // cuPointerGetAttributes
   int f32_bn = 0, f32_splits = 0;  // self-fetching fp32 GEMM: overrides of tile width and depth runs (0: by rule)
   int f32_gather = 0;            // ... and of its use: 0 by rule, 1 never, 2 wherever it can run
   uint64_t f32_gather_attr_mask = 0;

@@ -45,6 +45,42 @@ int mb_scratch(mb_context *ctx, size_t bytes, void **ptr) {
   return MB_SUCCESS;
 }
 
+namespace {
+
+// Results to page-locked host memory, by a kernel that writes there itself: behind other kernels of a stream the copy engine
+// takes its turn only after a handshake.  MobileNet, batch 1, input to host result: 129.7 -> 124.9 us.  (For the input the
+// engine is as fast, on an idle stream 1 .. 3 us faster, and large results it writes faster: RESULT_KERNEL_BYTES.)
+constexpr size_t RESULT_KERNEL_BYTES = 64 << 10;
+
+__global__ void __launch_bounds__(256) result_copy_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, int bytes) {
+  // (no launch of dependents: like a copy, this kernel is a full barrier in the stream)
+  const int i = (blockIdx.x * 256 + threadIdx.x) * 16;
+  if (i + 16 <= bytes) {
+    *reinterpret_cast<uint4 *>(dst + i) = *reinterpret_cast<const uint4 *>(src + i);
+  } else {
+    for (int j = i; j < bytes; ++j) dst[j] = src[j];
+  }
+}
+
+// The device's address of [host, host + bytes) where all of it lies inside one page-locked, mapped range, else null.
+uint8_t *mapped_host(const mb_context *ctx, const void *host, size_t bytes) {
+  if (ctx->pointer_attributes == nullptr) return nullptr;
+  unsigned type = 0;
+  CUdeviceptr mapped = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *into[4] = {&type, &mapped, &start, &size};
+  typedef CUresult (*AttributesFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(host);
+  if (reinterpret_cast<AttributesFn>(ctx->pointer_attributes)(4, what, into, at) != CUDA_SUCCESS ||
+      type != CU_MEMORYTYPE_HOST || mapped == 0 || at < start || at - start + bytes > size)
+    return nullptr;
+  return reinterpret_cast<uint8_t *>(mapped);
+}
+
+}  // namespace
+
 extern "C" {
 
 int mb_init(int device, mb_context **out) {
@@ -95,6 +131,12 @@ int mb_init(int device, mb_context **out) {
     fn = nullptr;
   }
   ctx->encode_im2col = fn;
+  fn = nullptr;
+  if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
+      qres != cudaDriverEntryPointSuccess) {
+    fn = nullptr;
+  }
+  ctx->pointer_attributes = fn;
   *out = ctx;
   return MB_SUCCESS;
 }
@@ -216,6 +258,22 @@ int mb_memcpy_d2h(mb_context *ctx, void *dst, const void *src, size_t bytes) {
   MB_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost,
                                ctx->stream));
   return MB_SUCCESS;
+}
+
+int mb_result_d2h(mb_context *ctx, void *dst, const void *src, size_t bytes) {
+  if (ctx == nullptr || (bytes && (!dst || !src))) return MB_INVALID_ARGS;
+  if (bytes != 0 && bytes <= RESULT_KERNEL_BYTES && !ctx->capturing &&
+      ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0) {
+    uint8_t *mapped = mapped_host(ctx, dst, bytes);
+    if (mapped != nullptr && (reinterpret_cast<uintptr_t>(mapped) & 15u) == 0) {
+      result_copy_kernel<<<static_cast<unsigned>((bytes + 4095) / 4096), 256, 0, ctx->stream>>>(
+          mapped, static_cast<const uint8_t *>(src), static_cast<int>(bytes));
+      MB_CUDA(ctx, cudaGetLastError());
+      ctx->launches++;
+      return MB_SUCCESS;
+    }
+  }
+  return mb_memcpy_d2h(ctx, dst, src, bytes);
 }
 
 int mb_memcpy_d2d(mb_context *ctx, void *dst, const void *src, size_t bytes) {

@@ -315,7 +315,7 @@ int mbh_run_host(mbh_engine *e, const char *input_name, const void *host_in, siz
   if (out == nullptr) return MaceStatus::MACE_INVALID_ARGS;
   if (output_bytes != static_cast<size_t>(out->raw_size()))
     return Fail(e, MaceStatus::MACE_INVALID_ARGS, "output size does not match the output tensor");
-  MBH_TRY(e, e->runtime.Status(mb_memcpy_d2h(e->runtime.ctx(), host_out, out->memory<void>(), output_bytes)));
+  MBH_TRY(e, e->runtime.Status(mb_result_d2h(e->runtime.ctx(), host_out, out->memory<void>(), output_bytes)));
   MBH_TRY(e, e->runtime.Status(mb_stream_sync(e->runtime.ctx())));
   return MaceStatus::MACE_SUCCESS;
 }

@@ -288,7 +288,7 @@ MaceStatus MaceEngine::Run(const std::map<std::string, MaceTensor> &inputs, std:
       // the staging buffer is reused by the next output
       MACE_RETURN_IF_ERROR(runtime_.Status(mb_stream_sync(ctx)));
     } else {
-      MACE_RETURN_IF_ERROR(runtime_.Status(mb_memcpy_d2h(ctx, mt.data_.get(), t->memory<void>(), bytes)));
+      MACE_RETURN_IF_ERROR(runtime_.Status(mb_result_d2h(ctx, mt.data_.get(), t->memory<void>(), bytes)));
     }
   }
   return runtime_.Status(mb_stream_sync(ctx));

@@ -1,5 +1,7 @@
 """uint8 GEMV, Conv2D, DepthwiseConv2d and pooling on the GPU against the CPU oracle
 (bit-exact), including the reference's two quantized known-answer tests."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -700,3 +702,45 @@ def test_quantize_dequantize_minmax(ctx, orc, size):
     assert np.array_equal(ctx.download(dy, (size,), np.float32), orc.dequantize(acc, 3.7e-4, 0))
     for b in (dx, dq, dy, da):
         b.free()
+
+
+# one output row per CTA, runs cut by rounds of CTAs, the longest runs that shared memory holds
+@pytest.mark.parametrize("shape", [(1, 9, 13, 32, 1), (3, 14, 14, 512, 2), (24, 56, 56, 128, 1), (20, 113, 111, 64, 2)])
+def test_dwconv_u8_row_runs(ctx, orc, shape):
+    N, H, W, C, stride = shape
+    rng = np.random.Generator(np.random.PCG64(H + C))
+    x = rng.integers(0, 256, size=(N, H, W, C), dtype=np.uint8)
+    f = rng.integers(0, 256, size=(3, 3, C, 1), dtype=np.uint8)
+    bias = np.rint(rng.normal(0, 500, size=C)).astype(np.int32)
+    mult, shift = orc.output_multiplier_and_shift(np.float32(0.02), np.float32(0.01),
+                                                  np.float32(0.02 * 0.01 * 3 * 74 * 74 * 3 / 127))
+    Ho, Wo, ph, pw = orc.calc_padding_and_output_size(H, W, 3, 3, (1, 1), (stride, stride), PAD["SAME"])
+    args = ((stride, stride), (1, 1), (ph >> 1, pw >> 1), (Ho, Wo), 0, 121, mult, shift, 0)
+    exp = orc.dwconv_u8(x, f, bias, *args)
+    dx, df, db = ctx.upload(x), ctx.upload(f), ctx.upload(bias)
+    do = ctx.alloc(exp.size)
+    ctx.dwconv_u8(dx, df, db, do, N, H, W, C, 1, 3, 3, *args)
+    assert np.array_equal(ctx.download(do, exp.shape, np.uint8), exp)
+    for b in (dx, df, db, do):
+        b.free()
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+@pytest.mark.parametrize("size,offset", [(1, 0), (15, 0), (16, 0), (1000, 16), (4097, 0), (65536, 0), (65537, 0), (100, 3)])
+def test_result_copies(ctx, pinned, size, offset):
+    from mace_b200 import capi
+
+    lib = capi.lib()
+    src = np.random.Generator(np.random.PCG64(size)).integers(0, 256, size=size, dtype=np.uint8)
+    d = ctx.upload(src)
+    ptr = ctypes.c_void_p()
+    assert lib.mb_host_alloc(ctx.h, size + 64, ctypes.byref(ptr)) == 0
+    host = (np.ctypeslib.as_array((ctypes.c_uint8 * (size + 64)).from_address(ptr.value)) if pinned
+            else np.empty(size + 64, np.uint8))
+    host[:] = 7
+    assert lib.mb_result_d2h(ctx.h, host.ctypes.data + offset, d.ptr, size) == 0
+    ctx.sync()
+    assert np.array_equal(host[offset:offset + size], src)
+    assert (host[:offset] == 7).all() and (host[offset + size:] == 7).all()
+    assert lib.mb_host_free(ctx.h, ptr) == 0
+    d.free()
