@@ -13,11 +13,11 @@
 // holds its pixel's valid filter rows and columns as bit masks, so padding costs one logic instruction per value.
 // W comes by TMA where its rows are 16-byte aligned, else through registers, and is split in shared memory.
 //
-// Roles (18 warps): two groups of four load X, taking the steps in turn (two steps of loads in flight; a third group
+// Roles (18 or 22 warps): two groups of four load X, taking the steps in turn (two steps of loads in flight; a third group
 // gained nothing and cost 0.5 us per launch; fetching with 4-byte asynchronous copies through shared memory instead took
-// twice as long, 128 of them per step), four split W, four store results, one thread issues the MMAs, one requests W.  Persistent over the tiles; where these do not fill
-// the SMs, one tile per cluster of 2 .. 8 CTAs with the depth cut between them, the partial tiles added up through
-// distributed shared memory.
+// twice as long, 128 of them per step), four split W, four or eight store results, one thread issues the MMAs, one
+// requests W.  Persistent over the tiles; where these do not fill the SMs, one tile per cluster of 2 .. 8 CTAs with the
+// depth cut between them, the partial tiles added up through distributed shared memory.
 //
 // What bounds it: the tensor pipe at three tf32 MMAs per product for long depths (12 MMAs x 92 cycles per step of
 // 128 x 128 x 32; a convolution's loads bring the step to 1400), the launch, first loads and results for small shapes.
@@ -40,8 +40,10 @@ using namespace sm100;
 constexpr int BM = 128;         // pixels (m) per tile == TMEM lanes
 constexpr int KB = 32;          // depth per step
 constexpr int XGROUPS = 2;      // of four warps each, taking the steps in turn
-constexpr int FIRST_W = 4 * XGROUPS, FIRST_E = FIRST_W + 4, EWARPS = 4, MMA_WARP = FIRST_E + EWARPS, TMA_WARP = MMA_WARP + 1;
-constexpr int THREADS = (TMA_WARP + 1) * 32;
+constexpr int FIRST_W = 4 * XGROUPS, FIRST_E = FIRST_W + 4;
+// EW warps for results: four, or eight where a tile's results take longer than its steps (see make_plan); then the MMA
+// warp and the one that requests W
+constexpr int threads(int ew) { return (FIRST_E + ew + 2) * 32; }
 constexpr int ACCS = 2;
 constexpr long long WAIT_BUDGET = 1ll << 31;        // ~1 s of SM clocks per wait
 enum { W_TMA = 0, W_ROWS = 1, W_COLS = 2 };         // k contiguous and 16-byte aligned; k contiguous; n contiguous
@@ -121,11 +123,11 @@ __device__ __forceinline__ int64_t out_offset(const Params &p, int m, int b) {
   return b * p.c_bs + m * p.c_ms;
 }
 
-template <int BN, int XK, int WK>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int BN, int XK, int WK, int EW>
+__global__ void __launch_bounds__(threads(EW), 1)
 gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Params p) {
   using C = Cfg<BN>;
-  constexpr int STAGES = C::STAGES;
+  constexpr int STAGES = C::STAGES, MMA_WARP = FIRST_E + EW, TMA_WARP = MMA_WARP + 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -147,7 +149,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     if (WK == W_TMA) prefetch_tensormap(&map_w);
     for (int a = 0; a < ACCS; ++a) {
       mbar_init(tfull_bar + 8 * a, 1);
-      mbar_init(tempty_bar + 8 * a, EWARPS);
+      mbar_init(tempty_bar + 8 * a, EW);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -420,6 +422,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   } else {
     // ---- results: a lane per pixel, one channel after the other, 32 adjacent pixels per store ----
     const int quarter = warp & 3;
+    const int c_begin = (warp - FIRST_E) / 4 * (BN * 4 / EW), c_end = c_begin + BN * 4 / EW;  // of eight, half the channels each
     int local = 0;
     mb_grid_dep_wait();
     for (TileIter t(p); t.valid(p); t.next(p), ++local) {
@@ -435,7 +438,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         // from there, one peer after the other, it took 2.1 us)
         const int share = BN / p.splits;  // channels per CTA: 8 .. 64
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 8) {
+        for (int c = c_begin; c < c_end; c += 8) {
           uint32_t r[8], r2[8];
           tmem_ld_32x32b_x8(src + c, r);
           if (C::WIDE) tmem_ld_32x32b_x8(src + BN + c, r2);
@@ -454,10 +457,10 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       const int n0 = t.tn * BN;
       // the next chunk's accumulators are on their way while this one is stored
       uint32_t r[16], r2[16];
-      tmem_ld_32x32b_x16(src, r);
-      if (C::WIDE) tmem_ld_32x32b_x16(src + BN, r2);
-#pragma unroll
-      for (int c = 0; c < BN; c += 16) {
+      tmem_ld_32x32b_x16(src + c_begin, r);
+      if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c_begin, r2);
+#pragma unroll 1
+      for (int c = c_begin; c < c_end; c += 16) {
         tmem_ld_wait_x16(r);
         if (C::WIDE) tmem_ld_wait_x16(r2);
         // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
@@ -465,7 +468,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         float x[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) x[j] = C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
-        if (c + 16 < BN) {
+        if (c + 16 < c_end) {
           tmem_ld_32x32b_x16(src + c + 16, r);
           if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c + 16, r2);
         } else {
@@ -550,11 +553,11 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   }
 }
 
-template <int BN, int XK, int WK>
+template <int BN, int XK, int WK, int EW>
 int launch_cfg(mb_context *ctx, Params &p) {
   using C = Cfg<BN>;
-  auto kern = gemm_f32_gather_kernel<BN, XK, WK>;
-  constexpr uint64_t bit = (BN == 128 ? 9 : 0) + XK * 3 + WK;
+  auto kern = gemm_f32_gather_kernel<BN, XK, WK, EW>;
+  constexpr uint64_t bit = (EW == 8 ? 18 : 0) + (BN == 128 ? 9 : 0) + XK * 3 + WK;
   CUtensorMap map;
   if (WK == W_TMA) MB_RETURN_IF_ERROR(mb_make_map_w_f32(ctx, &map, p.W, p.K, p.N, p.w_bs != 0 ? p.batch : 1, p.w_ns, p.w_bs, BN));
   else memset(&map, 0, sizeof(map));
@@ -567,7 +570,7 @@ int launch_cfg(mb_context *ctx, Params &p) {
   p.step_m = slots % p.tiles_m;
   p.step_n = (slots / p.tiles_m) % p.tiles_n;
   p.step_b = (slots / p.tiles_m) / p.tiles_n;
-  MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), THREADS,
+  MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), threads(EW),
                                   C::SMEM_BYTES + (p.splits > 1 ? C::PART_BYTES : 0), p.splits, map, p));
   ctx->launches++;
   ctx->launches_tc++;
@@ -575,7 +578,7 @@ int launch_cfg(mb_context *ctx, Params &p) {
 }
 
 struct Plan {
-  int bn = 64, splits = 1;
+  int bn = 64, splits = 1, warps = 4;
   int64_t cost = -1;
 };
 
@@ -597,13 +600,18 @@ Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
       if (s > 1 && rounds > 1 && asked == 0) continue;  // (one tile per CTA: a second round would start from nothing)
       const int64_t steps = ceil_div64(k_blocks, s);
       const int64_t step = g.conv ? (w == 128 ? 1450 : 1200) : (w == 128 ? 1250 : 1100);
-      const int64_t results = (w == 128 ? 10000 : 5000) * (g.residual != nullptr ? 2 : 1);
-      const int64_t last = (w == 128 ? 4000 : 1500) + (g.residual != nullptr ? 2000 : 0);
+      const bool res = g.residual != nullptr;
+      int64_t results = (w == 128 ? 10600 : 5400) * (res ? 2 : 1);
+      // eight warps for results: where they bound a 128-wide tile (at 64 eight are no faster), or the launch is one round of
+      // few steps; not elsewhere, as the warps that load X then have too few registers
+      const bool eight = s == 1 && steps * step <= results && (w == 128 || rounds == 1);
+      if (eight && w == 128) results = res ? 16000 : 7000;
+      const int64_t last = (w == 128 ? 4000 : 1500) + (res ? 2000 : 0) - (eight ? 700 : 0);
       const int64_t cost = s == 1 ? 8000 + (rounds - 1) * std::max<int64_t>(steps * step, results) + steps * step + last
                            : w == 128 ? 10500 + steps * 1350 + last
                                       : (s == 2 ? 11500 : s == 4 ? 10500 : 11000) + steps * (s == 2 ? 1150 : 1050) + last;
       if (best.cost < 0 || cost < best.cost) {
-        best.bn = w; best.splits = s; best.cost = cost;
+        best.bn = w; best.splits = s; best.warps = eight ? 8 : 4; best.cost = cost;
       }
     }
   }
@@ -653,19 +661,30 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
     fast_div_make(static_cast<uint32_t>(p.KW), &p.kw_mul, &p.kw_shift);
     fast_div_make(static_cast<uint32_t>(p.hw), &p.hw_mul, &p.hw_shift);
     fast_div_make(static_cast<uint32_t>(p.Wo), &p.wo_mul, &p.wo_shift);
-    if (plan.bn == 128) return w_tma ? launch_cfg<128, X_CONV, W_TMA>(ctx, p) : launch_cfg<128, X_CONV, W_ROWS>(ctx, p);
-    return w_tma ? launch_cfg<64, X_CONV, W_TMA>(ctx, p) : launch_cfg<64, X_CONV, W_ROWS>(ctx, p);
+#define MB_F32_CONV(BN_, EW_) \
+  return w_tma ? launch_cfg<BN_, X_CONV, W_TMA, EW_>(ctx, p) : launch_cfg<BN_, X_CONV, W_ROWS, EW_>(ctx, p);
+    if (plan.warps == 8) {
+      if (plan.bn == 128) { MB_F32_CONV(128, 8) }
+      MB_F32_CONV(64, 8)
+    }
+    if (plan.bn == 128) { MB_F32_CONV(128, 4) }
+    MB_F32_CONV(64, 4)
+#undef MB_F32_CONV
   }
   const bool cols = g.x_ms != 1;
   p.x_vec = cols && (reinterpret_cast<uintptr_t>(g.X) & 15u) == 0 && g.x_ms % 4 == 0 && g.x_bs % 4 == 0 && g.K % 4 == 0;
-#define MB_F32_W(BN_, XK_)                                          \
-  if (w_nc) return launch_cfg<BN_, XK_, W_COLS>(ctx, p);            \
-  return w_tma ? launch_cfg<BN_, XK_, W_TMA>(ctx, p) : launch_cfg<BN_, XK_, W_ROWS>(ctx, p);
-#define MB_F32(BN_)                     \
-  if (cols) { MB_F32_W(BN_, X_COLS) }   \
-  MB_F32_W(BN_, X_ROWS)
-  if (plan.bn == 128) { MB_F32(128) }
-  MB_F32(64)
+#define MB_F32_W(BN_, XK_, EW_)                                           \
+  if (w_nc) return launch_cfg<BN_, XK_, W_COLS, EW_>(ctx, p);              \
+  return w_tma ? launch_cfg<BN_, XK_, W_TMA, EW_>(ctx, p) : launch_cfg<BN_, XK_, W_ROWS, EW_>(ctx, p);
+#define MB_F32(BN_, EW_)                   \
+  if (cols) { MB_F32_W(BN_, X_COLS, EW_) } \
+  MB_F32_W(BN_, X_ROWS, EW_)
+  if (plan.warps == 8) {
+    if (plan.bn == 128) { MB_F32(128, 8) }
+    MB_F32(64, 8)
+  }
+  if (plan.bn == 128) { MB_F32(128, 4) }
+  MB_F32(64, 4)
 #undef MB_F32
 #undef MB_F32_W
 }
