@@ -286,6 +286,25 @@ def test_dwconv_f32_rows(ctx, orc, k, stride, shape):
         b.free()
 
 
+@pytest.mark.parametrize("stride,shape", [
+    # one word per row, a multiplier, ragged runs of 2, 4 and 8 rows
+    (1, (1, 1, 5, 4, 1)), (2, (1, 1, 5, 4, 1)), (1, (2, 3, 7, 8, 2)), (2, (2, 3, 7, 8, 2)), (1, (4, 64, 57, 112, 1)),
+    (2, (9, 64, 111, 108, 1)), (2, (25, 64, 113, 112, 1)), (1, (7, 64, 113, 112, 1)), (1, (13, 64, 115, 112, 1))])
+def test_dwconv_f32_whole_words(ctx, orc, stride, shape):
+    N, C, H, W, mult = shape
+    rng = np.random.Generator(np.random.PCG64(N + W))
+    x = rng.standard_normal((N, C, H, W)).astype(np.float32)
+    f = rng.standard_normal((mult, C, 3, 3)).astype(np.float32)
+    bias = rng.standard_normal(C * mult).astype(np.float32)
+    ho, wo, ph, pw = orc.calc_padding_and_output_size(H, W, 3, 3, (1, 1), (stride, stride), 1)
+    ref = orc.dwconv_f32(x, f, bias, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
+    dx, df, db, do = ctx.upload(x), ctx.upload(f), ctx.upload(bias), ctx.alloc(ref.nbytes)
+    ctx.dwconv_f32(dx, df, db, do, N, C, H, W, mult, 3, 3, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
+    assert rel_err(ctx.download(do, ref.shape, np.float32), ref, 1e-5, "dwconv_f32") <= 1e-5
+    for b in (dx, df, db, do):
+        b.free()
+
+
 def test_dwconv_f32(ctx, orc, kats):
     k = kats["dwconv_f32_2x2_valid"]  # SimpleValidTest, depthwise_conv2d_test.cc:26-84
     x = np.transpose(np.array(k["input"], np.float32).reshape(1, 3, 3, 2), (0, 3, 1, 2)).copy()
