@@ -291,6 +291,22 @@ int mb_gemm_u8_tc_launch_float_rule(mb_context *ctx, const uint8_t *A, const uin
                                     int64_t N, int64_t K, int32_t zp_a, int32_t zp_b, float mult_f,
                                     int32_t zp_c, int add_zp);
 
+// Whether the GEMM takes several vectors, or one of ragged length, faster than the kernel with a warp per row.  SM cycles from
+// times at 128 .. 8192 rows, 333 .. 8001 columns, 1 .. 4 vectors.  The GEMV: 1.6 to 2 us around the rows; a ragged row
+// costs 120 cycles per 32 bytes and 4.5 more per row that its SM holds (489 rows of 642: 3.2 us against 7.2 as a GEMM; 489
+// of 8001: 18.0 against 9.9), an aligned one 12 per such row and 512 bytes, and 93 per vector.  The GEMM on ragged rows: 960 per
+// step of 128 columns and 64 rows (its estimate in the plan is for tiles that are full of vectors).
+static bool gemm_is_faster(const mb_context *ctx, const mb_cut_plan &plan, int64_t batch, int64_t rows, int64_t K,
+                           int64_t batch_chunk, bool vec) {
+  const int64_t per_sm = ceil_div64(rows, 8) * 8 * ceil_div64(batch, batch_chunk) / ctx->num_sms + 1;
+  const int64_t gemv = vec ? 3000 + batch_chunk * 93 * per_sm + 12 * per_sm * ceil_div64(K, 512)
+                           : 4000 + 2500 * (batch_chunk - 1) + batch_chunk * ceil_div64(K, 32) * (120 + per_sm * 9 / 2);
+  if (plan.by_tma) return plan.cost < gemv;
+  const int64_t tiles = ceil_div64(batch, 128) * ceil_div64(rows, plan.bn);
+  const int64_t rounds = ceil_div64(tiles * plan.splits, ctx->num_sms), steps = ceil_div64(ceil_div64(K, 128), plan.splits);
+  return 10500 + rounds * steps * (plan.bn == 128 ? 1250 : 960) < gemv;
+}
+
 extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rhs,
                           const int32_t *bias, void *out, int out_is_int32, int64_t batch,
                           int64_t rows, int64_t K, int lhs_batched, int rhs_batched,
@@ -354,6 +370,15 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
     ctx->launches++;
     return MB_SUCCESS;
   }
+  const bool vec = (K % 16 == 0) && K > 0 && K <= 32768 &&
+                   ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) & 15u) == 0;
+  // a shared matrix: split the batch so that at least ~4 blocks per SM exist
+  int64_t chunks = 1;
+  if (!lhs_batched) {
+    chunks = std::min<int64_t>(batch, std::max<int64_t>(1, (4ll * ctx->num_sms) / ceil_div64(rows, 8)));
+    chunks = std::min<int64_t>(chunks, 65535);
+  }
+  const int64_t batch_chunk = ceil_div64(batch, chunks);
   // Several vectors against one matrix, of any length: the GEMM that fetches its own operands (the matrix is
   // read once, its depth cut over clusters where the rows do not fill the SMs).
   if (!lhs_batched && (rhs_batched || batch == 1) && ctx->use_tensor_cores && (batch >= 2 || K % 16 != 0) &&
@@ -363,7 +388,7 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
     g.M = batch; g.N = rows; g.K = K; g.zp_a = zp_rhs; g.zp_b = zp_lhs;
     g.rq_variant = 8; g.mult_f = multiplier; g.zp_f = add_zp_out ? static_cast<float>(zp_out) : 0.f;
     const mb_cut_plan plan = mb_gemm_u8_cut_plan(ctx, g);
-    if (plan.cost >= 0) return mb_gemm_u8_cut_launch(ctx, g, plan);
+    if (plan.cost >= 0 && gemm_is_faster(ctx, plan, batch, rows, K, batch_chunk, vec)) return mb_gemm_u8_cut_launch(ctx, g, plan);
   }
   GemvParams p;
   p.lhs = lhs; p.rhs = rhs; p.bias = bias; p.out = out;
@@ -371,15 +396,7 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
   p.lhs_batched = lhs_batched; p.rhs_batched = rhs_batched;
   p.out_is_int32 = out_is_int32; p.add_zp_out = add_zp_out;
   p.zp_lhs = zp_lhs; p.zp_rhs = zp_rhs; p.zp_out = zp_out; p.multiplier = multiplier;
-  const bool vec = (K % 16 == 0) && K > 0 && K <= 32768 &&
-                   ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) & 15u) == 0;
-  // a shared matrix: split the batch so that at least ~4 blocks per SM exist
-  int64_t chunks = 1;
-  if (!lhs_batched) {
-    chunks = std::min<int64_t>(batch, std::max<int64_t>(1, (4ll * ctx->num_sms) / ceil_div64(rows, 8)));
-    chunks = std::min<int64_t>(chunks, 65535);
-  }
-  p.batch_chunk = static_cast<int>(ceil_div64(batch, chunks));
+  p.batch_chunk = static_cast<int>(batch_chunk);
   dim3 grid(static_cast<unsigned>(ceil_div64(rows, 8)),
             lhs_batched ? static_cast<unsigned>(batch)
                         : static_cast<unsigned>(ceil_div64(batch, p.batch_chunk)));
