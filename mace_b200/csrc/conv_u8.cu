@@ -702,7 +702,13 @@ extern "C" int mb_conv2d_u8_nhwc(mb_context *ctx, const uint8_t *in, const uint8
   // k x k on the tensor cores, the windows fetched by TMA as the GEMM goes (gemm_u8_cut.cu).  Channel counts that are
   // no multiple of 16 (or a misaligned input) are first copied to one that is: the added channels
   // hold the input zero point and add nothing whatever the filter side holds.
-  if (ctx->use_tensor_cores && pixels * O * depth > (1 << 18)) {
+  // The kernel with a thread per pixel is the alternative for small ones: 220 ns per value of the depth and 32 channels (55 per
+  // 8, for up to 16).  2 x 7 x 7 x 75 -> 49, 1x1 stride 2: 38.7 us there, 8.2 here; 8 x 8 x 4 -> 8, 3x3: 5.2 and 6.4.
+  const size_t direct_smem = static_cast<size_t>(depth) * O * sizeof(int16_t);
+  const bool direct_fits = direct_smem <= 32 * 1024 && depth <= 256;
+  const int64_t direct_cost = !direct_fits || pixels * O * depth > (1 << 18) ? INT64_MAX
+                              : O > 16 ? 5000 + 420 * depth * ceil_div64(O, 32) : 7500 + 105 * depth * ceil_div64(O, 8);
+  if (ctx->use_tensor_cores) {
     const int64_t Cp = static_cast<int64_t>(align_up(static_cast<size_t>(C), 16));
     const bool copy_in = Cp != C || (reinterpret_cast<uintptr_t>(in) & 15u) != 0;
     const bool copy_f = Cp != C || (reinterpret_cast<uintptr_t>(filter) & 15u) != 0;
@@ -717,7 +723,8 @@ extern "C" int mb_conv2d_u8_nhwc(mb_context *ctx, const uint8_t *in, const uint8
     g.H = p.H; g.W = p.W; g.C_in = static_cast<int>(Cp); g.KH = p.KH; g.KW = p.KW; g.sh = p.stride_h; g.sw = p.stride_w;
     g.pad_t = p.pad_top; g.pad_l = p.pad_left; g.Ho = p.Ho; g.Wo = p.Wo;
     const mb_cut_plan plan = mb_gemm_u8_cut_plan(ctx, g);
-    if (plan.cost >= 0 && in_bytes < (1ull << 33) && f_bytes < (1ull << 33)) {
+    if (plan.cost >= 0 && plan.cost + (copy_in || copy_f ? 4500 : 0) < direct_cost && in_bytes < (1ull << 33) &&
+        f_bytes < (1ull << 33)) {
       if (copy_in || copy_f) {
         uint8_t *scratch = nullptr;
         MB_RETURN_IF_ERROR(mb_scratch(ctx, in_bytes + f_bytes, reinterpret_cast<void **>(&scratch)));
@@ -729,8 +736,7 @@ extern "C" int mb_conv2d_u8_nhwc(mb_context *ctx, const uint8_t *in, const uint8
       return mb_gemm_u8_cut_launch(ctx, g, plan);
     }
   }
-  const size_t direct_smem = static_cast<size_t>(depth) * O * sizeof(int16_t);
-  if (direct_smem <= 32 * 1024 && depth <= 256) {
+  if (direct_fits) {
     const unsigned blocks = static_cast<unsigned>(ceil_div64(pixels, 128));
     if (O % 32 == 0 || O > 16) MB_CUDA(ctx, mb_launch_chained(ctx, conv_u8_direct_kernel<32>, dim3(blocks), dim3(128), direct_smem, p));
     else MB_CUDA(ctx, mb_launch_chained(ctx, conv_u8_direct_kernel<8>, dim3(blocks), dim3(128), direct_smem, p));
