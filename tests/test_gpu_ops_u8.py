@@ -744,3 +744,24 @@ def test_result_copies(ctx, pinned, size, offset):
     assert (host[:offset] == 7).all() and (host[offset + size:] == 7).all()
     assert lib.mb_host_free(ctx.h, ptr) == 0
     d.free()
+
+
+# either side of the line between the thread-per-pixel kernel and the GEMM over windows
+@pytest.mark.parametrize("case", [(2, 7, 7, 75, 49, 1, 2, "VALID"), (3, 7, 7, 16, 32, 3, 2, "SAME"), (1, 4, 4, 32, 16, 3, 1, "SAME"),
+                                  (1, 8, 8, 4, 8, 3, 1, "SAME"), (1, 8, 8, 24, 8, 1, 2, "VALID"), (1, 3, 3, 16, 16, 1, 2, "VALID")])
+def test_conv2d_u8_small(ctx, orc, case):
+    N, H, W, C, O, k, stride, pad = case
+    _conv_case(ctx, orc, N, H, W, C, O, k, k, stride, pad)
+
+
+# a few rows against a row-major matrix of short depth
+@pytest.mark.parametrize("M,N,K", [(1, 512, 256), (3, 864, 256), (16, 864, 128), (16, 4096, 256)])
+def test_gemm_u8_few_rows_short_depth(ctx, M, N, K):
+    rng = np.random.Generator(np.random.PCG64(M + N))
+    a, b = rng.integers(0, 256, size=(M, K), dtype=np.uint8), rng.integers(0, 256, size=(K, N), dtype=np.uint8)
+    da, db, dc = ctx.upload(a), ctx.upload(b), ctx.alloc(M * N * 4)
+    ctx.gemm_u8(da, db, None, dc, 1, M, N, K, 7, 9, out_int32=True)
+    exp = (a.astype(np.int64) - 7) @ (b.astype(np.int64) - 9)
+    assert np.array_equal(ctx.download(dc, (M, N), np.int32), exp)
+    for x in (da, db, dc):
+        x.free()
