@@ -103,40 +103,42 @@ gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs, co
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
-  const int64_t b0 = static_cast<int64_t>(blockIdx.y) * VECS;
-  const float *lp = lhs + (lhs_batched ? b0 * rows * K : 0) + row * K;
-  const float *rp = rhs + (rhs_batched ? b0 * K : 0);
-  const int vecs = static_cast<int>(min(static_cast<int64_t>(VECS), batch - b0));
-  float s[VECS];
+  // (a grid has at most 65535 blocks along y; what the batch has beyond them is a further pass)
+  for (int64_t b0 = static_cast<int64_t>(blockIdx.y) * VECS; b0 < batch; b0 += static_cast<int64_t>(gridDim.y) * VECS) {
+    const float *lp = lhs + (lhs_batched ? b0 * rows * K : 0) + row * K;
+    const float *rp = rhs + (rhs_batched ? b0 * K : 0);
+    const int vecs = static_cast<int>(min(static_cast<int64_t>(VECS), batch - b0));
+    float s[VECS];
 #pragma unroll
-  for (int v = 0; v < VECS; ++v) s[v] = 0.f;
-  if (VEC4) {
+    for (int v = 0; v < VECS; ++v) s[v] = 0.f;
+    if (VEC4) {
 #pragma unroll 4
-    for (int64_t i = lane * 4; i < K; i += 128) {
-      const float4 a = __ldg(reinterpret_cast<const float4 *>(lp + i));
+      for (int64_t i = lane * 4; i < K; i += 128) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(lp + i));
 #pragma unroll
-      for (int v = 0; v < VECS; ++v) {
-        if (v < vecs) {
-          const float4 x = __ldg(reinterpret_cast<const float4 *>(rp + v * K + i));
-          s[v] = fmaf(a.x, x.x, s[v]); s[v] = fmaf(a.y, x.y, s[v]);
-          s[v] = fmaf(a.z, x.z, s[v]); s[v] = fmaf(a.w, x.w, s[v]);
+        for (int v = 0; v < VECS; ++v) {
+          if (v < vecs) {
+            const float4 x = __ldg(reinterpret_cast<const float4 *>(rp + v * K + i));
+            s[v] = fmaf(a.x, x.x, s[v]); s[v] = fmaf(a.y, x.y, s[v]);
+            s[v] = fmaf(a.z, x.z, s[v]); s[v] = fmaf(a.w, x.w, s[v]);
+          }
         }
       }
-    }
-  } else {
+    } else {
 #pragma unroll 4
-    for (int64_t i = lane; i < K; i += 32) {
-      const float a = __ldg(lp + i);
+      for (int64_t i = lane; i < K; i += 32) {
+        const float a = __ldg(lp + i);
 #pragma unroll
-      for (int v = 0; v < VECS; ++v)
-        if (v < vecs) s[v] = fmaf(a, __ldg(rp + v * K + i), s[v]);
+        for (int v = 0; v < VECS; ++v)
+          if (v < vecs) s[v] = fmaf(a, __ldg(rp + v * K + i), s[v]);
+      }
     }
-  }
 #pragma unroll
-  for (int v = 0; v < VECS; ++v) {
+    for (int v = 0; v < VECS; ++v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s[v] += __shfl_xor_sync(0xffffffffu, s[v], o);
-    if (lane == 0 && v < vecs) out[(b0 + v) * rows + row] = s[v] + (bias != nullptr ? __ldg(bias + row) : 0.f);
+      for (int o = 16; o > 0; o >>= 1) s[v] += __shfl_xor_sync(0xffffffffu, s[v], o);
+      if (lane == 0 && v < vecs) out[(b0 + v) * rows + row] = s[v] + (bias != nullptr ? __ldg(bias + row) : 0.f);
+    }
   }
 }
 
@@ -467,8 +469,8 @@ int mb_gemv_f32(mb_context *ctx, const float *lhs, const float *rhs, const float
   }
   const bool shared = !lhs_batched && rhs_batched;  // (one matrix, several vectors: up to eight per pass)
   const int vecs = !shared || batch == 1 ? 1 : batch == 2 ? 2 : batch <= 4 ? 4 : 8;
-  if (ceil_div64(batch, vecs) > 65535) return mb_fail(ctx, MB_UNSUPPORTED, "mb_gemv_f32: batch too large");
-  const dim3 grid(static_cast<unsigned>(ceil_div64(rows, 8)), static_cast<unsigned>(ceil_div64(batch, vecs)));
+  const dim3 grid(static_cast<unsigned>(ceil_div64(rows, 8)),
+                  static_cast<unsigned>(std::min<int64_t>(ceil_div64(batch, vecs), 65535)));
   const bool vec4 = K % 4 == 0 && ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) & 15u) == 0;
 #define MB_GEMV(V_)                                                                                                   \
   MB_CUDA(ctx, vec4 ? mb_launch_chained(ctx, gemv_f32_kernel<V_, true>, grid, dim3(256), 0, lhs, rhs, bias, out, batch, \

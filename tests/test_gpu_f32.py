@@ -103,6 +103,24 @@ def test_gemv_f32(ctx, orc, shape):
     assert rel_err(ctx.download(do, (batch * rows,), np.float32), ref, 1e-4, "gemv_f32") <= 1e-4
 
 
+@pytest.mark.parametrize("batch", [65535, 65536, 140001])
+@pytest.mark.parametrize("K", [5, 8])
+def test_gemv_f32_matrix_per_entry_many_entries(ctx, batch, K):
+    """A matrix per batch entry, more entries than a grid has blocks along y.  A sum of K <= 8 rounded products differs
+    from the exact one by at most K + 1 units of 2^-24 of the products' absolute sum."""
+    rows = 3
+    rng = np.random.Generator(np.random.PCG64(batch))
+    lhs = rng.standard_normal((batch, rows, K)).astype(np.float32)
+    rhs = rng.standard_normal((batch, K)).astype(np.float32)
+    dl, dr, do = ctx.upload(lhs), ctx.upload(rhs), ctx.alloc(batch * rows * 4)
+    ctx.gemv_f32(dl, dr, None, do, batch, rows, K, lhs_batched=True)
+    got = ctx.download(do, (batch, rows), np.float32)
+    terms = lhs.astype(np.float64) * rhs[:, None, :]
+    assert (np.abs(got - terms.sum(-1)) <= (K + 1) * 2.0 ** -24 * np.abs(terms).sum(-1)).all()
+    for b in (dl, dr, do):
+        b.free()
+
+
 def _conv_inputs(shape, fshape, seed):
     rng = np.random.Generator(np.random.PCG64(seed))
     x = rng.random(shape, dtype=np.float32)
