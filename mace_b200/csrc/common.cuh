@@ -54,7 +54,7 @@ struct mb_context {
   void *pointer_attributes = nullptr;  // cuPointerGetAttributes
   int f32_bn = 0, f32_splits = 0;  // self-fetching fp32 GEMM: overrides of tile width and depth runs (0: by rule)
   int f32_gather = 0;            // ... and of its use: 0 by rule, 1 never, 2 wherever it can run
-  uint64_t f32_gather_attr_mask = 0;
+  uint64_t f32_gather_attr_mask[2] = {0, 0};  // its kernels whose shared-memory limit was raised
   int cut_clusters[4] = {0, 0, 0, 0};  // CTAs of clusters of 2 / 4 / 8 that are resident at once, one CTA per SM (0: not asked)
   uint64_t cut_attr_mask = 0;    // kernels of gemm_u8_cut.cu / gemm_u8_gather.cu whose shared-memory limit was raised
   uint64_t func_attr_mask_plain = 0;  // the same for the GEMM's plain-store instances

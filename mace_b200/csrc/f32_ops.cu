@@ -25,9 +25,15 @@ int mb_dwconv_f32_launch(mb_context *ctx, const float *in, const float *filter, 
 
 namespace {
 
-// ---- GEMM: 64 x 64 tile per 256-thread block, 4 x 4 outputs per thread ----------
+// ---- GEMM: 64 x 64 tile per 128-thread block, 4 x 8 outputs per thread, one chain of FMAs in the order of k --------
+// What the tensor cores cannot take with this accuracy: products of depth below 48 and from 65 to 71 in a layout that TMA does
+// not take (mb_f32_gather_run).  Bound by latency: 12 warps per SM at best, of which 0.6 per scheduler are ready (FMA pipe 41 %
+// busy); a panel of 32 k is on its way to registers while the one before is multiplied.  Measured, a panel of 16 k loaded,
+// waited for and multiplied by 256 threads -> now: 16 x 16 x 16 4.2 -> 2.9 us, 64 x 64 x 64 9.3 -> 4.2, 384 x 384 x 64, batch 12,
+// 21.7 -> 10.9, 1536 x 1536 x 16 10.2 -> 4.7.
 constexpr int FT = 64;
-constexpr int FK = 16;
+constexpr int FK = 32;
+constexpr int FP = FT + 4;  // row pitch of a panel
 
 struct GemmF32Params {
   const float *A, *B;
@@ -40,53 +46,120 @@ struct GemmF32Params {
   float max_limit, coef;
 };
 
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmF32Params p) {
-  mb_grid_dep_launch();
-  mb_grid_dep_wait();
-  __shared__ float As[FK][FT + 4];
-  __shared__ float Bs[FK][FT + 4];
+// One thread's 16 values of a 64 x 32 panel.  Contiguous along k, a warp takes 4 rows x 8 k at a time: 32-byte sectors of
+// the operand, all banks of the panel; else 32 rows of one k.
+template <bool ALONG_K>
+struct PanelThread {
+  static constexpr int ROWS = ALONG_K ? 4 : 2;  // rows of this thread, 16 / ROWS values of each
+  const float *src;                             // its first row at its first k
+  int64_t rs, ks;
+  int row0, k0;
+  uint32_t in;
+  __device__ __forceinline__ PanelThread(const float *base, int64_t rows, int64_t first, int64_t rs_, int64_t ks_)
+      : rs(ALONG_K ? 4 * rs_ : 32), ks(ALONG_K ? 8 : ks_), in(0) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    row0 = ALONG_K ? warp * 16 + (lane >> 3) : lane;
+    k0 = ALONG_K ? lane & 7 : warp * 8;
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) in |= (first + row0 + q * (ALONG_K ? 4 : 32) < rows ? 1u : 0u) << q;
+    src = base + (first + row0) * rs_ + k0 * ks_;
+  }
+  __device__ __forceinline__ void load(float (&v)[16], int64_t kb, int64_t K) const {
+    const float *at = src + kb * (ALONG_K ? 1 : ks);
+    const int left = static_cast<int>(min(K - kb - k0, static_cast<int64_t>(FK)));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int q = i % ROWS, j = i / ROWS;
+      v[i] = (in >> q & 1u) != 0 && j * (ALONG_K ? 8 : 1) < left ? at[q * rs + j * ks] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void store(const float (&v)[16], float (*panel)[FP]) const {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int q = i % ROWS, j = i / ROWS;
+      panel[k0 + j * (ALONG_K ? 8 : 1)][row0 + q * (ALONG_K ? 4 : 32)] = v[i];
+    }
+  }
+};
+
+// Two FMAs per instruction, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t twice(float v) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+
+__device__ __forceinline__ void panel_fma(uint64_t (&acc)[4][4], const float *a, const float *b) {
+  const float4 a4 = *reinterpret_cast<const float4 *>(a);
+  const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(b), b1 = *reinterpret_cast<const ulonglong2 *>(b + 32);
+  const uint64_t av[4] = {twice(a4.x), twice(a4.y), twice(a4.z), twice(a4.w)}, bv[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) fma2(acc[i][j], av[i], bv[j]);
+}
+
+// AK, BK: the operand is contiguous along k (else along its rows, the columns of B)
+template <bool AK, bool BK>
+__global__ void __launch_bounds__(128) gemm_f32_kernel(const GemmF32Params p) {
+  __shared__ __align__(16) float As[2][FK][FP];
+  __shared__ __align__(16) float Bs[2][FK][FP];
   const int b = blockIdx.z;
   const int64_t m0 = static_cast<int64_t>(blockIdx.y) * FT, n0 = static_cast<int64_t>(blockIdx.x) * FT;
-  const float *A = p.A + b * p.a_bs, *B = p.B + b * p.b_bs;
+  const PanelThread<AK> pa(p.A + b * p.a_bs, p.M, m0, p.a_rs, p.a_cs);
+  const PanelThread<BK> pb(p.B + b * p.b_bs, p.N, n0, p.b_cs, p.b_rs);
   float *C = p.C + b * p.c_bs;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float acc[4][4] = {};
-  for (int64_t k0 = 0; k0 < p.K; k0 += FK) {
-    for (int i = threadIdx.x; i < FK * FT; i += 256) {
-      int kk, mm;
-      if (p.a_cs == 1) { kk = i % FK; mm = i / FK; } else { mm = i % FT; kk = i / FT; }
-      const int64_t m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < p.M && k < p.K) ? __ldg(A + m * p.a_rs + k * p.a_cs) : 0.f;
-      int nn;
-      if (p.b_cs == 1) { nn = i % FT; kk = i / FT; } else { kk = i % FK; nn = i / FK; }
-      const int64_t n = n0 + nn, kb = k0 + kk;
-      Bs[kk][nn] = (n < p.N && kb < p.K) ? __ldg(B + kb * p.b_rs + n * p.b_cs) : 0.f;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+  uint64_t acc2[4][4] = {};  // pairs of columns
+  float va[16], vb[16];
+  mb_grid_dep_launch();
+  mb_grid_dep_wait();
+  pa.load(va, 0, p.K);
+  pb.load(vb, 0, p.K);
+  int buf = 0;
+  for (int64_t k0 = 0; k0 < p.K; k0 += FK, buf ^= 1) {
+    pa.store(va, As[buf]);
+    pb.store(vb, Bs[buf]);
+    __syncthreads();  // (a thread is at most one panel ahead of the slowest, in the other buffer)
+    if (k0 + FK < p.K) {
+      pa.load(va, k0 + FK, p.K);
+      pb.load(vb, k0 + FK, p.K);
     }
-    __syncthreads();
+    const float *ap = &As[buf][0][ty * 4], *bp = &Bs[buf][0][tx * 4];
+    if (k0 + FK <= p.K) {
 #pragma unroll
-    for (int kk = 0; kk < FK; ++kk) {
-      const float4 a4 = *reinterpret_cast<const float4 *>(&As[kk][ty * 4]);
-      const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[kk][tx * 4]);
-      const float a[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], bv[j], acc[i][j]);
+      for (int kk = 0; kk < FK; ++kk) panel_fma(acc2, ap + kk * FP, bp + kk * FP);
+    } else {
+      for (int kk = 0; kk < static_cast<int>(p.K - k0); ++kk) panel_fma(acc2, ap + kk * FP, bp + kk * FP);
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int64_t m = m0 + ty * 4 + i;
     if (m >= p.M) continue;
-    const float bv = p.bias != nullptr ? p.bias[m] : 0.f;
+    float acc[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t n = n0 + tx * 4 + j;
-      if (n >= p.N) continue;
-      float v = acc[i][j];
-      if (p.bias != nullptr) v += bv;
-      C[m * p.c_rs + n * p.c_cs] = mb_activate(v, p.act, p.max_limit, p.coef);
+    for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * j]), "=f"(acc[2 * j + 1]) : "l"(acc2[i][j]));
+    if (p.bias != nullptr) {
+      const float bv = p.bias[m];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += bv;
+    }
+    mb_activate_n(acc, p.act, p.max_limit, p.coef);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t n = n0 + h * 32 + tx * 4;
+      float *dst = C + m * p.c_rs + n * p.c_cs;
+      if (p.c_cs == 1 && n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        *reinterpret_cast<float4 *>(dst) = make_float4(acc[h * 4], acc[h * 4 + 1], acc[h * 4 + 2], acc[h * 4 + 3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (n + j < p.N) dst[j * p.c_cs] = acc[h * 4 + j];
+      }
     }
   }
 }
@@ -275,10 +348,14 @@ unmerge_f32_kernel(const float *__restrict__ src, float *__restrict__ dst, int64
 }  // namespace
 
 // Whether the kernel that fetches its own operands takes a product (see gemm_f32_gather.cu); by_tma: the TMA-fed one of
-// gemm_f32_tc.cu could.
-static bool take_gather(mb_context *ctx, const mb_f32_gemm &g, bool by_tma) {
+// gemm_f32_tc.cu could; fp32_accuracy: the error may not be larger than that of fp32 FMAs, which is so for the products that
+// no other tensor-core route can take.
+static bool take_gather(mb_context *ctx, mb_f32_gemm &g, bool by_tma, bool fp32_accuracy) {
+  if (fp32_accuracy) g.run = mb_f32_gather_run(g.K);
   if (ctx->f32_gather == 1 || !mb_gemm_f32_gather_supported(ctx, g)) return false;
-  if (ctx->f32_gather == 2 || !by_tma) return true;
+  if (ctx->f32_gather == 2) return true;
+  if (fp32_accuracy && g.run == 0) return false;
+  if (!by_tma) return true;
   // The TMA-fed kernel: tiles of 128 columns of one image (or matrix), 1200 cycles per step, 2.6 us for the results of 128
   // channels (twice that with a residual), 4.4 us around them.
   const int64_t images = g.conv ? g.M / (static_cast<int64_t>(g.Ho) * g.Wo) : g.batch;
@@ -292,6 +369,23 @@ static bool take_gather(mb_context *ctx, const mb_f32_gemm &g, bool by_tma) {
     if (tma < 0 || cost < tma) tma = cost;
   }
   return mb_gemm_f32_gather_cost(ctx, g) < tma;
+}
+
+// A 1x1 convolution whose input is the product's operand as it lies ...
+static bool pointwise_in_place(int64_t KH, int64_t KW, int sh, int sw, int pad_t, int pad_l, int64_t H, int64_t W, int64_t Ho,
+                               int64_t Wo) {
+  return KH == 1 && KW == 1 && sh == 1 && sw == 1 && pad_t == 0 && pad_l == 0 && Ho == H && Wo == W;
+}
+// ... and with rows that fill the TMA-fed kernel's tiles.
+static bool long_rows(int64_t hw) { return hw % 4 == 0 && hw >= 128; }
+
+// Other convolutions of at least this much work go to the tensor cores by way of a column matrix (where the kernel that
+// fetches its own operands cannot run); smaller ones stay on the one-thread-per-output kernel.
+constexpr int64_t COLUMN_MIN_WORK = 1 << 18, COLUMN_MIN_POSITIONS = 32;
+
+static bool column_route(int64_t N, int64_t C, int64_t O, int64_t KH, int64_t KW, int64_t Ho, int64_t Wo) {
+  return N * O * Ho * Wo * C * KH * KW >= COLUMN_MIN_WORK && Ho * Wo * N >= COLUMN_MIN_POSITIONS && C * KH <= 65535 &&
+         Ho * Wo < (1ll << 30);
 }
 
 // The convolution as that kernel sees it.
@@ -332,15 +426,17 @@ int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *
   g.act = act; g.max_limit = max_limit; g.coef = coef;
   const bool by_tma = a_cs == 1 && b_cs == 1 && c_cs == 1 &&
                       mb_gemm_f32_tc_supported(ctx, B, A, N, M, K, b_rs, b_bs, a_rs, a_bs);
-  if (take_gather(ctx, g, by_tma)) return mb_gemm_f32_gather_launch(ctx, g);
+  if (take_gather(ctx, g, by_tma, !by_tma)) return mb_gemm_f32_gather_launch(ctx, g);
   // C = A * B with A [M x K] k-contiguous, B [K x N] n-contiguous and C n-contiguous is the
   // tensor-core kernel's layout with the roles X = B (pixels x channels side), W = A.
   if (by_tma) {
     return mb_gemm_f32_tc_launch(ctx, B, A, bias_per_row, C, batch, N, M, K, b_rs, b_bs, a_rs, a_bs,
                                  c_rs, c_bs, act, max_limit, coef, nullptr);
   }
-  if (batch > 65535 || ceil_div64(M, FT) > 65535)
+  if (batch > 65535 || ceil_div64(M, FT) > 65535) {
+    if (ctx->f32_gather != 1 && mb_gemm_f32_gather_supported(ctx, g)) return mb_gemm_f32_gather_launch(ctx, g);
     return mb_fail(ctx, MB_UNSUPPORTED, "fp32 GEMM: batch or M too large for this kernel");
+  }
   GemmF32Params p;
   p.A = A; p.B = B; p.C = C; p.bias = bias_per_row;
   p.M = M; p.N = N; p.K = K;
@@ -349,7 +445,9 @@ int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *
   p.act = act; p.max_limit = max_limit; p.coef = coef;
   dim3 grid(static_cast<unsigned>(ceil_div64(N, FT)), static_cast<unsigned>(ceil_div64(M, FT)),
             static_cast<unsigned>(batch));
-  MB_CUDA(ctx, mb_launch_chained(ctx, gemm_f32_kernel, dim3(grid), dim3(256), 0, p));
+  auto kern = a_cs == 1 ? (b_rs == 1 ? gemm_f32_kernel<true, true> : gemm_f32_kernel<true, false>)
+                        : (b_rs == 1 ? gemm_f32_kernel<false, true> : gemm_f32_kernel<false, false>);
+  MB_CUDA(ctx, mb_launch_chained(ctx, kern, grid, dim3(128), 0, p));
   MB_CUDA(ctx, cudaGetLastError());
   ctx->launches++;
   return MB_SUCCESS;
@@ -458,14 +556,17 @@ int mb_gemv_f32(mb_context *ctx, const float *lhs, const float *rhs, const float
   if (lhs == nullptr || rhs == nullptr || out == nullptr)
     return mb_fail(ctx, MB_INVALID_ARGS, "mb_gemv_f32: null operand");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  if (!lhs_batched && rhs_batched && (batch > 8 || ctx->f32_gather == 2)) {
-    // the vectors are the tensor core's M, the matrix its N (up to eight vectors share a pass of the CUDA-core kernel)
+  // Whole groups of 32 and more vectors against one matrix: the vectors are the tensor core's M, the matrix its N.  Fewer,
+  // and ragged ones, keep the accuracy of the CUDA-core kernel (a sum per lane, then over the lanes: 4e-8 to 2e-7 where the
+  // tensor cores' shortest runs give 1.3e-7 to 2e-7), in which up to eight vectors share a pass over the matrix.
+  const bool whole = batch >= 32 && batch % 4 == 0 && K % 4 == 0 && rows >= 16 && (reinterpret_cast<uintptr_t>(lhs) & 15u) == 0;
+  if (!lhs_batched && rhs_batched && (whole || ctx->f32_gather == 2)) {
     mb_f32_gemm g;
     g.X = rhs; g.x_ks = 1; g.x_ms = K;
     g.W = lhs; g.w_ns = K; g.w_ks = 1;
     g.bias = bias; g.C = out; g.c_ns = 1; g.c_ms = rows;
     g.M = batch; g.N = rows; g.K = K;
-    if (take_gather(ctx, g, false)) return mb_gemm_f32_gather_launch(ctx, g);
+    if (take_gather(ctx, g, false, false)) return mb_gemm_f32_gather_launch(ctx, g);
   }
   const bool shared = !lhs_batched && rhs_batched;  // (one matrix, several vectors: up to eight per pass)
   const int vecs = !shared || batch == 1 ? 1 : batch == 2 ? 2 : batch <= 4 ? 4 : 8;
@@ -516,16 +617,16 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
                                     Wo, activation, &empty));
   if (empty) return MB_SUCCESS;
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  const bool pointwise = KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 && Ho == H && Wo == W;
+  const bool pointwise = pointwise_in_place(KH, KW, stride_h, stride_w, pad_top, pad_left, H, W, Ho, Wo);
   {
-    const mb_f32_gemm g = conv_gemm(in, filter, bias, nullptr, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h,
-                                    dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);
-    if (N * O * Ho * Wo * C * KH * KW >= (1ll << 16) &&
-        take_gather(ctx, g, pointwise && (H * W) % 4 == 0 && H * W >= 128 &&
-                                mb_gemm_f32_tc_supported(ctx, in, filter, H * W, O, C, H * W, C * H * W, C, 0)))
+    const bool by_tma = pointwise && long_rows(H * W) && mb_gemm_f32_tc_supported(ctx, in, filter, H * W, O, C, H * W, C * H * W, C, 0);
+    const bool on_cores = pointwise && long_rows(H * W) ? !by_tma : !column_route(N, C, O, KH, KW, Ho, Wo);
+    mb_f32_gemm g = conv_gemm(in, filter, bias, nullptr, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h, dil_w, pad_top,
+                              pad_left, Ho, Wo, activation, max_limit, coefficient);
+    if (N * O * Ho * Wo * C * KH * KW >= (1ll << 16) && take_gather(ctx, g, by_tma, on_cores))
       return mb_gemm_f32_gather_launch(ctx, g);
   }
-  if (pointwise && ((H * W) % 4 == 0 && H * W >= 128 || !ctx->use_tensor_cores)) {
+  if (pointwise && (long_rows(H * W) || !ctx->use_tensor_cores)) {
     // out_n[O x HW] = filter[O x C] * in_n[C x HW] for every image n
     // (arm::Conv2dK1x1, mace/ops/arm/base/conv_2d_1x1.cc:61-68)
     const int64_t hw = H * W;
@@ -534,8 +635,7 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
   }
   // enough work to fill tensor-core tiles: gather columns and multiply; tiny problems stay on
   // the one-thread-per-output kernel
-  if (N * O * Ho * Wo * C * KH * KW >= (1ll << 18) && Ho * Wo * N >= 32 && C * KH <= 65535 &&
-      Ho * Wo < (1ll << 30)) {
+  if (column_route(N, C, O, KH, KW, Ho, Wo)) {
     return conv2d_f32_im2col(ctx, in, filter, bias, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h,
                              dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);
   }
@@ -569,19 +669,14 @@ int mb_conv2d_f32_nchw_residual(mb_context *ctx, const float *in, const float *f
   if (empty) return MB_SUCCESS;
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
   const int64_t hw = H * W;
-  {
-    const mb_f32_gemm g = conv_gemm(in, filter, bias, residual, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h,
-                                    dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);
-    if (take_gather(ctx, g, KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 && Ho == H &&
-                                Wo == W && hw % 4 == 0 && hw >= 128 &&
-                                mb_gemm_f32_tc_supported(ctx, in, filter, hw, O, C, hw, C * hw, C, 0)))
-      return mb_gemm_f32_gather_launch(ctx, g);
-  }
+  const bool pointwise_rows = pointwise_in_place(KH, KW, stride_h, stride_w, pad_top, pad_left, H, W, Ho, Wo) && long_rows(hw);
+  const bool by_tma = pointwise_rows && mb_gemm_f32_tc_supported(ctx, in, filter, hw, O, C, hw, C * hw, C, 0);
+  const bool on_cores = pointwise_rows ? !by_tma : !column_route(N, C, O, KH, KW, Ho, Wo);
+  mb_f32_gemm g = conv_gemm(in, filter, bias, residual, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h, dil_w, pad_top,
+                            pad_left, Ho, Wo, activation, max_limit, coefficient);
+  if (take_gather(ctx, g, by_tma, on_cores)) return mb_gemm_f32_gather_launch(ctx, g);
   // 1x1 stride 1 on the tensor cores: the sum and the activation ride in the GEMM's epilogue
-  if (KH == 1 && KW == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 && pad_left == 0 && Ho == H &&
-      Wo == W && hw % 4 == 0 && hw >= 128 &&
-      mb_gemm_f32_tc_supported(ctx, in, filter, hw, O, C, hw, C * hw, C, 0) &&
-      (reinterpret_cast<uintptr_t>(residual) & 3u) == 0) {
+  if (by_tma && (reinterpret_cast<uintptr_t>(residual) & 3u) == 0) {
     return mb_gemm_f32_tc_launch(ctx, in, filter, bias, out, N, hw, O, C, hw, C * hw, C, 0, hw, O * hw,
                                  activation, max_limit, coefficient, residual);
   }

@@ -19,11 +19,27 @@
 // requests W.  Persistent over the tiles; where these do not fill the SMs, one tile per cluster of 2 .. 8 CTAs with the
 // depth cut between them, the partial tiles added up through distributed shared memory.
 //
+// Accuracy.  tf32 products of split operands lose the last bit of some values, and the tensor core cuts its accumulator off
+// after every MMA (8 of k), so that an error of 2e-8 (values of either sign) to 5e-8 (of one sign) per MMA piles up with the
+// depth; a chain of fp32 FMAs rounds, and ends at 1.4e-7 / 1.2e-7 at k = 64, 5.7e-7 / 4.3e-7 at 1024.  (Relative errors in
+// the 2-norm against float64, normal / uniform [0, 1) operands.)  Three forms:
+//   WHOLE   one accumulator over the depth, hi cut off: what the TMA-fed kernel does, bit for bit (4.9e-7 / 5.1e-7 at k =
+//           64, 2.7e-6 / 6.7e-6 at 1024, three times that with 128 channels).
+//   RUNS    hi rounded; every `run` steps the result warps take the accumulator and carry the sum on in fp32, in shared
+//           memory; small products in columns of their own (64 channels) or first (128).  run = 1: 1.4e-7 / 1.3e-7, 2:
+//           2.1e-7 / 2.7e-7, 4: 3.5e-7 / 6.1e-7, whatever the depth.
+//   SPREAD  for up to two steps: three accumulators of at most three MMAs, handed over together: 1.2e-7 / 9.3e-8 at 64.
+// mb_f32_gather_run picks the run whose error is below the FMA chain's, for products that would otherwise run on CUDA cores;
+// none is up to k = 47 and from 65 to 71.  A 3x3 convolution in place of Winograd kernels takes the run whose error is below
+// theirs (F(2,3): 3.1e-8 times the root of the channels, F(6,3): 2e-6 and more).  The sums cost 384 x 384 x 64, batch
+// 12, 0.7 us of 6.7 (SPREAD), the 3x3 layers of ResNet-50 at batch 1 0.2 to 1.5 us each, and the largest products, whose
+// shared memory is busy with W already, a half (1536 x 1536 x 1024: 33 -> 49 us; 136 us on CUDA cores).
+//
 // What bounds it: the tensor pipe at three tf32 MMAs per product for long depths (12 MMAs x 92 cycles per step of
 // 128 x 128 x 32; a convolution's loads bring the step to 1400), the launch, first loads and results for small shapes.
 // Measured, before -> now: 7x7 stride 2 of 3 -> 64 channels, 224 x 224, batch 256, 1360 us (column matrix) -> 688;
-// 5x5 stride 2 of 48 -> 32, 112 x 112, batch 24, 341 -> 116; 3x3 of 512 channels, 7 x 7, batch 1, 70 (Winograd) -> 17;
-// 384 x 384 x 64 times a transposed matrix, batch 12, 16.4 (CUDA cores) -> 7.9; 736 x 176 x 384, batch 24, 152 -> 29.
+// 5x5 stride 2 of 48 -> 32, 112 x 112, batch 24, 341 -> 116; 3x3 of 512 channels, 7 x 7, batch 1, 39 (Winograd) -> 18;
+// 384 x 384 x 64 times a transposed matrix, batch 12, 10.9 (CUDA cores) -> 7.4; 736 x 176 x 384, batch 24, 76 -> 39.
 #include <algorithm>
 
 #include "gemm_f32_gather.cuh"
@@ -44,9 +60,9 @@ constexpr int FIRST_W = 4 * XGROUPS, FIRST_E = FIRST_W + 4;
 // EW warps for results: four, or eight where a tile's results take longer than its steps (see make_plan); then the MMA
 // warp and the one that requests W
 constexpr int threads(int ew) { return (FIRST_E + ew + 2) * 32; }
-constexpr int ACCS = 2;
 constexpr long long WAIT_BUDGET = 1ll << 31;        // ~1 s of SM clocks per wait
 enum { W_TMA = 0, W_ROWS = 1, W_COLS = 2 };         // k contiguous and 16-byte aligned; k contiguous; n contiguous
+enum { WHOLE = 0, RUNS = 1, SPREAD = 2 };           // see "Accuracy" above
 enum { X_CONV = 0, X_ROWS = 1, X_COLS = 2 };        // convolution; m contiguous; k contiguous
 
 struct Params {
@@ -57,6 +73,7 @@ struct Params {
   int step_m, step_n, step_b;  // gridDim.x in tile coordinates
   int64_t x_ks, x_ms, x_bs, w_ns, w_ks, w_bs, c_ns, c_ms, c_bs;
   int x_vec;                   // K-contiguous rows are 16-byte aligned
+  int run;                     // RUNS: steps per run
   int act;
   float max_limit, coef;
   int H, Wd, KW, taps, sh, sw, dh, dw, pad_t, pad_l, Wo, hw, KH;
@@ -65,21 +82,25 @@ struct Params {
   int *status;
 };
 
-template <int BN>
+template <int BN, int MODE>
 struct Cfg {
   static constexpr int W_BYTES = BN * KB * 4;            // hi (or lo) of a step
   static constexpr int STAGE_BYTES = 2 * W_BYTES;
   // 64 channels: hi x [w_hi | w_lo] is one MMA of 128 columns (see the MMA role)
   static constexpr bool WIDE = BN == 64;
   static constexpr int ACC_COLS = WIDE ? 2 * BN : BN;
-  static constexpr int A_COL0 = ACCS * ACC_COLS;         // TMEM: accumulators, then STAGES x 64 columns of A
+  // TMEM: accumulators, one or three of a tile and two or one tiles at a time, then STAGES x 64 columns of A
+  static constexpr int TILE_ACCS = MODE == SPREAD ? 3 : 1, ACCS = MODE == SPREAD ? 1 : 2;
+  static constexpr int A_COL0 = TILE_ACCS * ACCS * ACC_COLS;
   static constexpr int STAGES = (512 - A_COL0) / (2 * KB);
   static constexpr int RING = STAGES * STAGE_BYTES;
   static constexpr int TABLE_BYTES = FIRST_W * KB * 8;
   static constexpr int PART_BYTES = BN * BM * 4;         // the runs' shares of this CTA's channels: [rank][channel][128 m]
   // (PART_BYTES only where the depth is cut: what shared memory does not take is L1, which a convolution's windows live in)
   static constexpr int SMEM_BYTES = RING + 1024 /*align*/ + TABLE_BYTES + 256 /*barriers*/;
-  static_assert(SMEM_BYTES + PART_BYTES <= 227 * 1024, "shared memory budget");
+  // (twice where a depth that is cut has short runs as well, for the runs' sums, which no 128-channel tile has room for)
+  static constexpr int MAX_SMEM_BYTES = SMEM_BYTES + (BN == 64 ? 2 : 1) * PART_BYTES;
+  static_assert(MAX_SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
 
 struct TileIter {
@@ -101,10 +122,10 @@ struct TileIter {
   }
 };
 
-// (Rounding hi instead of cutting it off changed nothing: what error there is grows with the depth and comes from the
-// accumulator, which cuts off too.)
-__device__ __forceinline__ uint32_t tf32_hi(float v) { return __float_as_uint(v) & 0xffffe000u; }
-__device__ __forceinline__ uint32_t tf32_lo(float v) { return __float_as_uint(v - __uint_as_float(tf32_hi(v))); }
+// hi + lo == v; the MMA reads the upper 11 bits of each.  With hi rounded (half = 0x1000), lo has 12 bits of either sign, of
+// which at most the last is lost; with hi cut off (half = 0) lo has 13 bits and the sign of v.
+__device__ __forceinline__ uint32_t tf32_hi(float v, uint32_t half) { return (__float_as_uint(v) + half) & 0xffffe000u; }
+__device__ __forceinline__ uint32_t tf32_lo(float v, uint32_t half) { return __float_as_uint(v - __uint_as_float(tf32_hi(v, half))); }
 
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
@@ -123,11 +144,11 @@ __device__ __forceinline__ int64_t out_offset(const Params &p, int m, int b) {
   return b * p.c_bs + m * p.c_ms;
 }
 
-template <int BN, int XK, int WK, int EW>
+template <int BN, int XK, int WK, int EW, int MODE>
 __global__ void __launch_bounds__(threads(EW), 1)
 gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Params p) {
-  using C = Cfg<BN>;
-  constexpr int STAGES = C::STAGES, MMA_WARP = FIRST_E + EW, TMA_WARP = MMA_WARP + 1;
+  using C = Cfg<BN, MODE>;
+  constexpr int STAGES = C::STAGES, ACCS = C::ACCS, MMA_WARP = FIRST_E + EW, TMA_WARP = MMA_WARP + 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -138,6 +159,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + C::RING + C::TABLE_BYTES + 24 * STAGES + 16 * ACCS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr uint32_t half = MODE != WHOLE ? 0x1000u : 0u;
   mb_grid_dep_launch();
 
   if (threadIdx.x == MMA_WARP * 32) {
@@ -257,10 +279,10 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         for (int h = 0; h < 2; ++h) {
           uint32_t r[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] = tf32_hi(v[h * 16 + j]);
+          for (int j = 0; j < 16; ++j) r[j] = tf32_hi(v[h * 16 + j], half);
           tmem_st_32x32b_x16(slot + h * 16, r);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] = tf32_lo(v[h * 16 + j]);
+          for (int j = 0; j < 16; ++j) r[j] = tf32_lo(v[h * 16 + j], half);
           tmem_st_32x32b_x16(slot + KB + h * 16, r);
         }
         tmem_st_wait();
@@ -291,8 +313,8 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           for (int c = 0; c < C::W_BYTES / 2048; ++c) {
             const int at = (c * 128 + w4 * 32 + lane) * 16;
             const float4 v = *reinterpret_cast<const float4 *>(tile + at);
-            *reinterpret_cast<uint4 *>(tile + at) = make_uint4(tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w));
-            *reinterpret_cast<uint4 *>(tile + C::W_BYTES + at) = make_uint4(tf32_lo(v.x), tf32_lo(v.y), tf32_lo(v.z), tf32_lo(v.w));
+            *reinterpret_cast<uint4 *>(tile + at) = make_uint4(tf32_hi(v.x, half), tf32_hi(v.y, half), tf32_hi(v.z, half), tf32_hi(v.w, half));
+            *reinterpret_cast<uint4 *>(tile + C::W_BYTES + at) = make_uint4(tf32_lo(v.x, half), tf32_lo(v.y, half), tf32_lo(v.z, half), tf32_lo(v.w, half));
           }
           fence_proxy_async();
           __syncwarp();
@@ -341,8 +363,8 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
           const uint32_t at = swz_at(row[c], chunk[c]);
-          *reinterpret_cast<uint4 *>(tile + at) = make_uint4(tf32_hi(v[c].x), tf32_hi(v[c].y), tf32_hi(v[c].z), tf32_hi(v[c].w));
-          *reinterpret_cast<uint4 *>(tile + C::W_BYTES + at) = make_uint4(tf32_lo(v[c].x), tf32_lo(v[c].y), tf32_lo(v[c].z), tf32_lo(v[c].w));
+          *reinterpret_cast<uint4 *>(tile + at) = make_uint4(tf32_hi(v[c].x, half), tf32_hi(v[c].y, half), tf32_hi(v[c].z, half), tf32_hi(v[c].w, half));
+          *reinterpret_cast<uint4 *>(tile + C::W_BYTES + at) = make_uint4(tf32_lo(v[c].x, half), tf32_lo(v[c].y, half), tf32_lo(v[c].z, half), tf32_lo(v[c].w, half));
         }
         fence_proxy_async();
         __syncwarp();
@@ -376,132 +398,197 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       constexpr uint32_t idesc = make_idesc(/*c f32*/ 1, /*a tf32*/ 2, /*b tf32*/ 2, false, false, BM, BN);
       constexpr uint32_t idesc_wide = make_idesc(1, 2, 2, false, false, BM, C::WIDE ? 2 * BN : BN);
       const uint64_t wdesc = make_smem_desc(0, 16, 1024, 2);
-      int it = 0, local = 0;
+      const int run = MODE == RUNS ? p.run : steps;
+      const int third = steps == 1 ? 2 : 3;  // SPREAD: MMA depths per accumulator
+      int it = 0, filled = 0;  // steps, and accumulators handed to the result warps
       bool ok = true;
-      for (TileIter t(p); ok && t.valid(p); t.next(p), ++local) {
-        const int acc = local % ACCS;
-        if (local >= ACCS && !mbar_wait(tempty_bar + 8 * acc, ((local / ACCS) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
+      uint32_t d = 0;
+      // the next accumulator, once its last contents have been read
+      auto next_acc = [&]() {
+        const int acc = filled % ACCS;
+        if (filled >= ACCS && !mbar_wait(tempty_bar + 8 * acc, ((filled / ACCS) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
           fail(MB_DEV_TIMEOUT_MMA);
-          break;
+          return false;
         }
         tc_fence_after_sync();
-        const uint32_t d = tmem + acc * C::ACC_COLS;
-        for (int i = 0; i < steps; ++i, ++it) {
-          const int stage = it % STAGES;
-          if (!mbar_wait(full_bar + 8 * stage, (it / STAGES) & 1, abort_flag, WAIT_BUDGET)) {
-            fail(MB_DEV_TIMEOUT_MMA);
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          const uint32_t a_hi = tmem + C::A_COL0 + stage * (2 * KB), a_lo = a_hi + KB;
-          const uint32_t sw = smem_base + stage * C::STAGE_BYTES;
-          const uint64_t w_hi = wdesc | static_cast<uint64_t>((sw >> 4) & 0x3FFFu);
-          const uint64_t w_lo = wdesc | static_cast<uint64_t>(((sw + C::W_BYTES) >> 4) & 0x3FFFu);
-          // With A from tensor memory an MMA takes 92 cycles for 64 columns as for 128, so 64 channels take hi from there
-          // once for both halves of W, whose tiles lie one behind the other: 2 MMAs per 8 of k instead of 3, and hi * lo
-          // + lo * hi in columns of their own, which the epilogue adds.
-#pragma unroll
-          for (int j = 0; j < KB / 8; ++j) {
-            if (C::WIDE) {
-              mma_tf32_ts(d, a_hi + j * 8, w_hi + 2 * j, idesc_wide, (i > 0 || j > 0) ? 1u : 0u);
-              mma_tf32_ts(d + BN, a_lo + j * 8, w_hi + 2 * j, idesc, 1u);
-              continue;
+        d = tmem + acc * C::ACC_COLS;
+        return true;
+      };
+      for (TileIter t(p); ok && t.valid(p); t.next(p)) {
+        for (int i0 = 0; ok && i0 < steps; i0 += run) {
+          if (!(ok = next_acc())) break;
+          const int count = min(run, steps - i0);
+          // 128 channels in short runs: the small products first, while they do not cost the accumulator its last bits
+          constexpr bool small_first = MODE != WHOLE && !C::WIDE;
+          for (int i = 0; i < count; ++i) {
+            const int stage = (it + i) % STAGES;
+            if (!mbar_wait(full_bar + 8 * stage, ((it + i) / STAGES) & 1, abort_flag, WAIT_BUDGET)) {
+              fail(MB_DEV_TIMEOUT_MMA);
+              ok = false;
+              break;
             }
-            mma_tf32_ts(d, a_lo + j * 8, w_hi + 2 * j, idesc, (i > 0 || j > 0) ? 1u : 0u);
-            mma_tf32_ts(d, a_hi + j * 8, w_lo + 2 * j, idesc, 1u);
-            mma_tf32_ts(d, a_hi + j * 8, w_hi + 2 * j, idesc, 1u);
+            tc_fence_after_sync();
+            const uint32_t a_hi = tmem + C::A_COL0 + stage * (2 * KB), a_lo = a_hi + KB;
+            const uint32_t sw = smem_base + stage * C::STAGE_BYTES;
+            const uint64_t w_hi = wdesc | static_cast<uint64_t>((sw >> 4) & 0x3FFFu);
+            const uint64_t w_lo = wdesc | static_cast<uint64_t>(((sw + C::W_BYTES) >> 4) & 0x3FFFu);
+            // With A from tensor memory an MMA takes 92 cycles for 64 columns as for 128, so 64 channels take hi from
+            // there once for both halves of W, whose tiles lie one behind the other: 2 MMAs per 8 of k instead of 3, and
+            // hi * lo + lo * hi in columns of their own, which the result warps add.
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j) {
+              const uint32_t add = (i > 0 || j > 0) ? 1u : 0u;
+              if (C::WIDE) {
+                const int at = MODE == SPREAD ? (i * 4 + j) / third : 0;
+                const bool first = MODE == SPREAD ? (i * 4 + j) % third == 0 : add == 0;
+                const uint32_t da = d + at * C::ACC_COLS;
+                mma_tf32_ts(da, a_hi + j * 8, w_hi + 2 * j, idesc_wide, first ? 0u : 1u);
+                mma_tf32_ts(da + BN, a_lo + j * 8, w_hi + 2 * j, idesc, 1u);
+                continue;
+              }
+              mma_tf32_ts(d, a_lo + j * 8, w_hi + 2 * j, idesc, add);
+              mma_tf32_ts(d, a_hi + j * 8, w_lo + 2 * j, idesc, 1u);
+              if (!small_first) mma_tf32_ts(d, a_hi + j * 8, w_hi + 2 * j, idesc, 1u);
+            }
+            if (!small_first) mma_commit(empty_bar + 8 * stage);
           }
-          mma_commit(empty_bar + 8 * stage);
+          if (small_first && ok) {
+            for (int i = 0; i < count; ++i) {
+              const int stage = (it + i) % STAGES;
+              const uint32_t a_hi = tmem + C::A_COL0 + stage * (2 * KB);
+              const uint64_t w_hi = wdesc | static_cast<uint64_t>(((smem_base + stage * C::STAGE_BYTES) >> 4) & 0x3FFFu);
+#pragma unroll
+              for (int j = 0; j < KB / 8; ++j) {
+                const int at = MODE == SPREAD ? (i * 4 + j) / third : 0;
+                mma_tf32_ts(d + at * C::ACC_COLS, a_hi + j * 8, w_hi + 2 * j, idesc,
+                            at > 0 && (i * 4 + j) % third == 0 ? 0u : 1u);
+              }
+              mma_commit(empty_bar + 8 * stage);
+            }
+          }
+          if (ok) mma_commit(tfull_bar + 8 * (filled++ % ACCS));
+          it += count;
         }
-        if (!ok) break;
-        mma_commit(tfull_bar + 8 * acc);
       }
     }
     __syncwarp();
   } else {
     // ---- results: a lane per pixel, one channel after the other, 32 adjacent pixels per store ----
     const int quarter = warp & 3;
-    const int c_begin = (warp - FIRST_E) / 4 * (BN * 4 / EW), c_end = c_begin + BN * 4 / EW;  // of eight, half the channels each
-    int local = 0;
+    constexpr int CW = BN * 4 / EW;                  // channels per warp: of eight warps, half the channels each
+    const int c_begin = (warp - FIRST_E) / 4 * CW, c_end = c_begin + CW;
+    const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
+    int filled = 0;
     mb_grid_dep_wait();
-    for (TileIter t(p); t.valid(p); t.next(p), ++local) {
-      const int acc = local % ACCS;
-      if (!mbar_wait_warp(tfull_bar + 8 * acc, (local / ACCS) & 1, abort_flag, WAIT_BUDGET)) {
+    auto wait_acc = [&]() {
+      const int acc = filled % ACCS;
+      if (!mbar_wait_warp(tfull_bar + 8 * acc, (filled / ACCS) & 1, abort_flag, WAIT_BUDGET)) {
         fail(MB_DEV_TIMEOUT_EPILOGUE);
-        break;
+        return false;
       }
       tc_fence_after_sync();
-      const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * C::ACC_COLS;
-      if (p.splits > 1) {
-        // this CTA's run of the depth, each channel to the CTA that adds it up (writing it there takes nobody's time; read
-        // from there, one peer after the other, it took 2.1 us)
-        const int share = BN / p.splits;  // channels per CTA: 8 .. 64
-#pragma unroll 1
-        for (int c = c_begin; c < c_end; c += 8) {
-          uint32_t r[8], r2[8];
-          tmem_ld_32x32b_x8(src + c, r);
-          if (C::WIDE) tmem_ld_32x32b_x8(src + BN + c, r2);
-          tmem_ld_wait_x8(r);
-          if (C::WIDE) tmem_ld_wait_x8(r2);
-          const int owner = c / share;
-          const uint32_t dst = mapa_shared(part, owner) + ((rank * share + c - owner * share) * BM + quarter * 32 + lane) * 4;
+      return true;
+    };
+    auto release_acc = [&]() {
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty_bar + 8 * (filled % ACCS));
+      ++filled;
+    };
+    // this CTA's run of the depth, each channel to the CTA that adds it up (writing it there takes nobody's time; read
+    // from there, one peer after the other, it took 2.1 us)
+    const int share = BN / p.splits;  // channels per CTA: 8 .. 64
+    auto push8 = [&](const float *x, int c) {
+      const int owner = c / share;
+      const uint32_t dst = mapa_shared(part, owner) + ((rank * share + c - owner * share) * BM + quarter * 32 + lane) * 4;
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            st_cluster_f32(dst + j * (BM * 4), C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]));
-        }
-        break;
-      }
+      for (int j = 0; j < 8; ++j) st_cluster_f32(dst + j * (BM * 4), x[j]);
+    };
+    // the sums of the runs so far, each thread's own
+    float *sums = reinterpret_cast<float *>(smem + (part - smem_base) + (p.splits > 1 ? C::PART_BYTES : 0)) + quarter * 32 + lane;
+    const int runs = MODE == RUNS ? (steps + p.run - 1) / p.run : 1;
+    bool ok = true;
+    for (TileIter t(p); ok && t.valid(p); t.next(p)) {
       const int m = t.tm * BM + quarter * 32 + lane;
       const int64_t at = out_offset<XK>(p, m, t.b);
       const int n0 = t.tn * BN;
-      // the next chunk's accumulators are on their way while this one is stored
-      uint32_t r[16], r2[16];
-      tmem_ld_32x32b_x16(src + c_begin, r);
-      if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c_begin, r2);
 #pragma unroll 1
-      for (int c = c_begin; c < c_end; c += 16) {
-        tmem_ld_wait_x16(r);
-        if (C::WIDE) tmem_ld_wait_x16(r2);
-        // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
-        // latency per channel made a 128 x 128 tile take 19 us)
-        float x[16];
+      for (int i = 0; i < runs; ++i) {
+        if (!(ok = wait_acc())) break;
+        const uint32_t src = tmem + lanes + (filled % ACCS) * C::ACC_COLS;
+        // the next chunk's accumulators are on their way while this one is stored
+        uint32_t r[16], r2[16];
+        tmem_ld_32x32b_x16(src + c_begin, r);
+        if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c_begin, r2);
+#pragma unroll 1
+        for (int c = c_begin; c < c_end; c += 16) {
+          tmem_ld_wait_x16(r);
+          if (C::WIDE) tmem_ld_wait_x16(r2);
+          // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
+          // latency per channel made a 128 x 128 tile take 19 us)
+          float x[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
-        if (c + 16 < c_end) {
-          tmem_ld_32x32b_x16(src + c + 16, r);
-          if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c + 16, r2);
-        } else {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(tempty_bar + 8 * acc);
-        }
-        if (p.bias != nullptr) {
-          const float mine = n0 + c + (lane & 15) < p.N ? __ldg(p.bias + n0 + c + (lane & 15)) : 0.f;
+          for (int j = 0; j < 16; ++j) x[j] = C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
+          if (MODE == SPREAD) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) x[j] += __shfl_sync(0xffffffffu, mine, j);
-        }
-        if (p.residual != nullptr && m < p.M) {
-          const float *src_r = p.residual + at + static_cast<int64_t>(n0 + c) * p.c_ns;
-          float res[16];
+            for (int a = 1; a < C::TILE_ACCS; ++a) {
+              if (a == 2 && steps == 1) break;
+              tmem_ld_32x32b_x16(src + a * C::ACC_COLS + c, r);
+              if (C::WIDE) tmem_ld_32x32b_x16(src + a * C::ACC_COLS + BN + c, r2);
+              tmem_ld_wait_x16(r);
+              if (C::WIDE) tmem_ld_wait_x16(r2);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) res[j] = n0 + c + j < p.N ? __ldg(src_r + j * p.c_ns) : 0.f;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) x[j] += res[j];
-        }
-        mb_activate_n(x, p.act, p.max_limit, p.coef);
-        float *dst = p.C + at + static_cast<int64_t>(n0 + c) * p.c_ns;
-        if (n0 + c + 16 <= p.N) {
-          if (m < p.M) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) dst[j * p.c_ns] = x[j];
+              for (int j = 0; j < 16; ++j) x[j] += C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
+            }
           }
-        } else if (m < p.M) {
+          if (c + 16 < c_end) {
+            tmem_ld_32x32b_x16(src + c + 16, r);
+            if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c + 16, r2);
+          } else {
+            release_acc();
+          }
+          if (MODE == RUNS && i > 0) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (n0 + c + j < p.N) dst[j * p.c_ns] = x[j];
+            for (int j = 0; j < 16; ++j) x[j] += sums[(c + j) * BM];
+          }
+          if (MODE == RUNS && i + 1 < runs) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sums[(c + j) * BM] = x[j];
+            continue;
+          }
+          if (p.splits > 1) {
+            push8(x, c);
+            push8(x + 8, c + 8);
+            continue;
+          }
+          if (p.bias != nullptr) {
+            const float mine = n0 + c + (lane & 15) < p.N ? __ldg(p.bias + n0 + c + (lane & 15)) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] += __shfl_sync(0xffffffffu, mine, j);
+          }
+          if (p.residual != nullptr && m < p.M) {
+            const float *src_r = p.residual + at + static_cast<int64_t>(n0 + c) * p.c_ns;
+            float res[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) res[j] = n0 + c + j < p.N ? __ldg(src_r + j * p.c_ns) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] += res[j];
+          }
+          mb_activate_n(x, p.act, p.max_limit, p.coef);
+          float *dst = p.C + at + static_cast<int64_t>(n0 + c) * p.c_ns;
+          if (n0 + c + 16 <= p.N) {
+            if (m < p.M) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) dst[j * p.c_ns] = x[j];
+            }
+          } else if (m < p.M) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (n0 + c + j < p.N) dst[j * p.c_ns] = x[j];
+          }
         }
       }
+      if (p.splits > 1) break;
     }
   }
   __syncwarp();
@@ -553,17 +640,18 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   }
 }
 
-template <int BN, int XK, int WK, int EW>
+template <int BN, int XK, int WK, int EW, int MODE>
 int launch_cfg(mb_context *ctx, Params &p) {
-  using C = Cfg<BN>;
-  auto kern = gemm_f32_gather_kernel<BN, XK, WK, EW>;
-  constexpr uint64_t bit = (EW == 8 ? 18 : 0) + (BN == 128 ? 9 : 0) + XK * 3 + WK;
+  using C = Cfg<BN, MODE>;
+  auto kern = gemm_f32_gather_kernel<BN, XK, WK, EW, MODE>;
+  constexpr int bit = (MODE == SPREAD ? 54 : MODE == RUNS ? 36 : EW == 8 ? 18 : 0) + (BN == 128 ? 9 : 0) + XK * 3 + WK;
   CUtensorMap map;
   if (WK == W_TMA) MB_RETURN_IF_ERROR(mb_make_map_w_f32(ctx, &map, p.W, p.K, p.N, p.w_bs != 0 ? p.batch : 1, p.w_ns, p.w_bs, BN));
   else memset(&map, 0, sizeof(map));
-  if (!(ctx->f32_gather_attr_mask & (1ull << bit))) {
-    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES + C::PART_BYTES));
-    ctx->f32_gather_attr_mask |= 1ull << bit;
+  uint64_t &mask = ctx->f32_gather_attr_mask[bit >> 6];
+  if (!(mask & (1ull << (bit & 63)))) {
+    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::MAX_SMEM_BYTES));
+    mask |= 1ull << (bit & 63);
   }
   const int64_t tiles = static_cast<int64_t>(p.batch) * p.tiles_m * p.tiles_n;
   const int slots = p.splits > 1 ? static_cast<int>(tiles) : static_cast<int>(std::min<int64_t>(tiles, ctx->num_sms));
@@ -571,7 +659,8 @@ int launch_cfg(mb_context *ctx, Params &p) {
   p.step_n = (slots / p.tiles_m) % p.tiles_n;
   p.step_b = (slots / p.tiles_m) / p.tiles_n;
   MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), threads(EW),
-                                  C::SMEM_BYTES + (p.splits > 1 ? C::PART_BYTES : 0), p.splits, map, p));
+                                  C::SMEM_BYTES + ((p.splits > 1) + (MODE == RUNS && p.run < p.k_blocks)) * C::PART_BYTES,
+                                  p.splits, map, p));
   ctx->launches++;
   ctx->launches_tc++;
   return MB_SUCCESS;
@@ -596,6 +685,7 @@ Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
     const int64_t tiles = g.batch * tiles_m * ceil_div64(g.N, w);
     for (int s : {1, 2, 4, 8}) {
       if (asked != 0 ? s != asked : s > k_blocks) continue;
+      if (w == 128 && s > 1 && g.run != 0) continue;  // (no room for the runs' sums)
       const int64_t rounds = ceil_div64(tiles * s, s == 1 ? ctx->num_sms : mb_resident_cluster_ctas(ctx, s));
       if (s > 1 && rounds > 1 && asked == 0) continue;  // (one tile per CTA: a second round would start from nothing)
       const int64_t steps = ceil_div64(k_blocks, s);
@@ -642,6 +732,7 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
   p.tiles_n = static_cast<int>(ceil_div64(g.N, plan.bn));
   p.k_blocks = static_cast<int>(ceil_div64(g.K, KB));
   p.splits = plan.splits;
+  p.run = plan.bn == 128 ? std::min(g.run, 2) : g.run;  // (of the four steps that its ring holds)
   p.x_ks = g.x_ks; p.x_ms = g.x_ms; p.x_bs = g.x_bs;
   p.w_ns = g.w_ns; p.w_ks = g.w_ks; p.w_bs = g.w_bs;
   p.c_ns = g.c_ns; p.c_ms = g.c_ms; p.c_bs = g.c_bs;
@@ -661,30 +752,42 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
     fast_div_make(static_cast<uint32_t>(p.KW), &p.kw_mul, &p.kw_shift);
     fast_div_make(static_cast<uint32_t>(p.hw), &p.hw_mul, &p.hw_shift);
     fast_div_make(static_cast<uint32_t>(p.Wo), &p.wo_mul, &p.wo_shift);
-#define MB_F32_CONV(BN_, EW_) \
-  return w_tma ? launch_cfg<BN_, X_CONV, W_TMA, EW_>(ctx, p) : launch_cfg<BN_, X_CONV, W_ROWS, EW_>(ctx, p);
-    if (plan.warps == 8) {
-      if (plan.bn == 128) { MB_F32_CONV(128, 8) }
-      MB_F32_CONV(64, 8)
+#define MB_F32_CONV(BN_, EW_, MODE_) \
+  return w_tma ? launch_cfg<BN_, X_CONV, W_TMA, EW_, MODE_>(ctx, p) : launch_cfg<BN_, X_CONV, W_ROWS, EW_, MODE_>(ctx, p);
+    if (p.run != 0 && plan.bn == 128) { MB_F32_CONV(128, 8, RUNS) }
+    if (plan.bn == 64 && (p.run != 0 || plan.warps == 4)) {
+      // (one kernel for 64 channels with short runs or without: where a network's 1x1 and 3x3 layers took two in turn, every
+      // launch began with the other's instructions in the caches, 30 us of ResNet-50's 570 at batch 1)
+      if (p.run == 0) p.run = p.k_blocks;
+      MB_F32_CONV(64, 4, RUNS)
     }
-    if (plan.bn == 128) { MB_F32_CONV(128, 4) }
-    MB_F32_CONV(64, 4)
+    if (plan.bn == 64) { MB_F32_CONV(64, 8, WHOLE) }
+    if (plan.warps == 8) { MB_F32_CONV(128, 8, WHOLE) }
+    MB_F32_CONV(128, 4, WHOLE)
 #undef MB_F32_CONV
   }
   const bool cols = g.x_ms != 1;
   p.x_vec = cols && (reinterpret_cast<uintptr_t>(g.X) & 15u) == 0 && g.x_ms % 4 == 0 && g.x_bs % 4 == 0 && g.K % 4 == 0;
-#define MB_F32_W(BN_, XK_, EW_)                                           \
-  if (w_nc) return launch_cfg<BN_, XK_, W_COLS, EW_>(ctx, p);              \
-  return w_tma ? launch_cfg<BN_, XK_, W_TMA, EW_>(ctx, p) : launch_cfg<BN_, XK_, W_ROWS, EW_>(ctx, p);
-#define MB_F32(BN_, EW_)                   \
-  if (cols) { MB_F32_W(BN_, X_COLS, EW_) } \
-  MB_F32_W(BN_, X_ROWS, EW_)
-  if (plan.warps == 8) {
-    if (plan.bn == 128) { MB_F32(128, 8) }
-    MB_F32(64, 8)
+#define MB_F32_W(BN_, XK_, EW_, MODE_)                                           \
+  if (w_nc) return launch_cfg<BN_, XK_, W_COLS, EW_, MODE_>(ctx, p);              \
+  return w_tma ? launch_cfg<BN_, XK_, W_TMA, EW_, MODE_>(ctx, p) : launch_cfg<BN_, XK_, W_ROWS, EW_, MODE_>(ctx, p);
+#define MB_F32(BN_, EW_, MODE_)                   \
+  if (cols) { MB_F32_W(BN_, X_COLS, EW_, MODE_) } \
+  MB_F32_W(BN_, X_ROWS, EW_, MODE_)
+  if (p.run == 1 && p.k_blocks <= 2) {
+    if (plan.bn == 128) { MB_F32(128, 8, SPREAD) }
+    MB_F32(64, 4, SPREAD)
   }
-  if (plan.bn == 128) { MB_F32(128, 4) }
-  MB_F32(64, 4)
+  if (p.run != 0) {
+    if (plan.bn == 128) { MB_F32(128, 8, RUNS) }
+    MB_F32(64, 4, RUNS)
+  }
+  if (plan.warps == 8) {
+    if (plan.bn == 128) { MB_F32(128, 8, WHOLE) }
+    MB_F32(64, 8, WHOLE)
+  }
+  if (plan.bn == 128) { MB_F32(128, 4, WHOLE) }
+  MB_F32(64, 4, WHOLE)
 #undef MB_F32
 #undef MB_F32_W
 }

@@ -17,8 +17,15 @@ struct mb_f32_gemm {
   // conv: X is an NCHW tensor, M its output pixels over all images, k = (c * KH + kh) * KW + kw, and C an NCHW
   // tensor of N channels (x_*, c_* and the W strides unused)
   bool conv = false;
+  // How many steps of 32 of the depth the tensor core adds up before the sum is carried on in fp32; 0: all of them, as
+  // the TMA-fed kernel does.
+  int run = 0;
   int C_in = 0, H = 0, Wd = 0, KH = 1, KW = 1, sh = 1, sw = 1, dh = 1, dw = 1, pad_t = 0, pad_l = 0, Ho = 0, Wo = 0;
 };
+
+// The run that keeps the error of a product of this depth below that of a chain of fp32 FMAs, 0 where none does (see
+// "Accuracy" in gemm_f32_gather.cu).
+static inline int mb_f32_gather_run(int64_t K) { return K < 48 || (K > 64 && K < 72) ? 0 : K < 384 ? 1 : 2; }
 
 bool mb_gemm_f32_gather_supported(const mb_context *ctx, const mb_f32_gemm &g);
 // Estimated time of the launch in SM cycles.

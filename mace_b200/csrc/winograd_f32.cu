@@ -374,8 +374,8 @@ int pick_tile(int64_t H, int64_t W, int tile_override) {
 // Estimated SM cycles of the three Winograd kernels, from their times at 56 x 56 x 64 (batch 1: 13 us, 32: 56, 256: 400),
 // 28 x 28 x 128 (8: 21, 256: 290), 14 x 14 x 256 (256: 299) and 7 x 7 x 512 (256: 230): about 12 us of launches, the
 // transforms' bytes (the intermediates written and read once each) at 9.5 TB/s (part of them stays in L2), the batched
-// product at 1150 cycles per step and tile or 2.4 us for a tile's stores.  An odd column count keeps the product off TMA
-// (15 us at batch 1).
+// product at 1150 cycles per step and tile or 2.4 us for a tile's stores.  A column count that keeps the product off TMA costs
+// 0 to 4.6 us (128 channels, 28 x 28, batch 1 and 2; 256, 14 x 14, batch 3; 48, 28 x 28, batch 9: 7 us).
 static int64_t winograd_cost(const mb_context *ctx, int64_t N, int64_t C, int64_t H, int64_t W, int64_t O, int64_t Ho,
                              int64_t Wo, int tile_override) {
   const int tile = pick_tile(H, W, tile_override);
@@ -383,7 +383,7 @@ static int64_t winograd_cost(const mb_context *ctx, int64_t N, int64_t C, int64_
   const int64_t cols = N * ceil_div64(Ho, tile) * ceil_div64(Wo, tile);
   const int64_t bytes = 4 * (N * C * H * W + 2 * T * C * cols + 2 * T * O * cols + N * O * Ho * Wo + T * O * C);
   const int64_t rounds = ceil_div64(T * ceil_div64(cols, 128) * ceil_div64(O, O > 64 ? 128 : 64), ctx->num_sms);
-  return 23000 + bytes / 5000 + rounds * std::max<int64_t>(ceil_div64(C, 32) * 1150, 4500) + (cols % 4 != 0 ? 28000 : 0);
+  return 23000 + bytes / 5000 + rounds * std::max<int64_t>(ceil_div64(C, 32) * 1150, 4500) + (cols % 4 != 0 ? 6000 : 0);
 }
 
 extern "C" {
@@ -435,6 +435,8 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
     g.C_in = static_cast<int>(C); g.H = static_cast<int>(H); g.Wd = static_cast<int>(W);
     g.KH = 3; g.KW = 3; g.pad_t = pad_top; g.pad_l = pad_left;
     g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
+    // no larger an error than that of the Winograd kernels: 3.1e-8 times the root of C with F(2,3), 2e-6 and more with F(6,3)
+    g.run = pick_tile(H, W, tile_override) == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : 4;
     if (mb_gemm_f32_gather_supported(ctx, g) &&
         (ctx->f32_gather == 2 || mb_gemm_f32_gather_cost(ctx, g) < winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override)))
       return mb_gemm_f32_gather_launch(ctx, g);

@@ -268,6 +268,177 @@ def test_gemm_f32_of_any_layout_on_tensor_cores(ctx, orc, gather, maj, shape):
         b.free()
 
 
+def _norm_err(got, exact):
+    return float(np.linalg.norm(got.astype(np.float64) - exact) / np.linalg.norm(exact))
+
+
+def _with_options(ctx, call, **options):
+    for k, v in options.items():
+        ctx.set_option(k, v)
+    try:
+        return call()
+    finally:
+        for k in options:
+            ctx.set_option(k, 1 if k == "tensor_cores" else 0)
+
+
+# depths on both sides of every line of the rule, and long ones
+@pytest.mark.parametrize("K", [16, 47, 48, 64, 65, 72, 96, 200, 383, 384, 1024, 3000])
+@pytest.mark.parametrize("positive", [False, True])
+def test_gemm_f32_is_as_accurate_as_fmas(ctx, K, positive):
+    """A product in a layout that only the self-fetching kernel and the CUDA cores take: by rule its error against float64
+    is no larger than that of the CUDA cores' chain of fp32 FMAs (2 %: both are taken from 130 000 values)."""
+    batch, M, N = 2, 200, 333
+    rng = np.random.Generator(np.random.PCG64(K))
+    draw = rng.random if positive else rng.standard_normal
+    A, B = draw((batch, M, K)).astype(np.float32), draw((batch, N, K)).astype(np.float32)
+    exact = A.astype(np.float64) @ np.swapaxes(B, 1, 2).astype(np.float64)
+    dA, dB, dC = ctx.upload(A), ctx.upload(B), ctx.alloc(batch * M * N * 4)
+
+    def run():
+        ctx.gemm_f32(dA, dB, dC, batch, M, N, K, b_col_major=True)
+        return _norm_err(ctx.download(dC, (batch, M, N), np.float32), exact)
+
+    fma = _with_options(ctx, run, tensor_cores=0)
+    assert run() <= 1.02 * fma
+    if mb_f32_gather_run(K):   # the other tile width, and the depth cut
+        for bn, splits in ((64, 1), (64, 8), (128, 1)):
+            assert _with_options(ctx, run, f32_gather=2, f32_bn=bn, f32_splits=splits) <= 1.02 * fma, (bn, splits)
+    for b in (dA, dB, dC):
+        b.free()
+
+
+def mb_f32_gather_run(K):
+    """As in gemm_f32_gather.cuh."""
+    return 0 if K < 48 or 64 < K < 72 else 1 if K < 384 else 2
+
+
+@pytest.mark.parametrize("case", [
+    # few results, little work, 1x1 with rows that TMA does not take: kernel, N, C, HW, O, stride
+    (3, 1, 64, 4, 80, 1), (3, 1, 16, 14, 16, 1), (1, 2, 75, 28, 60, 1), (5, 1, 40, 7, 33, 2), (1, 1, 35, 12, 40, 1)])
+def test_small_conv2d_f32_is_as_accurate_as_fmas(ctx, orc, case):
+    k, N, C, HW, O, s = case
+    rng = np.random.Generator(np.random.PCG64(C))
+    x = rng.standard_normal((N, C, HW, HW)).astype(np.float32)
+    f = rng.standard_normal((O, C, k, k)).astype(np.float32)
+    ho, wo, ph, pw = orc.calc_padding_and_output_size(HW, HW, k, k, (1, 1), (s, s), PAD["SAME"])
+    padded = np.zeros((N, C, HW + 2 * k, HW + 2 * k))
+    padded[:, :, ph >> 1:(ph >> 1) + HW, pw >> 1:(pw >> 1) + HW] = x
+    exact = sum(np.einsum("ncyx,oc->noyx", padded[:, :, i:i + s * ho:s, j:j + s * wo:s], f[:, :, i, j].astype(np.float64))
+                for i in range(k) for j in range(k))
+    dx, df, do = ctx.upload(x), ctx.upload(f), ctx.alloc(exact.size * 4)
+
+    def run():
+        ctx.conv2d_f32(dx, df, None, do, N, C, HW, HW, O, k, k, (s, s), (1, 1), (ph >> 1, pw >> 1), (ho, wo))
+        return _norm_err(ctx.download(do, exact.shape, np.float32), exact)
+
+    fma = _with_options(ctx, run, tensor_cores=0)
+    assert run() <= 1.1 * fma  # (a few thousand values only)
+    for b in (dx, df, do):
+        b.free()
+
+
+@pytest.mark.parametrize("shape", [(9, 300, 256), (31, 200, 1000), (33, 300, 1001)])
+def test_gemv_f32_of_a_few_vectors_is_as_accurate_as_one_by_one(ctx, shape):
+    batch, rows, K = shape
+    rng = np.random.Generator(np.random.PCG64(batch))
+    w = rng.standard_normal((rows, K)).astype(np.float32)
+    x = rng.standard_normal((batch, K)).astype(np.float32)
+    exact = x.astype(np.float64) @ w.T.astype(np.float64)
+    dw, dx, do = ctx.upload(w), ctx.upload(x), ctx.alloc(batch * rows * 4)
+    ctx.gemv_f32(dw, dx, None, do, batch, rows, K)
+    together = _norm_err(ctx.download(do, (batch, rows), np.float32), exact)
+    one = np.empty((batch, rows), np.float32)
+    for b in range(batch):
+        d1 = ctx.upload(x[b])
+        ctx.gemv_f32(dw, d1, None, do, 1, rows, K)
+        one[b] = ctx.download(do, (rows,), np.float32)
+        d1.free()
+    assert together <= 1.02 * _norm_err(one, exact)
+    for b in (dw, dx, do):
+        b.free()
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, HW, O: 3x3 convolutions that the rule may take from the Winograd kernels, F(2,3) and F(6,3)
+    (1, 16, 7, 16), (3, 33, 9, 65), (7, 130, 14, 130), (1, 256, 14, 256), (1, 512, 7, 512), (2, 64, 56, 64), (9, 96, 17, 96)])
+def test_conv3x3_f32_is_as_accurate_as_winograd(ctx, orc, shape):
+    N, C, HW, O = shape
+    rng = np.random.Generator(np.random.PCG64(C))
+    x = rng.standard_normal((N, C, HW, HW)).astype(np.float32)
+    f = (rng.standard_normal((O, C, 3, 3)) * np.sqrt(2.0 / (9 * C))).astype(np.float32)
+    padded = np.pad(x.astype(np.float64), ((0, 0), (0, 0), (1, 1), (1, 1)))
+    exact = sum(np.einsum("ncyx,oc->noyx", padded[:, :, i:i + HW, j:j + HW], f[:, :, i, j].astype(np.float64), optimize=True)
+                for i in range(3) for j in range(3))
+    tile = 6 if HW > 16 else 2
+    dx, df, do = ctx.upload(x), ctx.upload(f), ctx.alloc(exact.size * 4)
+    dt = ctx.alloc((tile + 2) ** 2 * O * C * 4)
+    ctx.winograd_transform_filter(df, dt, C, O, tile)
+
+    def run():
+        ctx.winograd_f32(dx, df, None, do, N, C, HW, HW, O, (1, 1), (HW, HW), tile=tile, transformed=dt)
+        return _norm_err(ctx.download(do, exact.shape, np.float32), exact)
+
+    winograd = _with_options(ctx, run, f32_gather=1)
+    assert run() <= 1.05 * winograd
+    assert _with_options(ctx, run, f32_gather=2) <= 1.05 * winograd  # the direct convolution, whatever the rule says
+    for b in (dx, df, do, dt):
+        b.free()
+
+
+@pytest.mark.parametrize("maj", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("c_col", [False, True])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 63, 65, 31), (1, 64, 64, 32), (3, 65, 130, 33), (1, 130, 61, 65), (70000, 2, 3, 5)])
+def test_gemm_f32_on_cuda_cores(ctx, maj, c_col, shape):
+    """Edges of the 64 x 64 x 32 tiles in every layout.  A chain of K FMAs differs from the exact sum by at most K units of
+    2^-24 of the sum of the products' absolute values (to first order: one more for the rest)."""
+    batch, M, N, K = shape
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.standard_normal((batch, M, K)).astype(np.float32)
+    B = rng.standard_normal((batch, K, N)).astype(np.float32)
+    dA = ctx.upload(np.ascontiguousarray(np.swapaxes(A, 1, 2)) if maj[0] else A)
+    dB = ctx.upload(np.ascontiguousarray(np.swapaxes(B, 1, 2)) if maj[1] else B)
+    dC = ctx.alloc(batch * M * N * 4)
+    ctx.gemm_f32(dA, dB, dC, batch, M, N, K, bool(maj[0]), bool(maj[1]), c_col)
+    got = ctx.download(dC, (batch, N, M) if c_col else (batch, M, N), np.float32)
+    got = np.swapaxes(got, 1, 2) if c_col else got
+    A, B = A.astype(np.float64), B.astype(np.float64)
+    # (more entries than a grid has blocks along z: the tensor cores take them, three tf32 products)
+    units = K + 1 if batch <= 65535 else 32
+    assert (np.abs(got - A @ B) <= units * 2.0 ** -24 * (np.abs(A) @ np.abs(B))).all()
+    for b in (dA, dB, dC):
+        b.free()
+
+
+@pytest.mark.parametrize("maj", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("width,splits", [(64, 1), (64, 8), (128, 1)])
+@pytest.mark.parametrize("shape", [(1, 5, 63, 48), (2, 129, 65, 64), (1, 130, 129, 72), (1, 127, 200, 97), (20, 200, 300, 129),
+                                   (1, 128, 128, 384), (2, 140, 70, 449)])
+def test_gemm_f32_in_short_runs(ctx, maj, width, splits, shape):
+    """The forms whose sums leave the tensor core every few steps, at the edges of tiles, steps and runs, with several tiles
+    per CTA.  Per product 2^-22 from the split; per MMA of a run of at most 8 two units of 2^-23 from the accumulator; one of
+    2^-24 per run from the sums."""
+    batch, M, N, K = shape
+    rng = np.random.Generator(np.random.PCG64(K))
+    A = rng.standard_normal((batch, M, K)).astype(np.float32)
+    B = rng.standard_normal((batch, K, N)).astype(np.float32)
+    dA = ctx.upload(np.ascontiguousarray(np.swapaxes(A, 1, 2)) if maj[0] else A)
+    dB = ctx.upload(np.ascontiguousarray(np.swapaxes(B, 1, 2)) if maj[1] else B)
+    dC = ctx.alloc(batch * M * N * 4)
+    before = ctx.launches_tensor_core
+    _with_options(ctx, lambda: ctx.gemm_f32(dA, dB, dC, batch, M, N, K, bool(maj[0]), bool(maj[1])), f32_gather=2, f32_bn=width,
+                  f32_splits=splits)
+    assert ctx.launches_tensor_core == before + 1
+    got = ctx.download(dC, (batch, M, N), np.float32)
+    A, B = A.astype(np.float64), B.astype(np.float64)
+    bound = 2.0 ** -22 + 8 * 2 * 2.0 ** -23 + (K // 32 + 1) * 2.0 ** -24
+    if maj == (0, 0) and N % 4 == 0:  # (in TMA's layout: one run)
+        bound = 2.0 ** -21 + 3 * (K // 8 + 1) * 2 * 2.0 ** -23
+    assert (np.abs(got - A @ B) <= bound * (np.abs(A) @ np.abs(B))).all()
+    for b in (dA, dB, dC):
+        b.free()
+
+
 @pytest.mark.parametrize("shape", [(1, 1000, 2048), (3, 77, 1023), (40, 130, 516)])
 def test_gemv_f32_on_tensor_cores(ctx, orc, gather, shape):
     batch, rows, K = shape
