@@ -74,6 +74,7 @@ struct Params {
   int64_t x_ks, x_ms, x_bs, w_ns, w_ks, w_bs, c_ns, c_ms, c_bs;
   int x_vec;                   // K-contiguous rows are 16-byte aligned
   int run;                     // RUNS: steps per run
+  int exact;                   // results that are not finite are worked out again in fp32 (see store_exact4)
   int act;
   float max_limit, coef;
   int H, Wd, KW, taps, sh, sw, dh, dw, pad_t, pad_l, Wo, hw, KH;
@@ -144,6 +145,62 @@ __device__ __forceinline__ int64_t out_offset(const Params &p, int m, int b) {
   return b * p.c_bs + m * p.c_ms;
 }
 
+// Four results of a pixel by fp32 FMAs in the order of k, padding left out.  An infinity has no split (inf - inf) and neither
+// has a value that rounds beyond the largest tf32 one, so whatever they meet comes out of the tensor core as a NaN.  Results
+// that are not finite are stored as AGAIN, and when its tiles are done a CTA that stored one works those out again here,
+// which gives what the CUDA cores give.  (Results that are finite pay one FMA each for the check.  Called from the result
+// warps, tile by tile, the same code cost every launch 0.8 us, in registers that it never used; so it costs 0.2.)
+constexpr uint32_t AGAIN = 0x7fc0a6a1u;
+template <int XK>
+__device__ __noinline__ void store_exact4(const Params &p, int m, int b, int n, int n_end) {
+  const float *x = p.X, *w[4];
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) w[q] = p.W + b * p.w_bs + static_cast<int64_t>(min(n + q, n_end - 1)) * p.w_ns;
+  if (XK == X_CONV) {
+    const uint32_t img = fast_div(static_cast<uint32_t>(m), p.hw_mul, p.hw_shift);
+    const int pix = m - static_cast<int>(img) * p.hw;
+    const int ho = static_cast<int>(fast_div(static_cast<uint32_t>(pix), p.wo_mul, p.wo_shift));
+    const int h0 = ho * p.sh - p.pad_t, w0 = (pix - ho * p.Wo) * p.sw - p.pad_l;
+    x += static_cast<int64_t>(img) * p.image;
+    const int channels = p.K / p.taps;
+    int64_t k = 0;
+    for (int c = 0; c < channels; ++c, x += static_cast<int64_t>(p.H) * p.Wd)
+      for (int i = 0; i < p.KH; ++i)
+        for (int j = 0; j < p.KW; ++j, ++k) {
+          const int h = h0 + i * p.dh, col = w0 + j * p.dw;
+          if (h < 0 || h >= p.H || col < 0 || col >= p.Wd) continue;
+          const float v = x[static_cast<int64_t>(h) * p.Wd + col];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sum[q] = fmaf(v, w[q][k], sum[q]);
+        }
+  } else {
+    x += b * p.x_bs + m * p.x_ms;
+#pragma unroll 1
+    for (int k = 0; k < p.K; ++k) {
+      const float v = x[k * p.x_ks];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sum[q] = fmaf(v, w[q][k * p.w_ks], sum[q]);
+    }
+  }
+  const int64_t at = out_offset<XK>(p, m, b);
+  for (int q = 0; q < 4; ++q) {
+    const int c = n + q;
+    if (c >= n_end) return;
+    float v = sum[q];
+    if (p.bias != nullptr) v += p.bias[c];
+    if (p.residual != nullptr) v += p.residual[at + c * p.c_ns];
+    p.C[at + c * p.c_ns] = mb_activate(v, p.act, p.max_limit, p.coef);
+  }
+}
+template <int COUNT>
+__device__ __forceinline__ bool all_finite(const float (&x)[COUNT]) {
+  float z = 0.f;
+#pragma unroll
+  for (int j = 0; j < COUNT; ++j) z = fmaf(x[j], 0.f, z);
+  return z == 0.f;
+}
+
 template <int BN, int XK, int WK, int EW, int MODE>
 __global__ void __launch_bounds__(threads(EW), 1)
 gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Params p) {
@@ -158,6 +215,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   const uint32_t tfull_bar = wfull_bar + 8 * STAGES, tempty_bar = tfull_bar + 8 * ACCS;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + C::RING + C::TABLE_BYTES + 24 * STAGES + 16 * ACCS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  volatile int *again = abort_flag + 1;  // a result is not finite
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr uint32_t half = MODE != WHOLE ? 0x1000u : 0u;
   mb_grid_dep_launch();
@@ -174,6 +232,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       mbar_init(tempty_bar + 8 * a, EW);
     }
     *abort_flag = 0;
+    *again = 0;
     fence_barrier_init();
   }
   if (warp == FIRST_E) {
@@ -561,6 +620,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             push8(x + 8, c + 8);
             continue;
           }
+          const bool finite = MODE == WHOLE || !p.exact || all_finite(x);
           if (p.bias != nullptr) {
             const float mine = n0 + c + (lane & 15) < p.N ? __ldg(p.bias + n0 + c + (lane & 15)) : 0.f;
 #pragma unroll
@@ -575,6 +635,11 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             for (int j = 0; j < 16; ++j) x[j] += res[j];
           }
           mb_activate_n(x, p.act, p.max_limit, p.coef);
+          if (MODE != WHOLE && !finite) {
+            *again = 1;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(AGAIN);
+          }
           float *dst = p.C + at + static_cast<int64_t>(n0 + c) * p.c_ns;
           if (n0 + c + 16 <= p.N) {
             if (m < p.M) {
@@ -611,25 +676,26 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     if (warp < 16 && m < p.M) {
       // up to four channels per round, all loads before the first store (see above)
       for (int c0 = warp >> 2; c0 < share; c0 += 16) {
-        float x[4], add[4];
+        float x[4], bias[4], add[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int c = c0 + q * 4, n = n0 + c;
-          x[q] = add[q] = 0.f;
+          x[q] = bias[q] = add[q] = 0.f;
           if (c < share && n < p.N) {
             if (p.residual != nullptr) add[q] = __ldg(p.residual + at + static_cast<int64_t>(n) * p.c_ns);
-            const float b = p.bias != nullptr ? __ldg(p.bias + n) : 0.f;
+            if (p.bias != nullptr) bias[q] = __ldg(p.bias + n);
             for (int s = 0; s < p.splits; ++s) x[q] += mine[(s * share + c) * BM];
-            x[q] += b;
           }
         }
+        const bool finite = MODE == WHOLE || !p.exact || all_finite(x);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) x[q] += add[q];
+        for (int q = 0; q < 4; ++q) x[q] = (x[q] + bias[q]) + add[q];
+        if (MODE != WHOLE && !finite) *again = 1;
         mb_activate_n(x, p.act, p.max_limit, p.coef);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int c = c0 + q * 4, n = n0 + c;
-          if (c < share && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = x[q];
+          if (c < share && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = finite ? x[q] : __uint_as_float(AGAIN);
         }
       }
     }
@@ -637,6 +703,24 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   if (warp == FIRST_E) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, 512);
+  }
+  if (MODE != WHOLE && p.exact) {
+    if (p.splits > 1) __syncthreads();
+    if (*again == 0 || *abort_flag != 0) return;
+    mb_grid_dep_wait();  // (one of the warps may have had nothing to wait for so far)
+    const int width = BN / p.splits;
+    for (TileIter t(p); t.valid(p); t.next(p)) {
+      const int n_begin = t.tn * BN + rank * width, n_end = min(p.N, n_begin + width);
+      for (int i = threadIdx.x; i < BM * (width / 4); i += blockDim.x) {
+        const int m = t.tm * BM + (i & (BM - 1)), n = n_begin + (i / BM) * 4;
+        if (m >= p.M || n >= n_end) continue;
+        const float *stored = p.C + out_offset<XK>(p, m, t.b) + n * p.c_ns;
+        bool found = false;
+        for (int q = 0; q < 4 && n + q < n_end; ++q) found |= __float_as_uint(stored[q * p.c_ns]) == AGAIN;
+        if (found) store_exact4<XK>(p, m, t.b, n, n_end);
+      }
+      if (p.splits > 1) break;
+    }
   }
 }
 
@@ -733,6 +817,7 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
   p.k_blocks = static_cast<int>(ceil_div64(g.K, KB));
   p.splits = plan.splits;
   p.run = plan.bn == 128 ? std::min(g.run, 2) : g.run;  // (of the four steps that its ring holds)
+  p.exact = g.run != 0;
   p.x_ks = g.x_ks; p.x_ms = g.x_ms; p.x_bs = g.x_bs;
   p.w_ns = g.w_ns; p.w_ks = g.w_ks; p.w_bs = g.w_bs;
   p.c_ns = g.c_ns; p.c_ms = g.c_ms; p.c_bs = g.c_bs;

@@ -439,6 +439,65 @@ def test_gemm_f32_in_short_runs(ctx, maj, width, splits, shape):
         b.free()
 
 
+INF_CASES = [("inf", np.inf), ("-inf", -np.inf), ("largest", np.finfo(np.float32).max), ("nan", np.nan)]
+
+
+@pytest.mark.parametrize("name,value", INF_CASES)
+@pytest.mark.parametrize("maj", [(0, 1), (1, 0)])
+@pytest.mark.parametrize("shape", [(1, 30, 37, 20), (2, 130, 70, 64), (1, 140, 200, 100), (1, 129, 65, 1000)])
+def test_gemm_f32_of_infinite_operands(ctx, maj, shape, name, value):
+    """Infinities, values at the end of the range and NaNs give what IEEE arithmetic gives, at every tile width and with
+    the depth cut.  (The other operands are small powers of two, exact in every split, and no finite sum overflows.)"""
+    batch, M, N, K = shape
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.choice(np.float32([-0.5, -0.25, 0.25, 0.5]), (batch, M, K))
+    B = rng.choice(np.float32([-0.5, -0.25, 0.25, 0.5]), (batch, K, N))
+    A[0, M - 1, K // 2] = value      # a row with one of them,
+    A[0, 3, 1], B[0, 1, 5] = value, 0  # one that meets a zero,
+    B[-1, K - 1, N - 1] = value      # and a column
+    B[0, [K // 2, 1], N - 1] = A[0, [M - 1, 3], K - 1] = 0.25  # (where both meet, nothing cancels)
+    dA = ctx.upload(np.ascontiguousarray(np.swapaxes(A, 1, 2)) if maj[0] else A)
+    dB = ctx.upload(np.ascontiguousarray(np.swapaxes(B, 1, 2)) if maj[1] else B)
+    dC = ctx.alloc(batch * M * N * 4)
+    with np.errstate(all="ignore"):
+        exact = np.einsum("bmk,bkn->bmn", A.astype(np.float64), B.astype(np.float64))
+    settings = [{}] + ([dict(f32_gather=2, f32_bn=64, f32_splits=8), dict(f32_gather=2, f32_bn=128, f32_splits=1)]
+                       if mb_f32_gather_run(K) else [])
+    for options in settings:
+        _with_options(ctx, lambda: ctx.gemm_f32(dA, dB, dC, batch, M, N, K, bool(maj[0]), bool(maj[1])), **options)
+        got = ctx.download(dC, (batch, M, N), np.float32)
+        assert np.array_equal(np.isnan(got), np.isnan(exact)), options
+        with np.errstate(all="ignore"):
+            near = np.isnan(exact) | (got == exact) | (np.abs(got - exact) <= 1e-6 * (np.abs(exact) + K))
+        assert near.all(), options
+    for b in (dA, dB, dC):
+        b.free()
+
+
+@pytest.mark.parametrize("splits", [0, 1, 4])
+def test_conv2d_f32_of_an_infinite_pixel(ctx, orc, splits):
+    """A small convolution (padding taps left out, bias, activation, residual) around one infinite pixel and one infinite
+    weight."""
+    N, C, HW, O = 1, 32, 5, 70
+    rng = np.random.Generator(np.random.PCG64(0))
+    x = rng.choice(np.float32([-0.5, 0.25, 0.5]), (N, C, HW, HW))
+    f = rng.choice(np.float32([-0.5, 0.25, 0.5]), (O, C, 3, 3))
+    bias, r = rng.standard_normal(O).astype(np.float32), rng.standard_normal((N, O, HW, HW)).astype(np.float32)
+    x[0, 3, 0, 1], f[7, 2, 0, 0] = np.inf, -np.inf
+    ref = np.fmax(orc.conv2d_f32(x, f, bias, (1, 1), (1, 1), (1, 1), (HW, HW), 0) + r, 0)  # (a NaN becomes 0, as in ref::Activation)
+    assert np.isinf(ref).any() and np.isfinite(ref).any()
+    dx, df, db, dr, do = (ctx.upload(a) for a in (x, f, bias, r, np.zeros_like(ref)))
+    options = dict(f32_gather=2, f32_bn=64, f32_splits=splits) if splits else {}
+    _with_options(ctx, lambda: ctx.conv2d_f32_residual(dx, df, db, dr, do, N, C, HW, HW, O, 3, 3, (1, 1), (1, 1), (1, 1),
+                                                       (HW, HW), 1), **options)
+    got = ctx.download(do, ref.shape, np.float32)
+    assert np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(np.isnan(got), np.isnan(ref))
+    finite = np.isfinite(ref)
+    assert np.abs(got[finite] - ref[finite]).max() <= 1e-4
+    for b in (dx, df, db, dr, do):
+        b.free()
+
+
 @pytest.mark.parametrize("shape", [(1, 1000, 2048), (3, 77, 1023), (40, 130, 516)])
 def test_gemv_f32_on_tensor_cores(ctx, orc, gather, shape):
     batch, rows, K = shape
