@@ -122,6 +122,12 @@ __device__ __forceinline__ void mb_grid_dep_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A load of what the kernel in front may have written.  An ordinary one: the read-only path (__ldg, a pointer that is const and
+// __restrict__) is for data that do not change while the kernel runs, and the compiler may move such a load above
+// mb_grid_dep_wait(); but a chained kernel runs already while its predecessor writes.
+template <typename T>
+__device__ __forceinline__ T mb_load(const T *p) { return *p; }
+
 template <typename... KArgs, typename... Args>
 static inline cudaError_t mb_launch_chained(mb_context *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block,
                                             size_t smem, Args &&...args) {

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(128) conv_u8_direct_kernel(const ConvParams p)
         const uint8_t *ip = in_n + (static_cast<int64_t>(hi) * p.W + wi) * p.C;
         const int16_t *fp = fsm + ((kh * p.KW + kw) * p.C) * p.O + o0;
         for (int c = 0; c < p.C; ++c) {
-          const int32_t iv = static_cast<int32_t>(__ldg(ip + c)) - p.zp_in;
+          const int32_t iv = static_cast<int32_t>(mb_load(ip + c)) - p.zp_in;
 #pragma unroll
           for (int j = 0; j < OT; ++j)
             if (o0 + j < p.O) acc[j] += iv * fp[c * p.O + j];
@@ -209,7 +209,7 @@ __device__ __forceinline__ void gather_patch(const ConvParams &p, int64_t pix, u
 #pragma unroll
       for (int kh = 0; kh < 3; ++kh) {
         const uint32_t *wp = reinterpret_cast<const uint32_t *>(in_n + first[kh]);
-        const uint32_t w0 = __ldg(wp), w1 = __ldg(wp + 1), w2 = __ldg(wp + 2);
+        const uint32_t w0 = mb_load(wp), w1 = mb_load(wp + 1), w2 = mb_load(wp + 2);
         const uint32_t f0 = __funnelshift_r(w0, w1, sh[kh]), f1 = __funnelshift_r(w1, w2, sh[kh]), f2 = w2 >> sh[kh];
         r[kh][0] = row_ok[kh] ? ((f0 & m0) | (zi4 & ~m0)) : zi4;
         r[kh][1] = row_ok[kh] ? ((f1 & m1) | (zi4 & ~m1)) : zi4;
@@ -237,7 +237,7 @@ __device__ __forceinline__ void gather_patch(const ConvParams &p, int64_t pix, u
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         const int d = (kh * KW + kw) * C + c;  // compile-time
-        const uint32_t v = ok ? static_cast<uint32_t>(__ldg(ip + c)) : zi;
+        const uint32_t v = ok ? static_cast<uint32_t>(mb_load(ip + c)) : zi;
         patch[d >> 2] |= v << (8 * (d & 3));
       }
     }
@@ -368,14 +368,14 @@ __global__ void __launch_bounds__(128, 8) conv_u8_stem_mma_kernel(const Params q
     const int n = i / PLANES, piece = i % PLANES;
     uint4 v4;
     if (filter_words) {
-      v4 = __ldg(reinterpret_cast<const uint4 *>(p.filter + n * KD + piece * 16));
+      v4 = mb_load(reinterpret_cast<const uint4 *>(p.filter + n * KD + piece * 16));
     } else {
       uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
       for (int b = 0; b < 16; ++b) {
         const int k = piece * 16 + b;
         uint32_t v = 0;
-        if (k < KD) v = static_cast<uint32_t>(__ldg(p.filter + n * KD + k));
+        if (k < KD) v = static_cast<uint32_t>(mb_load(p.filter + n * KD + k));
         w[b >> 2] |= v << (8 * (b & 3));
       }
       v4 = make_uint4(w[0], w[1], w[2], w[3]);
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(128, 8) conv_u8_stem_mma_kernel(const Params q
         uint4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (p0 + j < PLANES) v[j] = pix < npix ? __ldg(row + p0 + j) : make_uint4(0, 0, 0, 0);
+          if (p0 + j < PLANES) v[j] = pix < npix ? mb_load(row + p0 + j) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           if (p0 + j < PLANES) {
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(256) im2col_u8_kernel(const ConvParams p, uint
     if ((p.C & 15) == 0 && (p.depth_padded & 15) == 0 &&
         ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0) {
       for (int c = 0; c < p.C; c += 16)
-        *reinterpret_cast<uint4 *>(dst + c) = __ldg(reinterpret_cast<const uint4 *>(src + c));
+        *reinterpret_cast<uint4 *>(dst + c) = mb_load(reinterpret_cast<const uint4 *>(src + c));
     } else {
       for (int c = 0; c < p.C; ++c) dst[c] = src[c];
     }
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(256) im2col_u8_kernel(const ConvParams p, uint
 }
 
 // Copy the [O x depth] filter into [O x depth_padded] with a zero tail.
-__global__ void __launch_bounds__(256) pad_rows_u8_kernel(const uint8_t *__restrict__ src,
+__global__ void __launch_bounds__(256) pad_rows_u8_kernel(const uint8_t *src,
                                                           uint8_t *__restrict__ dst, int64_t rows,
                                                           int len, int len_padded) {
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;

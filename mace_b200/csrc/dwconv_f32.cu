@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(256) dwconv_f32_rows_kernel(const DwF32Params 
   const uint32_t m = plane - n * static_cast<uint32_t>(p.C * p.mult_ch);
   const uint32_t c = fast_div(m, p.mc_mul, p.mc_shift);
   const uint32_t o = m - c * static_cast<uint32_t>(p.mult_ch);
-  const float *__restrict__ in = p.in + (static_cast<int64_t>(n) * p.C + c) * (static_cast<int64_t>(p.H) * p.W);
-  const float *__restrict__ fp = p.filter + (static_cast<int64_t>(o) * p.C + c) * (K * K);
+  const float *in = p.in + (static_cast<int64_t>(n) * p.C + c) * (static_cast<int64_t>(p.H) * p.W);
+  const float *fp = p.filter + (static_cast<int64_t>(o) * p.C + c) * (K * K);
   const int iw0 = w * S - p.pad_l, ih0 = h0 * S - p.pad_t;
   bool col_ok[K];
 #pragma unroll
@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(256) dwconv_f32_rows_kernel(const DwF32Params 
   mb_grid_dep_wait();
   float f[K * K];
 #pragma unroll
-  for (int i = 0; i < K * K; ++i) f[i] = __ldg(fp + i);
-  const float bias = p.bias != nullptr ? __ldg(p.bias + m) : 0.f;
+  for (int i = 0; i < K * K; ++i) f[i] = mb_load(fp + i);
+  const float bias = p.bias != nullptr ? mb_load(p.bias + m) : 0.f;
   float acc[RH];
 #pragma unroll
   for (int r = 0; r < RH; ++r) acc[r] = 0.f;
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256) dwconv_f32_rows_kernel(const DwF32Params 
     const bool row_ok = ih0 + i >= 0 && ih0 + i < p.H;
     float x[K];
 #pragma unroll
-    for (int j = 0; j < K; ++j) x[j] = (row_ok && col_ok[j]) ? __ldg(row + j) : 0.f;
+    for (int j = 0; j < K; ++j) x[j] = (row_ok && col_ok[j]) ? mb_load(row + j) : 0.f;
     row += p.W;
 #pragma unroll
     for (int r = 0; r < RH; ++r) {
@@ -101,15 +101,15 @@ __global__ void __launch_bounds__(256) dwconv_f32_wide_kernel(const DwF32Params 
   const uint32_t m = plane - n * static_cast<uint32_t>(p.C * p.mult_ch);
   const uint32_t c = fast_div(m, p.mc_mul, p.mc_shift);
   const uint32_t o = m - c * static_cast<uint32_t>(p.mult_ch);
-  const float *__restrict__ in = p.in + (static_cast<int64_t>(n) * p.C + c) * (static_cast<int64_t>(p.H) * p.W);
-  const float *__restrict__ fp = p.filter + (static_cast<int64_t>(o) * p.C + c) * 9;
+  const float *in = p.in + (static_cast<int64_t>(n) * p.C + c) * (static_cast<int64_t>(p.H) * p.W);
+  const float *fp = p.filter + (static_cast<int64_t>(o) * p.C + c) * 9;
   const int ih0 = h0 * S - p.pad_t;
   const bool left = w > 0, right = w * S + 4 < p.W;
   mb_grid_dep_wait();
   float f[9];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) f[i] = __ldg(fp + i);
-  const float bias = p.bias != nullptr ? __ldg(p.bias + m) : 0.f;
+  for (int i = 0; i < 9; ++i) f[i] = mb_load(fp + i);
+  const float bias = p.bias != nullptr ? mb_load(p.bias + m) : 0.f;
   float acc[RH * V];
 #pragma unroll
   for (int r = 0; r < RH * V; ++r) acc[r] = 0.f;
@@ -117,11 +117,11 @@ __global__ void __launch_bounds__(256) dwconv_f32_wide_kernel(const DwF32Params 
 #pragma unroll
   for (int i = 0; i < (RH - 1) * S + 3; ++i) {
     const bool row_ok = ih0 + i >= 0 && ih0 + i < p.H;
-    const float4 mid = row_ok ? __ldg(reinterpret_cast<const float4 *>(row)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float last = row_ok && right ? __ldg(row + 4) : 0.f;
+    const float4 mid = row_ok ? mb_load(reinterpret_cast<const float4 *>(row)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float last = row_ok && right ? mb_load(row + 4) : 0.f;
     float x[COLS];
     if (S == 1) {
-      x[0] = row_ok && left ? __ldg(row - 1) : 0.f;
+      x[0] = row_ok && left ? mb_load(row - 1) : 0.f;
       x[1] = mid.x; x[2] = mid.y; x[3] = mid.z; x[4] = mid.w;
     } else {
       x[0] = mid.x; x[1] = mid.y; x[2] = mid.z; x[3] = mid.w;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) dwconv_f32_kernel(const DwF32Params p) {
     for (int kw = 0; kw < p.KW; ++kw) {
       const int iw = -p.pad_l + w * p.sw + kw * p.dw;
       if (iw < 0 || iw >= p.W) continue;
-      sum = fmaf(__ldg(ib + ih * p.W + iw), __ldg(fp + kh * p.KW + kw), sum);
+      sum = fmaf(mb_load(ib + ih * p.W + iw), mb_load(fp + kh * p.KW + kw), sum);
     }
   }
   if (p.bias != nullptr) sum += p.bias[m];

@@ -78,7 +78,7 @@ __device__ __forceinline__ int32_t dp4a_u8_s8(uint32_t a, uint32_t b, int32_t c)
 }
 
 __global__ void __launch_bounds__(128)
-dwconv3x3_prepack_kernel(const uint8_t *__restrict__ filter, const int32_t *__restrict__ bias,
+dwconv3x3_prepack_kernel(const uint8_t *filter, const int32_t *bias,
                          uint4 *__restrict__ packed, int C, int32_t zp_in, int32_t zp_f) {
   const int groups = C >> 2;
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -86,7 +86,7 @@ dwconv3x3_prepack_kernel(const uint8_t *__restrict__ filter, const int32_t *__re
   int32_t w[9][4];
 #pragma unroll
   for (int t = 0; t < 9; ++t) {
-    const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(filter + t * C + g * 4));
+    const uint32_t v = mb_load(reinterpret_cast<const uint32_t *>(filter + t * C + g * 4));
 #pragma unroll
     for (int c = 0; c < 4; ++c) w[t][c] = static_cast<int32_t>((v >> (8 * c)) & 0xffu) - zp_f;
   }
@@ -113,7 +113,7 @@ dwconv3x3_prepack_kernel(const uint8_t *__restrict__ filter, const int32_t *__re
       v1[kh][0][c] = p1; v1[kh][1][c] = p1 << 8;
       v2[kh][0][c] = p2; v2[kh][1][c] = p2 << 8;
     }
-    const int32_t bv = bias != nullptr ? __ldg(bias + g * 4 + c) : 0;
+    const int32_t bv = bias != nullptr ? mb_load(bias + g * 4 + c) : 0;
     start[c] = bv - zp_in * sum;
   }
 #pragma unroll
@@ -147,7 +147,7 @@ struct DwRaw {
 // 32-bit offset (the host keeps the fast path to tensors below 4 GB), which keeps the
 // per-load address arithmetic to one 32-bit addition.
 template <int STRIDE>
-__device__ __forceinline__ void dw_load_raw(DwRaw<STRIDE> &raw, const uint8_t *__restrict__ in,
+__device__ __forceinline__ void dw_load_raw(DwRaw<STRIDE> &raw, const uint8_t *in,
                                             uint32_t thread_off, int hi, int H, uint32_t row_stride,
                                             const uint32_t (&col_off)[STRIDE == 1 ? 6 : 9],
                                             uint32_t col_ok, uint32_t zi4) {
@@ -162,11 +162,11 @@ __device__ __forceinline__ void dw_load_raw(DwRaw<STRIDE> &raw, const uint8_t *_
   if (col_ok == ALL) {
 #pragma unroll
     for (int j = 0; j < COLS; ++j)
-      raw.q[j] = __ldg(reinterpret_cast<const uint32_t *>(in + (row_off + col_off[j])));
+      raw.q[j] = mb_load(reinterpret_cast<const uint32_t *>(in + (row_off + col_off[j])));
   } else {
 #pragma unroll
     for (int j = 0; j < COLS; ++j)
-      raw.q[j] = ((col_ok >> j) & 1u) ? __ldg(reinterpret_cast<const uint32_t *>(in + (row_off + col_off[j]))) : zi4;
+      raw.q[j] = ((col_ok >> j) & 1u) ? mb_load(reinterpret_cast<const uint32_t *>(in + (row_off + col_off[j]))) : zi4;
   }
 }
 
@@ -220,7 +220,7 @@ __device__ __forceinline__ void dw_mac(int32_t (&acc)[4][4], const DwRow<STRIDE>
 // VAR: requantization variant (mb_requant_variant): 0..3 = mb_requant_t, 4 / 5 = packed form.
 template <int STRIDE, int VAR>
 __global__ void __launch_bounds__(DW_THREADS, DW_BLOCKS_PER_SM)
-dwconv3x3_u8_kernel(const DwParams p, const uint4 *__restrict__ packed, int rows_per_thread,
+dwconv3x3_u8_kernel(const DwParams p, const uint4 *packed, int rows_per_thread,
                     int segments, int weights_cached) {
   constexpr int COLS = STRIDE == 1 ? 6 : 9;
   mb_grid_dep_launch();
@@ -249,12 +249,12 @@ dwconv3x3_u8_kernel(const DwParams p, const uint4 *__restrict__ packed, int rows
   uint4 w1[3][2];
 #pragma unroll
   for (int kh = 0; kh < 3; ++kh) {
-    w1[kh][0] = __ldg(packed + (kh * 2 + 0) * groups + g);
-    if (STRIDE == 1) w1[kh][1] = __ldg(packed + (kh * 2 + 1) * groups + g);
+    w1[kh][0] = mb_load(packed + (kh * 2 + 0) * groups + g);
+    if (STRIDE == 1) w1[kh][1] = mb_load(packed + (kh * 2 + 1) * groups + g);
     else w1[kh][1] = w1[kh][0];
   }
-  const uint4 st4 = __ldg(packed + 12 * groups + g);
-  const uint4 flags = __ldg(packed + 13 * groups + g);
+  const uint4 st4 = mb_load(packed + 12 * groups + g);
+  const uint4 flags = mb_load(packed + 13 * groups + g);
   const int32_t start[4] = {static_cast<int32_t>(st4.x), static_cast<int32_t>(st4.y),
                             static_cast<int32_t>(st4.z), static_cast<int32_t>(st4.w)};
   const bool has_w2 = flags.x != 0;
@@ -278,7 +278,7 @@ dwconv3x3_u8_kernel(const DwParams p, const uint4 *__restrict__ packed, int rows
   const uint32_t out_row_stride = static_cast<uint32_t>(p.Wo) * p.C;
   const uint32_t out_off = n * static_cast<uint32_t>(p.Ho) * out_row_stride + g * 4 +
                            static_cast<uint32_t>(x0) * p.C;
-  const uint8_t *__restrict__ in = p.in;
+  const uint8_t *in = p.in;
   uint8_t *__restrict__ out = p.out;
   const int valid_cols = min(4, p.Wo - x0);
 
@@ -293,9 +293,9 @@ dwconv3x3_u8_kernel(const DwParams p, const uint4 *__restrict__ packed, int rows
     dw_mac<STRIDE>(acc, r1, w1[1][0], w1[1][1]);
     dw_mac<STRIDE>(acc, r2, w1[2][0], w1[2][1]);
     if (has_w2) {
-      if (rows_w2 & 1u) dw_mac<STRIDE>(acc, r0, __ldg(packed + 6 * groups + g), __ldg(packed + 7 * groups + g));
-      if (rows_w2 & 2u) dw_mac<STRIDE>(acc, r1, __ldg(packed + 8 * groups + g), __ldg(packed + 9 * groups + g));
-      if (rows_w2 & 4u) dw_mac<STRIDE>(acc, r2, __ldg(packed + 10 * groups + g), __ldg(packed + 11 * groups + g));
+      if (rows_w2 & 1u) dw_mac<STRIDE>(acc, r0, mb_load(packed + 6 * groups + g), mb_load(packed + 7 * groups + g));
+      if (rows_w2 & 2u) dw_mac<STRIDE>(acc, r1, mb_load(packed + 8 * groups + g), mb_load(packed + 9 * groups + g));
+      if (rows_w2 & 4u) dw_mac<STRIDE>(acc, r2, mb_load(packed + 10 * groups + g), mb_load(packed + 11 * groups + g));
     }
     uint32_t o = out_off + static_cast<uint32_t>(y) * out_row_stride;
 #pragma unroll
@@ -392,7 +392,7 @@ constexpr long long DW_WAIT_BUDGET = 1ll << 31;
 template <int STRIDE, int VAR, int GT = 0>
 __global__ void __launch_bounds__(DW_THREADS, DW_BLOCKS_PER_SM)
 dwconv3x3_u8_tma_kernel(const __grid_constant__ CUtensorMap tmap_in, const DwParams p,
-                        const uint4 *__restrict__ packed, const DwTmaTile t, int weights_cached) {
+                        const uint4 *packed, const DwTmaTile t, int weights_cached) {
   extern __shared__ uint8_t dw_smem_raw[];
   __shared__ int abort_flag;
   constexpr int COLS = STRIDE == 1 ? 6 : 9;
@@ -429,12 +429,12 @@ dwconv3x3_u8_tma_kernel(const __grid_constant__ CUtensorMap tmap_in, const DwPar
   uint4 w1[3][2];
 #pragma unroll
   for (int kh = 0; kh < 3; ++kh) {
-    w1[kh][0] = __ldg(packed + (kh * 2 + 0) * groups + gg);
-    if (STRIDE == 1) w1[kh][1] = __ldg(packed + (kh * 2 + 1) * groups + gg);
+    w1[kh][0] = mb_load(packed + (kh * 2 + 0) * groups + gg);
+    if (STRIDE == 1) w1[kh][1] = mb_load(packed + (kh * 2 + 1) * groups + gg);
     else w1[kh][1] = w1[kh][0];
   }
-  const uint4 st4 = __ldg(packed + 12 * groups + gg);
-  const uint4 flags = __ldg(packed + 13 * groups + gg);
+  const uint4 st4 = mb_load(packed + 12 * groups + gg);
+  const uint4 flags = mb_load(packed + 13 * groups + gg);
   const int32_t start[4] = {static_cast<int32_t>(st4.x), static_cast<int32_t>(st4.y),
                             static_cast<int32_t>(st4.z), static_cast<int32_t>(st4.w)};
   // the filter rows that have a 9-bit tap in ANY lane's channel group (rare: most warps skip most
@@ -482,9 +482,9 @@ dwconv3x3_u8_tma_kernel(const __grid_constant__ CUtensorMap tmap_in, const DwPar
     dw_mac<STRIDE>(acc, r0, w1[0][0], w1[0][1]);
     dw_mac<STRIDE>(acc, r1, w1[1][0], w1[1][1]);
     dw_mac<STRIDE>(acc, r2, w1[2][0], w1[2][1]);
-    if (rows_w2 & 1u) dw_mac<STRIDE>(acc, r0, __ldg(packed + 6 * groups + gg), __ldg(packed + 7 * groups + gg));
-    if (rows_w2 & 2u) dw_mac<STRIDE>(acc, r1, __ldg(packed + 8 * groups + gg), __ldg(packed + 9 * groups + gg));
-    if (rows_w2 & 4u) dw_mac<STRIDE>(acc, r2, __ldg(packed + 10 * groups + gg), __ldg(packed + 11 * groups + gg));
+    if (rows_w2 & 1u) dw_mac<STRIDE>(acc, r0, mb_load(packed + 6 * groups + gg), mb_load(packed + 7 * groups + gg));
+    if (rows_w2 & 2u) dw_mac<STRIDE>(acc, r1, mb_load(packed + 8 * groups + gg), mb_load(packed + 9 * groups + gg));
+    if (rows_w2 & 4u) dw_mac<STRIDE>(acc, r2, mb_load(packed + 10 * groups + gg), mb_load(packed + 11 * groups + gg));
     uint32_t o = out_off + static_cast<uint32_t>(y) * out_row_stride;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

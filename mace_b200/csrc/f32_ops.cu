@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(128) gemm_f32_kernel(const GemmF32Params p) {
 // many rows in flight as warps fit.
 template <int VECS, bool VEC4>
 __global__ void __launch_bounds__(256)
-gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs, const float *__restrict__ bias,
+gemv_f32_kernel(const float *lhs, const float *rhs, const float *bias,
                 float *__restrict__ out, int64_t batch, int64_t rows, int64_t K, int lhs_batched, int rhs_batched) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -187,11 +187,11 @@ gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs, co
     if (VEC4) {
 #pragma unroll 4
       for (int64_t i = lane * 4; i < K; i += 128) {
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(lp + i));
+        const float4 a = mb_load(reinterpret_cast<const float4 *>(lp + i));
 #pragma unroll
         for (int v = 0; v < VECS; ++v) {
           if (v < vecs) {
-            const float4 x = __ldg(reinterpret_cast<const float4 *>(rp + v * K + i));
+            const float4 x = mb_load(reinterpret_cast<const float4 *>(rp + v * K + i));
             s[v] = fmaf(a.x, x.x, s[v]); s[v] = fmaf(a.y, x.y, s[v]);
             s[v] = fmaf(a.z, x.z, s[v]); s[v] = fmaf(a.w, x.w, s[v]);
           }
@@ -200,17 +200,17 @@ gemv_f32_kernel(const float *__restrict__ lhs, const float *__restrict__ rhs, co
     } else {
 #pragma unroll 4
       for (int64_t i = lane; i < K; i += 32) {
-        const float a = __ldg(lp + i);
+        const float a = mb_load(lp + i);
 #pragma unroll
         for (int v = 0; v < VECS; ++v)
-          if (v < vecs) s[v] = fmaf(a, __ldg(rp + v * K + i), s[v]);
+          if (v < vecs) s[v] = fmaf(a, mb_load(rp + v * K + i), s[v]);
       }
     }
 #pragma unroll
     for (int v = 0; v < VECS; ++v) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s[v] += __shfl_xor_sync(0xffffffffu, s[v], o);
-      if (lane == 0 && v < vecs) out[(b0 + v) * rows + row] = s[v] + (bias != nullptr ? __ldg(bias + row) : 0.f);
+      if (lane == 0 && v < vecs) out[(b0 + v) * rows + row] = s[v] + (bias != nullptr ? mb_load(bias + row) : 0.f);
     }
   }
 }
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) conv2d_f32_direct_kernel(const ConvF32Par
       for (int kw = 0; kw < p.KW; ++kw) {
         const int iw = -p.pad_l + w * p.sw + kw * p.dw;
         if (iw < 0 || iw >= p.W) continue;
-        sum = fmaf(__ldg(ib + ih * p.W + iw), __ldg(fp + kh * p.KW + kw), sum);
+        sum = fmaf(mb_load(ib + ih * p.W + iw), mb_load(fp + kh * p.KW + kw), sum);
       }
     }
   }
@@ -273,7 +273,7 @@ struct ColF32Params {
 __global__ void __launch_bounds__(128) im2col_f32_kernel(const ColF32Params p, int rows_per_block) {
   const int h = blockIdx.x * blockDim.y + threadIdx.y, n = blockIdx.z;
   if (h >= p.Ho) return;
-  const float *__restrict__ in = p.in;
+  const float *in = p.in;
   float *__restrict__ col = p.col;
   const int y_end = min((static_cast<int>(blockIdx.y) + 1) * rows_per_block, p.C * p.KH);
   // Up to eight values are loaded before the first is stored: a store waits for the load that
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(128) im2col_f32_kernel(const ColF32Params p, i
           const int c = y / p.KH, kh = y - c * p.KH;
           const int ih = h * p.sh - p.pad_t + kh * p.dh;
           const bool ok = y < y_end && col_ok && ih >= 0 && ih < p.H;
-          v[j] = ok ? __ldg(in + ((static_cast<int64_t>(n) * p.C + c) * p.H + ih) * p.W + iw) : 0.f;
+          v[j] = ok ? mb_load(in + ((static_cast<int64_t>(n) * p.C + c) * p.H + ih) * p.W + iw) : 0.f;
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(128) im2col_f32_kernel(const ColF32Params p, i
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int iw = iw0 + (kw0 + j) * p.dw;
-          v[j] = (kw0 + j < p.KW && row_ok && iw >= 0 && iw < p.W) ? __ldg(src + iw) : 0.f;
+          v[j] = (kw0 + j < p.KW && row_ok && iw >= 0 && iw < p.W) ? mb_load(src + iw) : 0.f;
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -325,16 +325,16 @@ __global__ void __launch_bounds__(128) im2col_f32_kernel(const ColF32Params p, i
 
 // rows of K floats -> rows of Kp floats (a 16-byte multiple, which a tensor map's strides need)
 __global__ void __launch_bounds__(256)
-repack_rows_f32_kernel(const float *__restrict__ src, float *__restrict__ dst, int64_t rows, int K, int Kp) {
+repack_rows_f32_kernel(const float *src, float *__restrict__ dst, int64_t rows, int K, int Kp) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= rows * Kp) return;
   const int k = static_cast<int>(i % Kp);
-  dst[i] = k < K ? __ldg(src + (i / Kp) * K + k) : 0.f;
+  dst[i] = k < K ? mb_load(src + (i / Kp) * K + k) : 0.f;
 }
 
 // merged product [O][images * hw] (row stride src_rs) -> NCHW images
 __global__ void __launch_bounds__(256)
-unmerge_f32_kernel(const float *__restrict__ src, float *__restrict__ dst, int64_t total, int O, int hw,
+unmerge_f32_kernel(const float *src, float *__restrict__ dst, int64_t total, int O, int hw,
                    int64_t src_rs) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= total) return;
@@ -342,7 +342,7 @@ unmerge_f32_kernel(const float *__restrict__ src, float *__restrict__ dst, int64
   const int64_t r = i / hw;
   const int o = static_cast<int>(r % O);
   const int64_t n = r / O;
-  dst[i] = __ldg(src + o * src_rs + n * hw + pos);
+  dst[i] = mb_load(src + o * src_rs + n * hw + pos);
 }
 
 }  // namespace

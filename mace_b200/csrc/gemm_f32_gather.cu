@@ -293,12 +293,12 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #pragma unroll
             for (int j = 0; j < KB; j += 4) {
               const bool in = valid != 0 && k0 + j < p.K;
-              const float4 x = in ? __ldg(reinterpret_cast<const float4 *>(row + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              const float4 x = in ? mb_load(reinterpret_cast<const float4 *>(row + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
               v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < KB; ++j) v[j] = valid != 0 && k0 + j < p.K ? __ldg(row + j) : 0.f;
+            for (int j = 0; j < KB; ++j) v[j] = valid != 0 && k0 + j < p.K ? mb_load(row + j) : 0.f;
           }
         } else {
           const int k = k0 + lane;
@@ -323,8 +323,8 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #pragma unroll
           for (int j = 0; j < KB; j += 2) {
             const int4 t2 = *reinterpret_cast<const int4 *>(table + j);
-            v[j] = (valid & t2.y) == static_cast<uint32_t>(t2.y) ? __ldg(base + t2.x) : 0.f;
-            v[j + 1] = (valid & t2.w) == static_cast<uint32_t>(t2.w) ? __ldg(base + t2.z) : 0.f;
+            v[j] = (valid & t2.y) == static_cast<uint32_t>(t2.y) ? mb_load(base + t2.x) : 0.f;
+            v[j + 1] = (valid & t2.w) == static_cast<uint32_t>(t2.w) ? mb_load(base + t2.z) : 0.f;
           }
         }
         if (it >= STAGES && !mbar_wait_warp(empty_bar + 8 * stage, ((it / STAGES) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
@@ -395,10 +395,10 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             chunk[c] = (w4 / WARPS_N) * CH + c;
             const int k = k0 + chunk[c] * 4;
             const float *src = W + n0 + n + static_cast<int64_t>(k) * p.w_ks;
-            v[c].x = in && k < p.K ? __ldg(src) : 0.f;
-            v[c].y = in && k + 1 < p.K ? __ldg(src + p.w_ks) : 0.f;
-            v[c].z = in && k + 2 < p.K ? __ldg(src + 2 * p.w_ks) : 0.f;
-            v[c].w = in && k + 3 < p.K ? __ldg(src + 3 * p.w_ks) : 0.f;
+            v[c].x = in && k < p.K ? mb_load(src) : 0.f;
+            v[c].y = in && k + 1 < p.K ? mb_load(src + p.w_ks) : 0.f;
+            v[c].z = in && k + 2 < p.K ? mb_load(src + 2 * p.w_ks) : 0.f;
+            v[c].w = in && k + 3 < p.K ? mb_load(src + 3 * p.w_ks) : 0.f;
           }
         } else {
           const int c8 = lane & 7, k = k0 + c8 * 4;
@@ -408,10 +408,10 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             chunk[c] = c8;
             const float *src = W + static_cast<int64_t>(n0 + row[c]) * p.w_ns + k;
             const bool in = n0 + row[c] < p.N;
-            v[c].x = in && k < p.K ? __ldg(src) : 0.f;
-            v[c].y = in && k + 1 < p.K ? __ldg(src + 1) : 0.f;
-            v[c].z = in && k + 2 < p.K ? __ldg(src + 2) : 0.f;
-            v[c].w = in && k + 3 < p.K ? __ldg(src + 3) : 0.f;
+            v[c].x = in && k < p.K ? mb_load(src) : 0.f;
+            v[c].y = in && k + 1 < p.K ? mb_load(src + 1) : 0.f;
+            v[c].z = in && k + 2 < p.K ? mb_load(src + 2) : 0.f;
+            v[c].w = in && k + 3 < p.K ? mb_load(src + 3) : 0.f;
           }
         }
         if (it >= STAGES && !mbar_wait_warp(empty_bar + 8 * stage, ((it / STAGES) & 1) ^ 1, abort_flag, WAIT_BUDGET)) {
@@ -622,7 +622,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           }
           const bool finite = MODE == WHOLE || !p.exact || all_finite(x);
           if (p.bias != nullptr) {
-            const float mine = n0 + c + (lane & 15) < p.N ? __ldg(p.bias + n0 + c + (lane & 15)) : 0.f;
+            const float mine = n0 + c + (lane & 15) < p.N ? mb_load(p.bias + n0 + c + (lane & 15)) : 0.f;
 #pragma unroll
             for (int j = 0; j < 16; ++j) x[j] += __shfl_sync(0xffffffffu, mine, j);
           }
@@ -630,7 +630,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const float *src_r = p.residual + at + static_cast<int64_t>(n0 + c) * p.c_ns;
             float res[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) res[j] = n0 + c + j < p.N ? __ldg(src_r + j * p.c_ns) : 0.f;
+            for (int j = 0; j < 16; ++j) res[j] = n0 + c + j < p.N ? mb_load(src_r + j * p.c_ns) : 0.f;
 #pragma unroll
             for (int j = 0; j < 16; ++j) x[j] += res[j];
           }
@@ -682,8 +682,8 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           const int c = c0 + q * 4, n = n0 + c;
           x[q] = bias[q] = add[q] = 0.f;
           if (c < share && n < p.N) {
-            if (p.residual != nullptr) add[q] = __ldg(p.residual + at + static_cast<int64_t>(n) * p.c_ns);
-            if (p.bias != nullptr) bias[q] = __ldg(p.bias + n);
+            if (p.residual != nullptr) add[q] = mb_load(p.residual + at + static_cast<int64_t>(n) * p.c_ns);
+            if (p.bias != nullptr) bias[q] = mb_load(p.bias + n);
             for (int s = 0; s < p.splits; ++s) x[q] += mine[(s * share + c) * BM];
           }
         }

@@ -429,9 +429,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
     const float act_hi = p.act == 2 ? p.max_limit : INFINITY;
     const float act_slope = p.act == 6 ? p.coef : 0.f;
     const bool leaky = p.act == 6;
-    const float *__restrict__ bias = p.bias;
+    const float *bias = p.bias;
     const bool has_bias = bias != nullptr;
-    const float *__restrict__ residual = p.residual;
+    const float *residual = p.residual;
     const int64_t Ndim = p.Ndim;
     const int c_tma = p.c_tma;
     int acc_buf = 0;
@@ -483,7 +483,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
             prefetch_l2(nres + min(nn + c * 16, Ndim - 1) * p.c_row_stride);
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) r_next[j] = __ldg(res + min(n_first + j, Ndim - 1) * p.c_row_stride);
+        for (int j = 0; j < 16; ++j) r_next[j] = mb_load(res + min(n_first + j, Ndim - 1) * p.c_row_stride);
       }
       // staging, per set of four warps: [buffer][channel j][128 pixels]; a lane's 16 writes of
       // a chunk go to 16 different rows, a warp's write of one row covers all 32 banks.  The
@@ -516,7 +516,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
         for (int j = 0; j < 16; ++j) r_cur[j] = r_next[j];
         if (res != nullptr && i + 1 < CHUNKS) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) r_next[j] = __ldg(res + min(n0 + 16 + j, Ndim - 1) * p.c_row_stride);
+          for (int j = 0; j < 16; ++j) r_next[j] = mb_load(res + min(n0 + 16 + j, Ndim - 1) * p.c_row_stride);
         }
         float v[16];
         if constexpr (EPI == 1) {

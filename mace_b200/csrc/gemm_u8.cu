@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(256) repack_rows_u8_kernel(const RepackJob a, 
     const int off = static_cast<int>(reinterpret_cast<uintptr_t>(q) & 3u);
     const uint32_t *aligned = reinterpret_cast<const uint32_t *>(q - off);
     sh[s] = off * 8;
-    lo[s] = left[s] > 0 ? __ldg(aligned) : 0u;
-    hi[s] = left[s] + off > 4 ? __ldg(aligned + 1) : 0u;
+    lo[s] = left[s] > 0 ? mb_load(aligned) : 0u;
+    hi[s] = left[s] + off > 4 ? mb_load(aligned + 1) : 0u;
   }
 #pragma unroll
   for (int s = 0; s < REPACK_STEPS; ++s) {

@@ -57,12 +57,12 @@ __device__ __forceinline__ void load_bytes(const uint8_t *q, int valid, uint32_t
   const uint32_t *a = reinterpret_cast<const uint32_t *>(q - off);
   if (valid >= 16) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = __ldg(a + j);
-    w[4] = __ldg(a + (off != 0 ? 4 : 3));
+    for (int j = 0; j < 4; ++j) w[j] = mb_load(a + j);
+    w[4] = mb_load(a + (off != 0 ? 4 : 3));
   } else {
     const int need = valid > 0 ? valid + off : 0;
 #pragma unroll
-    for (int j = 0; j < 5; ++j) w[j] = 4 * j < need ? __ldg(a + j) : 0u;
+    for (int j = 0; j < 5; ++j) w[j] = 4 * j < need ? mb_load(a + j) : 0u;
   }
 }
 

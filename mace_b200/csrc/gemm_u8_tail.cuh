@@ -94,7 +94,7 @@ __device__ __forceinline__ void finish_tile(const TailParams &p, int32_t *tile, 
       int32_t add[4] = {p.kzz, p.kzz, p.kzz, p.kzz};
       if (p.bias != nullptr && !p.bias_per_row) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) add[j] += j < left ? __ldg(p.bias + n + j) : 0;
+        for (int j = 0; j < 4; ++j) add[j] += j < left ? mb_load(p.bias + n + j) : 0;
       }
       const int32_t *mine = tile + (lane % LANES) * 4;
       uint32_t peer[7];
@@ -117,7 +117,7 @@ __device__ __forceinline__ void finish_tile(const TailParams &p, int32_t *tile, 
         }
         const int m = m0 + row;
         if (p.bias_per_row && p.bias != nullptr) {
-          const int32_t rb = __ldg(p.bias + m);
+          const int32_t rb = mb_load(p.bias + m);
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] += rb;
         }

@@ -139,12 +139,12 @@ __device__ __forceinline__ uint32_t sum_partials(const uint32_t *p, int slices, 
   int sl = 0;
   for (; sl + 8 <= slices; sl += 8) {
     const uint32_t *q = p + sl * stride;
-    const uint32_t v0 = __ldg(q), v1 = __ldg(q + stride), v2 = __ldg(q + 2 * stride), v3 = __ldg(q + 3 * stride);
-    const uint32_t v4 = __ldg(q + 4 * stride), v5 = __ldg(q + 5 * stride), v6 = __ldg(q + 6 * stride),
-                   v7 = __ldg(q + 7 * stride);
+    const uint32_t v0 = mb_load(q), v1 = mb_load(q + stride), v2 = mb_load(q + 2 * stride), v3 = mb_load(q + 3 * stride);
+    const uint32_t v4 = mb_load(q + 4 * stride), v5 = mb_load(q + 5 * stride), v6 = mb_load(q + 6 * stride),
+                   v7 = mb_load(q + 7 * stride);
     a0 += v0; a1 += v1; a2 += v2; a3 += v3; a4 += v4; a5 += v5; a6 += v6; a7 += v7;
   }
-  for (; sl < slices; ++sl) a0 += __ldg(p + sl * stride);
+  for (; sl < slices; ++sl) a0 += mb_load(p + sl * stride);
   return ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
 }
 
@@ -647,14 +647,14 @@ gemm_u8_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
       // global inputs of the terms, requested before the main loop is followed
       const int64_t m = static_cast<int64_t>(tm) * TILE_M + rank * BM + r;
       int32_t row_bias = 0, col_bias[(BN + 127) / 128];
-      if (p.bias != nullptr && p.bias_per_row && m < p.M) row_bias = __ldg(p.bias + m);
+      if (p.bias != nullptr && p.bias_per_row && m < p.M) row_bias = mb_load(p.bias + m);
       if (!FUSE_SUMS && p.sum_a != nullptr && m < p.M) {
         sa_sum = sum_partials(p.sum_a + (p.a_batched ? b : 0) * p.sum_a_bstride + m, p.sum_a_slices, p.M);
       }
 #pragma unroll
       for (int j = 0; j < (BN + 127) / 128; ++j) {
         const int64_t n = static_cast<int64_t>(tn) * BN + j * 128 + r;
-        col_bias[j] = (p.bias != nullptr && !p.bias_per_row && n < p.N) ? __ldg(p.bias + n) : 0;
+        col_bias[j] = (p.bias != nullptr && !p.bias_per_row && n < p.N) ? mb_load(p.bias + n) : 0;
         if (!FUSE_SUMS && p.sum_b != nullptr && n < p.N) {
           sb_sum[j] = sum_partials(p.sum_b + (p.b_batched ? b : 0) * p.sum_b_bstride + n, p.sum_b_slices, p.N);
         }

@@ -58,12 +58,12 @@ __global__ void __launch_bounds__(256) gemv_u8_kernel(const GemvParams p) {
       if (b == b_begin || p.lhs_batched) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-          if (i < pre) l[i] = __ldg(l4 + lane + 32 * i);
+          if (i < pre) l[i] = mb_load(l4 + lane + 32 * i);
       }
       __syncthreads();  // previous batch entry's readers are done with xs
       uint32_t part = 0;
       for (int i = threadIdx.x; i < nvec; i += 256) {
-        const uint4 r = __ldg(r4 + i);
+        const uint4 r = mb_load(r4 + i);
         xs[i] = r;
         part = __dp4a(r.x, 0x01010101u, part);
         part = __dp4a(r.y, 0x01010101u, part);
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) gemv_u8_kernel(const GemvParams p) {
       }
 #pragma unroll 4
       for (int i = lane + 256; i < nvec; i += 32) {
-        const uint4 lv = __ldg(l4 + i);
+        const uint4 lv = mb_load(l4 + i);
         const uint4 r = xs[i];
         dot = __dp4a(lv.x, r.x, dot); dot = __dp4a(lv.y, r.y, dot);
         dot = __dp4a(lv.z, r.z, dot); dot = __dp4a(lv.w, r.w, dot);
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32) gemv_u8_stream_kernel(const Gem
     const uint4 *r4 = reinterpret_cast<const uint4 *>(p.rhs);
     uint32_t part = 0;
     for (int i = threadIdx.x; i < nvec; i += ST_WARPS * 32) {
-      const uint4 r = __ldg(r4 + i);
+      const uint4 r = mb_load(r4 + i);
       xs[i] = r;
       part = __dp4a(r.x, 0x01010101u, part);
       part = __dp4a(r.y, 0x01010101u, part);

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(const PoolF32Params p)
     for (int fw = 0; fw < p.KW; ++fw) {
       const int iw = iw0 + fw * p.dw;
       if (iw < 0 || iw >= p.W) continue;
-      const float v = __ldg(ip + ih * p.W + iw);
+      const float v = mb_load(ip + ih * p.W + iw);
       if (IS_MAX) res = fmaxf(res, v);
       else res += v;
       ++count;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(const PoolF32Params p)
 // after the other, each from a line of its own: 2048 planes of 7 x 7 took 9.0 us, now 4).  Several planes per warp where
 // there are enough of them: 524288 planes one by one took 77 us.
 template <int PLANES>
-__global__ void __launch_bounds__(256) global_avgpool_f32_kernel(const float *__restrict__ in, float *__restrict__ out,
+__global__ void __launch_bounds__(256) global_avgpool_f32_kernel(const float *in, float *__restrict__ out,
                                                                  int64_t planes, int size) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) global_avgpool_f32_kernel(const float *__
 #pragma unroll 2
   for (int i = lane; i < size; i += 32) {
 #pragma unroll
-    for (int q = 0; q < PLANES; ++q) s[q] += q < n ? __ldg(src + q * size + i) : 0.f;
+    for (int q = 0; q < PLANES; ++q) s[q] += q < n ? mb_load(src + q * size + i) : 0.f;
   }
   float mine = 0.f;
 #pragma unroll
@@ -108,13 +108,13 @@ __global__ void __launch_bounds__(256) maxpool3x3s2_f32_kernel(const PoolF32Para
     const float *row = ip + static_cast<int64_t>(ih) * p.W + iw0;
     float c[9];
     if (iw0 + 8 < p.W) {
-      const float4 a = __ldg(reinterpret_cast<const float4 *>(row));
-      const float4 b = __ldg(reinterpret_cast<const float4 *>(row) + 1);
+      const float4 a = mb_load(reinterpret_cast<const float4 *>(row));
+      const float4 b = mb_load(reinterpret_cast<const float4 *>(row) + 1);
       c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w; c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
-      c[8] = __ldg(row + 8);
+      c[8] = mb_load(row + 8);
     } else {
 #pragma unroll
-      for (int j = 0; j < 9; ++j) c[j] = iw0 + j < p.W ? __ldg(row + j) : -FLT_MAX;
+      for (int j = 0; j < 9; ++j) c[j] = iw0 + j < p.W ? mb_load(row + j) : -FLT_MAX;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) o[k] = fmaxf(o[k], fmaxf(c[2 * k], fmaxf(c[2 * k + 1], c[2 * k + 2])));
@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(256) eltwise_f32_kernel(const EltParams p, int
     const float4 *b4 = reinterpret_cast<const float4 *>(p.in1);
     float4 *o4 = reinterpret_cast<float4 *>(p.out);
     for (int64_t i = t0; i < n4; i += stride) {
-      const float4 a = __ldg(a4 + i);
-      const float4 b = b4 != nullptr ? __ldg(b4 + i) : make_float4(p.scalar, p.scalar, p.scalar, p.scalar);
+      const float4 a = mb_load(a4 + i);
+      const float4 b = b4 != nullptr ? mb_load(b4 + i) : make_float4(p.scalar, p.scalar, p.scalar, p.scalar);
       float4 o;
       o.x = elt_apply<TYPE>(a.x, b.x, p); o.y = elt_apply<TYPE>(a.y, b.y, p);
       o.z = elt_apply<TYPE>(a.z, b.z, p); o.w = elt_apply<TYPE>(a.w, b.w, p);
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) eltwise_f32_kernel(const EltParams p, int
 }
 
 __global__ void __launch_bounds__(256)
-activation_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t size, int vec4,
+activation_f32_kernel(const float *in, float *__restrict__ out, int64_t size, int vec4,
                       int act, float max_limit, float coef) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -207,7 +207,7 @@ activation_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int
     const float4 *a4 = reinterpret_cast<const float4 *>(in);
     float4 *o4 = reinterpret_cast<float4 *>(out);
     for (int64_t i = t0; i < n4; i += stride) {
-      float4 a = __ldg(a4 + i);
+      float4 a = mb_load(a4 + i);
       a.x = mb_activate(a.x, act, max_limit, coef); a.y = mb_activate(a.y, act, max_limit, coef);
       a.z = mb_activate(a.z, act, max_limit, coef); a.w = mb_activate(a.w, act, max_limit, coef);
       o4[i] = a;
@@ -220,7 +220,7 @@ activation_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int
 // One warp per (outer, inner) position; the classes are strided by `inner`.  The sum runs over
 // the lanes' partial sums instead of class order (difference: rounding of the last bits).
 __global__ void __launch_bounds__(256)
-softmax_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t positions,
+softmax_f32_kernel(const float *in, float *__restrict__ out, int64_t positions,
                    int64_t classes, int64_t inner, int use_log) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -229,12 +229,12 @@ softmax_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_
   if (pos >= positions) return;
   const int64_t base = (pos / inner) * classes * inner + pos % inner;
   float mx = -FLT_MAX;
-  for (int64_t c = lane; c < classes; c += 32) mx = fmaxf(mx, __ldg(in + base + c * inner));
+  for (int64_t c = lane; c < classes; c += 32) mx = fmaxf(mx, mb_load(in + base + c * inner));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float sum = 0.f;
   for (int64_t c = lane; c < classes; c += 32) {
-    const float e = expf(__ldg(in + base + c * inner) - mx);
+    const float e = expf(mb_load(in + base + c * inner) - mx);
     out[base + c * inner] = e;
     sum += e;
   }
@@ -263,7 +263,7 @@ static void launch_eltwise(mb_context *ctx, const EltParams &p, int vec4) {
 // whole: a thread takes four neighbouring outputs of a row, with two 16-byte loads where the column stride is 2 and rows
 // are aligned (one output per thread and 64-bit divisions: 56 x 56 x 256, batch 256, 187 us; now 111).
 __global__ void __launch_bounds__(256)
-subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t quads, int H, int W, int sh, int sw,
+subsample_f32_kernel(const float *in, float *__restrict__ out, int64_t quads, int H, int W, int sh, int sw,
                      int Ho, int Wo, int vec) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -277,7 +277,7 @@ subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int6
   const float *src = in + (pl * H + static_cast<int64_t>(ho) * sh) * W + static_cast<int64_t>(wo) * sw;
   float *dst = out + (pl * Ho + ho) * Wo + wo;
   if (vec && wo * 2 + 8 <= W) {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(src)), b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+    const float4 a = mb_load(reinterpret_cast<const float4 *>(src)), b = mb_load(reinterpret_cast<const float4 *>(src) + 1);
     if ((Wo & 3) == 0) {
       *reinterpret_cast<float4 *>(dst) = make_float4(a.x, a.z, b.x, b.z);
     } else {  // (eight columns of the input are there: so are four of the output)
@@ -287,7 +287,7 @@ subsample_f32_kernel(const float *__restrict__ in, float *__restrict__ out, int6
   }
   float v[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = wo + j < Wo ? __ldg(src + static_cast<int64_t>(j) * sw) : 0.f;
+  for (int j = 0; j < 4; ++j) v[j] = wo + j < Wo ? mb_load(src + static_cast<int64_t>(j) * sw) : 0.f;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     if (wo + j < Wo) dst[j] = v[j];

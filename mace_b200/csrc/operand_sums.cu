@@ -42,7 +42,7 @@ __device__ __forceinline__ void row_sums(const SumJob &j, int block) {
     uint32_t s = 0;
 #pragma unroll 8
     for (int64_t i = lane; i < nvec; i += 32) {
-      const uint4 v = __ldg(p + i);
+      const uint4 v = mb_load(p + i);
       s = __dp4a(v.x, 0x01010101u, s);
       s = __dp4a(v.y, 0x01010101u, s);
       s = __dp4a(v.z, 0x01010101u, s);
@@ -72,7 +72,7 @@ __device__ __forceinline__ void col_sums(const SumJob &j, int block, uint32_t (*
   if (active) {
 #pragma unroll 8
     for (int64_t r = r0 + ty; r < r1; r += WARPS) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(base + r * j.pitch) + c16);
+      const uint4 v = mb_load(reinterpret_cast<const uint4 *>(base + r * j.pitch) + c16);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {

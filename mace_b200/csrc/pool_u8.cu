@@ -10,7 +10,7 @@
 namespace {
 
 __global__ void __launch_bounds__(256)
-avgpool_u8_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int N, int H, int W,
+avgpool_u8_kernel(const uint8_t *in, uint8_t *__restrict__ out, int N, int H, int W,
                   int C, int KH, int KW, int sh, int sw, int pad_top, int pad_left, int Ho, int Wo) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -37,7 +37,7 @@ avgpool_u8_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int
 // Four adjacent channels per thread (one 32-bit word per pixel), all loads of a window row in
 // flight together; C % 4 == 0 and 4-byte aligned tensors.
 __global__ void __launch_bounds__(128)
-avgpool_u8_c4_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int N, int H, int W,
+avgpool_u8_c4_kernel(const uint8_t *in, uint8_t *__restrict__ out, int N, int H, int W,
                      int C, int KH, int KW, int sh, int sw, int pad_top, int pad_left, int Ho, int Wo) {
   mb_grid_dep_launch();
   mb_grid_dep_wait();
@@ -62,7 +62,7 @@ avgpool_u8_c4_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, 
     uint32_t v[49];
 #pragma unroll
     for (int i = 0; i < 49; ++i)
-      v[i] = __ldg(reinterpret_cast<const uint32_t *>(
+      v[i] = mb_load(reinterpret_cast<const uint32_t *>(
           base + (static_cast<int64_t>(h0 + i / 7) * W + (w0 + i % 7)) * C));
 #pragma unroll
     for (int i = 0; i < 49; ++i) {
@@ -76,7 +76,7 @@ avgpool_u8_c4_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, 
     const uint8_t *row = base + static_cast<int64_t>(h) * W * C;
 #pragma unroll 8
     for (int w = w0; w < w1; ++w) {
-      const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(row + static_cast<int64_t>(w) * C));
+      const uint32_t v = mb_load(reinterpret_cast<const uint32_t *>(row + static_cast<int64_t>(w) * C));
       s0 = __dp4a(v, 0x00000001u, s0);
       s1 = __dp4a(v, 0x00000100u, s1);
       s2 = __dp4a(v, 0x00010000u, s2);

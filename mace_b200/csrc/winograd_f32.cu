@@ -64,7 +64,7 @@ __device__ __forceinline__ float act_apply(float x, int act, float max_limit, fl
 
 // ---- filter transforms: OIHW -> U[T][O][C] ------------------------------------------
 __global__ void __launch_bounds__(256)
-wino_filter_2x2_kernel(const float *__restrict__ f, float *__restrict__ U, int C, int O) {
+wino_filter_2x2_kernel(const float *f, float *__restrict__ U, int C, int O) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= O * C) return;
   const float *g = f + static_cast<int64_t>(idx) * 9;
@@ -93,7 +93,7 @@ wino_filter_2x2_kernel(const float *__restrict__ f, float *__restrict__ U, int C
 }
 
 __global__ void __launch_bounds__(256)
-wino_filter_6x6_kernel(const float *__restrict__ f, float *__restrict__ U, int C, int O) {
+wino_filter_6x6_kernel(const float *f, float *__restrict__ U, int C, int O) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= O * C) return;
   const float G[8][3] = {{1.0f, 0.0f, 0.0f},
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) wino_input_kernel(const WinoParams p) {
     const bool row_ok = static_cast<unsigned>(h) < static_cast<unsigned>(p.H);
     const float *rowp = ip + ((row_ok ? h : 0) * p.W + w0);
 #pragma unroll
-    for (int j = 0; j < IN; ++j) d[i][j] = (row_ok && col_ok[j]) ? __ldg(rowp + j) : 0.f;
+    for (int j = 0; j < IN; ++j) d[i][j] = (row_ok && col_ok[j]) ? mb_load(rowp + j) : 0.f;
   }
   const int64_t ncols = static_cast<int64_t>(p.N) * tiles;
   float *op = p.V + static_cast<int64_t>(c) * ncols + static_cast<int64_t>(n) * tiles + tile;
