@@ -316,8 +316,16 @@ int64_t persistent_cost(const mb_context *ctx, const mb_cut_gemm &g) {
   return best + (fused ? 8300 : 13300);
 }
 
+// The same of the few-row kernel (gemm_u8_skinny.cu), which takes panels of 256 rows of B, from 1, 4, 8 and 16 rows against
+// 256 .. 1024 x 20004 .. 200004 (1 row: 6.2 us at 256 x 20004, 18.5 at 200004; 16 rows: 14.4, 191 at 1024 x 200004).
+int64_t skinny_cost(int64_t M, int64_t N, int64_t K) {
+  const int64_t bytes = ceil_div64(K, 256) * 256 * N;
+  return M <= 1 ? 9200 + bytes / 1950 : M <= 4 ? 13400 + bytes / 1950 : M <= 8 ? 16000 + bytes / 1200 : 22000 + bytes / 600;
+}
+
 // Runs the product on a cluster-cut kernel where that is estimated to be the fastest way: as it lies, or, with rows that
-// TMA cannot address, on copies that it can (2.4 us for the extra launch and the bytes at about 4 TB/s).
+// TMA cannot address, on copies that it can (2.4 us for the extra launch and the bytes at about 4 TB/s); or, few ragged
+// rows, on the kernel made for them.  Else the caller takes the persistent kernel, on copies.
 bool try_cut(mb_context *ctx, const mb_cut_gemm &g, bool a_copy, bool b_copy, int *status) {
   const mb_cut_plan direct = mb_gemm_u8_cut_plan(ctx, g);
   int64_t other = persistent_cost(ctx, g);
@@ -335,6 +343,14 @@ bool try_cut(mb_context *ctx, const mb_cut_gemm &g, bool a_copy, bool b_copy, in
   if (b_copy) { c.B = nullptr; c.ldb = ldb; }
   const mb_cut_plan copied = mb_gemm_u8_cut_plan(ctx, c);
   other += copy_cost;
+  if (g.M <= ctx->skinny_max_m && mb_gemm_u8_skinny_supported(g.batch, g.M, g.N, g.K, g.a_mn, g.b_mn, g.A, g.B)) {
+    const int64_t skinny = skinny_cost(g.M, g.N, g.K);
+    if (skinny < other && (direct.cost < 0 || skinny < direct.cost) && (copied.cost < 0 || skinny < copied.cost + copy_cost)) {
+      *status = mb_gemm_u8_skinny_launch(ctx, g.A, g.B, g.bias, g.C, g.out_is_int32, g.M, g.N, g.K, g.zp_a, g.zp_b, g.rq.mult,
+                                         g.rq.sh - 31, g.rq.zp, g.bias_per_row);
+      return true;
+    }
+  }
   if (direct.cost >= 0 && direct.cost <= other && (copied.cost < 0 || direct.cost <= copied.cost + copy_cost)) {
     *status = mb_gemm_u8_cut_launch(ctx, g, direct);
     return true;
@@ -371,7 +387,8 @@ int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, con
   // A ragged product of a few thousand multiplications per SM is not worth the copy: one launch of the
   // CUDA-core kernel is over before the copy's successor could start.
   if ((a_copy || b_copy) && batch * M * N * K <= (1 << 18)) use_tc = false;
-  if (use_tc && ctx->split_k && ctx->skinny_max_m > 0 && !ctx->pair_gemm && (ctx->force_bn == 0 || a_copy || b_copy)) {
+  const bool cut_rule = use_tc && ctx->split_k && ctx->skinny_max_m > 0 && !ctx->pair_gemm && (ctx->force_bn == 0 || a_copy || b_copy);
+  if (cut_rule) {
     mb_cut_gemm g;
     g.A = A; g.B = B; g.bias = bias; g.C = C; g.out_is_int32 = out_is_int32; g.bias_per_row = bias_per_row;
     g.batch = batch; g.M = M; g.N = N; g.K = K; g.a_mn = a_mn; g.b_mn = b_mn;
@@ -388,9 +405,9 @@ int mb_gemm_u8_rowmajor(mb_context *ctx, const uint8_t *A, const uint8_t *B, con
     }
     if (try_cut(ctx, g, a_copy, b_copy, &st)) return st;
   }
-  // (With the cluster-cut kernels off -- split_k or skinny_max_m = 0 --: a few rows against a large row-major B
-  // on CUDA cores, or on the tensor cores with the depth cut into runs through global memory.)
-  if (ctx->use_tensor_cores && M <= ctx->skinny_max_m && mb_gemm_u8_skinny_supported(batch, M, N, K, a_mn, b_mn, A, B)) {
+  // With the cluster-cut kernels off (split_k or skinny_max_m = 0), or beyond their depth: a few rows against a large
+  // row-major B on CUDA cores, or on the tensor cores with the depth cut into runs through global memory.
+  if (ctx->use_tensor_cores && !(cut_rule && (a_copy || b_copy)) && M <= ctx->skinny_max_m && mb_gemm_u8_skinny_supported(batch, M, N, K, a_mn, b_mn, A, B)) {
     int bn_unused = 0;
     const bool runs_apply = M >= ctx->runs_min_m && use_tc && !a_copy && !b_copy &&
                             split_k_choice(ctx, batch, M, N, K, &bn_unused) > 1;

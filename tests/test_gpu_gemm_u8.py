@@ -294,6 +294,19 @@ def test_few_rows_against_row_major_b(ctx, orc, shape, out_int32):
         assert len(np.unique(got)) > 16
 
 
+@pytest.mark.parametrize("shape,few_row_kernel", [((1, 20004, 256), True), ((4, 30004, 1000), True), ((16, 20004, 256), False),
+                                                  ((12, 50004, 260), False)])
+def test_few_ragged_rows_take_the_kernel_that_was_weighed(ctx, orc, shape, few_row_kernel):
+    """A short depth against many ragged columns: the few-row kernel on CUDA cores where its own estimate is the smallest,
+    else the tensor cores on a copy."""
+    M, N, K = shape
+    case = gemm_case(orc, N, 1, M, N, K, bias_len=N)
+    before = ctx.launches_tensor_core
+    got, exp = run_gemm(ctx, orc, case, 1, M, N, K)
+    assert np.array_equal(got, exp)
+    assert (ctx.launches_tensor_core == before) == few_row_kernel
+
+
 @pytest.mark.parametrize("shape", [(256, 256, 512, False, False, 1), (384, 320, 640, False, False, 1),
                                    (512, 256, 256, True, False, 1), (272, 528, 384, True, True, 2),
                                    (640, 1024, 2048, False, True, 1)])
