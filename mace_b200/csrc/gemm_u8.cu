@@ -297,12 +297,14 @@ int split_k_choice(const mb_context *ctx, int64_t batch, int64_t M, int64_t N, i
   return best >= 4 ? best : 1;
 }
 
+}  // namespace
+
 // ---- the choice between the tensor-core kernels ----------------------------------------
 // Estimated SM cycles of the persistent kernel (gemm_u8_tc.cu), from its times at 1024^3 (7.4 us), 512^3 (5.9 us),
 // 16 x 1024 x 1024 (7.3 us), 256 x 4096 x 4096 (17 us) and 4096^3 (58 us): about 4.4 us around the steps, a row-major
 // B whose column sums come from the tiles paces them; beyond a depth of 1024 (or with a column-major A) the sums
 // are a kernel of their own.
-int64_t persistent_cost(const mb_context *ctx, const mb_cut_gemm &g) {
+int64_t mb_gemm_u8_persistent_cost(const mb_context *ctx, const mb_cut_gemm &g) {
   const int64_t tiles_m = ceil_div64(g.M, 128), steps = ceil_div64(g.K, 128);
   const bool fused = !g.a_mn && g.K <= 1024;
   int64_t best = -1;
@@ -316,6 +318,8 @@ int64_t persistent_cost(const mb_context *ctx, const mb_cut_gemm &g) {
   return best + (fused ? 8300 : 13300);
 }
 
+namespace {
+
 // The same of the few-row kernel (gemm_u8_skinny.cu), which takes panels of 256 rows of B, from 1, 4, 8 and 16 rows against
 // 256 .. 1024 x 20004 .. 200004 (1 row: 6.2 us at 256 x 20004, 18.5 at 200004; 16 rows: 14.4, 191 at 1024 x 200004).
 int64_t skinny_cost(int64_t M, int64_t N, int64_t K) {
@@ -328,7 +332,7 @@ int64_t skinny_cost(int64_t M, int64_t N, int64_t K) {
 // rows, on the kernel made for them.  Else the caller takes the persistent kernel, on copies.
 bool try_cut(mb_context *ctx, const mb_cut_gemm &g, bool a_copy, bool b_copy, int *status) {
   const mb_cut_plan direct = mb_gemm_u8_cut_plan(ctx, g);
-  int64_t other = persistent_cost(ctx, g);
+  int64_t other = mb_gemm_u8_persistent_cost(ctx, g);
   if (!a_copy && !b_copy) {
     if (direct.cost < 0 || (ctx->cut_aligned == 0 ? direct.cost >= other : ctx->cut_aligned == 1)) return false;
     *status = mb_gemm_u8_cut_launch(ctx, g, direct);

@@ -35,6 +35,8 @@ struct mb_cut_plan {
 
 // The cheapest way for the product as it lies (by_tma only where every row is 16-byte aligned).
 mb_cut_plan mb_gemm_u8_cut_plan(mb_context *ctx, const mb_cut_gemm &g);
+// The same of the persistent kernel (gemm_u8_tc.cu; gemm_u8.cu has the estimate).
+int64_t mb_gemm_u8_persistent_cost(const mb_context *ctx, const mb_cut_gemm &g);
 int mb_gemm_u8_cut_launch(mb_context *ctx, const mb_cut_gemm &g, const mb_cut_plan &plan);
 int mb_gemm_u8_gather_launch(mb_context *ctx, const mb_cut_gemm &g, int bn, int splits);
 

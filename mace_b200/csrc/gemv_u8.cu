@@ -10,6 +10,8 @@
 // The kernel is bandwidth-bound: one warp streams one row of the matrix with
 // 128-bit loads and integer dot-product instructions.  When the matrix is shared by all
 // batch entries (the FullyConnected case) the warp keeps its row and loops over the vectors.
+#include <algorithm>
+
 #include "common.cuh"
 #include "gemm_u8_cut.cuh"
 #include "sm100_ptx.cuh"
@@ -291,20 +293,21 @@ int mb_gemm_u8_tc_launch_float_rule(mb_context *ctx, const uint8_t *A, const uin
                                     int64_t N, int64_t K, int32_t zp_a, int32_t zp_b, float mult_f,
                                     int32_t zp_c, int add_zp);
 
-// Whether the GEMM takes several vectors, or one of ragged length, faster than the kernel with a warp per row.  SM cycles from
-// times at 128 .. 8192 rows, 333 .. 8001 columns, 1 .. 4 vectors.  The GEMV: 1.6 to 2 us around the rows; a ragged row
-// costs 120 cycles per 32 bytes and 4.5 more per row that its SM holds (489 rows of 642: 3.2 us against 7.2 as a GEMM; 489
-// of 8001: 18.0 against 9.9), an aligned one 12 per such row and 512 bytes, and 93 per vector.  The GEMM on ragged rows: 960 per
-// step of 128 columns and 64 rows (its estimate in the plan is for tiles that are full of vectors).
-static bool gemm_is_faster(const mb_context *ctx, const mb_cut_plan &plan, int64_t batch, int64_t rows, int64_t K,
-                           int64_t batch_chunk, bool vec) {
+// SM cycles of the kernel with a warp per row, from times at 128 .. 8192 rows, 333 .. 8001 columns, 1 .. 4 vectors: 1.6 to 2 us
+// around the rows; a ragged row costs 120 cycles per 32 bytes and 4.5 more per row that its SM holds (489 rows of 642: 3.2 us
+// against 7.2 as a GEMM; 489 of 8001: 18.0 against 9.9), an aligned one 12 per such row and 512 bytes, and 93 per vector.
+static int64_t row_kernel_cost(const mb_context *ctx, int64_t batch, int64_t rows, int64_t K, int64_t batch_chunk, bool vec) {
   const int64_t per_sm = ceil_div64(rows, 8) * 8 * ceil_div64(batch, batch_chunk) / ctx->num_sms + 1;
-  const int64_t gemv = vec ? 3000 + batch_chunk * 93 * per_sm + 12 * per_sm * ceil_div64(K, 512)
-                           : 4000 + 2500 * (batch_chunk - 1) + batch_chunk * ceil_div64(K, 32) * (120 + per_sm * 9 / 2);
-  if (plan.by_tma) return plan.cost < gemv;
+  return vec ? 3000 + batch_chunk * 93 * per_sm + 12 * per_sm * ceil_div64(K, 512)
+             : 4000 + 2500 * (batch_chunk - 1) + batch_chunk * ceil_div64(K, 32) * (120 + per_sm * 9 / 2);
+}
+// The same of the cluster-cut GEMM.  On ragged rows 960 per step of 128 columns and 64 rows (the plan's own estimate is for
+// tiles that are full of vectors).
+static int64_t cut_cost(const mb_context *ctx, const mb_cut_plan &plan, int64_t batch, int64_t rows, int64_t K) {
+  if (plan.by_tma) return plan.cost;
   const int64_t tiles = ceil_div64(batch, 128) * ceil_div64(rows, plan.bn);
   const int64_t rounds = ceil_div64(tiles * plan.splits, ctx->num_sms), steps = ceil_div64(ceil_div64(K, 128), plan.splits);
-  return 10500 + rounds * steps * (plan.bn == 128 ? 1250 : 960) < gemv;
+  return 10500 + rounds * steps * (plan.bn == 128 ? 1250 : 960);
 }
 
 extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rhs,
@@ -321,17 +324,6 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
   if (lhs_batched && batch > 65535)
     return mb_fail(ctx, MB_UNSUPPORTED, "mb_gemv_u8: batch > 65535 with a batched matrix");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  // Many vectors against one matrix (FullyConnected on a batch) is a GEMM
-  // out[batch x rows] = rhs[batch x K] * lhs[rows x K]^T: the tensor-core kernel with the float
-  // requantization rule in its epilogue reads the matrix once instead of once per vector.
-  if (!lhs_batched && rhs_batched && batch >= 16 && K % 16 == 0 && K <= 1024 && ctx->use_tensor_cores &&
-      mb_gemm_u8_tc_supported(ctx, rhs, lhs, batch, rows, K, K, K)) {
-    ctx->gemm_b_const = ctx->gemv_lhs_const;  // the matrix is the GEMM's B
-    const int st = mb_gemm_u8_tc_launch_float_rule(ctx, rhs, lhs, bias, out, out_is_int32, batch, rows, K, zp_rhs,
-                                           zp_lhs, multiplier, zp_out, add_zp_out);
-    ctx->gemm_b_const = 0;
-    return st;
-  }
   // One vector against a large matrix: the streaming kernel (see gemv_u8_stream_kernel).
   if (batch == 1 && ctx->gemv_stream && K % 16 == 0 && K >= 256 && K <= 65536 && rows >= 2ll * ctx->num_sms &&
       ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) & 15u) == 0) {
@@ -379,16 +371,31 @@ extern "C" int mb_gemv_u8(mb_context *ctx, const uint8_t *lhs, const uint8_t *rh
     chunks = std::min<int64_t>(chunks, 65535);
   }
   const int64_t batch_chunk = ceil_div64(batch, chunks);
-  // Several vectors against one matrix, of any length: the GEMM that fetches its own operands (the matrix is
-  // read once, its depth cut over clusters where the rows do not fill the SMs).
+  // Several vectors against one matrix, of any length, are a GEMM out[batch x rows] = rhs[batch x K] * lhs[rows x K]^T with the
+  // float requantization rule in its epilogue: on the cluster-cut kernel (the matrix is read once, its depth cut over
+  // clusters where the rows do not fill the SMs) or, 16 and more of them, on the persistent one; by estimate.  Measured, row kernel
+  // or cut / persistent: 16 vectors of 64 -> 100 2.4 us / 4.3, 17 of 1024 -> 333 3.6 / 7.1, 16 of 1024 -> 1000 4.8 / 6.7, 64 4.9 / 6.9, 64
+  // of 512 -> 8000 6.8 / 5.3, 1000 of 1024 -> 1000 9.4 / 7.1, 4096 of 512 -> 4096 71 / 18.
   if (!lhs_batched && (rhs_batched || batch == 1) && ctx->use_tensor_cores && (batch >= 2 || K % 16 != 0) &&
-      batch * rows * K > (1 << 18)) {
+      (batch * rows * K > (1 << 18) || batch >= 16)) {
     mb_cut_gemm g;
     g.A = rhs; g.B = lhs; g.bias = bias; g.C = out; g.out_is_int32 = out_is_int32;
     g.M = batch; g.N = rows; g.K = K; g.zp_a = zp_rhs; g.zp_b = zp_lhs;
     g.rq_variant = 8; g.mult_f = multiplier; g.zp_f = add_zp_out ? static_cast<float>(zp_out) : 0.f;
     const mb_cut_plan plan = mb_gemm_u8_cut_plan(ctx, g);
-    if (plan.cost >= 0 && gemm_is_faster(ctx, plan, batch, rows, K, batch_chunk, vec)) return mb_gemm_u8_cut_launch(ctx, g, plan);
+    const int64_t best = row_kernel_cost(ctx, batch, rows, K, batch_chunk, vec);
+    const int64_t cut = batch * rows * K > (1 << 18) && plan.cost >= 0 ? cut_cost(ctx, plan, batch, rows, K) : best;
+    const bool persistent_can = rhs_batched && batch >= 16 && K % 16 == 0 && K <= 1024 &&
+                                mb_gemm_u8_tc_supported(ctx, rhs, lhs, batch, rows, K, K, K);
+    // (an eighth in favour of the persistent kernel: 64 of 1024 -> 8192 were estimated equal and are 7.5 us cut, 6.8 not)
+    if (persistent_can && mb_gemm_u8_persistent_cost(ctx, g) < std::min(best, cut + cut / 8)) {
+      ctx->gemm_b_const = ctx->gemv_lhs_const;  // the matrix is the GEMM's B
+      const int st = mb_gemm_u8_tc_launch_float_rule(ctx, rhs, lhs, bias, out, out_is_int32, batch, rows, K, zp_rhs,
+                                                     zp_lhs, multiplier, zp_out, add_zp_out);
+      ctx->gemm_b_const = 0;
+      return st;
+    }
+    if (cut < best) return mb_gemm_u8_cut_launch(ctx, g, plan);
   }
   GemvParams p;
   p.lhs = lhs; p.rhs = rhs; p.bias = bias; p.out = out;

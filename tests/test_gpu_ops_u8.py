@@ -87,6 +87,24 @@ def test_gemv_u8(ctx, orc, shape, lhs_batched):
         b.free()
 
 
+@pytest.mark.parametrize("shape,tensor_cores", [
+    # both sides of the lines between the row kernel, the cluster-cut GEMM and the persistent one
+    ((16, 100, 64), 0), ((17, 333, 1024), 0), ((16, 1000, 1024), 1), ((64, 1001, 1024), 1), ((64, 8000, 512), 1), ((130, 72, 48), 1)])
+def test_gemv_u8_of_many_vectors_by_estimate(ctx, orc, shape, tensor_cores):
+    batch, rows, K = shape
+    rng = np.random.Generator(np.random.PCG64(rows))
+    lhs = rng.integers(0, 256, size=(1, rows, K), dtype=np.uint8)
+    rhs = rng.integers(0, 256, size=(batch, K), dtype=np.uint8)
+    bias = np.rint(rng.normal(0, 1000, size=rows)).astype(np.int32)
+    mult = np.float32(127.0 / (3 * np.sqrt(K) * 74 * 74))
+    dl, dr, db, do = ctx.upload(lhs), ctx.upload(rhs), ctx.upload(bias), ctx.alloc(batch * rows)
+    before = ctx.launches_tensor_core
+    ctx.gemv_u8(dl, dr, db, do, batch, rows, K, 126, 121, mult, 128, True)
+    assert ctx.launches_tensor_core - before == tensor_cores
+    exp = orc.gemv_u8(lhs, rhs, bias, batch, rows, K, 126, 121, mult, 128, True)
+    assert np.array_equal(ctx.download(do, (batch * rows,), np.uint8), exp.ravel())
+
+
 @pytest.mark.parametrize("shape", [(4096, 4096), (1000, 1024), (300, 4112), (777, 20000), (5000, 256),
                                    (296, 65536), (1201, 8192)])
 def test_gemv_u8_streaming_kernel(ctx, orc, shape):
