@@ -37,7 +37,7 @@ struct mb_context {
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
   int *dev_status = nullptr;   // status word of bounded-wait failures: the device's address of host_status
-  int *host_status = nullptr;  // pinned mirror read at sync
+  int *host_status = nullptr;  // the word itself, in page-locked host memory: read there at sync
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
   void *encode_im2col = nullptr; // cuTensorMapEncodeIm2col
   int use_tensor_cores = 1;      // cleared by mb_set_option for A/B tests

@@ -13,10 +13,13 @@
 //   3x3 on 3 channels -> thread-per-pixel tensor-core kernel (namespace stem:
 //                        MobileNet's 3x3x3 first layer), or the packed-patch
 //                        dp4a kernel when the channel count is no multiple of 16
-//   small depth * O   -> direct kernel, one thread per output pixel, the whole
-//                        filter in shared memory
-//   everything else   -> patch gather into scratch (rows padded to 16 bytes)
-//                        + tensor-core GEMM
+//   k x k, any stride -> tensor-core GEMM that fetches the windows by TMA in im2col
+//                        mode (gemm_u8_cut.cu, or the persistent kernel), the
+//                        channels padded to 16 by a copy where they are ragged
+//   small work        -> direct kernel, one thread per output pixel, the whole
+//                        filter in shared memory, where its estimate is the smaller
+//   what TMA cannot   -> patch gather into scratch (rows padded to 16 bytes)
+//   describe             + tensor-core GEMM
 #include "common.cuh"
 #include "gemm_u8_cut.cuh"
 #include "sm100_ptx.cuh"

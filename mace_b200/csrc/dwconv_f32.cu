@@ -27,7 +27,8 @@ struct DwF32Params {
 // once for up to K output rows, all loads of a run are independent of each other (the
 // compiler issues them ahead of the arithmetic), and an index costs a few multiply-highs instead
 // of 64-bit divisions: one output per thread with 64-bit index arithmetic and bounds tests per tap ran
-// 64 channels of 112 x 112 -> 56 x 56, batch 32, in 105.7 us = 1.2 TB/s; this form takes 29.1 us = 4.4 TB/s.
+// 64 channels of 112 x 112 -> 56 x 56, batch 32, in 105.7 us = 1.2 TB/s; this form takes 29.1 us = 4.4 TB/s (and the next one,
+// which such rows now go to, 25.4).
 template <int K, int S, int RH>
 __global__ void __launch_bounds__(256) dwconv_f32_rows_kernel(const DwF32Params p) {
   mb_grid_dep_launch();
@@ -210,13 +211,17 @@ int launch_wide(mb_context *ctx, DwF32Params &p) {
 }
 
 // Rows per thread: long runs save loads (a row is read once for K output rows), short ones give a
-// small problem more threads.  The line: a run is as long as it can be while 32 warps per SM remain.
+// small problem more threads.  The line for the row kernel: a run is as long as it can be while 32 warps per SM remain
+// (64 channels, 111 x 111, runs of 1, 2, 4, 8: stride 1, batch 4, 19.0, 11.7, 8.3, 7.1 us; stride 2, batch 8, 10.5, 7.2, 6.0, 7.3;
+// 57 x 57, stride 1, batch 4, 6.1, 4.1, 3.9, 4.9).
 template <int K, int S>
 int launch_ks(mb_context *ctx, DwF32Params &p) {
   const int64_t outputs = static_cast<int64_t>(p.planes) * p.Ho * p.Wo;
   const int64_t want = static_cast<int64_t>(ctx->num_sms) * 1024;
-  // Whole words per row, and the padding that puts a word under each group of columns.  (Rows per thread: measured best
-  // while about 5 times 32 warps per SM remain at stride 2, 2.6 times at stride 1, whose threads hold more.)
+  // Whole words per row, and the padding that puts a word under each group of columns.  Runs are longer while twice 32 warps
+  // per SM remain at stride 1 (once for runs of two), four times at stride 2 (twice for two).  64 channels, 112 x 112, runs of 1, 2,
+  // 4, 8: stride 1, batch 8, 13.1, 10.0, 9.1, 8.6 us, batch 32, 50.0, 40.0, 38.8, 37.8; stride 2, batch 8, 6.4, 5.4, 6.0, batch 32, 26.4, 26.4,
+  // 25.4.
   if (K == 3 && p.W % 4 == 0 && p.Wo * S == p.W && p.pad_l == (S == 1 ? 1 : 0) &&
       ((reinterpret_cast<uintptr_t>(p.in) | reinterpret_cast<uintptr_t>(p.out)) & 15u) == 0) {
     if (S == 1 && outputs >= 64 * want) return launch_wide<S, S == 1 ? 8 : 4>(ctx, p);

@@ -623,8 +623,9 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
     const bool on_cores = pointwise && long_rows(H * W) ? !by_tma : !column_route(N, C, O, KH, KW, Ho, Wo);
     mb_f32_gemm g = conv_gemm(in, filter, bias, nullptr, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h, dil_w, pad_top,
                               pad_left, Ho, Wo, activation, max_limit, coefficient);
-    if (N * O * Ho * Wo * C * KH * KW >= (1ll << 16) && take_gather(ctx, g, by_tma, on_cores))
-      return mb_gemm_f32_gather_launch(ctx, g);
+    // However small: the one-thread-per-output kernel is a serial chain over the depth (depth 64, 4 x 4 pixels, 22.8 us against
+    // 6.5; 144, 3 x 3, 18.8 against 6.6; near the line, 48 to 54, 4.5 to 14 against 5.0 to 6.7).
+    if (take_gather(ctx, g, by_tma, on_cores)) return mb_gemm_f32_gather_launch(ctx, g);
   }
   if (pointwise && (long_rows(H * W) || !ctx->use_tensor_cores)) {
     // out_n[O x HW] = filter[O x C] * in_n[C x HW] for every image n
@@ -633,8 +634,8 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
     return mb_gemm_f32_strided(ctx, filter, in, out, bias, N, O, hw, C, C, 1, 0, hw, 1, C * hw, hw,
                                1, O * hw, activation, max_limit, coefficient);
   }
-  // enough work to fill tensor-core tiles: gather columns and multiply; tiny problems stay on
-  // the one-thread-per-output kernel
+  // (beyond the limits of the kernel that fetches its own operands:) enough work to fill tensor-core tiles: gather columns
+  // and multiply.  Else the one-thread-per-output kernel.
   if (column_route(N, C, O, KH, KW, Ho, Wo)) {
     return conv2d_f32_im2col(ctx, in, filter, bias, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h,
                              dil_w, pad_top, pad_left, Ho, Wo, activation, max_limit, coefficient);

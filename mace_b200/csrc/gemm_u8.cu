@@ -1,7 +1,11 @@
 // mb_gemm_u8: argument checks, operand preparation (row/column byte sums for
 // the zero-point correction, copies of rows that TMA cannot address) and the
-// choice between the tensor-core kernel (gemm_u8_tc.cu) and a CUDA-core kernel
-// that takes any depth and runs when the tensor cores are switched off.
+// choice between the kernels: the persistent one (gemm_u8_tc.cu), one tile per
+// CTA with the depth cut over a cluster (gemm_u8_cut.cu: operands by TMA;
+// gemm_u8_gather.cu: rows of any alignment), a few rows on CUDA cores
+// (gemm_u8_skinny.cu), and a CUDA-core kernel that takes any depth and size and
+// runs for ragged products of up to 2^18 multiplications, depths beyond 33000
+// and with the tensor cores switched off.
 //
 // Reference behaviour: MatMulFixpointImpl (mace/ops/matmul.cc:228-394) and the
 // GEMM of the quantized Conv2D (mace/ops/conv_2d.cc:301-315).

@@ -338,6 +338,32 @@ def test_small_conv2d_f32_is_as_accurate_as_fmas(ctx, orc, case):
         b.free()
 
 
+@pytest.mark.parametrize("case,tensor_core", [
+    # kernel, C, HW, O: a single pixel, a few, on both sides of the depth from which the tensor cores are accurate enough
+    ((1, 100, 1, 10), 1), ((1, 64, 4, 16), 1), ((3, 16, 3, 4), 1), ((1, 48, 2, 8), 1), ((1, 47, 2, 8), 0), ((3, 5, 9, 9), 0)])
+def test_smallest_conv2d_f32(ctx, orc, case, tensor_core):
+    """A chain of K FMAs differs from the exact sum by at most K units of 2^-24 of the sum of the products' absolute
+    values (to first order: one more for the rest); the tensor cores' short runs by less."""
+    k, C, HW, O = case
+    K = C * k * k
+    rng = np.random.Generator(np.random.PCG64(K))
+    x = rng.standard_normal((1, C, HW, HW)).astype(np.float32)
+    f = rng.standard_normal((O, C, k, k)).astype(np.float32)
+    pad = (k - 1) // 2
+    padded = np.pad(x.astype(np.float64), ((0, 0), (0, 0), (pad, pad), (pad, pad)))
+    windows = np.lib.stride_tricks.sliding_window_view(padded, (k, k), (2, 3))
+    dx, df, do = ctx.upload(x), ctx.upload(f), ctx.alloc(O * HW * HW * 4)
+    before = ctx.launches_tensor_core
+    ctx.conv2d_f32(dx, df, None, do, 1, C, HW, HW, O, k, k, (1, 1), (1, 1), (pad, pad), (HW, HW))
+    assert ctx.launches_tensor_core - before == tensor_core
+    got = ctx.download(do, (1, O, HW, HW), np.float32)
+    exact = np.einsum("nchwij,ocij->nohw", windows, f.astype(np.float64))
+    terms = np.einsum("nchwij,ocij->nohw", np.abs(windows), np.abs(f.astype(np.float64)))
+    assert (np.abs(got - exact) <= (K + 1) * 2.0 ** -24 * terms).all()
+    for b in (dx, df, do):
+        b.free()
+
+
 @pytest.mark.parametrize("shape", [(9, 300, 256), (31, 200, 1000), (33, 300, 1001)])
 def test_gemv_f32_of_a_few_vectors_is_as_accurate_as_one_by_one(ctx, shape):
     batch, rows, K = shape
@@ -518,8 +544,8 @@ def test_gemv_f32_on_tensor_cores(ctx, orc, gather, shape):
 @pytest.mark.parametrize("shape", [(1, 3, 7, 9, 1), (2, 300, 33, 31, 1), (3, 5, 20, 65, 2), (4, 130, 57, 112, 1),
                                    (8, 96, 56, 56, 1)])
 def test_dwconv_f32_rows(ctx, orc, k, stride, shape):
-    """The rows-per-thread kernel: every run length (the batch sizes make all of them reachable),
-    ragged last runs, narrow maps, a channel multiplier."""
+    """Runs of one and two rows, ragged last runs, narrow maps, a channel multiplier; 3x3 on rows of whole words takes the
+    kernel of test_dwconv_f32_whole_words.  The longer runs: test_dwconv_f32_long_runs."""
     N, C, H, W, mult = shape
     rng = np.random.Generator(np.random.PCG64(C + k))
     x = rng.standard_normal((N, C, H, W)).astype(np.float32)
@@ -548,6 +574,27 @@ def test_dwconv_f32_whole_words(ctx, orc, stride, shape):
     ref = orc.dwconv_f32(x, f, bias, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
     dx, df, db, do = ctx.upload(x), ctx.upload(f), ctx.upload(bias), ctx.alloc(ref.nbytes)
     ctx.dwconv_f32(dx, df, db, do, N, C, H, W, mult, 3, 3, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
+    assert rel_err(ctx.download(do, ref.shape, np.float32), ref, 1e-5, "dwconv_f32") <= 1e-5
+    for b in (dx, df, db, do):
+        b.free()
+
+
+@pytest.mark.parametrize("k,stride,shape", [
+    # rows that are no whole words, as many values per SM as make runs of 2, 4 and 8 rows (2, 4, 8 times 1024), ragged last runs
+    (3, 1, (2, 40, 75, 75)), (3, 1, (4, 64, 57, 57)), (3, 1, (3, 64, 89, 91)), (3, 2, (6, 64, 59, 57)), (3, 2, (5, 64, 87, 91)),
+    (3, 2, (8, 64, 101, 99)), (5, 1, (3, 64, 89, 91)), (5, 2, (8, 64, 101, 99)), (5, 1, (4, 64, 57, 56)), (5, 2, (3, 64, 89, 88))])
+def test_dwconv_f32_long_runs(ctx, orc, k, stride, shape):
+    N, C, H, W = shape
+    rng = np.random.Generator(np.random.PCG64(C + W))
+    x = rng.standard_normal((N, C, H, W)).astype(np.float32)
+    f = rng.standard_normal((1, C, k, k)).astype(np.float32)
+    bias = rng.standard_normal(C).astype(np.float32)
+    ho, wo, ph, pw = orc.calc_padding_and_output_size(H, W, k, k, (1, 1), (stride, stride), 1)
+    values = N * C * ho * wo / (1024 * 148)
+    assert values >= 2  # (runs of 2 from there, of 4 from 4, of 8 from 8)
+    ref = orc.dwconv_f32(x, f, bias, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
+    dx, df, db, do = ctx.upload(x), ctx.upload(f), ctx.upload(bias), ctx.alloc(ref.nbytes)
+    ctx.dwconv_f32(dx, df, db, do, N, C, H, W, 1, k, k, (stride, stride), (1, 1), (ph >> 1, pw >> 1), (ho, wo), 1)
     assert rel_err(ctx.download(do, ref.shape, np.float32), ref, 1e-5, "dwconv_f32") <= 1e-5
     for b in (dx, df, db, do):
         b.free()
