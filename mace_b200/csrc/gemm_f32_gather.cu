@@ -32,14 +32,15 @@
 // mb_f32_gather_run picks the run whose error is below the FMA chain's, for products that would otherwise run on CUDA cores;
 // none is up to k = 47 and from 65 to 71.  A 3x3 convolution in place of Winograd kernels takes the run whose error is below
 // theirs (F(2,3): 3.1e-8 times the root of the channels, F(6,3): 2e-6 and more).  The sums cost 384 x 384 x 64, batch
-// 12, 0.7 us of 6.7 (SPREAD), the 3x3 layers of ResNet-50 at batch 1 0.2 to 1.5 us each, and the largest products, whose
-// shared memory is busy with W already, a half (1536 x 1536 x 1024: 33 -> 49 us; 136 us on CUDA cores).
+// 12, 0.9 us of 6.7 (SPREAD), the 3x3 layers of ResNet-50 at batch 1 0.2 to 1.5 us each, and the largest products, whose
+// shared memory is busy with W already, a half (1536 x 1536 x 1024: 33 -> 50 us; 136 us on CUDA cores).  Sums in registers
+// instead spilled: 96 registers for four result warps, 80 for eight.
 //
 // What bounds it: the tensor pipe at three tf32 MMAs per product for long depths (12 MMAs x 92 cycles per step of
 // 128 x 128 x 32; a convolution's loads bring the step to 1400), the launch, first loads and results for small shapes.
 // Measured, before -> now: 7x7 stride 2 of 3 -> 64 channels, 224 x 224, batch 256, 1360 us (column matrix) -> 688;
 // 5x5 stride 2 of 48 -> 32, 112 x 112, batch 24, 341 -> 116; 3x3 of 512 channels, 7 x 7, batch 1, 39 (Winograd) -> 18;
-// 384 x 384 x 64 times a transposed matrix, batch 12, 10.9 (CUDA cores) -> 7.4; 736 x 176 x 384, batch 24, 76 -> 39.
+// 384 x 384 x 64 times a transposed matrix, batch 12, 10.9 (CUDA cores) -> 7.7; 736 x 176 x 384, batch 24, 76 -> 39.
 #include <algorithm>
 
 #include "gemm_f32_gather.cuh"
@@ -571,16 +572,21 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       const int m = t.tm * BM + quarter * 32 + lane;
       const int64_t at = out_offset<XK>(p, m, t.b);
       const int n0 = t.tn * BN;
+      const int c_stop = MODE == WHOLE ? c_end : min(c_end, p.N - n0);  // (runs: no sums of channels that do not exist)
 #pragma unroll 1
       for (int i = 0; i < runs; ++i) {
         if (!(ok = wait_acc())) break;
         const uint32_t src = tmem + lanes + (filled % ACCS) * C::ACC_COLS;
         // the next chunk's accumulators are on their way while this one is stored
         uint32_t r[16], r2[16];
+        if (MODE != WHOLE && c_begin >= c_stop) {
+          release_acc();
+          continue;
+        }
         tmem_ld_32x32b_x16(src + c_begin, r);
         if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c_begin, r2);
 #pragma unroll 1
-        for (int c = c_begin; c < c_end; c += 16) {
+        for (int c = c_begin; c < c_stop; c += 16) {
           tmem_ld_wait_x16(r);
           if (C::WIDE) tmem_ld_wait_x16(r2);
           // (everything is loaded before the first store: the compiler may not move a load above a store, and one load
@@ -600,7 +606,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
               for (int j = 0; j < 16; ++j) x[j] += C::WIDE ? __uint_as_float(r[j]) + __uint_as_float(r2[j]) : __uint_as_float(r[j]);
             }
           }
-          if (c + 16 < c_end) {
+          if (c + 16 < c_stop) {
             tmem_ld_32x32b_x16(src + c + 16, r);
             if (C::WIDE) tmem_ld_32x32b_x16(src + BN + c + 16, r2);
           } else {
@@ -773,7 +779,7 @@ Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
       const int64_t rounds = ceil_div64(tiles * s, s == 1 ? ctx->num_sms : mb_resident_cluster_ctas(ctx, s));
       if (s > 1 && rounds > 1 && asked == 0) continue;  // (one tile per CTA: a second round would start from nothing)
       const int64_t steps = ceil_div64(k_blocks, s);
-      const int64_t step = g.conv ? (w == 128 ? 1450 : 1200) : (w == 128 ? 1250 : 1100);
+      const int64_t step = g.conv ? (w == 128 ? 1450 : g.run != 0 ? 1280 : 1200) : (w == 128 ? 1250 : 1100);
       const bool res = g.residual != nullptr;
       int64_t results = (w == 128 ? 10600 : 5400) * (res ? 2 : 1);
       // eight warps for results: where they bound a 128-wide tile (at 64 eight are no faster), or the launch is one round of
@@ -781,9 +787,12 @@ Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
       const bool eight = s == 1 && steps * step <= results && (w == 128 || rounds == 1);
       if (eight && w == 128) results = res ? 16000 : 7000;
       const int64_t last = (w == 128 ? 4000 : 1500) + (res ? 2000 : 0) - (eight ? 700 : 0);
-      const int64_t cost = s == 1 ? 8000 + (rounds - 1) * std::max<int64_t>(steps * step, results) + steps * step + last
+      // products in TMA's layout: 64 channels undivided take 13.6 us for 16 of 512 x 48 x 512 and 8.6 for 16 of 256 x 48 x 256, 128
+      // with the depth cut 16.4 and 10.3, the TMA-fed kernel 13.9 and 9.2
+      const int64_t product = g.conv || g.run != 0 ? 0 : w == 64 && s == 1 ? -1500 : w == 128 && s > 1 ? 3500 : 0;
+      const int64_t cost = product + (s == 1 ? 8000 + (rounds - 1) * std::max<int64_t>(steps * step, results) + steps * step + last
                            : w == 128 ? 10500 + steps * 1350 + last
-                                      : (s == 2 ? 11500 : s == 4 ? 10500 : 11000) + steps * (s == 2 ? 1150 : 1050) + last;
+                                      : (s == 2 ? 11500 : s == 4 ? 10500 : 11000) + steps * (s == 2 ? 1150 : 1050) + last);
       if (best.cost < 0 || cost < best.cost) {
         best.bn = w; best.splits = s; best.warps = eight ? 8 : 4; best.cost = cost;
       }
@@ -865,7 +874,7 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
   }
   if (p.run != 0) {
     if (plan.bn == 128) { MB_F32(128, 8, RUNS) }
-    MB_F32(64, 4, RUNS)
+    MB_F32(64, 8, RUNS)
   }
   if (plan.warps == 8) {
     if (plan.bn == 128) { MB_F32(128, 8, WHOLE) }
