@@ -157,10 +157,13 @@ int mb_pair_clusters(const mb_context *ctx);
  * over the SM pairs run on clusters of two CTAs -- tcgen05.mma.cta_group::2,
  * each CTA loading half of a tile's operands; 2: wherever that kernel can
  * run, for tests.  Measured no faster than one CTA per 128 x 256 tile),
- * "split_k" (1 default: a product with fewer output tiles than a quarter of
- * the SMs and a depth of 2048 or more is computed as 4 or 8 depth runs on as
- * many times the SMs, their exact int32 results added by a second kernel;
- * 0 keeps one CTA per output tile),
+ * "split_k" (1 default: a product with few output tiles and a long depth is
+ * cut along the depth over a cluster of CTAs whose exact int32 results are
+ * added through distributed shared memory, where the estimate says so; 0
+ * keeps one CTA per output tile), "skinny_max_m" (16 default: row counts up
+ * to this may take the few-row kernel on CUDA cores; 0, with split_k on, cuts
+ * the depth into runs through global memory instead of over clusters, for
+ * tests),
  * "gemv_lhs_const" (0 default; 1 promises that the matrix of the following
  * mb_gemv_u8 calls is not written by work enqueued ahead of them -- a weight,
  * the reference's Tensor::is_weight(), mace/core/tensor.h -- so its first
