@@ -748,8 +748,9 @@ int launch_cfg(mb_context *ctx, Params &p) {
   p.step_m = slots % p.tiles_m;
   p.step_n = (slots / p.tiles_m) % p.tiles_n;
   p.step_b = (slots / p.tiles_m) / p.tiles_n;
+  const bool sums = MODE == RUNS && p.run < ceil_div64(p.k_blocks, p.splits);  // (some CTA has more than one run)
   MB_CUDA(ctx, mb_launch_clusters(ctx, kern, static_cast<unsigned>(slots * p.splits), threads(EW),
-                                  C::SMEM_BYTES + ((p.splits > 1) + (MODE == RUNS && p.run < p.k_blocks)) * C::PART_BYTES,
+                                  C::SMEM_BYTES + ((p.splits > 1) + sums) * C::PART_BYTES,
                                   p.splits, map, p));
   ctx->launches++;
   ctx->launches_tc++;

@@ -436,7 +436,7 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
     g.KH = 3; g.KW = 3; g.pad_t = pad_top; g.pad_l = pad_left;
     g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
     // no larger an error than that of the Winograd kernels: 3.1e-8 times the root of C with F(2,3), 2e-6 and more with F(6,3)
-    g.run = pick_tile(H, W, tile_override) == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : 4;
+    g.run = pick_tile(H, W, tile_override) == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : C < 200 ? 4 : 6;
     if (mb_gemm_f32_gather_supported(ctx, g) &&
         (ctx->f32_gather == 2 || mb_gemm_f32_gather_cost(ctx, g) < winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override)))
       return mb_gemm_f32_gather_launch(ctx, g);
