@@ -849,6 +849,10 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
     fast_div_make(static_cast<uint32_t>(p.Wo), &p.wo_mul, &p.wo_shift);
 #define MB_F32_CONV(BN_, EW_, MODE_) \
   return w_tma ? launch_cfg<BN_, X_CONV, W_TMA, EW_, MODE_>(ctx, p) : launch_cfg<BN_, X_CONV, W_ROWS, EW_, MODE_>(ctx, p);
+    if (p.run == 1 && p.k_blocks <= 2) {
+      if (plan.bn == 128) { MB_F32_CONV(128, 8, SPREAD) }
+      MB_F32_CONV(64, 4, SPREAD)
+    }
     if (p.run != 0 && plan.bn == 128) { MB_F32_CONV(128, 8, RUNS) }
     if (plan.bn == 64 && (p.run != 0 || plan.warps == 4)) {
       // (one kernel for 64 channels with short runs or without: where a network's 1x1 and 3x3 layers took two in turn, every

@@ -338,6 +338,29 @@ def test_small_conv2d_f32_is_as_accurate_as_fmas(ctx, orc, case):
         b.free()
 
 
+@pytest.mark.parametrize("positive", [False, True])
+@pytest.mark.parametrize("C,O", [(48, 20), (64, 18), (64, 5), (80, 14)])
+def test_short_conv2d_f32_is_as_accurate_as_fmas(ctx, C, O, positive):
+    """1x1 convolutions of 14 x 15 pixels with too little work for a column matrix, at the depths of three accumulators.
+    (6 %: from a few thousand values.)"""
+    rng = np.random.Generator(np.random.PCG64(C + O))
+    draw = rng.random if positive else rng.standard_normal
+    x, f = draw((1, C, 14, 15)).astype(np.float32), draw((O, C, 1, 1)).astype(np.float32)
+    exact = np.einsum("nchw,oc->nohw", x.astype(np.float64), f[:, :, 0, 0].astype(np.float64))
+    dx, df, do = ctx.upload(x), ctx.upload(f), ctx.alloc(exact.size * 4)
+
+    def run():
+        ctx.conv2d_f32(dx, df, None, do, 1, C, 14, 15, O, 1, 1, (1, 1), (1, 1), (0, 0), (14, 15))
+        return _norm_err(ctx.download(do, exact.shape, np.float32), exact)
+
+    fma = _with_options(ctx, run, tensor_cores=0)
+    before = ctx.launches_tensor_core
+    assert run() <= 1.06 * fma
+    assert ctx.launches_tensor_core == before + 1
+    for b in (dx, df, do):
+        b.free()
+
+
 @pytest.mark.parametrize("case,tensor_core", [
     # kernel, C, HW, O: a single pixel, a few, on both sides of the depth from which the tensor cores are accurate enough
     ((1, 100, 1, 10), 1), ((1, 64, 4, 16), 1), ((3, 16, 3, 4), 1), ((1, 48, 2, 8), 1), ((1, 47, 2, 8), 0), ((3, 5, 9, 9), 0)])
