@@ -32,7 +32,7 @@
 // mb_f32_gather_run picks the run whose error is below the FMA chain's, for products that would otherwise run on CUDA cores;
 // none is up to k = 47 and from 65 to 71.  A 3x3 convolution in place of Winograd kernels takes the run whose error is below
 // theirs (F(2,3): 3.1e-8 times the root of the channels, F(6,3): 2e-6 and more).  The sums cost 384 x 384 x 64, batch
-// 12, 0.9 us of 6.7 (SPREAD), the 3x3 layers of ResNet-50 at batch 1 0.2 to 1.5 us each, and the largest products, whose
+// 12, 1.1 us of 6.7 (SPREAD, with the check of its results), the 3x3 layers of ResNet-50 at batch 1 0.2 to 1.5 us each, and the largest products, whose
 // shared memory is busy with W already, a half (1536 x 1536 x 1024: 33 -> 50 us; 136 us on CUDA cores).  Sums in registers
 // instead spilled: 96 registers for four result warps, 80 for eight.
 //
