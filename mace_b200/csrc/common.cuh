@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -36,6 +38,13 @@ struct mb_context {
   // call carves from the start; contents do not survive the call.
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
+  // W of fp32 products split in front of them (gemm_f32_pairs.cu); blocks that a recorded graph may refer to are kept
+  void *weight_scratch = nullptr;
+  size_t weight_scratch_bytes = 0;
+  std::vector<void *> weight_scratch_kept;
+  bool captured_any = false;   // a graph has been recorded on this context
+  int f32_pairs = 0;           // gemm_f32_pairs.cu: 0 by rule, 1 never, 2 wherever it can run
+  uint32_t f32_pairs_attr_mask = 0;  // kernels of gemm_f32_pairs.cu whose shared-memory limit was raised
   int *dev_status = nullptr;   // status word of bounded-wait failures: the device's address of host_status
   int *host_status = nullptr;  // the word itself, in page-locked host memory: read there at sync
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
@@ -108,6 +117,9 @@ int mb_check_cuda(mb_context *ctx, cudaError_t e, const char *what);
 // Returns a device pointer to at least `bytes` of scratch (256-byte aligned),
 // growing the arena if needed.  offset allows several carve-outs per call.
 int mb_scratch(mb_context *ctx, size_t bytes, void **ptr);
+// Another such arena, for a call that may run inside one that has carved the first.  *ptr is null where it would have to grow
+// inside a graph capture: the caller then does without.  Never freed before the context once a graph may refer to it.
+int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr);
 
 // ---- programmatic dependent launch ------------------------------------------------------------
 // A kernel launched through mb_launch_chained may be started before the kernel in front of it in

@@ -45,6 +45,26 @@ int mb_scratch(mb_context *ctx, size_t bytes, void **ptr) {
   return MB_SUCCESS;
 }
 
+int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr) {
+  *ptr = nullptr;
+  if (bytes > ctx->weight_scratch_bytes) {
+    if (ctx->capturing) return MB_SUCCESS;
+    const size_t want = align_up(bytes + bytes / 2, 1 << 20);  // (so few blocks, each half as large again, are ever kept)
+    void *block = nullptr;
+    if (ctx->captured_any) ctx->weight_scratch_kept.reserve(ctx->weight_scratch_kept.size() + 1);
+    MB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    MB_CUDA(ctx, cudaMalloc(&block, want));
+    if (ctx->weight_scratch != nullptr) {
+      if (ctx->captured_any) ctx->weight_scratch_kept.push_back(ctx->weight_scratch);
+      else cudaFree(ctx->weight_scratch);
+    }
+    ctx->weight_scratch = block;
+    ctx->weight_scratch_bytes = want;
+  }
+  *ptr = ctx->weight_scratch;
+  return MB_SUCCESS;
+}
+
 namespace {
 
 // Results to page-locked host memory, by a kernel that writes there itself: behind other kernels of a stream the copy engine
@@ -156,6 +176,8 @@ int mb_destroy(mb_context *ctx) {
     cudaStreamDestroy(ctx->upload_stream);
   }
   if (ctx->scratch) cudaFree(ctx->scratch);
+  if (ctx->weight_scratch) cudaFree(ctx->weight_scratch);
+  for (void *block : ctx->weight_scratch_kept) cudaFree(block);
   if (ctx->skinny_ws) cudaFree(ctx->skinny_ws);
   if (ctx->host_status) cudaFreeHost(ctx->host_status);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -410,6 +432,7 @@ int mb_graph_begin(mb_context *ctx) {
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
   MB_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   ctx->capturing = 1;
+  ctx->captured_any = true;
   ctx->capture_launches0 = ctx->launches;
   ctx->capture_launches_tc0 = ctx->launches_tc;
   return MB_SUCCESS;
@@ -485,6 +508,9 @@ int mb_set_option(mb_context *ctx, const char *name, int value) {
     // accepted and without effect: MN-major operands always reach the tensor core in place
   } else if (strcmp(name, "f32_gather") == 0) {
     ctx->f32_gather = value;
+  } else if (strcmp(name, "f32_pairs") == 0) {
+    if (value < 0 || value > 2) return mb_fail(ctx, MB_INVALID_ARGS, "f32_pairs must be 0, 1 or 2");
+    ctx->f32_pairs = value;
   } else if (strcmp(name, "f32_bn") == 0) {
     if (value != 0 && value != 64 && value != 128) return mb_fail(ctx, MB_INVALID_ARGS, "f32_bn must be 0, 64 or 128");
     ctx->f32_bn = value;

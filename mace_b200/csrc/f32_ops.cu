@@ -18,6 +18,8 @@ int mb_gemm_f32_tc_launch(mb_context *ctx, const float *X, const float *W, const
                           int64_t c_row_stride, int64_t c_batch_stride, int act, float max_limit,
                           float coef, const float *residual);
 
+bool mb_gemm_f32_pairs_pays(const mb_context *ctx, int64_t batch, int64_t Mdim, int64_t Ndim, int64_t K, int w_batched);
+
 int mb_dwconv_f32_launch(mb_context *ctx, const float *in, const float *filter, const float *bias, float *out,
                          int64_t N, int64_t C, int64_t H, int64_t W, int64_t mult_ch, int64_t KH, int64_t KW,
                          int stride_h, int stride_w, int dil_h, int dil_w, int pad_top, int pad_left, int64_t Ho,
@@ -356,16 +358,19 @@ static bool take_gather(mb_context *ctx, mb_f32_gemm &g, bool by_tma, bool fp32_
   if (ctx->f32_gather == 2) return true;
   if (fp32_accuracy && g.run == 0) return false;
   if (!by_tma) return true;
-  // The TMA-fed kernel: tiles of 128 columns of one image (or matrix), 1200 cycles per step, 2.6 us for the results of 128
-  // channels (twice that with a residual), 4.4 us around them.
+  // The TMA-fed kernels: tiles of 128 columns of one image (or matrix), 1200 cycles per step, 2.6 us for the results of 128
+  // channels (twice that with a residual), 4.4 us around them; from the size on where W is split in front (gemm_f32_pairs.cu) 750
+  // (600 for 64 channels), 2 us for the results, 6 us around them.
   const int64_t images = g.conv ? g.M / (static_cast<int64_t>(g.Ho) * g.Wo) : g.batch;
-  const int64_t tiles_m = ceil_div64(g.M / (g.conv ? images : 1), 128), steps = ceil_div64(g.K, 32);
+  const int64_t columns = g.M / (g.conv ? images : 1), tiles_m = ceil_div64(columns, 128), steps = ceil_div64(g.K, 32);
+  const bool pairs = mb_gemm_f32_pairs_pays(ctx, images, columns, g.N, g.K, g.w_bs != 0);
   int64_t tma = -1;
   for (int w : {128, 64}) {
     if (w == 128 && g.N <= 64) continue;
     const int64_t rounds = ceil_div64(images * tiles_m * ceil_div64(g.N, w), ctx->num_sms);
-    const int64_t results = (w == 128 ? 5000 : 3000) * (g.residual != nullptr ? 2 : 1);
-    const int64_t cost = 8300 + rounds * std::max<int64_t>(steps * 1200, results);
+    const int64_t results = pairs ? (w == 128 ? 3800 : 2400) : (w == 128 ? 5000 : 3000) * (g.residual != nullptr ? 2 : 1);
+    const int64_t step = !pairs ? 1200 : w == 128 ? 750 : 600;
+    const int64_t cost = (pairs ? 11500 : 8300) + rounds * std::max<int64_t>(steps * step, results);
     if (tma < 0 || cost < tma) tma = cost;
   }
   return mb_gemm_f32_gather_cost(ctx, g) < tma;

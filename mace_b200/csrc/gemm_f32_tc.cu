@@ -654,11 +654,25 @@ bool mb_gemm_f32_tc_supported(const mb_context *ctx, const float *X, const float
   return true;
 }
 
+bool mb_gemm_f32_pairs_pays(const mb_context *ctx, int64_t batch, int64_t Mdim, int64_t Ndim, int64_t K, int w_batched);
+int mb_gemm_f32_pairs_launch(mb_context *ctx, const float *X, const float *W, const float *bias, float *C,
+                             int64_t batch, int64_t Mdim, int64_t Ndim, int64_t K, int64_t x_row_stride,
+                             int64_t x_batch_stride, int64_t w_row_stride, int64_t w_batch_stride,
+                             int64_t c_row_stride, int64_t c_batch_stride, int act, float max_limit,
+                             float coef, const float *residual, bool *done);
+
 int mb_gemm_f32_tc_launch(mb_context *ctx, const float *X, const float *W, const float *bias, float *C,
                           int64_t batch, int64_t Mdim, int64_t Ndim, int64_t K, int64_t x_row_stride,
                           int64_t x_batch_stride, int64_t w_row_stride, int64_t w_batch_stride,
                           int64_t c_row_stride, int64_t c_batch_stride, int act, float max_limit,
                           float coef, const float *residual) {
+  if (mb_gemm_f32_pairs_pays(ctx, batch, Mdim, Ndim, K, w_batch_stride != 0)) {
+    bool done = false;
+    MB_RETURN_IF_ERROR(mb_gemm_f32_pairs_launch(ctx, X, W, bias, C, batch, Mdim, Ndim, K, x_row_stride, x_batch_stride,
+                                                w_row_stride, w_batch_stride, c_row_stride, c_batch_stride, act, max_limit, coef,
+                                                residual, &done));
+    if (done) return MB_SUCCESS;
+  }
   const int BN = Ndim > 64 ? 128 : 64;
   F32TcParams p;
   p.Mdim = Mdim; p.Ndim = Ndim; p.K = K; p.batch = batch;

@@ -1,0 +1,137 @@
+"""The fp32 GEMM on pairs of halves (gemm_f32_pairs.cu) against float64, with bounds derived from its arithmetic, at the edges of
+its tiles, and where its split of a value into two halves does not reach."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import mace_b200
+    c = mace_b200.Context(0)
+    yield c
+    c.close()
+
+
+def _bound(A, B):
+    """hi + lo of a value is within 2^-22 of it, or 2^-26 of the largest value of its row or column; the accumulator is cut off by
+    at most 2^-23 of what it holds after each of three MMAs per 16 of the depth."""
+    A, B = np.abs(A), np.abs(B)
+    K = A.shape[-1]
+    return (A @ B) * (2.0 ** -21 + (3 * K / 16 + 4) * 2.0 ** -23) + \
+        K * A.max(axis=-1)[..., :, None] * B.max(axis=-2)[..., None, :] * 2.0 ** -25 + 1e-30
+
+
+def _matmul(ctx, A, B, pairs=2):
+    batch, M, K = A.shape
+    N = B.shape[2]
+    dA, dB, dC = ctx.upload(A), ctx.upload(B), ctx.upload(np.full((batch, M, N), 7, np.float32))
+    ctx.set_option("f32_gather", 1)
+    ctx.set_option("f32_pairs", pairs)
+    ctx.gemm_f32(dA, dB, dC, batch, M, N, K)
+    for name in ("f32_gather", "f32_pairs"):
+        ctx.set_option(name, 0)
+    got = ctx.download(dC, (batch, M, N), np.float32)
+    for b in (dA, dB, dC):
+        b.free()
+    return got
+
+
+@pytest.mark.parametrize("shape", [
+    # batch, M (channels), N (pixels), K: narrow and wide column tiles, depths of one to many steps with odd halves of the last one,
+    # more tiles than SMs, results that TMA does not store (fewer than 16 rows)
+    (1, 16, 128, 4), (1, 64, 132, 16), (2, 65, 32, 20), (3, 7, 260, 48), (1, 128, 256, 32), (2, 200, 100, 64), (5, 33, 1000, 260),
+    (30, 130, 640, 36), (1, 1000, 40, 1028), (9, 64, 3000, 100)])
+def test_gemm_f32_pairs(ctx, shape):
+    batch, M, N, K = shape
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.standard_normal((batch, M, K)).astype(np.float32)
+    B = rng.standard_normal((batch, K, N)).astype(np.float32)
+    before = ctx.launches_tensor_core, ctx.launches
+    got = _matmul(ctx, A, B)
+    assert (ctx.launches_tensor_core, ctx.launches) == (before[0] + 1, before[1] + 2)
+    A, B = A.astype(np.float64), B.astype(np.float64)
+    assert (np.abs(got - A @ B) <= _bound(A, B)).all()
+
+
+@pytest.mark.parametrize("shape", [(2, 32, 144, 64), (3, 100, 576, 130), (1, 20, 196, 8), (2, 260, 784, 256)])
+@pytest.mark.parametrize("act", [0, 1, 2, 6])
+@pytest.mark.parametrize("residual", [False, True])
+def test_conv1x1_f32_pairs(ctx, shape, act, residual):
+    """Bias, residual sum and activation of a 1x1 convolution (the residual lands where the result leaves from)."""
+    N, C, HW, O = shape
+    rng = np.random.Generator(np.random.PCG64(O))
+    x = rng.standard_normal((N, C, HW)).astype(np.float32)
+    f = (rng.standard_normal((O, C)) * 0.2).astype(np.float32)
+    bias = rng.standard_normal(O).astype(np.float32) if act != 1 else None
+    r = rng.standard_normal((N, O, HW)).astype(np.float32)
+    dx, df, dr, do = ctx.upload(x), ctx.upload(f), ctx.upload(r), ctx.upload(np.zeros((N, O, HW), np.float32))
+    db = ctx.upload(bias) if bias is not None else None
+    side = (HW // 4, 4)
+    for name, value in (("f32_gather", 1), ("f32_pairs", 2)):
+        ctx.set_option(name, value)
+    if residual:
+        ctx.conv2d_f32_residual(dx, df, db, dr, do, N, C, *side, O, 1, 1, (1, 1), (1, 1), (0, 0), side, act, 0.6, 0.25)
+    else:
+        ctx.conv2d_f32(dx, df, db, do, N, C, *side, O, 1, 1, (1, 1), (1, 1), (0, 0), side, act, 0.6, 0.25)
+    for name in ("f32_gather", "f32_pairs"):
+        ctx.set_option(name, 0)
+    got = ctx.download(do, (N, O, HW), np.float32)
+    x, f = x.astype(np.float64), np.broadcast_to(f.astype(np.float64), (N, O, C))
+    ref = f @ x + (bias.astype(np.float64)[None, :, None] if bias is not None else 0) + (r if residual else 0)
+    size = np.abs(ref)
+    ref = {0: ref, 1: np.maximum(ref, 0), 2: np.clip(ref, 0, np.float32(0.6)), 6: np.where(ref > 0, ref, ref * 0.25)}[act]
+    assert (np.abs(got - ref) <= _bound(f, x) + 2.0 ** -22 * (size + 1)).all()
+    for b in (dx, df, dr, do) + ((db,) if db else ()):
+        b.free()
+
+
+@pytest.mark.parametrize("M", [40, 150])
+@pytest.mark.parametrize("what", ["zeros", "late", "tiny", "huge", "steep", "inf", "nan", "inf_row"])
+def test_gemm_f32_pairs_beyond_the_split(ctx, M, what):
+    """Rows and columns of zeros, scales that a later step exceeds, values that halves do not hold: FMAs take over."""
+    batch, N, K = 2, 300, 132
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.standard_normal((batch, M, K)).astype(np.float32)
+    B = rng.standard_normal((batch, K, N)).astype(np.float32)
+    if what == "zeros":
+        A[:, 3], B[:, :, 7], B[0, :100], B[1, :40, 128:] = 0, 0, 0, 0
+    elif what == "late":
+        B[:, 96:, ::3] *= np.float32(2.0 ** 18)
+    elif what == "tiny":
+        A *= np.float32(1e-25)
+        B *= np.float32(1e-3)
+    elif what == "huge":
+        A *= np.float32(1e25)
+        B *= np.float32(1e-22)
+    elif what == "steep":
+        A *= np.float32(10.0) ** rng.integers(-9, 9, (1, M, 1)).astype(np.float32)
+        B *= np.float32(10.0) ** rng.integers(-9, 9, (1, 1, N)).astype(np.float32)
+    elif what == "inf":
+        B[1, 50, 9] = np.inf
+    elif what == "nan":
+        B[0, 131, 299] = np.nan
+    elif what == "inf_row":
+        A[0, 5, 0] = -np.inf
+    got = _matmul(ctx, A, B)
+    with np.errstate(all="ignore"):
+        A, B = A.astype(np.float64), B.astype(np.float64)
+        ref = np.einsum("bmk,bkn->bmn", A, B)
+        assert np.array_equal(np.isnan(got), np.isnan(ref))
+        assert np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+        finite = np.isfinite(ref)
+        A, B = np.where(np.isfinite(A), A, 0), np.where(np.isfinite(B), B, 0)
+        # (worked out again, a sum of K products rounds K times)
+        bound = _bound(A, B) + (np.abs(A) @ np.abs(B)) * K * 2.0 ** -24
+        assert (np.abs(got - ref)[finite] <= bound[finite]).all()
+
+
+def test_gemm_f32_pairs_choice(ctx):
+    """By rule for a product of many steps, with an error no larger than the other kernel's."""
+    rng = np.random.Generator(np.random.PCG64(0))
+    A = rng.standard_normal((1, 256, 512)).astype(np.float32)
+    B = rng.standard_normal((1, 512, 128 * 600)).astype(np.float32)
+    exact = A[0].astype(np.float64) @ B[0].astype(np.float64)
+    err = [np.linalg.norm(_matmul(ctx, A, B, pairs)[0] - exact) for pairs in (0, 1, 2)]
+    assert err[0] == err[2] < err[1]
