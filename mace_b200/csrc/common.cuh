@@ -38,12 +38,15 @@ struct mb_context {
   // call carves from the start; contents do not survive the call.
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
-  // W of fp32 products split in front of them (gemm_f32_pairs.cu); blocks that a recorded graph may refer to are kept
+  // W of fp32 products split in front of them (gemm_f32_pairs.cu, conv_f32_direct.cu); blocks that a recorded graph may refer to are kept
   void *weight_scratch = nullptr;
   size_t weight_scratch_bytes = 0;
   std::vector<void *> weight_scratch_kept;
   bool captured_any = false;   // a graph has been recorded on this context
   int f32_pairs = 0;           // gemm_f32_pairs.cu: 0 by rule, 1 never, 2 wherever it can run
+  int f32_direct = 0;          // fp32 convolutions of conv_f32_direct.cu: 0 by rule, 1 never, 2 wherever they can run
+  bool f32_conv_presplit_smem = false;  // the limit of the kernel that splits their filter was raised
+  int f32_direct_smem[4] = {0, 0, 0, 0};  // shared-memory limits its kernels were given
   uint32_t f32_pairs_attr_mask = 0;  // kernels of gemm_f32_pairs.cu whose shared-memory limit was raised
   int *dev_status = nullptr;   // status word of bounded-wait failures: the device's address of host_status
   int *host_status = nullptr;  // the word itself, in page-locked host memory: read there at sync

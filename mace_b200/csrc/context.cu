@@ -508,6 +508,9 @@ int mb_set_option(mb_context *ctx, const char *name, int value) {
     // accepted and without effect: MN-major operands always reach the tensor core in place
   } else if (strcmp(name, "f32_gather") == 0) {
     ctx->f32_gather = value;
+  } else if (strcmp(name, "f32_direct") == 0) {
+    if (value < 0 || value > 2) return mb_fail(ctx, MB_INVALID_ARGS, "f32_direct must be 0, 1 or 2");
+    ctx->f32_direct = value;
   } else if (strcmp(name, "f32_pairs") == 0) {
     if (value < 0 || value > 2) return mb_fail(ctx, MB_INVALID_ARGS, "f32_pairs must be 0, 1 or 2");
     ctx->f32_pairs = value;

@@ -1,0 +1,20 @@
+// Stride-1 fp32 convolutions with SAME padding as a direct product on the tensor cores (conv_f32_direct.cu).
+#pragma once
+
+#include "common.cuh"
+
+struct mb_f32_conv {
+  const float *X = nullptr, *filter = nullptr, *bias = nullptr;  // NCHW, OIHW, null or one per output channel
+  float *out = nullptr;
+  int64_t N = 0, C = 0, H = 0, W = 0, O = 0;
+  int KH = 3, KW = 3;  // odd; the output is as large as the input
+  int act = 0;
+  float max_limit = 0.f, coef = 0.f;
+  int run = 1;         // filter rows of 32 channels that the tensor core adds up before the sum is carried on in fp32
+};
+
+bool mb_conv_f32_direct_supported(const mb_context *ctx, const mb_f32_conv &g);
+// Estimated time in SM cycles.
+int64_t mb_conv_f32_direct_cost(const mb_context *ctx, const mb_f32_conv &g);
+// *done is false where nothing was launched, for want of room for the split filter inside a graph capture.
+int mb_conv_f32_direct_launch(mb_context *ctx, const mb_f32_conv &g, bool *done);

@@ -7,6 +7,7 @@
 // index order; these kernels accumulate in fp32 in a tiled order, so results
 // agree to rounding (tests bound the difference at 1e-4 of the output range).
 #include "common.cuh"
+#include "conv_f32_direct.cuh"
 #include "gemm_f32_gather.cuh"
 
 bool mb_gemm_f32_tc_supported(const mb_context *ctx, const float *X, const float *W, int64_t Mdim,
@@ -628,6 +629,23 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
     const bool on_cores = pointwise && long_rows(H * W) ? !by_tma : !column_route(N, C, O, KH, KW, Ho, Wo);
     mb_f32_gemm g = conv_gemm(in, filter, bias, nullptr, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h, dil_w, pad_top,
                               pad_left, Ho, Wo, activation, max_limit, coefficient);
+    // Stride 1, the output as large as the input: every input value split once instead of once per tap.  Nine taps and more:
+    // with fewer the input's way through registers is what a block waits for (512 -> 128 channels, 1x1, 28 x 28, batch 16:
+    // 35 us against 17; 64 -> 64, 5x5, 56 x 56, batch 24: 69 against 130).
+    mb_f32_conv d;
+    d.X = in; d.filter = filter; d.bias = bias; d.out = out;
+    d.N = N; d.C = C; d.H = H; d.W = W; d.O = O; d.KH = static_cast<int>(std::min<int64_t>(KH, 99)); d.KW = static_cast<int>(std::min<int64_t>(KW, 99));
+    d.act = activation; d.max_limit = max_limit; d.coef = coefficient;
+    d.run = static_cast<int>(std::max<int64_t>(1, 10 / KW));  // an error of 3.5e-7 to 4e-7, the self-fetching kernel's at depth 60
+    if (stride_h == 1 && stride_w == 1 && dil_h == 1 && dil_w == 1 && pad_top == KH / 2 && pad_left == KW / 2 && Ho == H && Wo == W &&
+        ctx->f32_direct != 1 && mb_conv_f32_direct_supported(ctx, d) &&
+        (ctx->f32_direct == 2 || (ctx->f32_gather == 0 && !on_cores && KH * KW >= 9 && C * KH * KW >= 128 &&
+                                  mb_gemm_f32_gather_supported(ctx, g) &&
+                                  mb_conv_f32_direct_cost(ctx, d) < mb_gemm_f32_gather_cost(ctx, g)))) {
+      bool done = false;
+      MB_RETURN_IF_ERROR(mb_conv_f32_direct_launch(ctx, d, &done));
+      if (done) return MB_SUCCESS;
+    }
     // However small: the one-thread-per-output kernel is a serial chain over the depth (depth 64, 4 x 4 pixels, 22.8 us against
     // 6.5; 144, 3 x 3, 18.8 against 6.6; near the line, 48 to 54, 4.5 to 14 against 5.0 to 6.7).
     if (take_gather(ctx, g, by_tma, on_cores)) return mb_gemm_f32_gather_launch(ctx, g);

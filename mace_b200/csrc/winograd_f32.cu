@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "conv_f32_direct.cuh"
 #include "gemm_f32_gather.cuh"
 
 int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *C,
@@ -426,7 +427,9 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
   // A direct convolution where the three launches cost more.  Only with both forms of the filter at hand: a call with one of
   // them gives bit for bit what a call with the other does.
-  if (filter != nullptr && transformed_filter != nullptr && ctx->f32_gather != 1) {
+  if (filter != nullptr && transformed_filter != nullptr) {
+    const int tile = pick_tile(H, W, tile_override);
+    int64_t best = winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override);
     mb_f32_gemm g;
     g.X = in; g.W = filter; g.bias = bias; g.C = out;
     g.M = N * Ho * Wo; g.N = O; g.K = C * 9;
@@ -436,10 +439,27 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
     g.KH = 3; g.KW = 3; g.pad_t = pad_top; g.pad_l = pad_left;
     g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
     // no larger an error than that of the Winograd kernels: 3.1e-8 times the root of C with F(2,3), 2e-6 and more with F(6,3)
-    g.run = pick_tile(H, W, tile_override) == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : C < 200 ? 4 : 6;
-    if (mb_gemm_f32_gather_supported(ctx, g) &&
-        (ctx->f32_gather == 2 || mb_gemm_f32_gather_cost(ctx, g) < winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override)))
-      return mb_gemm_f32_gather_launch(ctx, g);
+    g.run = tile == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : C < 200 ? 4 : 6;
+    bool gather = false;
+    if (ctx->f32_gather != 1 && mb_gemm_f32_gather_supported(ctx, g)) {
+      const int64_t cost = mb_gemm_f32_gather_cost(ctx, g);
+      gather = ctx->f32_gather == 2 || cost < best;
+      if (gather) best = cost;
+    }
+    // (errors of 1.3e-7, 3.5e-7 and 1.4e-6 with runs of one, three and twelve filter rows)
+    mb_f32_conv d;
+    d.X = in; d.filter = filter; d.bias = bias; d.out = out;
+    d.N = N; d.C = C; d.H = H; d.W = W; d.O = O;
+    d.act = activation; d.max_limit = max_limit; d.coef = coefficient;
+    d.run = gather || (tile == 2 && C <= 128) ? 1 : tile == 6 ? 12 : 3;
+    if (Ho == H && Wo == W && pad_top == 1 && pad_left == 1 && ctx->f32_direct != 1 && mb_conv_f32_direct_supported(ctx, d) &&
+        (ctx->f32_direct == 2 ||
+         (ctx->f32_gather == 0 && mb_conv_f32_direct_cost(ctx, d) < best))) {
+      bool done = false;
+      MB_RETURN_IF_ERROR(mb_conv_f32_direct_launch(ctx, d, &done));
+      if (done) return MB_SUCCESS;
+    }
+    if (gather) return mb_gemm_f32_gather_launch(ctx, g);
   }
   const int tile = pick_tile(H, W, tile_override);
   const int T = (tile + 2) * (tile + 2);
