@@ -12,7 +12,7 @@
 //
 // A row's scale is that of the first step of 32 in which it has a value other than zero (zeros need none), so that nothing has
 // to be read twice.  Later values may be 2^14 times larger; beyond that hi is infinite and the results of that row come out as
-// NaN, like those of an infinite value or of a row below 2^-61, and are worked out again by fp32 FMAs (store_exact4).
+// NaN, like those of an infinite value or of a row below 2^-61, and are marked, and worked out again by fp32 FMAs.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -47,14 +47,4 @@ __device__ __forceinline__ void f32_split2(uint64_t v, uint64_t s, uint32_t &hi,
   const __half2 l = __floats2half2_rn(r0, r1);
   hi = *reinterpret_cast<const uint32_t *>(&h);
   lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-
-// Where four k (chunk 0 .. 7 of a step of 32) of channel n's hi half lie in a step of W in shared memory; its lo half lies at
-// F32_W_LO ^ that.  128 channels: rows of 128 bytes, hi in the first half, in the tensor core's 128-byte swizzle; 64: rows of 64
-// bytes in the 64-byte swizzle, hi in row 2 n and lo in 2 n + 1.  Either way a channel keeps to the 128 bytes in which its
-// fp32 values land.
-constexpr uint32_t F32_W_LO = 64;
-template <int BN>
-__device__ __forceinline__ uint32_t f32_w_at(int n, int chunk) {
-  return static_cast<uint32_t>(n * 128 + (((chunk >> 1) ^ (n & (BN == 64 ? 3 : 7))) << 4) + (chunk & 1) * 8);
 }

@@ -759,7 +759,7 @@ int launch_cfg(mb_context *ctx, Params &p) {
 
 struct Plan {
   int bn = 64, splits = 1, warps = 4;
-  int64_t cost = -1;
+  int64_t cost = -1, steps = 0;  // (steps of a CTA beyond the first two of a tile)
 };
 
 // Tile width and depth runs with the smallest estimate, in SM cycles.  Measured: a step is bound by the MMAs, whose A
@@ -795,7 +795,7 @@ Plan make_plan(mb_context *ctx, const mb_f32_gemm &g) {
                            : w == 128 ? 10500 + steps * 1350 + last
                                       : (s == 2 ? 11500 : s == 4 ? 10500 : 11000) + steps * (s == 2 ? 1150 : 1050) + last);
       if (best.cost < 0 || cost < best.cost) {
-        best.bn = w; best.splits = s; best.warps = eight ? 8 : 4; best.cost = cost;
+        best.bn = w; best.splits = s; best.warps = eight ? 8 : 4; best.cost = cost; best.steps = rounds * std::max<int64_t>(0, steps - 2);
       }
     }
   }
@@ -815,7 +815,11 @@ bool mb_gemm_f32_gather_supported(const mb_context *ctx, const mb_f32_gemm &g) {
   return g.x_ms != 1 || g.K * g.x_ks < (1ll << 31);
 }
 
-int64_t mb_gemm_f32_gather_cost(mb_context *ctx, const mb_f32_gemm &g) { return make_plan(ctx, g).cost; }
+int64_t mb_gemm_f32_gather_cost(mb_context *ctx, const mb_f32_gemm &g) {
+  const Plan plan = make_plan(ctx, g);
+  // (X with its depth contiguous is a lane per row, 32 lines per load: 2550 cycles per step of 128 columns, 1950 of 64)
+  return plan.cost + (!g.conv && g.x_ms != 1 ? plan.steps * (plan.bn == 128 ? 1300 : 850) : 0);
+}
 
 int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
   const Plan plan = make_plan(ctx, g);

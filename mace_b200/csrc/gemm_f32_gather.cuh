@@ -31,3 +31,7 @@ bool mb_gemm_f32_gather_supported(const mb_context *ctx, const mb_f32_gemm &g);
 // Estimated time of the launch in SM cycles.
 int64_t mb_gemm_f32_gather_cost(mb_context *ctx, const mb_f32_gemm &g);
 int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g);
+// The same where both operands have their depth contiguous and lie as TMA wants them (gemm_f32_rows.cu).
+bool mb_gemm_f32_rows_supported(const mb_context *ctx, const mb_f32_gemm &g);
+int64_t mb_gemm_f32_rows_cost(const mb_context *ctx, const mb_f32_gemm &g);
+int mb_gemm_f32_rows_launch(mb_context *ctx, const mb_f32_gemm &g);

@@ -435,36 +435,9 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem,
       : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem], half-precision inputs, fp32 accumulation: lane = row of A, two k per 32-bit column.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same with A in shared memory.
-__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same called by a whole warp with the same operands, one of whose threads issues: the operands then come from uniform
-// registers (issued inside a branch that one thread takes, each is moved there first: 85 cycles per MMA).
+// D[tmem] (+)= A * B, half-precision inputs, fp32 accumulation, B in shared memory, A there (ss) or in tensor memory (ts: lane = row,
+// two k per 32-bit column).  Called by a whole warp with the same operands, one of whose threads issues: the operands then
+// come from uniform registers (issued inside a branch that one thread takes, each is moved there first: 85 cycles per MMA).
 __device__ __forceinline__ void mma_f16_ss_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                  uint32_t accumulate) {
   asm volatile(
