@@ -149,7 +149,7 @@ int mb_pair_clusters(const mb_context *ctx);
  * "f32_bn" (0 / 64 / 128) and "f32_splits" (0 / 1 / 2 / 4 / 8) its tile width and
  * depth runs (0: by rule), "f32_pairs" (0 default: by rule; 1 never, 2 wherever it can run:
  * the fp32 GEMM on pairs of halves), "f32_direct" (the same of the direct stride-1 fp32
- * convolution), "f32_rows" (of the fp32 GEMM whose operands both have their depth contiguous), "wino_plane" (1 default; 0 takes the one-thread-per-tile Winograd
+ * convolution), "f32_stem" (fp32 convolutions of up to four channels with a stride of two as direct products), "f32_rows" (of the fp32 GEMM whose operands both have their depth contiguous), "wino_plane" (1 default; 0 takes the one-thread-per-tile Winograd
  * output transform instead of the plane-at-a-time one, for A/B tests), "pdl"
  * (1 default; 0 launches the kernels of the uint8 operator chain in plain
  * stream order instead of with programmatic stream serialization),

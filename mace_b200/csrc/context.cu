@@ -511,6 +511,9 @@ int mb_set_option(mb_context *ctx, const char *name, int value) {
   } else if (strcmp(name, "f32_direct") == 0) {
     if (value < 0 || value > 2) return mb_fail(ctx, MB_INVALID_ARGS, "f32_direct must be 0, 1 or 2");
     ctx->f32_direct = value;
+  } else if (strcmp(name, "f32_stem") == 0) {
+    if (value < 0 || value > 2) return mb_fail(ctx, MB_INVALID_ARGS, "f32_stem must be 0, 1 or 2");
+    ctx->f32_stem = value;
   } else if (strcmp(name, "f32_rows") == 0) {
     if (value < 0 || value > 2) return mb_fail(ctx, MB_INVALID_ARGS, "f32_rows must be 0, 1 or 2");
     ctx->f32_rows = value;

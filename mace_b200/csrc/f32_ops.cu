@@ -655,6 +655,13 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter, co
       MB_RETURN_IF_ERROR(mb_conv_f32_direct_launch(ctx, d, &done));
       if (done) return MB_SUCCESS;
     }
+    // Few input channels, a stride of two columns: input values split once, not once per tap, where the estimate is the smaller
+    // (3 -> 64 channels, 7x7, 224 x 224, batch 8: 30 us fetching its own operands, 22 this way; 2: 12.9 and 13.6).  Up to 64 deep
+    // the self-fetching kernel's form with three accumulators is the more accurate.
+    if (dil_h == 1 && dil_w == 1 && ctx->f32_stem != 1 && mb_conv_f32_stem_supported(ctx, d, stride_h, stride_w, pad_left, Ho, Wo) &&
+        (ctx->f32_stem == 2 || (ctx->f32_gather == 0 && !on_cores && C * KH * KW > 64 && mb_gemm_f32_gather_supported(ctx, g) &&
+                                mb_conv_f32_stem_cost(ctx, d, stride_h, Ho, Wo) < mb_gemm_f32_gather_cost(ctx, g))))
+      return mb_conv_f32_stem_launch(ctx, d, stride_h, pad_top, pad_left, Ho, Wo);
     // However small: the one-thread-per-output kernel is a serial chain over the depth (depth 64, 4 x 4 pixels, 22.8 us against
     // 6.5; 144, 3 x 3, 18.8 against 6.6; near the line, 48 to 54, 4.5 to 14 against 5.0 to 6.7).
     if (take_gather(ctx, g, by_tma, on_cores)) return mb_gemm_f32_gather_launch(ctx, g);
