@@ -9,7 +9,8 @@
 // in another, both twice.  Every `run` steps the result warps take them and carry the sums on in registers: with one step the
 // error is 1.16e-7, with three 1.76e-7 (2-norm against float64; the self-fetching kernel on tf32: 1.37e-7, 2.06e-7).
 //
-// What bounds it: launch, first copies and results for few steps; shared memory else, 144 KB or 1150 cycles per step of 128 x 128.
+// What bounds it: launch, first copies and results for few steps; the shared-memory pipe else (57 % busy: 1150 cycles per step of 128 x 128
+// for copies, split and MMAs, with waits between the three).
 // Against the kernel whose warps fetch X from where it lies (a lane a row: 32 lines per instruction): see cost_of.
 //
 // Roles: warp 0 copies, warp 1 MMAs, 8 warps split, 8 or 16 results (32 columns of n per thread).  Persistent over the tiles.
