@@ -46,7 +46,7 @@ struct mb_context {
   int f32_pairs = 0;           // gemm_f32_pairs.cu: 0 by rule, 1 never, 2 wherever it can run
   int f32_direct = 0;          // fp32 convolutions of conv_f32_direct.cu: 0 by rule, 1 never, 2 wherever they can run
   bool f32_conv_presplit_smem = false;  // the limit of the kernel that splits their filter was raised
-  int f32_direct_smem[4] = {0, 0, 0, 0};  // shared-memory limits its kernels were given
+  bool f32_direct_smem[4] = {false, false, false, false};  // its kernels whose shared-memory limit was raised
   int f32_stem = 0;            // conv_f32_stem.cu: 0 by rule, 1 never, 2 wherever it can run
   int f32_stem_smem[4] = {0, 0, 0, 0};  // shared-memory limits its kernels were given
   int f32_rows = 0;            // gemm_f32_rows.cu: 0 by rule, 1 never, 2 wherever it can run

@@ -513,10 +513,11 @@ int launch(mb_context *ctx, Params &p, const void *split) {
   if (p.w_stays) p.w_stages = p.blocks * p.KH;
   const int smem = around + p.w_stages * row;
   auto kern = conv_f32_direct_kernel<BN, TAPS>;
-  int &limit = ctx->f32_direct_smem[(BN == 128) * 2 + (TAPS != 0)];
-  if (smem > limit) {
-    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    limit = smem;
+  // (the limit is the device's, not this context's: the largest for all, or a context's small call would take room from another's)
+  bool &raised = ctx->f32_direct_smem[(BN == 128) * 2 + (TAPS != 0)];
+  if (!raised) {
+    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    raised = true;
   }
   const int grid = std::min<int64_t>(static_cast<int64_t>(p.tiles_m) * p.tiles_n, ctx->num_sms);
   MB_CUDA(ctx, mb_launch_chained(ctx, kern, dim3(grid), dim3(Cf::THREADS), smem, map, p));

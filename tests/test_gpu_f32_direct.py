@@ -170,3 +170,17 @@ def test_direct_conv2d_f32_inside_a_capture(ctx):
         check()
         c._check(L.mb_graph_destroy(c.h, g))
     c.close()
+
+
+@pytest.mark.parametrize("O", [64, 128])
+def test_direct_conv2d_f32_in_two_contexts(ctx, O):
+    """A call that needs little shared memory, in a context of its own, takes none from a larger one's next call."""
+    import mace_b200
+    rng = np.random.Generator(np.random.PCG64(1))
+    large, small = [(rng.standard_normal((1, c, hw, hw)).astype(np.float32), rng.standard_normal((O, c, 3, 3)).astype(np.float32))
+                    for c, hw in ((256, 56), (16, 8))]
+    first = _run(ctx, *large, None)
+    other = mace_b200.Context(0)
+    _run(other, *small, None)
+    other.close()
+    assert np.array_equal(_run(ctx, *large, None), first)
