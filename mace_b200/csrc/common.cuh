@@ -48,7 +48,7 @@ struct mb_context {
   bool f32_conv_presplit_smem = false;  // the limit of the kernel that splits their filter was raised
   bool f32_direct_smem[4] = {false, false, false, false};  // its kernels whose shared-memory limit was raised
   int f32_stem = 0;            // conv_f32_stem.cu: 0 by rule, 1 never, 2 wherever it can run
-  int f32_stem_smem[4] = {0, 0, 0, 0};  // shared-memory limits its kernels were given
+  bool f32_stem_smem[4] = {false, false, false, false};  // its kernels whose shared-memory limit was raised
   int f32_rows = 0;            // gemm_f32_rows.cu: 0 by rule, 1 never, 2 wherever it can run
   bool f32_rows_smem[2] = {false, false};  // its kernels whose shared-memory limit was raised
   uint32_t f32_pairs_attr_mask = 0;  // kernels of gemm_f32_pairs.cu whose shared-memory limit was raised

@@ -501,10 +501,11 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
 template <int CI>
 int launch(mb_context *ctx, Params &p, int smem) {
   auto kern = conv_f32_stem_kernel<CI>;
-  int &limit = ctx->f32_stem_smem[CI - 1];
-  if (smem > limit) {
-    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    limit = smem;
+  // (the limit is the device's, not this context's: the largest for all, or a context's small call would take room from another's)
+  bool &raised = ctx->f32_stem_smem[CI - 1];
+  if (!raised) {
+    MB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    raised = true;
   }
   MB_CUDA(ctx, mb_launch_chained(ctx, kern, dim3(std::min(p.units, ctx->num_sms)), dim3(THREADS), smem, p));
   ctx->launches++;

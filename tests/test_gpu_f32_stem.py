@@ -152,3 +152,20 @@ def test_conv_f32_stem_refuses(ctx, geometry):
     for b in (dx, df):
         b.free()
     assert np.array_equal(got[0], got[1])
+
+
+def test_conv_f32_stem_in_two_contexts(ctx):
+    """A call that needs little shared memory, in a context of its own, takes none from a larger one's next call."""
+    import mace_b200
+    rng = np.random.Generator(np.random.PCG64(1))
+    large, small = [(rng.standard_normal((1, c, 16, 16)).astype(np.float32), rng.standard_normal((64, c, k, k)).astype(np.float32), k)
+                    for c, k in ((3, 7), (3, 1))]
+    bias = np.zeros(64, np.float32)
+
+    def run(c, x, f, k):
+        return _conv(c, x, f, bias, 2 if k > 1 else 1, (k // 2, k // 2), (8, 8) if k > 1 else (16, 8))
+    first = run(ctx, *large)
+    other = mace_b200.Context(0)
+    run(other, *small)
+    other.close()
+    assert np.array_equal(run(ctx, *large), first)
