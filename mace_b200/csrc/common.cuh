@@ -119,6 +119,11 @@ struct mb_context {
   char last_error[512] = {0};
 };
 
+// The type of mb_context::encode_tiled.
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
 int mb_fail(mb_context *ctx, int code, const char *fmt, ...);
 int mb_check_cuda(mb_context *ctx, cudaError_t e, const char *what);
 // Returns a device pointer to at least `bytes` of scratch (256-byte aligned),

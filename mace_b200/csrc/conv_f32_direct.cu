@@ -42,7 +42,6 @@ constexpr int FIRST_IN = 2, IN_WARPS = 8;         // input warps per group
 constexpr long long WAIT_BUDGET = 1ll << 31;       // ~1 s of SM clocks per wait
 constexpr int SCALE_SLOTS = 8;                     // input is at most two patches ahead of the MMAs, these two tiles of the results
 constexpr int MAX_W_STAGES = 12;
-constexpr uint32_t AGAIN = 0x7fc0a6a1u;            // a result to be worked out again (see f32_split.cuh)
 
 struct Params {
   const float *X, *filter, *bias, *w_unscale;
@@ -83,41 +82,16 @@ __device__ __forceinline__ int64_t value_at(const Params &p, int64_t f) {
   return static_cast<int64_t>(img) * p.C_in * p.H * p.W + y * p.W + x;
 }
 
-// A result by fp32 FMAs in the order of k, padding left out.
+// A result by fp32 FMAs.
 __device__ __noinline__ void store_exact(const Params &p, int64_t f, int o) {
   const uint32_t img = fast_div(static_cast<uint32_t>(f), p.image_mul, p.image_shift);
   const uint32_t in = static_cast<uint32_t>(f) - img * p.image;
   const int y = static_cast<int>(fast_div(in, p.pitch_mul, p.pitch_shift)), x = static_cast<int>(in) - y * p.pitch;
   const int64_t hw = static_cast<int64_t>(p.H) * p.W;
-  const float *src = p.X + static_cast<int64_t>(img) * p.C_in * hw, *w = p.filter + static_cast<int64_t>(o) * p.C_in * p.taps;
-  float sum = 0.f;
-  for (int c = 0; c < p.C_in; ++c, src += hw)
-    for (int i = 0; i < p.KH; ++i)
-      for (int j = 0; j < p.KW; ++j, ++w) {
-        const int h = y + i - p.ph, v = x + j - p.pw;
-        if (h >= 0 && h < p.H && v >= 0 && v < p.W) sum = fmaf(src[static_cast<int64_t>(h) * p.W + v], *w, sum);
-      }
+  float sum = f32_chain_window(p.X + static_cast<int64_t>(img) * p.C_in * hw, p.filter + static_cast<int64_t>(o) * p.C_in * p.taps,
+                               p.C_in, p.H, p.W, p.KH, p.KW, y - p.ph, x - p.pw);
   if (p.bias != nullptr) sum += p.bias[o];
   p.C[(static_cast<int64_t>(img) * p.O + o) * hw + static_cast<int64_t>(y) * p.W + x] = mb_activate(sum, p.act, p.max_limit, p.coef);
-}
-
-// The scale of a tile whose input warps found these largest values (all zero: 0).  A tile's places share one, so it leaves less
-// room above (2^9 instead of 2^14) and more below: 2^-31 of the largest value is the smallest step, and a place may be 2^-9 of it
-// without losing a bit.  What does not fit (values that are not finite, and those beyond 2^13 times all that the other warps
-// have) is left out: its places come out as NaN and are worked out again, and the others keep their bits.
-__device__ __forceinline__ float finite_abs(float v) {
-  v = fabsf(v);
-  return v < INFINITY ? v : 0.f;
-}
-__device__ __forceinline__ float tile_scale(const float *most) {
-  float first = 0.f, second = 0.f;
-#pragma unroll
-  for (int i = 0; i < IN_WARPS; ++i) {
-    second = fmaxf(second, fminf(first, most[i]));
-    first = fmaxf(first, most[i]);
-  }
-  if (second > 0.f && first * (1.f / 8192.f) > second) first = second;
-  return first > 0.f ? f32_row_scale(first * (1.f / 32.f)) : 0.f;
 }
 
 // OIHW filter -> [block][tap][hi, lo][O][32 channels] halves and 1 / scale per output channel, a block of threads per channel,
@@ -342,22 +316,22 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         };
         load(w8);
         if (scale == 0.f) {
-          // the scale of the first block with a value other than zero serves the tile (see tile_scale)
+          // the scale of the first block with a value other than zero serves the tile (see f32_shared_scale)
           float most = 0.f;
 #pragma unroll
-          for (int c = 0; c < KC; ++c) most = fmaxf(most, finite_abs(v[c]));
+          for (int c = 0; c < KC; ++c) most = fmaxf(most, f32_finite_abs(v[c]));
           for (int rb = w8 + IN_WARPS; rb < row_blocks; rb += IN_WARPS) {
             const int64_t at = value_at(p, f0 + rb * 32);
             const float *src = p.X + max(at, static_cast<int64_t>(0)) + static_cast<int64_t>(blk) * KC * hw;
             const int channels = at >= 0 ? min(KC, p.C_in - blk * KC) : 0;
 #pragma unroll 8
-            for (int c = 0; c < channels; ++c) most = fmaxf(most, finite_abs(mb_load(src + c * hw)));
+            for (int c = 0; c < channels; ++c) most = fmaxf(most, f32_finite_abs(mb_load(src + c * hw)));
           }
 #pragma unroll
           for (int d = 1; d < 32; d *= 2) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
           if (lane == 0) group_most[(looked & 1) * IN_WARPS + w8] = most;
           named_bar_sync(1 + group, IN_WARPS * 32);
-          scale = tile_scale(group_most + (looked & 1) * IN_WARPS);
+          scale = f32_shared_scale<IN_WARPS>(group_most + (looked & 1) * IN_WARPS);
           ++looked;
           if (w8 == 0 && lane == 0) scales[tile % SCALE_SLOTS] = f32_row_unscale(scale);
         }
@@ -452,7 +426,7 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       if (z != 0.f) {
         *again = 1;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(AGAIN);
+        for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(F32_AGAIN);
       }
       if (dst != nullptr) {
         if (n0 + 32 <= p.O) {
@@ -486,13 +460,9 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       const int64_t at = value_at(p, f);
       if (at < 0) continue;
       const int64_t hw = static_cast<int64_t>(p.H) * p.W, img = at / (p.C_in * hw), pix = at - img * p.C_in * hw;
-      if (__float_as_uint(p.C[(img * p.O + o) * hw + pix]) == AGAIN) store_exact(p, f, o);
+      if (__float_as_uint(p.C[(img * p.O + o) * hw + pix]) == F32_AGAIN) store_exact(p, f, o);
     }
 }
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 template <int BN, int TAPS>
 int launch(mb_context *ctx, Params &p, const void *split) {

@@ -11,7 +11,7 @@
 // products (hi times the filter's lo, lo times its hi) and one per two for the large ones (hi * hi), of 16 of the depth; each
 // kind has an accumulator: an error of 2.2e-7 (2-norm against float64, depth 147) against the self-fetching kernel's 2.8e-7.
 //
-// Input is scaled by strips of output rows (see strip_scale); three warps look for the largest value of the strips ahead.
+// Input is scaled by strips of output rows (see f32_shared_scale); three warps look for the largest value of the strips ahead.
 //
 // What bounds it: the input warps' instructions and waits, 2900 cycles per output row of three channels and 7 x 7 taps, of which the
 // MMAs (48 cycles each with 64 columns) are busy 1760.  With the input in shared memory the MMAs' reads left little of its
@@ -41,7 +41,6 @@ constexpr int MAX_SLOTS = 16, UNITS_AHEAD = 4;
 constexpr int DEPTH = 8, ITEM_BYTES = 32 * 8;  // input items on their way per warp, two columns per lane each
 constexpr int HEAD = 2048;                    // barriers, scales, channel table
 constexpr long long WAIT_BUDGET = 1ll << 31;  // ~1 s of SM clocks per wait
-constexpr uint32_t AGAIN = 0x7fc0a6a1u;       // a result to be worked out again (see f32_split.cuh)
 
 __host__ __device__ constexpr int mmas(int channels) { return channels + (channels + 1) / 2; }  // per filter row
 
@@ -73,38 +72,11 @@ struct Unit {
   }
 };
 
-// The scale of a strip from the largest finite values that the warps which looked at it found (all zero: 0).  Its pixels share
-// one, so it leaves less room above (2^9) and more below: the smallest step is 2^-31 of the largest value.  What does not fit
-// (values that are not finite, and those beyond 2^13 times all that the other warps have) is left out: its results come out
-// as NaN and are worked out again, and the others keep their bits.
-__device__ __forceinline__ float strip_scale(const volatile float *most) {
-  float first = 0.f, second = 0.f;
-#pragma unroll
-  for (int i = 0; i < SCAN_WARPS; ++i) {
-    const float m = most[i];
-    second = fmaxf(second, fminf(first, m));
-    first = fmaxf(first, m);
-  }
-  if (second > 0.f && first * (1.f / 8192.f) > second) first = second;
-  return first > 0.f ? f32_row_scale(first * (1.f / 32.f)) : 0.f;
-}
-
-__device__ __forceinline__ float finite_abs(float v) {
-  v = fabsf(v);
-  return v < INFINITY ? v : 0.f;
-}
-
-// A result by fp32 FMAs in the order of k, padding left out.
+// A result by fp32 FMAs.
 __device__ __noinline__ void store_exact(const Params &p, int channels, float *dst, int img, int o, int y, int x) {
   const int64_t hw = static_cast<int64_t>(p.H) * p.W;
-  const float *src = p.X + img * channels * hw, *w = p.filter + o * channels * p.KH * p.KW;
-  float sum = 0.f;
-  for (int c = 0; c < channels; ++c, src += hw)
-    for (int i = 0; i < p.KH; ++i)
-      for (int j = 0; j < p.KW; ++j, ++w) {
-        const int h = y * p.sh - p.pt + i, v = x * 2 - p.pl + j;
-        if (h >= 0 && h < p.H && v >= 0 && v < p.W) sum = fmaf(src[static_cast<int64_t>(h) * p.W + v], *w, sum);
-      }
+  float sum = f32_chain_window(p.X + img * channels * hw, p.filter + o * channels * p.KH * p.KW, channels, p.H, p.W, p.KH, p.KW,
+                               y * p.sh - p.pt, x * 2 - p.pl);
   if (p.bias != nullptr) sum += p.bias[o];
   *dst = mb_activate(sum, p.act, p.max_limit, p.coef);
 }
@@ -196,10 +168,10 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
         if (p.vec)  // (rows are whole groups of four)
           look(src, [](const float *at) {
             const float4 v = mb_load(reinterpret_cast<const float4 *>(at));
-            return fmaxf(fmaxf(finite_abs(v.x), finite_abs(v.y)), fmaxf(finite_abs(v.z), finite_abs(v.w)));
+            return fmaxf(fmaxf(f32_finite_abs(v.x), f32_finite_abs(v.y)), fmaxf(f32_finite_abs(v.z), f32_finite_abs(v.w)));
           });
         else
-          look(src, [](const float *at) { return finite_abs(mb_load(at)); });
+          look(src, [](const float *at) { return f32_finite_abs(mb_load(at)); });
       }
 #pragma unroll
       for (int d = 1; d < 32; d *= 2) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
@@ -255,7 +227,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
         fail(MB_DEV_TIMEOUT_EPILOGUE);
         break;
       }
-      const float scale = strip_scale(most_of + uslot * SCAN_WARPS);
+      const float scale = f32_shared_scale<SCAN_WARPS>(most_of + uslot * SCAN_WARPS);
       const uint64_t scales = f32_pair(scale, scale);
       int open = -1;  // the row whose slot is this warp's to write
       auto advance = [&](int row) {  // ... becomes this one
@@ -411,7 +383,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
           fail(MB_DEV_TIMEOUT_EPILOGUE);
           break;
         }
-        const float unscale = f32_row_unscale(strip_scale(most_of + uslot * SCAN_WARPS));
+        const float unscale = f32_row_unscale(f32_shared_scale<SCAN_WARPS>(most_of + uslot * SCAN_WARPS));
         const int x = t.x0 + quarter * p.per + lane;
         float *dst = p.C + ((static_cast<int64_t>(t.img) * p.O + n0) * p.Ho + t.y0) * p.Wo + x;
         for (int y = 0; y < t.rows; ++y, dst += p.Wo) {
@@ -455,7 +427,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
             if (z != 0.f) {
               *again = 1;
 #pragma unroll
-              for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(AGAIN);
+              for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(F32_AGAIN);
             }
             if (n0 + 32 <= p.O) {
 #pragma unroll
@@ -493,7 +465,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
     for (int i = threadIdx.x; i < p.O * t.rows * width; i += THREADS) {
       const int o = i / (t.rows * width), in = i - o * t.rows * width, y = t.y0 + in / width, x = t.x0 + in % width;
       float *dst = p.C + ((static_cast<int64_t>(t.img) * p.O + o) * p.Ho + y) * p.Wo + x;
-      if (__float_as_uint(*reinterpret_cast<volatile float *>(dst)) == AGAIN) store_exact(p, CI, dst, t.img, o, y, x);
+      if (__float_as_uint(*reinterpret_cast<volatile float *>(dst)) == F32_AGAIN) store_exact(p, CI, dst, t.img, o, y, x);
     }
   }
 }

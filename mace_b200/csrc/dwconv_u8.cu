@@ -709,10 +709,6 @@ static int dwconv_u8_impl(mb_context *ctx, const uint8_t *in, const uint8_t *fil
                                          static_cast<cuuint64_t>(H * W * C)};
           const cuuint32_t box[4] = {static_cast<cuuint32_t>(t.CB), static_cast<cuuint32_t>(t.TWB), 1, 1};
           const cuuint32_t estr[4] = {1, 1, 1, 1};
-          typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                            const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
-                                            CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                            CUtensorMapFloatOOBfill);
           const CUresult r = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(
               &tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<uint8_t *>(in), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -16,7 +16,10 @@
 #pragma once
 
 #include <cuda_fp16.h>
-#include <stdint.h>
+
+#include "common.cuh"
+
+constexpr uint32_t F32_AGAIN = 0x7fc0a6a1u;  // stored for a result to be worked out again
 
 // The scale of a row whose largest value is m > 0.  NaN below 2^-61: its products are then worked out again.
 __device__ __forceinline__ float f32_row_scale(float m) {
@@ -47,4 +50,46 @@ __device__ __forceinline__ void f32_split2(uint64_t v, uint64_t s, uint32_t &hi,
   const __half2 l = __floats2half2_rn(r0, r1);
   hi = *reinterpret_cast<const uint32_t *>(&h);
   lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+__device__ __forceinline__ float f32_finite_abs(float v) {
+  v = fabsf(v);
+  return v < INFINITY ? v : 0.f;
+}
+
+// The scale of values that share one although they belong to several rows (the places of a convolution's tile or strip), from the
+// largest finite ones that the warps which looked at them found (all zero: 0).  It leaves less room above (2^9 instead of 2^14)
+// and more below: 2^-31 of the largest value is the smallest step, and a place may be 2^-9 of it without losing a bit.  What does
+// not fit (values that are not finite, and those beyond 2^13 times all that the other warps have) is left out: its results come
+// out as NaN and are worked out again, and the others keep their bits.
+template <int WARPS>
+__device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
+  float first = 0.f, second = 0.f;
+#pragma unroll
+  for (int i = 0; i < WARPS; ++i) {
+    const float m = most[i];
+    second = fmaxf(second, fminf(first, m));
+    first = fmaxf(first, m);
+  }
+  if (second > 0.f && first * (1.f / 8192.f) > second) first = second;
+  return first > 0.f ? f32_row_scale(first * (1.f / 32.f)) : 0.f;
+}
+
+// What a result is worked out again by: fp32 FMAs in the order of the depth, of a product's row and column ...
+__device__ __forceinline__ float f32_chain(const float *x, int64_t x_ks, const float *w, int64_t K) {
+  float sum = 0.f;
+  for (int64_t k = 0; k < K; ++k) sum = fmaf(x[k * x_ks], w[k], sum);
+  return sum;
+}
+// ... and of a convolution's window with its corner at (top, left) of an image, padding left out.
+__device__ __forceinline__ float f32_chain_window(const float *image, const float *filter, int channels, int H, int W, int KH, int KW,
+                                                  int top, int left) {
+  float sum = 0.f;
+  for (int c = 0; c < channels; ++c, image += static_cast<int64_t>(H) * W)
+    for (int i = 0; i < KH; ++i)
+      for (int j = 0; j < KW; ++j, ++filter) {
+        const int h = top + i, v = left + j;
+        if (h >= 0 && h < H && v >= 0 && v < W) sum = fmaf(image[static_cast<int64_t>(h) * W + v], *filter, sum);
+      }
+  return sum;
 }

@@ -43,6 +43,7 @@
 // 384 x 384 x 64 times a transposed matrix, batch 12, 10.9 (CUDA cores) -> 7.7; 736 x 176 x 384, batch 24, 76 -> 39.
 #include <algorithm>
 
+#include "f32_split.cuh"
 #include "gemm_f32_gather.cuh"
 #include "gemm_u8_cut.cuh"  // mb_launch_clusters
 #include "sm100_ptx.cuh"
@@ -148,10 +149,9 @@ __device__ __forceinline__ int64_t out_offset(const Params &p, int m, int b) {
 
 // Four results of a pixel by fp32 FMAs in the order of k, padding left out.  An infinity has no split (inf - inf) and neither
 // has a value that rounds beyond the largest tf32 one, so whatever they meet comes out of the tensor core as a NaN.  Results
-// that are not finite are stored as AGAIN, and when its tiles are done a CTA that stored one works those out again here,
+// that are not finite are stored as F32_AGAIN, and when its tiles are done a CTA that stored one works those out again here,
 // which gives what the CUDA cores give.  (Results that are finite pay one FMA each for the check.  Called from the result
 // warps, tile by tile, the same code cost every launch 0.8 us, in registers that it never used; so it costs 0.2.)
-constexpr uint32_t AGAIN = 0x7fc0a6a1u;
 template <int XK>
 __device__ __noinline__ void store_exact4(const Params &p, int m, int b, int n, int n_end) {
   const float *x = p.X, *w[4];
@@ -644,7 +644,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           if (MODE != WHOLE && !finite) {
             *again = 1;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(AGAIN);
+            for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(F32_AGAIN);
           }
           float *dst = p.C + at + static_cast<int64_t>(n0 + c) * p.c_ns;
           if (n0 + c + 16 <= p.N) {
@@ -701,7 +701,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int c = c0 + q * 4, n = n0 + c;
-          if (c < share && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = finite ? x[q] : __uint_as_float(AGAIN);
+          if (c < share && n < p.N) p.C[at + static_cast<int64_t>(n) * p.c_ns] = finite ? x[q] : __uint_as_float(F32_AGAIN);
         }
       }
     }
@@ -722,7 +722,7 @@ gemm_f32_gather_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         if (m >= p.M || n >= n_end) continue;
         const float *stored = p.C + out_offset<XK>(p, m, t.b) + n * p.c_ns;
         bool found = false;
-        for (int q = 0; q < 4 && n + q < n_end; ++q) found |= __float_as_uint(stored[q * p.c_ns]) == AGAIN;
+        for (int q = 0; q < 4 && n + q < n_end; ++q) found |= __float_as_uint(stored[q * p.c_ns]) == F32_AGAIN;
         if (found) store_exact4<XK>(p, m, t.b, n, n_end);
       }
       if (p.splits > 1) break;

@@ -114,18 +114,16 @@ __device__ __forceinline__ int my_tiles(const F32TcParams &p) {
   return static_cast<int>((p.batch * p.tiles_m * p.tiles_n - blockIdx.x + gridDim.x - 1) / gridDim.x);
 }
 
-// A result that came out of the tensor core as no finite number (see f32_split.cuh) is stored as F_AGAIN; when its tiles are done
+// A result that came out of the tensor core as no finite number (see f32_split.cuh) is stored as F32_AGAIN; when its tiles are done
 // a CTA that stored one works those out again, by fp32 FMAs in the order of k.
-constexpr uint32_t F_AGAIN = 0x7fc0a6a1u;
 __device__ __noinline__ void tile_again(const F32TcParams &p, int m0, int n0, int bn, int b) {
   for (int i = threadIdx.x; i < FBM * bn; i += blockDim.x) {
     const int64_t m = m0 + (i & (FBM - 1)), n = n0 + i / FBM;
     if (m >= p.Mdim || n >= p.Ndim) continue;
     const int64_t at = b * p.c_batch_stride + n * p.c_row_stride + m;
-    if (__float_as_uint(*reinterpret_cast<volatile float *>(p.C + at)) != F_AGAIN) continue;
+    if (__float_as_uint(*reinterpret_cast<volatile float *>(p.C + at)) != F32_AGAIN) continue;
     const float *x = p.X + b * p.x_bs + m, *w = p.W + b * p.w_bs + n * p.w_rs;
-    float sum = 0.f;
-    for (int64_t k = 0; k < p.K; ++k) sum = fmaf(x[k * p.x_rs], w[k], sum);
+    float sum = f32_chain(x, p.x_rs, w, p.K);
     if (p.bias != nullptr) sum += p.bias[n];
     if (p.residual != nullptr) sum += p.residual[at];
     p.C[at] = mb_activate(sum, p.act, p.max_limit, p.coef);
@@ -514,7 +512,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
         if (z[0] + z[1] != 0.f) {
           *again = 1;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) a[j] = __uint_as_float(F_AGAIN);
+          for (int j = 0; j < 16; ++j) a[j] = __uint_as_float(F32_AGAIN);
         }
         if (c_tma) {
 #pragma unroll
@@ -596,11 +594,6 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     for (FTileIter it(p); it.valid(p); it.next(p)) tile_again(p, it.tm * FBM, it.tn * BN, BN, it.b);
   }
 }
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 // 3-D fp32 tensor map: dims {inner, rows, batch} in elements, no swizzle, zero fill.
 // Every stride must be a multiple of 16 bytes, that of a batch dimension of extent 1 too:

@@ -32,7 +32,6 @@ constexpr int FIRST_SPLIT = 2, SPLIT_WARPS = 8, FIRST_OUT = FIRST_SPLIT + SPLIT_
 constexpr int STAGES = 4;
 constexpr int SCALE_SLOTS = 8;  // tiles: the split is at most STAGES tiles of one step ahead of the MMAs, these two of the results
 constexpr long long WAIT_BUDGET = 1ll << 31;  // ~1 s of SM clocks per wait
-constexpr uint32_t AGAIN = 0x7fc0a6a1u;       // a result to be worked out again (see f32_split.cuh)
 
 // Where four k (chunk 0 .. 7 of a step) of a row's hi half lie: in the first 64 of its 128 bytes, in the tensor core's 128-byte
 // swizzle.  Its lo half lies at 64 ^ that.
@@ -67,10 +66,9 @@ __device__ __noinline__ void tile_again(const Params &p, int m0, int n0, int bn,
     const int m = m0 + (i & (BM - 1)), n = n0 + i / BM;
     if (m >= p.M || n >= p.N) continue;
     float *c = p.C + b * p.c_bs + n * p.c_ns + m;
-    if (__float_as_uint(*c) != AGAIN) continue;
+    if (__float_as_uint(*c) != F32_AGAIN) continue;
     const float *x = p.X + b * p.x_bs + m * p.x_ms, *w = p.W + b * p.w_bs + n * p.w_ns;
-    float sum = 0.f;
-    for (int k = 0; k < p.K; ++k) sum = fmaf(x[k], w[k], sum);
+    float sum = f32_chain(x, 1, w, p.K);
     if (p.bias != nullptr) sum += p.bias[n];
     *c = mb_activate(sum, p.act, p.max_limit, p.coef);
   }
@@ -308,7 +306,7 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       if (z != 0.f) {
         *again = 1;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(AGAIN);
+        for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(F32_AGAIN);
       }
       if (m < p.M) {
         float *dst = p.C + b * p.c_bs + n0 * p.c_ns + m;

@@ -585,11 +585,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_x,
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // 3-D fp32 tensor map: dims {inner, rows, batch} in elements, 128-byte swizzle, zero fill.
 // Every stride must be a multiple of 16 bytes, that of a batch dimension of extent 1 too:
 // callers pass row stride x rows there.

@@ -48,11 +48,6 @@ int mb_tc_dispatch_plain(mb_context *ctx, const TcChoice &c, const CUtensorMap &
 int mb_tc_dispatch_conv_plain(mb_context *ctx, int bn, int kb, const CUtensorMap &ta, const CUtensorMap &tb,
                               const CUtensorMap &tc, ConvTcParams &p);
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // 3-D uint8 tensor map: dims {inner, rows, batch}; 128-byte swizzle for the operand
 // tiles, 32-byte swizzle for the output staging boxes; row_pitch 0: no gaps.
 int mb_make_map_u8(mb_context *ctx, CUtensorMap *map, const void *base, uint64_t inner,
