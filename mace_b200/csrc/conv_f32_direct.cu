@@ -407,7 +407,7 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           tmem_ld_wait_x8(r);
           tmem_ld_wait_x8(s);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) sum[j + k] += __uint_as_float(r[k]) + __uint_as_float(s[k]);
+          for (int k = 0; k < 8; ++k) sum[j + k] += fmaf(__uint_as_float(s[k]), F32_LO, __uint_as_float(r[k]));
         }
         tc_fence_before_sync();
         __syncwarp();

@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
             tmem_ld_wait_x16(r);
             tmem_ld_wait_x16(s);
 #pragma unroll
-            for (int k = 0; k < 16; ++k) sum[j + k] = __uint_as_float(r[k]) + __uint_as_float(s[k]);
+            for (int k = 0; k < 16; ++k) sum[j + k] = fmaf(__uint_as_float(s[k]), F32_LO, __uint_as_float(r[k]));
           }
           tc_fence_before_sync();
           __syncwarp();

@@ -1,10 +1,11 @@
 // fp32 operands as pairs of half-precision numbers for tcgen05.mma kind::f16.
 //
-// v * s = hi + lo with s a power of two that brings the largest value of a row to 2 .. 4 (a row: what shares one index of the
+// v * s = hi + 2^-11 lo with s a power of two that brings the largest value of a row to 2 .. 4 (a row: what shares one index of the
 // result, a pixel's or an output channel's values over the depth): hi is v * s rounded to 11 bits, lo the rest rounded to
-// 11 bits, together 22 bits and a sign, or 2^-25 absolute where that is more, 2^-26 of the row's largest value.  Three MMAs, hi * hi +
-// hi * lo + lo * hi, in fp32 accumulators make a product to 2^-24 of the row's norm; the result is multiplied by the two
-// inverse powers of two, which is exact.
+// 11 bits, together 22 bits and a sign, or 2^-36 absolute where that is more, 2^-37 of the row's largest value.  (At the scale of hi,
+// lo would end at 2^-25: values below 2^-12 of the row's largest lost bits, which shows where small values meet large ones of the
+// other operand: 6e-6 instead of 8e-8 with a column of X times 1000 and W's divided by it.)  Three MMAs, hi * hi in one fp32
+// accumulator and hi * lo + lo * hi in another; the second one's 2^-11 and the two inverse powers of two are exact.
 //
 // Against tf32 pairs (11 + 11 bits cut off, as many MMAs): an operand takes half the bytes in shared and tensor memory and
 // an MMA covers 16 of the depth in the time of 8.  Those kernels were bound by shared memory: 144 KB per step of 128 x 128 x 32
@@ -37,17 +38,34 @@ __device__ __forceinline__ uint64_t f32_pair(float x, float y) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
   return r;
 }
+__device__ __forceinline__ float2 f32_parts(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t f32_mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f32_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+constexpr float F32_LO = 1.f / 2048.f;  // what the accumulator of the small products is multiplied by
+
 // Two values v (packed) times s as hi and lo halves, the first value in the low half.
 __device__ __forceinline__ void f32_split2(uint64_t v, uint64_t s, uint32_t &hi, uint32_t &lo) {
-  uint64_t a, r;
-  float a0, a1, r0, r1;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(v), "l"(s));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
-  const __half2 h = __floats2half2_rn(a0, a1);
+  const uint64_t a = f32_mul2(v, s);
+  const float2 a2 = f32_parts(a);
+  const __half2 h = __floats2half2_rn(a2.x, a2.y);
   const float2 f = __half22float2(h);
+  uint64_t r;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(f32_pair(f.x, f.y)));  // (exact)
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r0), "=f"(r1) : "l"(r));
-  const __half2 l = __floats2half2_rn(r0, r1);
+  const float2 r2 = f32_parts(f32_mul2(r, f32_pair(1.f / F32_LO, 1.f / F32_LO)));
+  const __half2 l = __floats2half2_rn(r2.x, r2.y);
   hi = *reinterpret_cast<const uint32_t *>(&h);
   lo = *reinterpret_cast<const uint32_t *>(&l);
 }

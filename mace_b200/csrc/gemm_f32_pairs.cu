@@ -23,7 +23,9 @@
 //   warps 2..9    X split, two warps per TMEM lane quarter, 16 k each
 //   warps 10..17  epilogue: two sets of four warps (one per TMEM lane quarter), each on half of the tile's columns
 //   warps 18, 19  a set's result and residual copies (one thread each)
-// TMEM columns: two accumulators of 128 columns, then STAGES x 32 columns of A (hi 16, lo 16).
+// TMEM columns: with 64 channels two accumulators of 64 columns of large products and 64 of small ones; with 128 two of large
+// products and one of small ones, which the epilogue adds to the large ones first, in tensor memory, so that it is free some
+// 500 cycles into the next tile, whose large products run ahead meanwhile.  Then STAGES x 32 columns of A (hi 16, lo 16).
 // Every wait is bounded; on a timeout the kernel records a status word, lets outstanding
 // copies land, frees its TMEM and returns.
 #include "common.cuh"
@@ -76,17 +78,18 @@ struct F32Cfg {
   static constexpr int FIXED = STAGING_BYTES + XSCALE_BYTES + UB_BYTES + BAR_BYTES + 1024;
   static constexpr int NUM_ACC = 2;
   static constexpr int TMEM_COLS = 512;
-  // 64 channels: hi and lo of W are rows of their own, an MMA covers both and writes columns 2 n and 2 n + 1
+  // 64 channels: the hi rows of W with the lo rows behind them, hi of X times both is one MMA of 128 columns
   static constexpr bool WIDE = BN == 64;
   static constexpr int ACC_COLS = 128;
-  static constexpr int A_COL0 = NUM_ACC * ACC_COLS;  // first TMEM column of the A ring
+  static constexpr int SMALL_COL0 = WIDE ? 64 : NUM_ACC * ACC_COLS;  // small products (WIDE: of the accumulator)
+  static constexpr int A_COL0 = (NUM_ACC + (WIDE ? 0 : 1)) * ACC_COLS;  // first TMEM column of the A ring
   static constexpr int MAX_TMEM_STAGES = (TMEM_COLS - A_COL0) / FKB;
   static constexpr int SMEM_STAGES = (227 * 1024 - FIXED) / STAGE_BYTES;
   static constexpr int STAGES = SMEM_STAGES < MAX_TMEM_STAGES ? SMEM_STAGES : MAX_TMEM_STAGES;
   static_assert(STAGES >= 2, "pipeline needs two stages");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + FIXED;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-  static_assert(3 * STAGES * 8 + 2 * NUM_ACC * 8 + 4 * F_BUFS * 8 + 16 <= BAR_BYTES, "barrier area");
+  static_assert(3 * STAGES * 8 + 2 * NUM_ACC * 8 + 4 * F_BUFS * 8 + 8 + 16 <= BAR_BYTES, "barrier area");
 };
 
 // Column tiles first: the CTAs that read one tile of X run side by side and fetch it from HBM once.
@@ -208,7 +211,8 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const uint32_t tempty_bar = tfull_bar + 8 * NUM_ACC;   // [NUM_ACC] accumulator drained
   const uint32_t free_bar = tempty_bar + 8 * NUM_ACC;    // [2][F_BUFS] result buffer free, its residual landed
   const uint32_t ready_bar = free_bar + 8 * 2 * F_BUFS;  // [2][F_BUFS] result buffer written
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * STAGES + 2 * NUM_ACC + 4 * F_BUFS);
+  const uint32_t sempty_bar = ready_bar + 8 * 2 * F_BUFS;  // accumulator of the small products drained (128 channels)
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * STAGES + 2 * NUM_ACC + 4 * F_BUFS + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *again = abort_flag + 1;
 
@@ -230,6 +234,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
       mbar_init(tfull_bar + 8 * b, 1);
       mbar_init(tempty_bar + 8 * b, F_EPI_WARPS);
     }
+    mbar_init(sempty_bar, F_EPI_WARPS);
     for (int b = 0; b < 2 * F_BUFS; ++b) {
       mbar_init(free_bar + 8 * b, 1);
       mbar_init(ready_bar + 8 * b, F_EPI_WARPS / 2);
@@ -274,7 +279,9 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
           const uint32_t sw = sx + Cfg::X_BYTES;
           mbar_arrive_expect_tx(fb, Cfg::X_BYTES + Cfg::W_BYTES);
           tma_load_3d(sx, &tmap_x, fb, it.tm * FBM, kb * FKB, xb);  // [32 k][128 m], 512-byte rows
-          tma_load_3d(sw, &tmap_w, fb, 0, Cfg::WIDE ? 2 * kb : kb, wb * static_cast<int>(p.Ndim) + it.tn * BN);
+          const int w_row = wb * static_cast<int>(p.Ndim) + it.tn * BN;
+          tma_load_3d(sw, &tmap_w, fb, 0, Cfg::WIDE ? 2 * kb : kb, w_row);
+          if (Cfg::WIDE) tma_load_3d(sw + Cfg::W_BYTES / 2, &tmap_w, fb, 0, 2 * kb + 1, w_row);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -291,21 +298,26 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     // registers, the common case is unrolled, the next step's barrier is asked ahead.
     {
       constexpr uint32_t idesc = make_idesc(/*c f32*/ 1, /*a f16*/ 0, /*b f16*/ 0, /*a mn*/ false, /*b mn*/ false, FBM, 128);
+      constexpr uint32_t idesc_64 = make_idesc(1, 0, 0, false, false, FBM, 64);
       // W (K-major), 16 of k are 32 bytes inside the swizzled row (+2 in the descriptor's address field): rows of 128 bytes, hi
-      // then lo; or of 64 bytes, hi and lo of a channel in turn.
+      // then lo; or of 64 bytes, the hi rows before the lo rows.
       const uint64_t w0 = Cfg::WIDE ? make_smem_desc(smem_base + Cfg::X_BYTES, 16, 512, 4)
                                     : make_smem_desc(smem_base + Cfg::X_BYTES, 16, 1024, 2);
       const int k_blocks = p.k_blocks;
       const bool odd_end = (p.K + 15) / 16 % 2 != 0;  // the last step has only 16 of k
       uint32_t stage = 0, phase = 0;
       uint32_t acc_buf = 0, acc_phase = 0;
+      uint32_t small_phase = 1;  // (of sempty_bar, which the first tile need not wait for)
       bool ok = true, ready = false;
-      for (int tiles = my_tiles(p); ok && tiles > 0; --tiles) {
+      for (int tiles = my_tiles(p); ok && tiles > 0; --tiles, small_phase ^= 1) {
         if (!mbar_wait_warp(tempty_bar + 8 * acc_buf, acc_phase ^ 1, abort_flag, F_WAIT_BUDGET)) {
           fail(MB_DEV_TIMEOUT_MMA);
           break;
         }
-        const uint32_t d_tmem = tmem_base + acc_buf * Cfg::ACC_COLS;
+        const uint32_t d_tmem = tmem_base + acc_buf * Cfg::ACC_COLS, s_tmem = (Cfg::WIDE ? d_tmem : tmem_base) + Cfg::SMALL_COL0;
+        bool small_free = Cfg::WIDE;
+        int owed = 0;              // steps whose small products are still to be issued: the last ones, up to this one
+        uint32_t owed_stage = stage;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!ready && !mbar_wait_warp(split_bar + 8 * stage, phase, abort_flag, F_WAIT_BUDGET)) {
             fail(MB_DEV_TIMEOUT_MMA);
@@ -319,15 +331,56 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
           // A (TMEM): lane = pixel, two k per column; hi in the first 16 columns of the stage's slot, lo in the next 16
           const uint32_t a_hi = tmem_base + Cfg::A_COL0 + stage * FKB, a_lo = a_hi + 16;
           const uint64_t w_hi = w0 + stage * (Cfg::STAGE_BYTES >> 4);
-          mma_f16_ts_elect(d_tmem, a_lo, w_hi, idesc, kb > 0 ? 1u : 0u);
-          if (!Cfg::WIDE) mma_f16_ts_elect(d_tmem, a_hi, w_hi + 4, idesc, 1u);
-          mma_f16_ts_elect(d_tmem, a_hi, w_hi, idesc, 1u);
-          if (!odd_end || kb + 1 < k_blocks) {
-            mma_f16_ts_elect(d_tmem, a_lo + 8, w_hi + 2, idesc, 1u);
-            if (!Cfg::WIDE) mma_f16_ts_elect(d_tmem, a_hi + 8, w_hi + 6, idesc, 1u);
-            mma_f16_ts_elect(d_tmem, a_hi + 8, w_hi + 2, idesc, 1u);
+          const bool both = !odd_end || kb + 1 < k_blocks;
+          if (Cfg::WIDE) {
+            mma_f16_ts_elect(d_tmem, a_hi, w_hi, idesc, kb > 0 ? 1u : 0u);
+            mma_f16_ts_elect(s_tmem, a_lo, w_hi, idesc_64, 1u);
+            if (both) {
+              mma_f16_ts_elect(d_tmem, a_hi + 8, w_hi + 2, idesc, 1u);
+              mma_f16_ts_elect(s_tmem, a_lo + 8, w_hi + 2, idesc_64, 1u);
+            }
+            mma_commit_elect(empty_bar + 8 * stage);
+          } else if (small_free) {
+            mma_f16_ts_elect(d_tmem, a_hi, w_hi, idesc, 1u);
+            mma_f16_ts_elect(s_tmem, a_hi, w_hi + 4, idesc, 1u);
+            mma_f16_ts_elect(s_tmem, a_lo, w_hi, idesc, 1u);
+            if (both) {
+              mma_f16_ts_elect(d_tmem, a_hi + 8, w_hi + 2, idesc, 1u);
+              mma_f16_ts_elect(s_tmem, a_hi + 8, w_hi + 6, idesc, 1u);
+              mma_f16_ts_elect(s_tmem, a_lo + 8, w_hi + 2, idesc, 1u);
+            }
+            mma_commit_elect(empty_bar + 8 * stage);
+          } else {
+            mma_f16_ts_elect(d_tmem, a_hi, w_hi, idesc, kb > 0 ? 1u : 0u);
+            if (both) mma_f16_ts_elect(d_tmem, a_hi + 8, w_hi + 2, idesc, 1u);
+            ++owed;
+            small_free = __all_sync(0xffffffffu, mbar_test_wait(sempty_bar, small_phase));
+            if (!small_free && (owed == STAGES || kb + 1 == k_blocks)) {
+              if (!mbar_wait_warp(sempty_bar, small_phase, abort_flag, F_WAIT_BUDGET)) {
+                fail(MB_DEV_TIMEOUT_MMA);
+                ok = false;
+                break;
+              }
+              small_free = true;
+            }
+            if (small_free) {
+              tc_fence_after_sync();
+#pragma unroll 1
+              for (; owed > 0; --owed) {
+                const int step = kb + 1 - owed;
+                const uint32_t x_hi = tmem_base + Cfg::A_COL0 + owed_stage * FKB, x_lo = x_hi + 16;
+                const uint64_t w = w0 + owed_stage * (Cfg::STAGE_BYTES >> 4);
+                mma_f16_ts_elect(s_tmem, x_hi, w + 4, idesc, step > 0 ? 1u : 0u);
+                mma_f16_ts_elect(s_tmem, x_lo, w, idesc, 1u);
+                if (both || owed > 1) {
+                  mma_f16_ts_elect(s_tmem, x_hi + 8, w + 6, idesc, 1u);
+                  mma_f16_ts_elect(s_tmem, x_lo + 8, w + 2, idesc, 1u);
+                }
+                mma_commit_elect(empty_bar + 8 * owed_stage);
+                if (++owed_stage == STAGES) owed_stage = 0;
+              }
+            }
           }
-          mma_commit_elect(empty_bar + 8 * stage);
           stage = next;
           phase = next_phase;
         }
@@ -419,7 +472,8 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     // Result buffers of a set: [buffer][channel j][128 pixels]; a lane's 16 accesses of a chunk go to 16 different rows, a
     // warp's access to one row covers all 32 banks.
     float *stage_f = reinterpret_cast<float *>(smem_aligned + STAGING_AT) + set * (F_BUFS * 16 * FBM);
-    float2 *table = reinterpret_cast<float2 *>(smem_aligned + UB_AT) + (warp - FIRST_EPI) * (BN / 2);
+    // of two channels each: 1 / scale, bias
+    float4 *table = reinterpret_cast<float4 *>(smem_aligned + UB_AT) + (warp - FIRST_EPI) * (BN / 4);
     const uint32_t my_free_bar = free_bar + 8 * (set * F_BUFS), my_ready_bar = ready_bar + 8 * (set * F_BUFS);
     int acc_buf = 0;
     uint32_t acc_phase = 0;
@@ -444,31 +498,50 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
         break;
       }
       tc_fence_after_sync();
-      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc_buf * Cfg::ACC_COLS +
-                             set * (Cfg::ACC_COLS / 2);
+      const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+      const uint32_t tbase = lanes + acc_buf * Cfg::ACC_COLS + set * (BN / 2);
+      const uint32_t sbase = (Cfg::WIDE ? tbase : lanes + set * (BN / 2)) + Cfg::SMALL_COL0;
       uint32_t r[16], r2[16];
+      if (!Cfg::WIDE) {
+        // the small products join the large ones (the first chunk's in registers), and leave their accumulator to the next tile
+#pragma unroll
+        for (int i = CHUNKS - 1; i >= 0; --i) {
+          tmem_ld_32x32b_x16(tbase + i * 16, r);
+          tmem_ld_32x32b_x16(sbase + i * 16, r2);
+          tmem_ld_wait_x16(r);
+          tmem_ld_wait_x16(r2);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(fmaf(__uint_as_float(r2[j]), F32_LO, __uint_as_float(r[j])));
+          if (i > 0) tmem_st_32x32b_x16(tbase + i * 16, r);
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sempty_bar);
+        tmem_st_wait();
+      }
       auto load = [&](int i) {
-        tmem_ld_32x32b_x16(tbase + i * (Cfg::WIDE ? 32 : 16), r);
-        if (Cfg::WIDE) tmem_ld_32x32b_x16(tbase + i * 32 + 16, r2);
+        tmem_ld_32x32b_x16(tbase + i * 16, r);
+        if (Cfg::WIDE) tmem_ld_32x32b_x16(sbase + i * 16, r2);
       };
-      load(0);
+      if (Cfg::WIDE) load(0);
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
-        table[j * 32 + lane] = make_float2(u[j], b[j]);
+        float *entry = reinterpret_cast<float *>(table + j * 16 + (lane >> 1)) + (lane & 1);
+        entry[0] = u[j];
+        entry[2] = b[j];
       }
       const float unscale = x_unscale[(tile % F_SCALE_SLOTS) * FBM + quarter * 32 + lane];
+      const uint64_t unscales = f32_pair(unscale, unscale);
       __syncwarp();
       float *c = p.C + it.b * p.c_batch_stride + m;
 #pragma unroll
       for (int i = 0; i < CHUNKS; ++i, ++q) {
-        tmem_ld_wait_x16(r);
+        if (Cfg::WIDE || i > 0) tmem_ld_wait_x16(r);
         if (Cfg::WIDE) tmem_ld_wait_x16(r2);
         float a[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          if (!Cfg::WIDE) a[j] = __uint_as_float(r[j]);
-          else if (j < 8) a[j] = __uint_as_float(r[(2 * j) & 15]) + __uint_as_float(r[(2 * j + 1) & 15]);
-          else a[j] = __uint_as_float(r2[(2 * j) & 15]) + __uint_as_float(r2[(2 * j + 1) & 15]);
+          a[j] = Cfg::WIDE ? fmaf(__uint_as_float(r2[j]), F32_LO, __uint_as_float(r[j])) : __uint_as_float(r[j]);
         }
         if (i + 1 < CHUNKS) load(i + 1);
         if (i == CHUNKS - 1) {
@@ -489,18 +562,20 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
 #pragma unroll
           for (int j = 0; j < 16; ++j) buf[j * FBM] = mb_load(res + min(n0 + j, Ndim - 1) * p.c_row_stride);
         }
-        float z[2] = {0.f, 0.f};
+        uint64_t z2 = 0;
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
-          const float4 t = *reinterpret_cast<const float4 *>(table + i * 16 + j);
+          const float4 t = table[i * 8 + j / 2];
+          // (the products with powers of two are exact, so the sum with the bias rounds once)
+          uint64_t x2 = f32_mul2(f32_pair(a[j], a[j + 1]), unscales);
+          x2 = EPI == 0 ? f32_mul2(x2, f32_pair(t.x, t.y)) : f32_fma2(x2, f32_pair(t.x, t.y), f32_pair(t.z, t.w));
+          z2 = f32_fma2(x2, 0, z2);
+          const float2 both = f32_parts(x2);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            // (the product of two powers of two and its product with a are exact, so the sum with the bias rounds once)
-            float x = a[j + h] * (unscale * (h == 0 ? t.x : t.z));
-            z[h] = fmaf(x, 0.f, z[h]);
+            float x = h == 0 ? both.x : both.y;
             if (EPI != 0) {
               // (acc + bias) + residual: the rounding order of a convolution followed by a sum
-              x += h == 0 ? t.y : t.w;
               if (RES) x += buf[(j + h) * FBM];
               const float neg = LEAKY ? fminf(x, 0.f) * act_slope : 0.f;
               x = fminf(fmaxf(x, act_lo), act_hi);
@@ -509,7 +584,8 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
             a[j + h] = x;
           }
         }
-        if (z[0] + z[1] != 0.f) {
+        const float2 z = f32_parts(z2);
+        if (z.x + z.y != 0.f) {
           *again = 1;
 #pragma unroll
           for (int j = 0; j < 16; ++j) a[j] = __uint_as_float(F32_AGAIN);
@@ -614,12 +690,12 @@ int make_map_f32(mb_context *ctx, CUtensorMap *map, const void *base, uint64_t i
   return MB_SUCCESS;
 }
 
-// The split W as f32_presplit_kernel lays it out: boxes of bn rows' 128 bytes of one step (64 rows: as rows of 64 bytes).
+// The split W as f32_presplit_kernel lays it out: boxes of bn rows' 128 bytes of one step (64 rows: of their 64 bytes of hi or lo).
 int make_map_split(mb_context *ctx, CUtensorMap *map, const void *base, uint64_t k_blocks, uint64_t rows, int bn) {
   const uint32_t per = bn == 64 ? 2 : 1, halves = 64 / per;
   const cuuint64_t dims[3] = {halves, k_blocks * per, rows};
   const cuuint64_t strides[2] = {halves * 2, k_blocks * 128};
-  const cuuint32_t box[3] = {halves, per, static_cast<cuuint32_t>(bn)};
+  const cuuint32_t box[3] = {halves, 1, static_cast<cuuint32_t>(bn)};
   const cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(
       map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr,

@@ -283,7 +283,7 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
           tmem_ld_wait_x8(s);
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            const float x = __uint_as_float(r[k]) + __uint_as_float(s[k]);
+            const float x = fmaf(__uint_as_float(s[k]), F32_LO, __uint_as_float(r[k]));
             sum[j + k] = i == 0 ? x : sum[j + k] + x;
           }
         }

@@ -27,14 +27,13 @@ def _exact(x, f):
 
 
 def _bound(x, f):
-    """hi + lo of a value is within 2^-22 of it, or 2^-31 of the largest value around (half of that for a weight's row), and the
-    accumulator is cut off by at most 2^-23 of what it holds after each of its MMAs (18 of large products between two hand-overs
-    with the default runs here, a rounding for each hand-over)."""
+    """hi + lo of a value is within 2^-22 of it, and the accumulator is cut off by at most 2^-23 of what it holds after each of its
+    MMAs (18 of large products between two hand-overs with the default runs here, a rounding for each hand-over)."""
     ax, af = np.abs(x), np.abs(f)
     K = f[0].size
     terms = _exact(ax, af)
     cut = min(K, 32 * f.shape[2] * f.shape[3]) / 16 + K / 32 + 4
-    return terms * (2.0 ** -21 + cut * 2.0 ** -23) + K * ax.max() * af.max(axis=(1, 2, 3))[None, :, None, None] * 2.0 ** -30 + 1e-30
+    return terms * (2.0 ** -21 + cut * 2.0 ** -23) + 1e-30
 
 
 def _run(ctx, x, f, bias, act=0, max_limit=0.0, coef=0.0, direct=2):
@@ -119,6 +118,28 @@ def test_direct_conv2d_f32_beyond_the_split(ctx, O, what):
         scale = np.abs(xs).max() * np.abs(fs).max(axis=(1, 2, 3))[None, :, None, None]
         bound = terms * 2.0 ** -17 + f[0].size * scale * 2.0 ** -30
         assert (np.abs(got - ref)[finite] <= bound[finite]).all()
+
+
+@pytest.mark.parametrize("spread", [2.0 ** 8, 2.0 ** 12])
+@pytest.mark.parametrize("O", [20, 100])
+def test_direct_conv2d_f32_spread(ctx, O, spread):
+    """Small values that meet large weights keep their bits, and so do dark regions beside bright ones."""
+    rng = np.random.Generator(np.random.PCG64(O))
+    x = rng.standard_normal((2, 70, 15, 15)).astype(np.float32)
+    f = (rng.standard_normal((O, 70, 3, 3)) * 0.1).astype(np.float32)
+    def error(x, f, part):
+        got, exact = _run(ctx, x, f, None), _exact(x.astype(np.float64), f.astype(np.float64))
+        assert (np.abs(got - exact) <= _bound(x, f)).all()
+        return np.linalg.norm((got - exact)[part]) / np.linalg.norm(exact[part])
+
+    for dim, dark in ((np.s_[:, :, :8], np.s_[:, :, :7]), (np.s_[:, :, :, 8:], np.s_[:, :, :, 9:])):
+        plain, y = error(x, f, dark), x.copy()
+        y[dim] *= np.float32(1 / spread)
+        assert error(y, f, dark) <= 1.05 * plain
+    plain = error(x, f, np.s_[:])
+    x[:, ::7] *= np.float32(1 / spread)
+    f[:, ::7] *= np.float32(spread)
+    assert error(x, f, np.s_[:]) <= 1.05 * plain
 
 
 def test_direct_conv2d_f32_choice(ctx):

@@ -15,12 +15,11 @@ def ctx():
 
 
 def _bound(A, B):
-    """hi + lo of a value is within 2^-22 of it, or 2^-26 of the largest value of its row or column; the accumulator is cut off by
-    at most 2^-23 of what it holds after each of three MMAs per 16 of the depth."""
+    """hi + lo of a value is within 2^-22 of it; the accumulator is cut off by at most 2^-23 of what it holds after each of three MMAs
+    per 16 of the depth."""
     A, B = np.abs(A), np.abs(B)
     K = A.shape[-1]
-    return (A @ B) * (2.0 ** -21 + (3 * K / 16 + 4) * 2.0 ** -23) + \
-        K * A.max(axis=-1)[..., :, None] * B.max(axis=-2)[..., None, :] * 2.0 ** -25 + 1e-30
+    return (A @ B) * (2.0 ** -21 + (3 * K / 16 + 4) * 2.0 ** -23) + 1e-30
 
 
 def _matmul(ctx, A, B, pairs=2):
@@ -125,6 +124,21 @@ def test_gemm_f32_pairs_beyond_the_split(ctx, M, what):
         # (worked out again, a sum of K products rounds K times)
         bound = _bound(A, B) + (np.abs(A) @ np.abs(B)) * K * 2.0 ** -24
         assert (np.abs(got - ref)[finite] <= bound[finite]).all()
+
+
+@pytest.mark.parametrize("spread", [2.0 ** 8, 2.0 ** 12])
+@pytest.mark.parametrize("M", [40, 150])
+def test_gemm_f32_pairs_spread(ctx, M, spread):
+    """Small values that meet large ones of the other operand keep their bits."""
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.standard_normal((2, M, 260)).astype(np.float32)
+    B = rng.standard_normal((2, 260, 300)).astype(np.float32)
+    plain, exact = _matmul(ctx, A, B), A.astype(np.float64) @ B.astype(np.float64)
+    A[:, :, ::7] *= np.float32(1 / spread)
+    B[:, ::7] *= np.float32(spread)
+    got = _matmul(ctx, A, B)
+    assert (np.abs(got - exact) <= _bound(A, B)).all()
+    assert np.linalg.norm(got - exact) <= 1.05 * np.linalg.norm(plain - exact)
 
 
 def test_gemm_f32_pairs_choice(ctx):

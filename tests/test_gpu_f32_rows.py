@@ -31,12 +31,11 @@ def _matmul(ctx, A, B, rows=2, bn=0):
 
 
 def _bound(A, B):
-    """hi + lo of a value is within 2^-22 of it, or 2^-26 of the largest value of its row; an accumulator holds at most three steps (six
-    MMAs of large products, each cut off by at most 2^-23 of it), and the sums of the runs round once each."""
+    """hi + lo of a value is within 2^-22 of it; an accumulator holds at most three steps (six MMAs of large products, each cut off by
+    at most 2^-23 of it), and the sums of the runs round once each."""
     A, B = np.abs(A), np.swapaxes(np.abs(B), -1, -2)
     K = A.shape[-1]
-    return (A @ B) * (2.0 ** -21 + (6 + K / 32 + 4) * 2.0 ** -23) + \
-        K * A.max(axis=-1)[..., :, None] * B.max(axis=-2)[..., None, :] * 2.0 ** -25 + 1e-30
+    return (A @ B) * (2.0 ** -21 + (6 + K / 32 + 4) * 2.0 ** -23) + 1e-30
 
 
 @pytest.mark.parametrize("bn", [64, 128])
@@ -94,6 +93,21 @@ def test_gemm_f32_rows_beyond_the_split(ctx, bn, what):
         # (worked out again, a sum of K products rounds K times)
         bound = _bound(A, B) + (np.abs(A) @ np.swapaxes(np.abs(B), 1, 2)) * K * 2.0 ** -24
         assert (np.abs(got - ref)[finite] <= bound[finite]).all()
+
+
+@pytest.mark.parametrize("spread", [2.0 ** 8, 2.0 ** 12])
+@pytest.mark.parametrize("bn", [64, 128])
+def test_gemm_f32_rows_spread(ctx, bn, spread):
+    """Small values that meet large ones of the other operand keep their bits."""
+    rng = np.random.Generator(np.random.PCG64(bn))
+    A = rng.standard_normal((2, 150, 420)).astype(np.float32)
+    B = rng.standard_normal((2, 140, 420)).astype(np.float32)
+    plain, exact = _matmul(ctx, A, B, bn=bn), A.astype(np.float64) @ np.swapaxes(B, 1, 2).astype(np.float64)
+    A[:, :, ::7] *= np.float32(1 / spread)
+    B[:, :, ::7] *= np.float32(spread)
+    got = _matmul(ctx, A, B, bn=bn)
+    assert (np.abs(got - exact) <= _bound(A, B)).all()
+    assert np.linalg.norm(got - exact) <= 1.05 * np.linalg.norm(plain - exact)
 
 
 @pytest.mark.parametrize("shape", [(9, 300, 200, 352), (1, 1024, 1024, 1024)])

@@ -39,13 +39,10 @@ def _exact(x, f, sh, pad, out_hw):
 
 
 def _bound(x, f, bias, sh, pad, out_hw, ref):
-    """hi + lo of a value is within 2^-22 of it, or 2^-31 of its strip's largest (2^-26 of a channel's); an accumulator holds at most
-    six MMAs per filter row, each of which cuts off at most 2^-23 of it; the bias and the sum of the two accumulators round once."""
-    C, KH, KW = f.shape[1:]
+    """hi + lo of a value is within 2^-22 of it; an accumulator holds at most six MMAs per filter row, each of which cuts off at most
+    2^-23 of it; the bias and the sum of the two accumulators round once."""
     size = _exact(np.abs(x), np.abs(f), sh, pad, out_hw)
-    steps = np.abs(x).max() * np.abs(f).max(axis=(1, 2, 3))[None, :, None, None] * C * KH * KW
-    return size * (2.0 ** -21 + (6 * KH + 2) * 2.0 ** -23) + steps * (2.0 ** -30 + 2.0 ** -25) + \
-        (np.abs(ref) + np.abs(bias)[None, :, None, None]) * 2.0 ** -23 + 1e-30
+    return size * (2.0 ** -21 + (6 * f.shape[2] + 2) * 2.0 ** -23) + (np.abs(ref) + np.abs(bias)[None, :, None, None]) * 2.0 ** -23 + 1e-30
 
 
 @pytest.mark.parametrize("shape", [
@@ -115,6 +112,28 @@ def test_conv_f32_stem_beyond_the_split(ctx, what):
             rest[1, 2, 30, 31] = 0
             tight = _bound(rest, f, bias, sh, pad, out_hw, ref)
             assert (np.abs(got - ref) <= tight)[:, :, far].all()
+
+
+@pytest.mark.parametrize("spread", [2.0 ** 8, 2.0 ** 12])
+def test_conv_f32_stem_spread(ctx, spread):
+    """Small values that meet large weights keep their bits, and so do dark regions beside bright ones."""
+    rng = np.random.Generator(np.random.PCG64(6))
+    x = rng.standard_normal((2, 3, 60, 60)).astype(np.float32)
+    f = rng.standard_normal((40, 3, 7, 7)).astype(np.float32)
+    args = (np.zeros(40, np.float32), 2, (3, 3), (30, 30))
+
+    def error(x, f, part):
+        got, exact = _conv(ctx, x, f, *args), _exact(x, f, *args[1:])
+        assert (np.abs(got - exact) <= _bound(x, f, *args, exact)).all()
+        return np.linalg.norm((got - exact)[part]) / np.linalg.norm(exact[part])
+
+    plain, all_of_it = error(x, f, np.s_[:, :, :, :18]), error(x, f, np.s_[:])
+    dim = x.copy()
+    dim[:, :, :, :40] *= np.float32(1 / spread)
+    assert error(dim, f, np.s_[:, :, :, :18]) <= 1.05 * plain
+    x[:, 1] *= np.float32(1 / spread)
+    f[:, 1] *= np.float32(spread)
+    assert error(x, f, np.s_[:]) <= 1.05 * all_of_it
 
 
 def test_conv_f32_stem_choice(ctx):
