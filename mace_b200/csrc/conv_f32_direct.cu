@@ -418,7 +418,7 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       float z = 0.f;
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float x = sum[j] * (unscale * __shfl_sync(0xffffffffu, w_mine, j));
+        const float x = sum[j] * unscale * __shfl_sync(0xffffffffu, w_mine, j);
         z = fmaf(x, 0.f, z);
         sum[j] = x + __shfl_sync(0xffffffffu, b_mine, j);
       }

@@ -417,8 +417,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
           for (int j = 0; j < 32; j += 2) {
             // (the products are exact, so the sum with the bias rounds once)
             const float4 ub = *reinterpret_cast<const float4 *>(table + n0 + j);
-            sum[j] = fmaf(sum[j], unscale * ub.x, ub.y);
-            sum[j + 1] = fmaf(sum[j + 1], unscale * ub.z, ub.w);
+            sum[j] = fmaf(sum[j] * unscale, ub.x, ub.y);
+            sum[j + 1] = fmaf(sum[j + 1] * unscale, ub.z, ub.w);
             z = fmaf(sum[j], 0.f, z);
             z = fmaf(sum[j + 1], 0.f, z);
           }

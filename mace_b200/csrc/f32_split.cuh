@@ -13,7 +13,7 @@
 //
 // A row's scale is that of the first step of 32 in which it has a value other than zero (zeros need none), so that nothing has
 // to be read twice.  Later values may be 2^14 times larger; beyond that hi is infinite and the results of that row come out as
-// NaN, like those of an infinite value or of a row below 2^-61, and are marked, and worked out again by fp32 FMAs.
+// NaN, like those of an infinite value, and are marked, and worked out again by fp32 FMAs.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -22,13 +22,14 @@
 
 constexpr uint32_t F32_AGAIN = 0x7fc0a6a1u;  // stored for a result to be worked out again
 
-// The scale of a row whose largest value is m > 0.  NaN below 2^-61: its products are then worked out again.
+// The scale of a row whose largest value is m > 0: at least 2^-126 and at most 2^126, so that its inverse is a normal number too.
+// (Rows below 2^-125 stay below 2, but have no bits that lo does not hold.)
 __device__ __forceinline__ float f32_row_scale(float m) {
   const uint32_t e = __float_as_uint(m) >> 23;  // biased; the scale's is 254 - e + 1
-  if (e < 66u) return __uint_as_float(0x7fc00000u);
-  return __uint_as_float((255u - min(e, 190u)) << 23);
+  return __uint_as_float(min(255u - min(e, 254u), 253u) << 23);
 }
-// What a result is multiplied by: 1 / s, 0 for a row of zeros only (its scale is still 0).
+// What a result is multiplied by: 1 / s, 0 for a row of zeros only (its scale is still 0).  X's and W's one after the other: their
+// product may leave the range of fp32 where the result does not.
 __device__ __forceinline__ float f32_row_unscale(float s) {
   return s == 0.f ? 0.f : __uint_as_float(0x7f000000u - __float_as_uint(s));
 }

@@ -298,7 +298,7 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       float z = 0.f;
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float x = sum[j] * (unscale * __shfl_sync(0xffffffffu, w_mine, j));
+        const float x = sum[j] * unscale * __shfl_sync(0xffffffffu, w_mine, j);
         z = fmaf(x, 0.f, z);
         sum[j] = p.bias != nullptr ? x + __shfl_sync(0xffffffffu, b_mine, j) : x;
       }

@@ -142,6 +142,20 @@ def test_direct_conv2d_f32_spread(ctx, O, spread):
     assert error(x, f, np.s_[:]) <= 1.05 * plain
 
 
+@pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
+@pytest.mark.parametrize("O", [20, 100])
+def test_direct_conv2d_f32_scales(ctx, O, powers):
+    """Results are those of operands of ordinary size, bit for bit: nothing is worked out again because a row is small or large."""
+    rng = np.random.Generator(np.random.PCG64(O))
+    x = rng.standard_normal((2, 40, 12, 12)).astype(np.float32)
+    f = (rng.standard_normal((O, 40, 3, 3)) * 0.1).astype(np.float32)
+    plain = _run(ctx, x, f, None)
+    a, b = (np.float32(2.0) ** p for p in powers)
+    f[::3] *= a
+    plain[:, ::3] *= a
+    assert np.array_equal(_run(ctx, x * b, f, None), plain * b)
+
+
 def test_direct_conv2d_f32_choice(ctx):
     """By rule: a batch of 3x3 and 5x5 layers, and no smaller an accuracy there than the other kernels have."""
     rng = np.random.Generator(np.random.PCG64(0))

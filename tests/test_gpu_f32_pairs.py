@@ -141,6 +141,22 @@ def test_gemm_f32_pairs_spread(ctx, M, spread):
     assert np.linalg.norm(got - exact) <= 1.05 * np.linalg.norm(plain - exact)
 
 
+@pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
+@pytest.mark.parametrize("M", [40, 150])
+def test_gemm_f32_pairs_scales(ctx, M, powers):
+    """Results are those of operands of ordinary size, bit for bit: nothing is worked out again because a row is small or large."""
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.standard_normal((2, M, 100)).astype(np.float32)
+    B = rng.standard_normal((2, 100, 300)).astype(np.float32)
+    plain = _matmul(ctx, A, B)
+    a, b = (np.float32(2.0) ** p for p in powers)
+    A[:, ::3] *= a
+    B[:, :, 5:200] *= b
+    plain[:, ::3] *= a
+    plain[:, :, 5:200] *= b
+    assert np.array_equal(_matmul(ctx, A, B), plain)
+
+
 def test_gemm_f32_pairs_choice(ctx):
     """By rule for a product of many steps, with an error no larger than the other kernel's."""
     rng = np.random.Generator(np.random.PCG64(0))

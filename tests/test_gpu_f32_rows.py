@@ -110,6 +110,22 @@ def test_gemm_f32_rows_spread(ctx, bn, spread):
     assert np.linalg.norm(got - exact) <= 1.05 * np.linalg.norm(plain - exact)
 
 
+@pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
+@pytest.mark.parametrize("bn", [64, 128])
+def test_gemm_f32_rows_scales(ctx, bn, powers):
+    """Results are those of operands of ordinary size, bit for bit: nothing is worked out again because a row is small or large."""
+    rng = np.random.Generator(np.random.PCG64(bn))
+    A = rng.standard_normal((2, 150, 100)).astype(np.float32)
+    B = rng.standard_normal((2, 140, 100)).astype(np.float32)
+    plain = _matmul(ctx, A, B, bn=bn)
+    a, b = (np.float32(2.0) ** p for p in powers)
+    A[:, ::3] *= a
+    B[:, 5:100] *= b
+    plain[:, ::3] *= a
+    plain[:, :, 5:100] *= b
+    assert np.array_equal(_matmul(ctx, A, B, bn=bn), plain)
+
+
 @pytest.mark.parametrize("shape", [(9, 300, 200, 352), (1, 1024, 1024, 1024)])
 def test_gemm_f32_rows_choice(ctx, shape):
     """By rule, with an error no larger than that of the kernel that fetches its own operands."""

@@ -136,6 +136,20 @@ def test_conv_f32_stem_spread(ctx, spread):
     assert error(x, f, np.s_[:]) <= 1.05 * all_of_it
 
 
+@pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
+def test_conv_f32_stem_scales(ctx, powers):
+    """Results are those of operands of ordinary size, bit for bit: nothing is worked out again because a row is small or large."""
+    rng = np.random.Generator(np.random.PCG64(6))
+    x = rng.standard_normal((2, 3, 60, 60)).astype(np.float32)
+    f = rng.standard_normal((40, 3, 7, 7)).astype(np.float32)
+    args = (np.zeros(40, np.float32), 2, (3, 3), (30, 30))
+    plain = _conv(ctx, x, f, *args)
+    a, b = (np.float32(2.0) ** p for p in powers)
+    f[::3] *= a
+    plain[:, ::3] *= a
+    assert np.array_equal(_conv(ctx, x * b, f, *args), plain * b)
+
+
 def test_conv_f32_stem_choice(ctx):
     """By rule: large ones, with an error no larger than that of the kernel that fetches its own operands."""
     rng = np.random.Generator(np.random.PCG64(9))
