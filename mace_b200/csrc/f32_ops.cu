@@ -437,10 +437,8 @@ int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *
   // 48.8 this way; 4 of 240 x 64 x 80: 6.4 and 7.3.  Up to 64 deep the former's three accumulators are the more accurate.
   if (!by_tma && ctx->f32_rows != 1 && mb_gemm_f32_rows_supported(ctx, g) &&
       (ctx->f32_rows == 2 ||
-       (gather && ctx->f32_gather == 0 && g.run != 0 && K > 64 && mb_gemm_f32_rows_cost(ctx, g) < mb_gemm_f32_gather_cost(ctx, g)))) {
-    if (g.run == 0) g.run = 1;
+       (gather && ctx->f32_gather == 0 && g.run != 0 && K > 64 && mb_gemm_f32_rows_cost(ctx, g) < mb_gemm_f32_gather_cost(ctx, g))))
     return mb_gemm_f32_rows_launch(ctx, g);
-  }
   if (gather) return mb_gemm_f32_gather_launch(ctx, g);
   // C = A * B with A [M x K] k-contiguous, B [K x N] n-contiguous and C n-contiguous is the
   // tensor-core kernel's layout with the roles X = B (pixels x channels side), W = A.

@@ -7,10 +7,12 @@
 // rewrite in place as 32 halves of hi and 32 of lo.  Both operands of the MMA then lie in shared memory, so that all of
 // tensor memory is there for accumulators: the large products hi * hi in one, cut off once per 16 of k, hi * lo + lo * hi
 // in another, both twice.  Every `run` steps the result warps take them and carry the sums on in registers: with one step the
-// error is 1.16e-7, with three 1.76e-7 (2-norm against float64; the self-fetching kernel on tf32: 1.37e-7, 2.06e-7).
+// error is 1.16e-7, with three 1.76e-7 (2-norm against float64; the self-fetching kernel on tf32: 1.37e-7, 2.06e-7).  A run's rows
+// have scales of their own, for which the warps that split look at all of its steps first.  (With a scale per tile, from its first
+// step, rows that grew beyond 2^14 times that were worked out again by FMAs.)
 //
-// What bounds it: launch, first copies and results for few steps; the shared-memory pipe else (57 % busy: 1150 cycles per step of 128 x 128
-// for copies, split and MMAs, with waits between the three).
+// What bounds it: launch, first copies and results for few steps; else the split, whose warps wait for a run, look at it, split
+// it step by step and hand each on (1860 cycles per step of 128 x 128 in runs of three, 2150 in runs of one).
 // Against the kernel whose warps fetch X from where it lies (a lane a row: 32 lines per instruction): see cost_of.
 //
 // Roles: warp 0 copies, warp 1 MMAs, 8 warps split, 8 or 16 results (32 columns of n per thread).  Persistent over the tiles.
@@ -29,8 +31,8 @@ using namespace sm100;
 
 constexpr int BM = 128, KB = 32;
 constexpr int FIRST_SPLIT = 2, SPLIT_WARPS = 8, FIRST_OUT = FIRST_SPLIT + SPLIT_WARPS;
-constexpr int STAGES = 4;
-constexpr int SCALE_SLOTS = 8;  // tiles: the split is at most STAGES tiles of one step ahead of the MMAs, these two of the results
+constexpr int MAX_RUN = 3;
+constexpr int SCALE_SLOTS = 16;  // runs: the split is at most STAGES ahead of the MMAs, these two of the results
 constexpr long long WAIT_BUDGET = 1ll << 31;  // ~1 s of SM clocks per wait
 
 // Where four k (chunk 0 .. 7 of a step) of a row's hi half lie: in the first 64 of its 128 bytes, in the tensor core's 128-byte
@@ -53,6 +55,8 @@ struct Params {
 template <int BN>
 struct Cfg {
   static constexpr int ROWS = BM + BN, STAGE_BYTES = ROWS * 128;
+  static constexpr int STAGES = BN == 128 ? 6 : 8;  // (two runs and more)
+  static_assert(STAGES >= MAX_RUN && STAGES + 3 <= SCALE_SLOTS, "a run is split when all of it has landed");
   static constexpr int OUT_WARPS = BN / 8, THREADS = (FIRST_OUT + OUT_WARPS) * 32;
   static constexpr int ACC_COLS = 2 * BN, ACCS = 2, TMEM_COLS = ACCS * ACC_COLS;
   static constexpr int SCALE_AT = STAGES * STAGE_BYTES, BAR_AT = SCALE_AT + SCALE_SLOTS * ROWS * 4;
@@ -79,6 +83,7 @@ __global__ void __launch_bounds__(Cfg<BN>::THREADS, 1)
 gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                      const __grid_constant__ Params p) {
   using C = Cfg<BN>;
+  constexpr int STAGES = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -198,57 +203,63 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const int r0 = (warp - FIRST_SPLIT) * 4 + (lane >> 3);  // row of chunk i: i * 32 + r0
     const int chunk = (lane & 7) ^ (r0 & 7);                // (TMA lays the rows out in the 128-byte swizzle)
     const bool swap = ((lane >> 3) & 1) != 0;               // of two rows that share their banks, one writes lo first
-    uint32_t stage = 0, phase = 0;
-    int tile = 0;
+    uint32_t stage = 0, phase = 0, run = 0;
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++tile) {
-      const int tn = t % p.tiles_n, tm = t / p.tiles_n % p.tiles_m;
-      float *slot = unscales + (tile % SCALE_SLOTS) * C::ROWS;
-      float scale[CH];
+    float4 v[CH];
+    auto load = [&](uint32_t at) {
+      const uint8_t *rows = smem + at * C::STAGE_BYTES + r0 * 128 + (lane & 7) * 16;
 #pragma unroll
-      for (int i = 0; i < CH; ++i) scale[i] = 0.f;
-      bool known = false;  // every row of the warp has its scale
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_warp(landed_bar + 8 * stage, phase, abort_flag, WAIT_BUDGET)) {
-          fail(MB_DEV_TIMEOUT_EPILOGUE);
-          ok = false;
-          break;
-        }
-        uint8_t *rows = smem + stage * C::STAGE_BYTES;
-        float4 v[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) v[i] = *reinterpret_cast<const float4 *>(rows + (i * 32 + r0) * 128 + (lane & 7) * 16);
-        __syncwarp();  // (a row is rewritten by the warp that read it)
-        if (!known) {
-          bool all = true;
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            float most = fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
-#pragma unroll
-            for (int d = 1; d < 8; d *= 2) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
-            if (scale[i] == 0.f && most > 0.f) scale[i] = f32_row_scale(most);
-            const int row = i * 32 + r0;
-            all = all && (scale[i] != 0.f || (row < BM ? tm * BM + row >= p.M : tn * BN + row - BM >= p.N));
-            if ((lane & 7) == 0) slot[row] = f32_row_unscale(scale[i]);
+      for (int i = 0; i < CH; ++i) v[i] = *reinterpret_cast<const float4 *>(rows + i * 4096);
+    };
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+      for (int kb = 0; ok && kb < k_blocks; kb += p.run, ++run) {
+        // the largest values of the run's rows, its first step last, whose values stay: the eight lanes of a row halve their rows
+        // between them and end with one each
+        const int steps = min(p.run, k_blocks - kb);
+        float most[8] = {};
+        for (int i = steps - 1; i >= 0; --i) {
+          const uint32_t at = stage + i, wrapped = at >= static_cast<uint32_t>(STAGES) ? 1u : 0u;
+          if (!mbar_wait_warp(landed_bar + 8 * (at - wrapped * STAGES), phase ^ wrapped, abort_flag, WAIT_BUDGET)) {
+            fail(MB_DEV_TIMEOUT_EPILOGUE);
+            ok = false;
+            break;
           }
-          known = __all_sync(0xffffffffu, all);
-        }
+          load(at - wrapped * STAGES);
 #pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const uint64_t scales = f32_pair(scale[i], scale[i]);
-          uint2 hi, lo;
-          f32_split2(f32_pair(v[i].x, v[i].y), scales, hi.x, lo.x);
-          f32_split2(f32_pair(v[i].z, v[i].w), scales, hi.y, lo.y);
-          const uint32_t at = hi_at(i * 32 + r0, chunk);
-          *reinterpret_cast<uint2 *>(rows + (swap ? at ^ 64 : at)) = swap ? lo : hi;
-          *reinterpret_cast<uint2 *>(rows + (swap ? at : at ^ 64)) = swap ? hi : lo;
+          for (int j = 0; j < CH; ++j) most[j] = fmaxf(fmaxf(most[j], fmaxf(fabsf(v[j].x), fabsf(v[j].y))), fmaxf(fabsf(v[j].z), fabsf(v[j].w)));
         }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(full_bar + 8 * stage);
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
+        if (!ok) break;
+#pragma unroll
+        for (int d = 4; d > 0; d /= 2)
+#pragma unroll
+          for (int i = 0; i < d; ++i) {
+            const bool up = (lane & d) != 0;
+            most[i] = fmaxf(up ? most[i + d] : most[i], __shfl_xor_sync(0xffffffffu, up ? most[i] : most[i + d], d));
+          }
+        const float mine = most[0] > 0.f ? f32_row_scale(most[0]) : 0.f;
+        if ((lane & 7) < CH) unscales[(run % SCALE_SLOTS) * C::ROWS + (lane & 7) * 32 + r0] = f32_row_unscale(mine);
+        for (int i = 0; i < steps; ++i) {
+          if (i > 0) load(stage);
+          __syncwarp();  // (a row is rewritten by the warp that read it)
+          uint8_t *rows = smem + stage * C::STAGE_BYTES;
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            const float scale = __shfl_sync(0xffffffffu, mine, (lane & 24) + j);
+            const uint64_t scales = f32_pair(scale, scale);
+            uint2 hi, lo;
+            f32_split2(f32_pair(v[j].x, v[j].y), scales, hi.x, lo.x);
+            f32_split2(f32_pair(v[j].z, v[j].w), scales, hi.y, lo.y);
+            const uint32_t at = hi_at(j * 32 + r0, chunk);
+            *reinterpret_cast<uint2 *>(rows + (swap ? at ^ 64 : at)) = swap ? lo : hi;
+            *reinterpret_cast<uint2 *>(rows + (swap ? at : at ^ 64)) = swap ? hi : lo;
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full_bar + 8 * stage);
+          if (++stage == static_cast<uint32_t>(STAGES)) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
     }
@@ -256,17 +267,17 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     // ---- results: a lane per m, 32 of n per thread ----
     const int quarter = warp & 3, c0 = (warp - FIRST_OUT) / 4 * 32;
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
-    const int runs = (k_blocks + p.run - 1) / p.run;
-    uint32_t acc = 0, acc_phase = 0;
-    int tile = 0;
+    uint32_t acc = 0, acc_phase = 0, run = 0;
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++tile) {
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
       const int tn = t % p.tiles_n, q = t / p.tiles_n, tm = q % p.tiles_m, b = q / p.tiles_m;
       const int m = tm * BM + quarter * 32 + lane, n0 = tn * BN + c0;
       const float b_mine = p.bias != nullptr && n0 + lane < p.N ? mb_load(p.bias + n0 + lane) : 0.f;
-      float sum[32];
+      uint64_t sums[16];  // of two channels each
+#pragma unroll
+      for (int j = 0; j < 16; ++j) sums[j] = 0;
 #pragma unroll 1
-      for (int i = 0; i < runs; ++i) {
+      for (int kb = 0; kb < k_blocks; kb += p.run, ++run) {
         if (!mbar_wait_warp(tfull_bar + 8 * acc, acc_phase, abort_flag, WAIT_BUDGET)) {
           fail(MB_DEV_TIMEOUT_EPILOGUE);
           ok = false;
@@ -274,6 +285,8 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         }
         tc_fence_after_sync();
         const uint32_t src = tmem + lanes + acc * C::ACC_COLS + c0;
+        const float *slot = unscales + (run % SCALE_SLOTS) * C::ROWS;
+        const uint64_t unscale = f32_pair(slot[quarter * 32 + lane], slot[quarter * 32 + lane]);
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
           uint32_t r[8], s[8];
@@ -282,9 +295,14 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
           tmem_ld_wait_x8(r);
           tmem_ld_wait_x8(s);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float x = fmaf(__uint_as_float(s[k]), F32_LO, __uint_as_float(r[k]));
-            sum[j + k] = i == 0 ? x : sum[j + k] + x;
+          for (int k = 0; k < 8; k += 4) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(slot + BM + c0 + j + k);  // (one address: a broadcast)
+#pragma unroll
+            for (int h = 0; h < 4; h += 2) {
+              const uint64_t x = f32_fma2(f32_pair(__uint_as_float(s[k + h]), __uint_as_float(s[k + h + 1])), f32_pair(F32_LO, F32_LO),
+                                          f32_pair(__uint_as_float(r[k + h]), __uint_as_float(r[k + h + 1])));
+              sums[(j + k + h) / 2] = f32_fma2(f32_mul2(x, unscale), h == 0 ? w.x : w.y, sums[(j + k + h) / 2]);
+            }
           }
         }
         tc_fence_before_sync();
@@ -293,12 +311,11 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         if ((acc ^= 1) == 0) acc_phase ^= 1;
       }
       if (!ok) break;
-      const float *slot = unscales + (tile % SCALE_SLOTS) * C::ROWS;
-      const float unscale = slot[quarter * 32 + lane], w_mine = slot[BM + c0 + lane];
-      float z = 0.f;
+      float z = 0.f, sum[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float x = sum[j] * unscale * __shfl_sync(0xffffffffu, w_mine, j);
+        const float2 both = f32_parts(sums[j / 2]);
+        const float x = j % 2 == 0 ? both.x : both.y;
         z = fmaf(x, 0.f, z);
         sum[j] = p.bias != nullptr ? x + __shfl_sync(0xffffffffu, b_mine, j) : x;
       }
@@ -355,11 +372,12 @@ int launch(mb_context *ctx, Params &p) {
   return MB_SUCCESS;
 }
 
-// Estimated SM cycles, from 1536 x 1536 x 1024 (128 columns 35.8 us, 64 43.0), 1024^3 (35.2, 23.8), 736 x 176 x 384, batch 24 (29.9,
-// 36.0), 1024 x 1024 x 64, batch 8 (19.7, 21.6) and single tiles (7.3, 5.8).  The self-fetching kernel: 49.6, 36.4, 39.6, 21.0, 6.2 us.
+// Estimated SM cycles, from 1536 x 1536 x 1024 (128 columns 37.8 us, 64 49.3), 1024^3 (37.5, 26.9), 257 x 200 x 260, batch 5 (17.4,
+// 12.8), 1024 x 1024 x 64, batch 8 (19.7, 20.0) and single tiles (6.5, 4.9).  The self-fetching kernel: 49.6, 36.4, -, 21.0, 6.2 us.
 int64_t cost_of(const mb_context *ctx, const mb_f32_gemm &g, int bn) {
   const int64_t rounds = ceil_div64(g.batch * ceil_div64(g.M, BM) * ceil_div64(g.N, bn), ctx->num_sms);
-  return (bn == 128 ? 12000 : 10000) + rounds * std::max<int64_t>(ceil_div64(g.K, KB) * (bn == 128 ? 1800 : 1150), bn == 128 ? 6200 : 4400);
+  const int64_t step = g.run > 1 ? (bn == 128 ? 1860 : 1300) : (bn == 128 ? 2150 : 1560);  // (runs of three steps, of one)
+  return (bn == 128 ? 12000 : 10000) + rounds * std::max<int64_t>(ceil_div64(g.K, KB) * step, bn == 128 ? 6200 : 4400);
 }
 int pick_bn(const mb_context *ctx, const mb_f32_gemm &g) {
   if (ctx->f32_bn != 0) return ctx->f32_bn;
@@ -388,7 +406,7 @@ int mb_gemm_f32_rows_launch(mb_context *ctx, const mb_f32_gemm &g) {
   p.tiles_m = static_cast<int>(ceil_div64(g.M, BM));
   p.tiles_n = static_cast<int>(ceil_div64(g.N, bn));
   p.k_blocks = static_cast<int>(ceil_div64(g.K, KB));
-  p.run = g.run != 0 ? 2 * g.run - 1 : p.k_blocks;
+  p.run = g.run > 1 ? MAX_RUN : 1;
   p.act = g.act; p.max_limit = g.max_limit; p.coef = g.coef;
   p.status = ctx->dev_status;
   return bn == 128 ? launch<128>(ctx, p) : launch<64>(ctx, p);

@@ -126,6 +126,22 @@ def test_gemm_f32_rows_scales(ctx, bn, powers):
     assert np.array_equal(_matmul(ctx, A, B, bn=bn), plain)
 
 
+@pytest.mark.parametrize("power", [-40, -16, 16, 40])
+@pytest.mark.parametrize("K", [164, 420])
+@pytest.mark.parametrize("bn", [64, 128])
+def test_gemm_f32_rows_steps(ctx, bn, K, power):
+    """Steps of another size than the first, in which the other operand makes up for it: the same results, bit for bit, and so none
+    of them is worked out again."""
+    rng = np.random.Generator(np.random.PCG64(bn))
+    A = rng.standard_normal((2, 150, K)).astype(np.float32)
+    B = rng.standard_normal((2, 140, K)).astype(np.float32)
+    plain = _matmul(ctx, A, B, bn=bn)
+    for k0, k1 in ((32, 64), (96, 164)) if K < 384 else ((96, 192), (288, 420)):  # (runs of one step and of three)
+        A[:, :, k0:k1] *= np.float32(2.0) ** power
+        B[:, :, k0:k1] *= np.float32(2.0) ** -power
+    assert np.array_equal(_matmul(ctx, A, B, bn=bn), plain)
+
+
 @pytest.mark.parametrize("shape", [(9, 300, 200, 352), (1, 1024, 1024, 1024)])
 def test_gemm_f32_rows_choice(ctx, shape):
     """By rule, with an error no larger than that of the kernel that fetches its own operands."""
