@@ -14,10 +14,11 @@
 //
 // W (the filter) comes split by f32_conv_presplit_kernel, a step being 32 channels of one tap: a tile of hi rows with a tile
 // of lo rows behind it, so that hi x [w_hi | w_lo] is one MMA of twice the columns, lo x w_hi goes to the second half, and the
-// large products have an accumulator of their own, which is cut off once per 16 of k (2e-8 each time).  Every `run` filter rows the
-// result warps take both and carry the sums on in registers, where they round: errors (2-norm against float64, 3x3) of 1.3e-7 with a row
-// at a time, 3.5e-7 with three, 1.4e-6 with twelve, whatever the depth; Winograd's are 3.1e-8 times the root of the channels with F(2,3)
-// and 2e-6 and more with F(6,3).
+// large products have an accumulator of their own, which is cut off once per 16 of k (2e-8 each time).  Every `run` filter rows of
+// 32 channels the result warps take both and carry the sums on in registers, where they round: errors (2-norm against float64, 3x3) of
+// 1.3e-7 with a row at a time, 3.5e-7 with three, whatever the depth; Winograd's are 3.1e-8 times the root of the channels with
+// F(2,3) and 2e-6 and more with F(6,3).  So every patch may have a scale of its own: it takes that of the one before where its largest
+// value allows it, which is known when the patch has been written, and else its own, and is written again.
 //
 // What bounds it: shared memory, 470 cycles per tap of 128 channels (40 KB into the MMAs, 16 KB of W in), of which the MMAs are
 // busy 384, at the clocks that the power limit leaves; with 64 channels the issue of small MMAs, 350 against 235.
@@ -40,7 +41,7 @@ using namespace sm100;
 constexpr int BM = 128, KC = 32;                   // places per tile, channels per block
 constexpr int FIRST_IN = 2, IN_WARPS = 8;         // input warps per group
 constexpr long long WAIT_BUDGET = 1ll << 31;       // ~1 s of SM clocks per wait
-constexpr int SCALE_SLOTS = 8;                     // input is at most two patches ahead of the MMAs, these two tiles of the results
+constexpr int SCALE_SLOTS = 8;                     // patches: input is at most two ahead of the MMAs, these two runs of the results
 constexpr int MAX_W_STAGES = 12;
 
 struct Params {
@@ -49,7 +50,7 @@ struct Params {
   int N, C_in, H, W, O, KH, KW, ph, pw;
   int pitch, image;          // places per row and per image
   int64_t places;            // all of them
-  int tiles_m, tiles_n, blocks, taps, run;
+  int tiles_m, tiles_n, blocks, taps, run;  // run: filter rows, of one block
   int patch_rows;            // a multiple of 32
   int w_stages;              // filter rows in shared memory
   int w_stays;               // ... which are all there are
@@ -62,7 +63,7 @@ struct Params {
 template <int BN>
 struct Cfg {
   // Input in two groups that take the tiles in turn where a tile's MMAs are over sooner than the first loads of the next one
-  // and the look at its scale (64 channels, 56 x 56, batch 32: 45.3 -> 42.3 us).
+  // (64 channels, 56 x 56, batch 32: 45.3 -> 42.3 us).
   static constexpr int IN_GROUPS = BN == 64 ? 2 : 1;
   static constexpr int FIRST_OUT = FIRST_IN + IN_GROUPS * IN_WARPS;
   static constexpr int OUT_WARPS = BN / 8;         // 32 channels per thread
@@ -155,8 +156,8 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(more);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *again = abort_flag + 1;
-  float *scales = reinterpret_cast<float *>(more + 16);     // [SCALE_SLOTS] of the tiles' input
-  float *warp_most = scales + SCALE_SLOTS;                  // [IN_GROUPS][2][IN_WARPS]
+  float *scales = reinterpret_cast<float *>(more + 16);     // [SCALE_SLOTS] of the patches
+  float *warp_most = scales + SCALE_SLOTS;                  // [IN_GROUPS][IN_WARPS]
   const int patch_bytes = p.patch_rows * 128;
   const uint32_t w_row_bytes = p.KW * C::W_BYTES, w_stages = p.w_stages;
   const uint32_t w_base = smem_base + 1024, patch0 = w_base + w_stages * w_row_bytes;
@@ -234,7 +235,7 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       bool ok = true, ready = false;
       for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
         uint32_t d = 0;
-        int left = 0, rows = blocks * taps_h;  // filter rows of this run and of the tile still to come
+        int left = 0;                          // filter rows of this run still to come
         const bool here = w_stays && t != blockIdx.x;  // the whole filter
         for (int blk = 0; ok && blk < blocks; ++blk) {
           if (!mbar_wait_warp(pfull_bar + 8 * patch, patch_phase, abort_flag, WAIT_BUDGET)) {
@@ -252,7 +253,7 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 break;
               }
               d = tmem + acc * C::ACC_COLS;
-              left = min(run, rows);
+              left = min(run, taps_h - i);
               add = 0u;
             }
             // (a barrier per filter row: what the thread does around one takes as long as four MMAs)
@@ -279,7 +280,6 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             if (!w_stays) mma_commit_elect(wempty_bar + 8 * stage);
             stage = next;
             phase = next_phase;
-            --rows;
             if (--left == 0) {
               mma_commit_elect(tfull_bar + 8 * acc);
               if ((acc ^= 1) == 0) acc_phase ^= 1;
@@ -295,14 +295,13 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   } else if (warp < C::FIRST_OUT) {
     // ---- input: tensor -> registers -> hi / lo planes ----
     const int w8 = (warp - FIRST_IN) % IN_WARPS, group = (warp - FIRST_IN) / IN_WARPS;
-    float *group_most = warp_most + group * 2 * IN_WARPS;
+    float *group_most = warp_most + group * IN_WARPS;
     const int row_blocks = p.patch_rows / 32;
     const int64_t hw = static_cast<int64_t>(p.H) * p.W;
-    uint32_t looked = 0;
+    float scale = 0.f;  // of the patch before, which the next one tries first
     // (A wait that gives up ends none of these warps, which meet at a barrier: the waits that follow it return at once.)
     for (int tile = group, t = blockIdx.x + group * gridDim.x; t < tiles; t += C::IN_GROUPS * gridDim.x, tile += C::IN_GROUPS) {
       const int64_t f0 = static_cast<int64_t>(t / p.tiles_n) * BM - static_cast<int64_t>(p.ph) * p.pitch - p.pw + lane;
-      float scale = 0.f;
       for (int blk = 0; blk < p.blocks; ++blk) {
         const uint32_t nth = static_cast<uint32_t>(tile) * p.blocks + blk, patch = nth & 1, phase = (nth >> 1) & 1;
         uint8_t *to = smem + (patch0 - smem_base) + patch * patch_bytes;
@@ -315,47 +314,65 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           for (int c = 0; c < KC; ++c) v[c] = c < channels ? mb_load(src + c * hw) : 0.f;
         };
         load(w8);
-        if (scale == 0.f) {
-          // the scale of the first block with a value other than zero serves the tile (see f32_shared_scale)
-          float most = 0.f;
-#pragma unroll
-          for (int c = 0; c < KC; ++c) most = fmaxf(most, f32_finite_abs(v[c]));
-          for (int rb = w8 + IN_WARPS; rb < row_blocks; rb += IN_WARPS) {
-            const int64_t at = value_at(p, f0 + rb * 32);
-            const float *src = p.X + max(at, static_cast<int64_t>(0)) + static_cast<int64_t>(blk) * KC * hw;
-            const int channels = at >= 0 ? min(KC, p.C_in - blk * KC) : 0;
-#pragma unroll 8
-            for (int c = 0; c < channels; ++c) most = fmaxf(most, f32_finite_abs(mb_load(src + c * hw)));
-          }
-#pragma unroll
-          for (int d = 1; d < 32; d *= 2) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
-          if (lane == 0) group_most[(looked & 1) * IN_WARPS + w8] = most;
-          named_bar_sync(1 + group, IN_WARPS * 32);
-          scale = f32_shared_scale<IN_WARPS>(group_most + (looked & 1) * IN_WARPS);
-          ++looked;
-          if (w8 == 0 && lane == 0) scales[tile % SCALE_SLOTS] = f32_row_unscale(scale);
-        }
-        const uint64_t ss = f32_pair(scale, scale);
         // The groups write in turn, tile by tile (and load ahead of it): a patch's barrier tells its last use from the one
         // before, not from two before, so its uses have to be waited for one after the other.
         if (C::IN_GROUPS > 1 && blk == 0 && tile > 0 &&
             !mbar_wait_warp(turn_bar + 8 * group, ((tile - 1) >> 1) & 1, abort_flag, WAIT_BUDGET))
           fail(MB_DEV_TIMEOUT_PRODUCER);
         if (!mbar_wait_warp(pempty_bar + 8 * patch, phase ^ 1, abort_flag, WAIT_BUDGET)) fail(MB_DEV_TIMEOUT_PRODUCER);
-        for (int rb = w8; rb < row_blocks; rb += IN_WARPS) {
-          if (rb != w8) load(rb);
+        float most = 0.f;
+        auto split = [&]() {
+          most = 0.f;
+          const uint64_t ss = f32_pair(scale, scale);
+#pragma unroll 1
+          for (int rb = w8; rb < row_blocks; rb += IN_WARPS) {
+            if (rb != w8) load(rb);
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 hi, lo;
-            f32_split2(f32_pair(v[8 * g], v[8 * g + 1]), ss, hi.x, lo.x);
-            f32_split2(f32_pair(v[8 * g + 2], v[8 * g + 3]), ss, hi.y, lo.y);
-            f32_split2(f32_pair(v[8 * g + 4], v[8 * g + 5]), ss, hi.z, lo.z);
-            f32_split2(f32_pair(v[8 * g + 6], v[8 * g + 7]), ss, hi.w, lo.w);
-            uint8_t *row = to + (rb * 32 + lane) * 128;
-            *reinterpret_cast<uint4 *>(row + ((g ^ (lane & 7)) << 4)) = hi;
-            *reinterpret_cast<uint4 *>(row + (((g + 4) ^ (lane & 7)) << 4)) = lo;
+            for (int c = 0; c < KC; ++c) most = fmaxf(most, fabsf(v[c]));
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              uint4 hi, lo;
+              f32_split2(f32_pair(v[8 * g], v[8 * g + 1]), ss, hi.x, lo.x);
+              f32_split2(f32_pair(v[8 * g + 2], v[8 * g + 3]), ss, hi.y, lo.y);
+              f32_split2(f32_pair(v[8 * g + 4], v[8 * g + 5]), ss, hi.z, lo.z);
+              f32_split2(f32_pair(v[8 * g + 6], v[8 * g + 7]), ss, hi.w, lo.w);
+              uint8_t *row = to + (rb * 32 + lane) * 128;
+              *reinterpret_cast<uint4 *>(row + ((g ^ (lane & 7)) << 4)) = hi;
+              *reinterpret_cast<uint4 *>(row + (((g + 4) ^ (lane & 7)) << 4)) = lo;
+            }
+          }
+        };
+        const bool first = scale == 0.f;  // (the same for all warps of the group)
+        uint32_t votes = 0;
+        if (!first) {
+          split();
+          // Whether the scale was right: how many warps have values beyond what hi holds (16 each), how many have one that is large
+          // enough for a patch's largest (1 each).
+          const bool high = __any_sync(0xffffffffu, most * scale >= F32_HIGH), fair = __any_sync(0xffffffffu, most * scale >= F32_LOW);
+          votes = named_bar_popc(1 + group, IN_WARPS * 32, lane < 16 ? high : lane == 16 && fair);
+        }
+        if (votes >= 16 || votes == 0) {
+          // its own, and once more if that is another one
+          float finite = 0.f;
+#pragma unroll 1
+          for (int rb = w8; rb < row_blocks; rb += IN_WARPS) {
+            if (!first || rb != w8) load(rb);
+#pragma unroll
+            for (int c = 0; c < KC; ++c) finite = fmaxf(finite, f32_finite_abs(v[c]));
+          }
+#pragma unroll
+          for (int d = 1; d < 32; d *= 2) finite = fmaxf(finite, __shfl_xor_sync(0xffffffffu, finite, d));
+          if (lane == 0) group_most[w8] = finite;
+          named_bar_sync(1 + group, IN_WARPS * 32);
+          const float own = f32_shared_scale<IN_WARPS>(group_most);
+          named_bar_sync(1 + group, IN_WARPS * 32);
+          if (first || (own != 0.f && own != scale)) {
+            scale = own;
+            if (row_blocks > IN_WARPS) load(w8);
+            split();
           }
         }
+        if (w8 == 0 && lane == 0) scales[nth % SCALE_SLOTS] = f32_row_unscale(scale);
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
@@ -369,11 +386,10 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const int quarter = warp & 3, c0 = (warp - C::FIRST_OUT) / 4 * 32;
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
     const int64_t hw = static_cast<int64_t>(p.H) * p.W;
-    const int runs = (p.blocks * p.KH + p.run - 1) / p.run;
-    uint32_t acc = 0, acc_phase = 0;
-    int tile = 0;
+    const int runs = (p.KH + p.run - 1) / p.run;  // of a block
+    uint32_t acc = 0, acc_phase = 0, nth = 0;
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++tile) {
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
       const int64_t f = static_cast<int64_t>(t / p.tiles_n) * BM + quarter * 32 + lane;
       const int n0 = t % p.tiles_n * BN + c0;
       // this lane's channel: what its results are multiplied by, its bias
@@ -387,11 +403,11 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         if (static_cast<int>(y) < p.H && static_cast<int>(x) < p.W)
           dst = p.C + (static_cast<int64_t>(img) * p.O + n0) * hw + static_cast<int64_t>(y) * p.W + x;
       }
-      float sum[32];
+      uint64_t sums[16];  // of two channels each
 #pragma unroll
-      for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+      for (int j = 0; j < 16; ++j) sums[j] = 0;
 #pragma unroll 1
-      for (int i = 0; i < runs; ++i) {
+      for (int i = 0; i < p.blocks * runs; ++i) {
         if (!mbar_wait_warp(tfull_bar + 8 * acc, acc_phase, abort_flag, WAIT_BUDGET)) {
           fail(MB_DEV_TIMEOUT_EPILOGUE);
           ok = false;
@@ -399,6 +415,8 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
         tc_fence_after_sync();
         const uint32_t src = tmem + lanes + acc * C::ACC_COLS + c0;
+        const uint32_t patch = nth + static_cast<uint32_t>(runs == 1 ? i : i / runs);
+        const uint64_t unscale = f32_pair(scales[patch % SCALE_SLOTS], scales[patch % SCALE_SLOTS]);
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
           uint32_t r[8], s[8];
@@ -407,18 +425,23 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           tmem_ld_wait_x8(r);
           tmem_ld_wait_x8(s);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) sum[j + k] += fmaf(__uint_as_float(s[k]), F32_LO, __uint_as_float(r[k]));
+          for (int k = 0; k < 8; k += 2) {
+            const uint64_t x = f32_fma2(f32_pair(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), f32_pair(F32_LO, F32_LO),
+                                        f32_pair(__uint_as_float(r[k]), __uint_as_float(r[k + 1])));
+            sums[(j + k) / 2] = f32_fma2(x, unscale, sums[(j + k) / 2]);
+          }
         }
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(tempty_bar + 8 * acc);
         if ((acc ^= 1) == 0) acc_phase ^= 1;
       }
-      const float unscale = scales[tile % SCALE_SLOTS];
-      float z = 0.f;
+      nth += p.blocks;
+      float z = 0.f, sum[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float x = sum[j] * unscale * __shfl_sync(0xffffffffu, w_mine, j);
+        const float2 both = f32_parts(sums[j / 2]);
+        const float x = (j % 2 == 0 ? both.x : both.y) * __shfl_sync(0xffffffffu, w_mine, j);
         z = fmaf(x, 0.f, z);
         sum[j] = x + __shfl_sync(0xffffffffu, b_mine, j);
       }
@@ -540,7 +563,7 @@ int mb_conv_f32_direct_launch(mb_context *ctx, const mb_f32_conv &g, bool *done)
   p.tiles_n = static_cast<int>(ceil_div64(p.O, bn));
   p.blocks = static_cast<int>(ceil_div64(p.C_in, KC));
   p.taps = p.KH * p.KW;
-  p.run = std::max(1, std::min(g.run, p.blocks * p.KH));
+  p.run = std::max(1, std::min(g.run, p.KH));
   p.patch_rows = patch_rows(p.W, p.KH, p.KW);
   p.act = g.act; p.max_limit = g.max_limit; p.coef = g.coef;
   p.status = ctx->dev_status;

@@ -10,7 +10,7 @@ struct mb_f32_conv {
   int KH = 3, KW = 3;  // (conv_f32_direct.cu: odd; the output is as large as the input)
   int act = 0;
   float max_limit = 0.f, coef = 0.f;
-  int run = 1;         // filter rows of 32 channels that the tensor core adds up before the sum is carried on in fp32
+  int run = 1;         // filter rows of 32 channels, KH at most, that the tensor core adds up before the sum is carried on in fp32
 };
 
 // ... and few input channels with a stride of two columns (conv_f32_stem.cu); the geometry of g plus stride, padding and output.

@@ -76,11 +76,12 @@ __device__ __forceinline__ float f32_finite_abs(float v) {
   return v < INFINITY ? v : 0.f;
 }
 
-// The scale of values that share one although they belong to several rows (the places of a convolution's tile or strip), from the
-// largest finite ones that the warps which looked at them found (all zero: 0).  It leaves less room above (2^9 instead of 2^14)
-// and more below: 2^-31 of the largest value is the smallest step, and a place may be 2^-9 of it without losing a bit.  What does
-// not fit (values that are not finite, and those beyond 2^13 times all that the other warps have) is left out: its results come
-// out as NaN and are worked out again, and the others keep their bits.
+// The scale of values that share one although they belong to several rows (the places of a convolution's patch or strip), from the
+// largest finite ones that the warps which looked at them found (all zero: 0).  It brings the largest to 2^12 .. 2^13, and is fair
+// for others whose largest comes to F32_LOW at least and stays below F32_HIGH.  A value of 2^-14 and more is then held to 22 bits,
+// 2^-22 of the largest or less.  What does not fit (values that are not finite, and those beyond 2^13 times all that the other
+// warps have) is left out: its results come out as NaN and are worked out again, and the others keep their bits.
+constexpr float F32_LOW = 256.f, F32_HIGH = 65504.f;
 template <int WARPS>
 __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
   float first = 0.f, second = 0.f;
@@ -91,7 +92,7 @@ __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
     first = fmaxf(first, m);
   }
   if (second > 0.f && first * (1.f / 8192.f) > second) first = second;
-  return first > 0.f ? f32_row_scale(first * (1.f / 32.f)) : 0.f;
+  return first > 0.f ? f32_row_scale(first * (1.f / 2048.f)) : 0.f;
 }
 
 // What a result is worked out again by: fp32 FMAs in the order of the depth, of a product's row and column ...

@@ -169,6 +169,21 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The same, with the number of those threads whose `vote` is true.
+__device__ __forceinline__ uint32_t named_bar_popc(int id, int threads, bool vote) {
+  uint32_t count;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "bar.red.popc.u32 %0, %1, %2, p;\n\t"
+      "}\n"
+      : "=r"(count)
+      : "r"(id), "r"(threads), "r"(static_cast<uint32_t>(vote))
+      : "memory");
+  return count;
+}
+
 // ---- TMA ----------------------------------------------------------------------
 
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {

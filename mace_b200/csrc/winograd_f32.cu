@@ -446,12 +446,12 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
       gather = ctx->f32_gather == 2 || cost < best;
       if (gather) best = cost;
     }
-    // (errors of 1.3e-7, 3.5e-7 and 1.4e-6 with runs of one, three and twelve filter rows)
+    // (errors of 1.3e-7 and 3.5e-7 with runs of one and three filter rows)
     mb_f32_conv d;
     d.X = in; d.filter = filter; d.bias = bias; d.out = out;
     d.N = N; d.C = C; d.H = H; d.W = W; d.O = O;
     d.act = activation; d.max_limit = max_limit; d.coef = coefficient;
-    d.run = gather || (tile == 2 && C <= 128) ? 1 : tile == 6 ? 12 : 3;
+    d.run = gather || (tile == 2 && C <= 128) ? 1 : 3;
     if (Ho == H && Wo == W && pad_top == 1 && pad_left == 1 && ctx->f32_direct != 1 && mb_conv_f32_direct_supported(ctx, d) &&
         (ctx->f32_direct == 2 ||
          (ctx->f32_gather == 0 && mb_conv_f32_direct_cost(ctx, d) < best))) {

@@ -156,6 +156,23 @@ def test_direct_conv2d_f32_scales(ctx, O, powers):
     assert np.array_equal(_run(ctx, x * b, f, None), plain * b)
 
 
+@pytest.mark.parametrize("power", [-8, 8])
+@pytest.mark.parametrize("KH", [3, 5])
+@pytest.mark.parametrize("O", [20, 100])
+def test_direct_conv2d_f32_blocks(ctx, O, KH, power):
+    """Blocks of channels of another size than the first, for which the weights make up: the same results, bit for bit, and so none of
+    them is worked out again."""
+    rng = np.random.Generator(np.random.PCG64(O))
+    x = rng.standard_normal((2, 100, 12, 70)).astype(np.float32)
+    f = (rng.standard_normal((O, 100, KH, 3)) * 0.1).astype(np.float32)
+    f = np.sign(f) * np.clip(np.abs(f), 2.0 ** -7, 0.5)  # (all of them within reach of both halves)
+    plain = _run(ctx, x, f, None)
+    for c0, c1 in ((32, 64), (96, 100)):
+        x[:, c0:c1] *= np.float32(2.0) ** power
+        f[:, c0:c1] *= np.float32(2.0) ** -power
+    assert np.array_equal(_run(ctx, x, f, None), plain)
+
+
 def test_direct_conv2d_f32_choice(ctx):
     """By rule: a batch of 3x3 and 5x5 layers, and no smaller an accuracy there than the other kernels have."""
     rng = np.random.Generator(np.random.PCG64(0))
