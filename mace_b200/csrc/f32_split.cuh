@@ -1,19 +1,18 @@
 // fp32 operands as pairs of half-precision numbers for tcgen05.mma kind::f16.
 //
-// v * s = hi + 2^-11 lo with s a power of two that brings the largest value of a row to 2 .. 4 (a row: what shares one index of the
-// result, a pixel's or an output channel's values over the depth): hi is v * s rounded to 11 bits, lo the rest rounded to
-// 11 bits, together 22 bits and a sign, or 2^-36 absolute where that is more, 2^-37 of the row's largest value.  (At the scale of hi,
-// lo would end at 2^-25: values below 2^-12 of the row's largest lost bits, which shows where small values meet large ones of the
-// other operand: 6e-6 instead of 8e-8 with a column of X times 1000 and W's divided by it.)  Three MMAs, hi * hi in one fp32
+// v * s = hi + 2^-11 lo with s a power of two that brings the largest value of a row to 2^14 .. 2^15, where it is known (a row: what
+// shares one index of the result, a pixel's or an output channel's values over the depth): hi is v * s rounded to 11 bits, lo the rest
+// rounded to 11 bits, together 22 bits and a sign, or 2^-36 absolute where that is more, below 2^-28 of the row's largest value.  (At
+// the scale of hi, lo would end at 2^-25; and with the largest at 2 .. 4 values below 2^-12 of it lost bits, which shows where small
+// values meet large ones of the other operand: 6e-6 instead of 8e-8 with a column of X times 1000 and W's divided by it.)  Three MMAs, hi * hi in one fp32
 // accumulator and hi * lo + lo * hi in another; the second one's 2^-11 and the two inverse powers of two are exact.
 //
 // Against tf32 pairs (11 + 11 bits cut off, as many MMAs): an operand takes half the bytes in shared and tensor memory and
 // an MMA covers 16 of the depth in the time of 8.  Those kernels were bound by shared memory: 144 KB per step of 128 x 128 x 32
 // at 128 bytes a cycle, 1150 cycles of which the MMAs were busy 768; 72 KB and 384 cycles now.
 //
-// A row's scale is that of the first step of 32 in which it has a value other than zero (zeros need none), so that nothing has
-// to be read twice.  Later values may be 2^14 times larger; beyond that hi is infinite and the results of that row come out as
-// NaN, like those of an infinite value, and are marked, and worked out again by fp32 FMAs.
+// Where a row's largest value is not known beforehand its scale is one that the values at hand allow, and follows them when they
+// grow.  Results of an infinite value come out as NaN, and are marked, and worked out again by fp32 FMAs.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -22,12 +21,14 @@
 
 constexpr uint32_t F32_AGAIN = 0x7fc0a6a1u;  // stored for a result to be worked out again
 
-// The scale of a row whose largest value is m > 0: at least 2^-126 and at most 2^126, so that its inverse is a normal number too.
-// (Rows below 2^-125 stay below 2, but have no bits that lo does not hold.)
+// The scale that brings a row's largest value m > 0 to 2^TOP .. 2^(TOP + 1): at most 2^126, so that its inverse is a normal number
+// too.  (Rows that it leaves smaller are below 2^-111 and have no bits that lo does not hold.)
+template <int TOP = 14>
 __device__ __forceinline__ float f32_row_scale(float m) {
-  const uint32_t e = __float_as_uint(m) >> 23;  // biased; the scale's is 254 - e + 1
-  return __uint_as_float(min(255u - min(e, 254u), 253u) << 23);
+  const uint32_t e = __float_as_uint(m) >> 23;  // biased; the scale's is 254 - e + TOP
+  return __uint_as_float(min(254u + TOP - min(e, 254u), 253u) << 23);
 }
+constexpr float F32_HIGH = 65504.f;  // what no value times its scale may reach
 // What a result is multiplied by: 1 / s, 0 for a row of zeros only (its scale is still 0).  X's and W's one after the other: their
 // product may leave the range of fp32 where the result does not.
 __device__ __forceinline__ float f32_row_unscale(float s) {
@@ -81,7 +82,7 @@ __device__ __forceinline__ float f32_finite_abs(float v) {
 // for others whose largest comes to F32_LOW at least and stays below F32_HIGH.  A value of 2^-14 and more is then held to 22 bits,
 // 2^-22 of the largest or less.  What does not fit (values that are not finite, and those beyond 2^13 times all that the other
 // warps have) is left out: its results come out as NaN and are worked out again, and the others keep their bits.
-constexpr float F32_LOW = 256.f, F32_HIGH = 65504.f;
+constexpr float F32_LOW = 256.f;
 template <int WARPS>
 __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
   float first = 0.f, second = 0.f;
@@ -92,7 +93,7 @@ __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
     first = fmaxf(first, m);
   }
   if (second > 0.f && first * (1.f / 8192.f) > second) first = second;
-  return first > 0.f ? f32_row_scale(first * (1.f / 2048.f)) : 0.f;
+  return first > 0.f ? f32_row_scale<12>(first) : 0.f;
 }
 
 // What a result is worked out again by: fp32 FMAs in the order of the depth, of a product's row and column ...

@@ -431,7 +431,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
           float most = 0.f;
 #pragma unroll
           for (int k = 0; k < 16; ++k) most = fmaxf(most, fmaxf(fabsf(v[k]), fabsf(other[k * FBM])));
-          if (scale == 0.f && most > 0.f) scale = f32_row_scale(most);
+          if (scale == 0.f && most > 0.f) scale = f32_row_scale<4>(most);
           if (half == 0) x_unscale[(tile % F_SCALE_SLOTS) * FBM + quarter * 32 + lane] = f32_row_unscale(scale);
           known = __all_sync(0xffffffffu, scale != 0.f || !inside);
         }

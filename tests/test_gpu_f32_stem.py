@@ -114,7 +114,7 @@ def test_conv_f32_stem_beyond_the_split(ctx, what):
             assert (np.abs(got - ref) <= tight)[:, :, far].all()
 
 
-@pytest.mark.parametrize("spread", [2.0 ** 8, 2.0 ** 12])
+@pytest.mark.parametrize("spread", [2.0 ** 10, 2.0 ** 20])
 def test_conv_f32_stem_spread(ctx, spread):
     """Small values that meet large weights keep their bits, and so do dark regions beside bright ones."""
     rng = np.random.Generator(np.random.PCG64(6))
