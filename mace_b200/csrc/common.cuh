@@ -41,6 +41,7 @@ struct mb_context {
   // W of fp32 products split in front of them (gemm_f32_pairs.cu, conv_f32_direct.cu); blocks that a recorded graph may refer to are kept
   void *weight_scratch = nullptr;
   size_t weight_scratch_bytes = 0;
+  size_t weight_scratch_refused = SIZE_MAX;  // a size that could not be had: not asked for again before something has been freed
   std::vector<void *> weight_scratch_kept;
   bool captured_any = false;   // a graph has been recorded on this context
   int f32_pairs = 0;           // gemm_f32_pairs.cu: 0 by rule, 1 never, 2 wherever it can run
@@ -130,7 +131,9 @@ int mb_check_cuda(mb_context *ctx, cudaError_t e, const char *what);
 // growing the arena if needed.  offset allows several carve-outs per call.
 int mb_scratch(mb_context *ctx, size_t bytes, void **ptr);
 // Another such arena, for a call that may run inside one that has carved the first.  *ptr is null where it would have to grow
-// inside a graph capture: the caller then does without.  Never freed before the context once a graph may refer to it.
+// inside a graph capture or there is no memory: the caller then does without.  Never freed before the context once a graph may
+// refer to it.
+constexpr size_t WEIGHT_SCRATCH_BYTES = 256u << 20;  // what is asked of it at most
 int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr);
 
 // ---- programmatic dependent launch ------------------------------------------------------------

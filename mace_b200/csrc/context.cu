@@ -48,18 +48,29 @@ int mb_scratch(mb_context *ctx, size_t bytes, void **ptr) {
 int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr) {
   *ptr = nullptr;
   if (bytes > ctx->weight_scratch_bytes) {
-    if (ctx->capturing) return MB_SUCCESS;
-    const size_t want = align_up(bytes + bytes / 2, 1 << 20);  // (so few blocks, each half as large again, are ever kept)
-    void *block = nullptr;
-    if (ctx->captured_any) ctx->weight_scratch_kept.reserve(ctx->weight_scratch_kept.size() + 1);
+    if (ctx->capturing || bytes >= ctx->weight_scratch_refused) return MB_SUCCESS;
     MB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    MB_CUDA(ctx, cudaMalloc(&block, want));
-    if (ctx->weight_scratch != nullptr) {
-      if (ctx->captured_any) ctx->weight_scratch_kept.push_back(ctx->weight_scratch);
-      else cudaFree(ctx->weight_scratch);
+    if (!ctx->captured_any && ctx->weight_scratch != nullptr) {
+      cudaFree(ctx->weight_scratch);
+      ctx->weight_scratch = nullptr;
+      ctx->weight_scratch_bytes = 0;
     }
-    ctx->weight_scratch = block;
-    ctx->weight_scratch_bytes = want;
+    // half as large again, so that few blocks are ever taken, or where that is not left what was asked for
+    void *block = nullptr;
+    for (const size_t want : {align_up(bytes + bytes / 2, 1 << 20), align_up(bytes, 256)}) {
+      if (mb_should_mock_runtime_failure() || cudaMalloc(&block, want) != cudaSuccess) {
+        cudaGetLastError();  // (the caller does without)
+        continue;
+      }
+      if (ctx->weight_scratch != nullptr) ctx->weight_scratch_kept.push_back(ctx->weight_scratch);
+      ctx->weight_scratch = block;
+      ctx->weight_scratch_bytes = want;
+      break;
+    }
+    if (block == nullptr) {
+      ctx->weight_scratch_refused = bytes;
+      return MB_SUCCESS;
+    }
   }
   *ptr = ctx->weight_scratch;
   return MB_SUCCESS;
@@ -243,6 +254,7 @@ int mb_malloc(mb_context *ctx, size_t bytes, void **dptr) {
 int mb_free(mb_context *ctx, void *dptr) {
   if (ctx == nullptr) return MB_INVALID_ARGS;
   if (dptr == nullptr) return MB_SUCCESS;
+  ctx->weight_scratch_refused = SIZE_MAX;
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
   MB_CUDA(ctx, cudaFree(dptr));
   return MB_SUCCESS;

@@ -530,7 +530,8 @@ bool mb_conv_f32_direct_supported(const mb_context *ctx, const mb_f32_conv &g) {
   if (g.KH % 2 == 0 || g.KW % 2 == 0 || g.KH > 7 || g.KW > 7) return false;
   const int64_t image = (g.H + g.KH / 2) * (g.W + g.KW / 2);
   if (g.W >= (1 << 14) || g.H >= (1 << 14) || g.N * image >= (1ll << 31) - 4096) return false;
-  if (g.C >= (1 << 20) || g.O >= (1 << 20) || g.C * g.O * g.KH * g.KW >= (1ll << 29)) return false;
+  if (g.C >= (1 << 20) || g.O >= (1 << 20) || ceil_div64(g.C, KC) * KC * g.O * g.KH * g.KW * 4 > static_cast<int64_t>(WEIGHT_SCRATCH_BYTES))
+    return false;
   const int bn = g.O > 64 ? 128 : 64;
   if (ceil_div64(g.N * image, BM) * ceil_div64(g.O, bn) >= (1ll << 30)) return false;
   return 2 * 1024 + 2 * patch_rows(g.W, g.KH, g.KW) * 128 + 2 * g.KW * bn * 128 <= 227 * 1024;
@@ -548,7 +549,7 @@ int64_t mb_conv_f32_direct_cost(const mb_context *ctx, const mb_f32_conv &g) {
   return 15000 + g.C * g.O * g.KH * g.KW / 200 + rounds * std::max(steps, input);
 }
 
-// *done is false where the filter's split has no room (inside a graph capture): nothing has been launched then.
+// *done is false where the filter's split has no room (see mb_weight_scratch): nothing has been launched then.
 int mb_conv_f32_direct_launch(mb_context *ctx, const mb_f32_conv &g, bool *done) {
   *done = false;
   Params p = {};

@@ -21,5 +21,5 @@ int mb_conv_f32_stem_launch(mb_context *ctx, const mb_f32_conv &g, int sh, int p
 bool mb_conv_f32_direct_supported(const mb_context *ctx, const mb_f32_conv &g);
 // Estimated time in SM cycles.
 int64_t mb_conv_f32_direct_cost(const mb_context *ctx, const mb_f32_conv &g);
-// *done is false where nothing was launched, for want of room for the split filter inside a graph capture.
+// *done is false where nothing was launched, for want of room for the split filter (see mb_weight_scratch).
 int mb_conv_f32_direct_launch(mb_context *ctx, const mb_f32_conv &g, bool *done);

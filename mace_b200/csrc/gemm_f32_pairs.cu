@@ -43,7 +43,6 @@ constexpr int F_THREADS = (FIRST_STORE + 2) * 32;
 constexpr long long F_WAIT_BUDGET = 1ll << 31;
 // Scales of so many tiles: X is at most F32Cfg::STAGES tiles of one step ahead of the MMAs, these are two ahead of the epilogue.
 constexpr int F_SCALE_SLOTS = 16;
-constexpr size_t SPLIT_BYTES = 256u << 20;  // of W at most
 constexpr int F_BUFS = 4;      // result buffers per set, 16 channels x 128 pixels each
 
 struct F32TcParams {
@@ -740,7 +739,7 @@ bool mb_gemm_f32_pairs_pays(const mb_context *ctx, int64_t batch, int64_t Mdim, 
   return (steps - 60) * 400 > (w_batched ? batch : 1) * Ndim * K * 8 / 1700;
 }
 
-// *done is false where nothing was launched, for want of room for the split W.
+// *done is false where nothing was launched, for want of room for the split W (see mb_weight_scratch).
 int mb_gemm_f32_pairs_launch(mb_context *ctx, const float *X, const float *W, const float *bias, float *C,
                           int64_t batch, int64_t Mdim, int64_t Ndim, int64_t K, int64_t x_row_stride,
                           int64_t x_batch_stride, int64_t w_row_stride, int64_t w_batch_stride,
@@ -775,7 +774,7 @@ int mb_gemm_f32_pairs_launch(mb_context *ctx, const float *X, const float *W, co
   }
   const int64_t w_rows = Ndim * (p.w_batched ? batch : 1);
   const size_t split_bytes = static_cast<size_t>(w_rows) * p.k_blocks * 128;
-  if (w_rows >= (1ll << 31) || split_bytes > SPLIT_BYTES) return MB_SUCCESS;
+  if (w_rows >= (1ll << 31) || split_bytes > WEIGHT_SCRATCH_BYTES) return MB_SUCCESS;
   uint8_t *split = nullptr;
   MB_RETURN_IF_ERROR(mb_weight_scratch(ctx, align_up(split_bytes, 256) + w_rows * 4, reinterpret_cast<void **>(&split)));
   if (split == nullptr) return MB_SUCCESS;

@@ -105,3 +105,37 @@ def test_allocator_failures_come_out_of_the_net_and_the_engine_recovers(orc):
             assert np.array_equal(got.reshape(2, 1000), mn.oracle_forward(orc, layers, xin))
     finally:
         L.mb_set_runtime_failure_ratio(0.0)
+
+
+@pytest.mark.parametrize("option", ["f32_pairs", "f32_direct"])
+def test_no_memory_for_split_weights_is_another_kernel_not_an_error(option):
+    """fp32 products whose kernel keeps a split form of the weights, where there is no memory for it."""
+    import mace_b200
+    L = mace_b200.lib()
+    ctx = mace_b200.Context(0)
+    rng = np.random.Generator(np.random.PCG64(5))
+    k = 1 if option == "f32_pairs" else 3
+    x = rng.standard_normal((1, 64, 16, 8)).astype(np.float32)
+    f = (rng.standard_normal((64, 64, k, k)) * 0.1).astype(np.float32)
+    dx, df, do = ctx.upload(x), ctx.upload(f), ctx.alloc(64 * 128 * 4)
+
+    def call():
+        before = ctx.launches
+        ctx.conv2d_f32(dx, df, None, do, 1, 64, 16, 8, 64, k, k, (1, 1), (1, 1), (k // 2, k // 2), (16, 8))
+        return ctx.launches - before, ctx.download(do, (64, 128), np.float32)
+
+    exact = call()[1]  # (too small for a kernel that splits weights in front)
+    try:
+        ctx.set_option("f32_gather", 1)
+        ctx.set_option(option, 2)
+        assert L.mb_set_runtime_failure_ratio(1.0) == 0
+        for _ in range(2):
+            assert np.abs(call()[1] - exact).max() <= 1e-5 * np.abs(exact).max()
+        assert L.mb_set_runtime_failure_ratio(0.0) == 0
+        ctx.upload(x).free()  # (something has been freed: the memory is asked for again)
+        launches, got = call()
+        assert launches == 2 and np.abs(got - exact).max() <= 1e-5 * np.abs(exact).max()
+        ctx.sync()
+    finally:
+        L.mb_set_runtime_failure_ratio(0.0)
+        ctx.close()
