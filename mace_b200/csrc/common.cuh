@@ -130,9 +130,8 @@ int mb_check_cuda(mb_context *ctx, cudaError_t e, const char *what);
 // Returns a device pointer to at least `bytes` of scratch (256-byte aligned),
 // growing the arena if needed.  offset allows several carve-outs per call.
 int mb_scratch(mb_context *ctx, size_t bytes, void **ptr);
-// Another such arena, for a call that may run inside one that has carved the first.  *ptr is null where it would have to grow
-// inside a graph capture or there is no memory: the caller then does without.  Never freed before the context once a graph may
-// refer to it.
+// Another such arena, for a call that may run inside one that has carved the first; it grows inside a graph capture too.  *ptr is
+// null where there is no memory: the caller then does without.  Never freed before the context once a graph may refer to it.
 constexpr size_t WEIGHT_SCRATCH_BYTES = 256u << 20;  // what is asked of it at most
 int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr);
 

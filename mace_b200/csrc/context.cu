@@ -48,15 +48,19 @@ int mb_scratch(mb_context *ctx, size_t bytes, void **ptr) {
 int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr) {
   *ptr = nullptr;
   if (bytes > ctx->weight_scratch_bytes) {
-    if (ctx->capturing || bytes >= ctx->weight_scratch_refused) return MB_SUCCESS;
-    MB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (bytes >= ctx->weight_scratch_refused) return MB_SUCCESS;
     if (!ctx->captured_any && ctx->weight_scratch != nullptr) {
+      MB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
       cudaFree(ctx->weight_scratch);
       ctx->weight_scratch = nullptr;
       ctx->weight_scratch_bytes = 0;
     }
     // half as large again, so that few blocks are ever taken, or where that is not left what was asked for
     void *block = nullptr;
+    // (While this thread records a graph memory is had in the relaxed mode only.  Without it a call's kernel, and the rounding of its
+    // results, would depend on the calls before the recording.)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (ctx->capturing) MB_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
     for (const size_t want : {align_up(bytes + bytes / 2, 1 << 20), align_up(bytes, 256)}) {
       if (mb_should_mock_runtime_failure() || cudaMalloc(&block, want) != cudaSuccess) {
         cudaGetLastError();  // (the caller does without)
@@ -67,6 +71,7 @@ int mb_weight_scratch(mb_context *ctx, size_t bytes, void **ptr) {
       ctx->weight_scratch_bytes = want;
       break;
     }
+    if (ctx->capturing) MB_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
     if (block == nullptr) {
       ctx->weight_scratch_refused = bytes;
       return MB_SUCCESS;

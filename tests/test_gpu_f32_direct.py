@@ -186,8 +186,7 @@ def test_direct_conv2d_f32_choice(ctx):
 
 
 def test_direct_conv2d_f32_inside_a_capture(ctx):
-    """A first call inside a capture has no room for the split filter and takes another kernel; one after a call outside
-    keeps its block although later calls need a larger one."""
+    """A graph keeps the block of its split filter although later calls need a larger one."""
     import mace_b200
     c = mace_b200.Context(0)
     rng = np.random.Generator(np.random.PCG64(1))
@@ -221,6 +220,44 @@ def test_direct_conv2d_f32_inside_a_capture(ctx):
         c._check(L.mb_graph_launch(c.h, g))
         check()
         c._check(L.mb_graph_destroy(c.h, g))
+    c.close()
+
+
+def test_direct_conv2d_f32_first_inside_a_capture():
+    """The same bits whether or not calls before the recording left room for the split filters."""
+    import mace_b200
+    c = mace_b200.Context(0)
+    L = mace_b200.lib()
+    rng = np.random.Generator(np.random.PCG64(2))
+    layers = []
+    for C, O in ((32, 64), (256, 256)):  # (the second one's block is a larger one)
+        x, f = rng.standard_normal((2, C, 12, 12)).astype(np.float32), rng.standard_normal((O, C, 3, 3)).astype(np.float32)
+        layers.append((c.upload(x), c.upload(f), c.alloc(2 * O * 144 * 4), C, O))
+
+    def calls():
+        for x, f, out, C, O in layers:
+            c.conv2d_f32(x, f, None, out, 2, C, 12, 12, O, 3, 3, (1, 1), (1, 1), (1, 1), (12, 12))
+
+    def results():
+        got = [c.download(out, (2, O, 144), np.float32) for _, _, out, _, O in layers]
+        for layer in layers:
+            c._check(L.mb_memset(c.h, layer[2].ptr, 0, layer[2].nbytes))
+        return got
+
+    c.set_option("f32_direct", 2)
+    c._check(L.mb_graph_begin(c.h))
+    calls()
+    g = ctypes.c_void_p()
+    c._check(L.mb_graph_end(c.h, ctypes.byref(g)))
+    c._check(L.mb_graph_launch(c.h, g))
+    recorded = results()
+    calls()
+    for a, b in zip(recorded, results()):
+        assert np.array_equal(a, b)
+    c._check(L.mb_graph_launch(c.h, g))
+    for a, b in zip(recorded, results()):
+        assert np.array_equal(a, b)
+    c._check(L.mb_graph_destroy(c.h, g))
     c.close()
 
 
