@@ -179,6 +179,11 @@ static inline cudaError_t mb_launch_chained(mb_context *ctx, void (*kern)(KArgs.
 #define MB_CUDA(ctx, expr) MB_RETURN_IF_ERROR(mb_check_cuda((ctx), (expr), #expr))
 
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
+// Whether two stretches of memory of so many bytes have one in common (null: no).
+static inline bool mb_ranges_meet(const void *a, const void *b, int64_t bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b), n = static_cast<uintptr_t>(bytes);
+  return a != nullptr && b != nullptr && (x < y ? y - x : x - y) < n;
+}
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Division of a dividend below 2^31 by a divisor fixed at launch: with s = ceil(log2 d) and

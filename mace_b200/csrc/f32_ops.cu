@@ -719,6 +719,8 @@ int mb_conv2d_f32_nchw_residual(mb_context *ctx, const float *in, const float *f
                                  activation, max_limit, coefficient, residual);
   }
   // every other shape: the convolution without activation, then sum + activation in place
+  if (mb_ranges_meet(residual, out, N * O * Ho * Wo * 4))
+    return mb_fail(ctx, MB_UNSUPPORTED, "mb_conv2d_f32_nchw_residual: the residual lies in the output, which is written before the sum");
   MB_RETURN_IF_ERROR(mb_conv2d_f32_nchw(ctx, in, filter, bias, out, N, C, H, W, O, KH, KW, stride_h, stride_w,
                                         dil_h, dil_w, pad_top, pad_left, Ho, Wo, 0, 0.f, 0.f));
   return mb_eltwise_act_f32(ctx, out, residual, out, N * O * Ho * Wo, 0, 0.f, 0, 0.f, 0.f, 0, activation,

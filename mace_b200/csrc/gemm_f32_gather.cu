@@ -831,7 +831,8 @@ int mb_gemm_f32_gather_launch(mb_context *ctx, const mb_f32_gemm &g) {
   p.k_blocks = static_cast<int>(ceil_div64(g.K, KB));
   p.splits = plan.splits;
   p.run = plan.bn == 128 ? std::min(g.run, 2) : g.run;  // (of the four steps that its ring holds)
-  p.exact = g.run != 0;
+  // (a residual that lies where the results do is gone by then)
+  p.exact = g.run != 0 && !mb_ranges_meet(g.residual, g.C, g.batch * g.M * g.N * 4);
   p.x_ks = g.x_ks; p.x_ms = g.x_ms; p.x_bs = g.x_bs;
   p.w_ns = g.w_ns; p.w_ks = g.w_ks; p.w_bs = g.w_bs;
   p.c_ns = g.c_ns; p.c_ms = g.c_ms; p.c_bs = g.c_bs;

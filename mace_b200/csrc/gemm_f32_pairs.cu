@@ -739,13 +739,15 @@ bool mb_gemm_f32_pairs_pays(const mb_context *ctx, int64_t batch, int64_t Mdim, 
   return (steps - 60) * 400 > (w_batched ? batch : 1) * Ndim * K * 8 / 1700;
 }
 
-// *done is false where nothing was launched, for want of room for the split W (see mb_weight_scratch).
+// *done is false where nothing was launched: the residual lies in C, or there is no room for the split W (see mb_weight_scratch).
 int mb_gemm_f32_pairs_launch(mb_context *ctx, const float *X, const float *W, const float *bias, float *C,
                           int64_t batch, int64_t Mdim, int64_t Ndim, int64_t K, int64_t x_row_stride,
                           int64_t x_batch_stride, int64_t w_row_stride, int64_t w_batch_stride,
                           int64_t c_row_stride, int64_t c_batch_stride, int act, float max_limit,
                           float coef, const float *residual, bool *done) {
   *done = false;
+  // A result that is worked out again needs its residual once more, which must not lie where the first one was stored.
+  if (mb_ranges_meet(residual, C, ((batch - 1) * c_batch_stride + (Ndim - 1) * c_row_stride + Mdim) * 4)) return MB_SUCCESS;
   const int BN = Ndim > 64 ? 128 : 64;
   F32TcParams p = {};
   p.X = X; p.W = W;
