@@ -12,7 +12,8 @@
 // at 128 bytes a cycle, 1150 cycles of which the MMAs were busy 768; 72 KB and 384 cycles now.
 //
 // Where a row's largest value is not known beforehand its scale is one that the values at hand allow, and follows them when they
-// grow.  Results of an infinite value come out as NaN, and are marked, and worked out again by fp32 FMAs.
+// grow, or the tile is done once more.  Results of an infinite value come out as NaN, and are marked, and worked out again by fp32
+// FMAs.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -99,6 +100,7 @@ __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
 // What a result is worked out again by: fp32 FMAs in the order of the depth, of a product's row and column ...
 __device__ __forceinline__ float f32_chain(const float *x, int64_t x_ks, const float *w, int64_t K) {
   float sum = 0.f;
+#pragma unroll 16  // (so many loads on their way)
   for (int64_t k = 0; k < K; ++k) sum = fmaf(x[k * x_ks], w[k], sum);
   return sum;
 }

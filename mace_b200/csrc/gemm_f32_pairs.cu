@@ -13,9 +13,13 @@
 // What bounds it: shared memory at 128 bytes a cycle and the clocks that the power limit leaves.  A step of 128 x 128 x 32 moves
 // 16 KB of X in and out, 16 KB of W in and 24 KB into the MMAs: 576 cycles, of which the MMAs are busy 384 (tf32 pairs split
 // in the kernel: 144 KB, 1150 cycles, 768 busy; 750 measured now).  A tile of few steps is bound by HBM.
-// Measured, tf32 pairs -> this kernel (1x1 convolutions, batch 256, us): 64 -> 256 channels at 56 x 56 254 -> 234, 256 -> 64 218 ->
-// 186, 512 -> 128 at 28 x 28 150 -> 120, 128 -> 512 175 -> 155, 256 -> 1024 at 14 x 14 165 -> 130, 1024 -> 256 151 -> 114, 512 ->
-// 1024 302 -> 223.
+// Measured, tf32 pairs -> this kernel (1x1 convolutions, batch 256, us; in brackets with a residual): 64 -> 256 channels at 56 x 56
+// 220 -> 226 (394 -> 346), 256 -> 64 214 -> 180, 512 -> 128 at 28 x 28 148 -> 128, 128 -> 512 170 -> 148 (258 -> 206), 256 -> 1024 at
+// 14 x 14 156 -> 139 (194 -> 154), 1024 -> 256 147 -> 123, 1024 -> 512 282 -> 227.
+//
+// A row of X has the scale of its first step that has a value.  Where a later one is beyond 2^11 times that the row's results are no
+// finite numbers; the tiles that have some are marked, and a second pass over them has scales from all of a row.  512 -> 128 at
+// 28 x 28 with channels 2^14 times larger from the 32nd on: in all pixels 497 us (7170 by FMAs), in one of 1000 233 (1863).
 //
 // Structure (one persistent CTA per SM):
 //   warp 0        TMA producer: X as one [32 k x 128 m] box (no swizzle) and a step of W, mbarrier ring
@@ -43,6 +47,7 @@ constexpr int F_THREADS = (FIRST_STORE + 2) * 32;
 constexpr long long F_WAIT_BUDGET = 1ll << 31;
 // Scales of so many tiles: X is at most F32Cfg::STAGES tiles of one step ahead of the MMAs, these are two ahead of the epilogue.
 constexpr int F_SCALE_SLOTS = 16;
+constexpr int MARKS = 512;     // tiles of a CTA with a mark of their own (of results that are no finite numbers)
 constexpr int F_BUFS = 4;      // result buffers per set, 16 channels x 128 pixels each
 
 struct F32TcParams {
@@ -73,7 +78,7 @@ struct F32Cfg {
   static constexpr int STAGING_BYTES = 2 * F_BUFS * BUF_BYTES;
   static constexpr int XSCALE_BYTES = F_SCALE_SLOTS * FBM * 4;
   static constexpr int UB_BYTES = F_EPI_WARPS * (BN / 2) * 8;  // (1 / scale, bias) of the channels of an epilogue warp
-  static constexpr int BAR_BYTES = 512;
+  static constexpr int BAR_BYTES = 512 + 2 * MARKS;
   static constexpr int FIXED = STAGING_BYTES + XSCALE_BYTES + UB_BYTES + BAR_BYTES + 1024;
   static constexpr int NUM_ACC = 2;
   static constexpr int TMEM_COLS = 512;
@@ -88,36 +93,46 @@ struct F32Cfg {
   static_assert(STAGES >= 2, "pipeline needs two stages");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + FIXED;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-  static_assert(3 * STAGES * 8 + 2 * NUM_ACC * 8 + 4 * F_BUFS * 8 + 8 + 16 <= BAR_BYTES, "barrier area");
+  static constexpr int BARRIERS = 3 * STAGES + 2 * NUM_ACC + 4 * F_BUFS + 1;
+  static_assert(8 * BARRIERS + 2 * MARKS + 16 <= BAR_BYTES, "barriers, marks, flags");
 };
 
-// Column tiles first: the CTAs that read one tile of X run side by side and fetch it from HBM once.
+// Column tiles first: the CTAs that read one tile of X run side by side and fetch it from HBM once.  With `only` the CTA's nth tiles
+// that are marked there (the nth + i * MARKS ones with them).
 struct FTileIter {
-  int tm, tn, b;
-  __device__ __forceinline__ FTileIter(const F32TcParams &p) {
+  int tm, tn, b, nth = 0;
+  const volatile uint8_t *only;
+  __device__ __forceinline__ FTileIter(const F32TcParams &p, const volatile uint8_t *marked = nullptr) : only(marked) {
     const unsigned t = blockIdx.x;
     tn = t % p.tiles_n;
     const unsigned q = t / p.tiles_n;
     tm = q % p.tiles_m;
     b = q / p.tiles_m;
+    skip(p);
   }
   __device__ __forceinline__ bool valid(const F32TcParams &p) const { return b < p.batch; }
   __device__ __forceinline__ void next(const F32TcParams &p) {
+    step(p);
+    skip(p);
+  }
+
+ private:
+  __device__ __forceinline__ void step(const F32TcParams &p) {
+    ++nth;
     tm += p.step_m;
     tn += p.step_n;
     b += p.step_b;
     if (tn >= p.tiles_n) { tn -= p.tiles_n; ++tm; }
     if (tm >= p.tiles_m) { tm -= p.tiles_m; ++b; }
   }
+  __device__ __forceinline__ void skip(const F32TcParams &p) {
+    if (only == nullptr) return;
+    while (valid(p) && only[nth % MARKS] == 0) step(p);
+  }
 };
 
-// Tiles of this CTA.
-__device__ __forceinline__ int my_tiles(const F32TcParams &p) {
-  return static_cast<int>((p.batch * p.tiles_m * p.tiles_n - blockIdx.x + gridDim.x - 1) / gridDim.x);
-}
-
-// A result that came out of the tensor core as no finite number (see f32_split.cuh) is stored as F32_AGAIN; when its tiles are done
-// a CTA that stored one works those out again, by fp32 FMAs in the order of k.
+// A result that the second pass has as no finite number either is stored as F32_AGAIN; when its tiles are done a CTA that stored
+// one works those out again, by fp32 FMAs in the order of k.
 __device__ __noinline__ void tile_again(const F32TcParams &p, int m0, int n0, int bn, int b) {
   for (int i = threadIdx.x; i < FBM * bn; i += blockDim.x) {
     const int64_t m = m0 + (i & (FBM - 1)), n = n0 + i / FBM;
@@ -184,52 +199,44 @@ f32_presplit_kernel(const float *W, uint8_t *dst, float *unscale, int64_t rows, 
   }
 }
 
-// EPI selects the epilogue's arithmetic: 0 = the accumulator is the result (the Winograd products); 1 = bias and a clamp
-// (NOOP / RELU / RELUX), 2 = with a residual too; 3 and 4 = the same with the leaky term.
-template <int BN, int EPI>
-__global__ void __launch_bounds__(F_THREADS, 1)
-gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
-                   const __grid_constant__ CUtensorMap tmap_w,
-                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
-                   const __grid_constant__ F32TcParams p) {
+// Where what lies in shared memory behind the stages.
+template <int BN>
+struct FShared {
   using Cfg = F32Cfg<BN>;
-  constexpr int STAGES = Cfg::STAGES;
-  constexpr int NUM_ACC = Cfg::NUM_ACC;
-  constexpr bool RES = EPI == 2 || EPI == 4, LEAKY = EPI >= 3;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t *smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
-  constexpr int STAGING_AT = STAGES * Cfg::STAGE_BYTES, XSCALE_AT = STAGING_AT + Cfg::STAGING_BYTES;
-  constexpr int UB_AT = XSCALE_AT + Cfg::XSCALE_BYTES, BAR_AT = UB_AT + Cfg::UB_BYTES;
-  float *x_unscale = reinterpret_cast<float *>(smem_aligned + XSCALE_AT);  // [F_SCALE_SLOTS][FBM]
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem_aligned + BAR_AT);
-  const uint32_t full_bar = smem_u32(bars);              // [STAGES] raw tiles landed
-  const uint32_t split_bar = full_bar + 8 * STAGES;      // [STAGES] hi/lo ready
-  const uint32_t empty_bar = split_bar + 8 * STAGES;     // [STAGES] stage consumed
-  const uint32_t tfull_bar = empty_bar + 8 * STAGES;     // [NUM_ACC] accumulator complete
-  const uint32_t tempty_bar = tfull_bar + 8 * NUM_ACC;   // [NUM_ACC] accumulator drained
-  const uint32_t free_bar = tempty_bar + 8 * NUM_ACC;    // [2][F_BUFS] result buffer free, its residual landed
-  const uint32_t ready_bar = free_bar + 8 * 2 * F_BUFS;  // [2][F_BUFS] result buffer written
-  const uint32_t sempty_bar = ready_bar + 8 * 2 * F_BUFS;  // accumulator of the small products drained (128 channels)
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * STAGES + 2 * NUM_ACC + 4 * F_BUFS + 1);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  volatile int *again = abort_flag + 1;
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  mb_grid_dep_launch();  // the kernel behind this one may start its own prologue
-
-  if (threadIdx.x == 0) {
-    prefetch_tensormap(&tmap_x);
-    prefetch_tensormap(&tmap_w);
-    if (p.c_tma) prefetch_tensormap(&tmap_c);
-    if (RES && p.c_tma) prefetch_tensormap(&tmap_r);
-    for (int s = 0; s < STAGES; ++s) {
+  static constexpr int STAGING_AT = Cfg::STAGES * Cfg::STAGE_BYTES, XSCALE_AT = STAGING_AT + Cfg::STAGING_BYTES;
+  static constexpr int UB_AT = XSCALE_AT + Cfg::XSCALE_BYTES, BAR_AT = UB_AT + Cfg::UB_BYTES;
+  uint8_t *base;             // 1024-byte aligned
+  uint32_t base_u32;
+  uint32_t full_bar, split_bar, empty_bar;  // [STAGES] raw tiles landed, hi/lo ready, stage consumed
+  uint32_t tfull_bar, tempty_bar;           // [NUM_ACC] accumulator complete, drained
+  uint32_t free_bar, ready_bar;             // [2][F_BUFS] result buffer free (its residual landed), written
+  uint32_t sempty_bar;                      // accumulator of the small products drained (128 channels)
+  volatile uint8_t *marks;   // [2][MARKS] tiles with a result that is no finite number, of the first pass and the second
+  uint32_t *tmem_slot;
+  volatile int *abort_flag, *again;         // again: [2] any such tile
+  __device__ __forceinline__ explicit FShared(uint8_t *raw) {
+    base_u32 = (smem_u32(raw) + 1023u) & ~1023u;
+    base = raw + (base_u32 - smem_u32(raw));
+    full_bar = base_u32 + BAR_AT;
+    split_bar = full_bar + 8 * Cfg::STAGES;
+    empty_bar = split_bar + 8 * Cfg::STAGES;
+    tfull_bar = empty_bar + 8 * Cfg::STAGES;
+    tempty_bar = tfull_bar + 8 * Cfg::NUM_ACC;
+    free_bar = tempty_bar + 8 * Cfg::NUM_ACC;
+    ready_bar = free_bar + 8 * 2 * F_BUFS;
+    sempty_bar = ready_bar + 8 * 2 * F_BUFS;
+    marks = base + BAR_AT + 8 * Cfg::BARRIERS;
+    tmem_slot = reinterpret_cast<uint32_t *>(base + BAR_AT + 8 * Cfg::BARRIERS + 2 * MARKS);
+    abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    again = abort_flag + 1;
+  }
+  __device__ __forceinline__ void init_barriers() const {
+    for (int s = 0; s < Cfg::STAGES; ++s) {
       mbar_init(full_bar + 8 * s, 1);
       mbar_init(split_bar + 8 * s, F_X_WARPS);
       mbar_init(empty_bar + 8 * s, 1);
     }
-    for (int b = 0; b < NUM_ACC; ++b) {
+    for (int b = 0; b < Cfg::NUM_ACC; ++b) {
       mbar_init(tfull_bar + 8 * b, 1);
       mbar_init(tempty_bar + 8 * b, F_EPI_WARPS);
     }
@@ -238,25 +245,33 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
       mbar_init(free_bar + 8 * b, 1);
       mbar_init(ready_bar + 8 * b, F_EPI_WARPS / 2);
     }
-    *abort_flag = 0;
-    *again = 0;
     fence_barrier_init();
   }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), Cfg::TMEM_COLS);
-    tmem_relinquish();
-  }
+};
+
+// The warps' roles over the CTA's tiles.  EPI selects the epilogue's arithmetic: 0 = the accumulator is the result (the Winograd
+// products); 1 = bias and a clamp (NOOP / RELU / RELUX), 2 = with a residual too; 3 and 4 = the same with the leaky term.
+// SECOND: once more over the tiles that the first pass marked; the split warps look at all of a row first.
+template <int BN, int EPI, bool SECOND>
+__device__ __forceinline__ void run_tiles(const CUtensorMap &tmap_x, const CUtensorMap &tmap_w, const CUtensorMap &tmap_c,
+                                          const CUtensorMap &tmap_r, const F32TcParams &p, const FShared<BN> &sh,
+                                          const uint32_t tmem_base, const int warp, const int lane) {
+  using Cfg = F32Cfg<BN>;
+  constexpr int STAGES = Cfg::STAGES;
+  constexpr int NUM_ACC = Cfg::NUM_ACC;
+  constexpr bool RES = EPI == 2 || EPI == 4, LEAKY = EPI >= 3;
+  constexpr int STAGING_AT = FShared<BN>::STAGING_AT, UB_AT = FShared<BN>::UB_AT;
+  const uint32_t smem_base = sh.base_u32;
+  uint8_t *smem_aligned = sh.base;
+  float *x_unscale = reinterpret_cast<float *>(smem_aligned + FShared<BN>::XSCALE_AT);  // [F_SCALE_SLOTS][FBM]
+  const uint32_t full_bar = sh.full_bar, split_bar = sh.split_bar, empty_bar = sh.empty_bar, tfull_bar = sh.tfull_bar;
+  const uint32_t tempty_bar = sh.tempty_bar, free_bar = sh.free_bar, ready_bar = sh.ready_bar, sempty_bar = sh.sempty_bar;
+  volatile int *abort_flag = sh.abort_flag;
+  const volatile uint8_t *only = SECOND ? sh.marks : nullptr;
   auto fail = [&](int code) {
     *abort_flag = 1;
     atomicCAS(p.status, 0, code);
   };
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  // everything above touched only this CTA's shared and tensor memory; from here on the roles read
-  // and write global memory, which the kernel in front of this one may still be producing
-  mb_grid_dep_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -265,7 +280,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (FTileIter it(p); ok && it.valid(p); it.next(p)) {
+      for (FTileIter it(p, only); ok && it.valid(p); it.next(p)) {
         const int xb = p.x_batched ? it.b : 0, wb = p.w_batched ? it.b : 0;
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait(empty_bar + 8 * stage, phase ^ 1, abort_flag, F_WAIT_BUDGET)) {
@@ -285,6 +300,17 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
             stage = 0;
             phase ^= 1;
           }
+        }
+      }
+      // (the MMAs have released every stage when the pass ends)
+      for (int s = 0; ok && s < STAGES; ++s) {
+        if (!mbar_wait(empty_bar + 8 * stage, phase ^ 1, abort_flag, F_WAIT_BUDGET)) {
+          fail(MB_DEV_TIMEOUT_PRODUCER);
+          ok = false;
+        }
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
@@ -308,7 +334,12 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
       uint32_t acc_buf = 0, acc_phase = 0;
       uint32_t small_phase = 1;  // (of sempty_bar, which the first tile need not wait for)
       bool ok = true, ready = false;
-      for (int tiles = my_tiles(p); ok && tiles > 0; --tiles, small_phase ^= 1) {
+      int tiles = static_cast<int>((p.batch * p.tiles_m * p.tiles_n - blockIdx.x + gridDim.x - 1) / gridDim.x);
+      if (SECOND) {
+        tiles = 0;
+        for (FTileIter it(p, only); it.valid(p); it.next(p)) ++tiles;
+      }
+      for (; ok && tiles > 0; --tiles, small_phase ^= 1) {
         if (!mbar_wait_warp(tempty_bar + 8 * acc_buf, acc_phase ^ 1, abort_flag, F_WAIT_BUDGET)) {
           fail(MB_DEV_TIMEOUT_MMA);
           break;
@@ -408,10 +439,20 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
       for (int k = 0; k < 16; ++k) v[k] = xs[k * FBM];
     };
     bool loaded = false;  // v holds this step's values
-    for (FTileIter it(p); ok && it.valid(p); it.next(p), ++tile) {
-      const bool inside = static_cast<int64_t>(it.tm) * FBM + quarter * 32 + lane < p.Mdim;
+    for (FTileIter it(p, only); ok && it.valid(p); it.next(p), ++tile) {
+      const int64_t m = static_cast<int64_t>(it.tm) * FBM + quarter * 32 + lane;
+      const bool inside = m < p.Mdim;
       float scale = 0.f;
       bool known = false;  // every pixel of the warp has its scale
+      if (SECOND) {
+        const float *x = p.X + it.b * p.x_bs + min(m, p.Mdim - 1);
+        float most = 0.f;
+#pragma unroll 16
+        for (int64_t k = 0; k < p.K; ++k) most = fmaxf(most, f32_finite_abs(mb_load(x + k * p.x_rs)));
+        if (most > 0.f) scale = f32_row_scale(most);
+        if (half == 0) x_unscale[(tile % F_SCALE_SLOTS) * FBM + quarter * 32 + lane] = f32_row_unscale(scale);
+        known = true;
+      }
       for (int kb = 0; kb < p.k_blocks; ++kb) {
         if (!loaded) {
           if (!mbar_wait_warp(full_bar + 8 * stage, phase, abort_flag, F_WAIT_BUDGET)) {
@@ -479,7 +520,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     int tile = 0;
     int q = 0;        // chunks of this set so far
     bool ok = true;
-    for (FTileIter it(p); ok && it.valid(p); it.next(p), ++tile) {
+    for (FTileIter it(p, only); ok && it.valid(p); it.next(p), ++tile) {
       const int64_t m = static_cast<int64_t>(it.tm) * FBM + quarter * 32 + lane;
       const bool m_ok = m < p.Mdim;
       const int64_t n_first = static_cast<int64_t>(it.tn) * BN + set * (BN / 2);
@@ -585,9 +626,10 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
         const float2 z = f32_parts(z2);
         if (z.x + z.y != 0.f) {
-          *again = 1;
+          sh.again[SECOND] = 1;
+          sh.marks[SECOND * MARKS + (SECOND ? it.nth : tile) % MARKS] = 1;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) a[j] = __uint_as_float(F32_AGAIN);
+          for (int j = 0; SECOND && j < 16; ++j) a[j] = __uint_as_float(F32_AGAIN);
         }
         if (c_tma) {
 #pragma unroll
@@ -616,7 +658,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     const int set = warp - FIRST_STORE;
     const uint32_t bufs = smem_base + STAGING_AT + set * (F_BUFS * Cfg::BUF_BYTES);
     const uint32_t my_free_bar = free_bar + 8 * (set * F_BUFS), my_ready_bar = ready_bar + 8 * (set * F_BUFS);
-    FTileIter rt(p);  // where the next chunk to be given out lies
+    FTileIter rt(p, only);  // where the next chunk to be given out lies
     int rc = 0, rq = 0;
     auto give = [&]() {
       if (RES) {
@@ -636,7 +678,7 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     for (int i = 0; i < F_BUFS; ++i) give();
     int q = 0;
     bool ok = true;
-    for (FTileIter it(p); ok && it.valid(p); it.next(p)) {
+    for (FTileIter it(p, only); ok && it.valid(p); it.next(p)) {
       const int n_first = it.tn * BN + set * (BN / 2);
       for (int i = 0; i < CHUNKS; ++i, ++q) {
         if (!mbar_wait(my_ready_bar + 8 * (q & 3), (q >> 2) & 1, abort_flag, F_WAIT_BUDGET)) {
@@ -654,19 +696,69 @@ gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
     }
     bulk_wait_group<0>();  // staging must outlive the stores' reads
   }
+}
 
+template <int BN, int EPI>
+__global__ void __launch_bounds__(F_THREADS, 1)
+gemm_f32_pairs_kernel(const __grid_constant__ CUtensorMap tmap_x,
+                   const __grid_constant__ CUtensorMap tmap_w,
+                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
+                   const __grid_constant__ F32TcParams p) {
+  using Cfg = F32Cfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  const FShared<BN> sh(smem_raw);
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  mb_grid_dep_launch();  // the kernel behind this one may start its own prologue
+
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&tmap_x);
+    prefetch_tensormap(&tmap_w);
+    if (p.c_tma) prefetch_tensormap(&tmap_c);
+    if ((EPI == 2 || EPI == 4) && p.c_tma) prefetch_tensormap(&tmap_r);
+    sh.init_barriers();
+    *sh.abort_flag = 0;
+    sh.again[0] = sh.again[1] = 0;
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(sh.tmem_slot), Cfg::TMEM_COLS);
+    tmem_relinquish();
+    for (int i = lane; i < 2 * MARKS; i += 32) sh.marks[i] = 0;
+  }
+  tc_fence_before_sync();
   __syncthreads();
-  if (*abort_flag != 0) {
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *sh.tmem_slot;
+  // everything above touched only this CTA's shared and tensor memory; from here on the roles read
+  // and write global memory, which the kernel in front of this one may still be producing
+  mb_grid_dep_wait();
+
+  run_tiles<BN, EPI, false>(tmap_x, tmap_w, tmap_c, tmap_r, p, sh, tmem_base, warp, lane);
+  __syncwarp();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (sh.again[0] != 0 && *sh.abort_flag == 0) {
+    // (no copy, MMA or arrival of the first pass is on its way any more)
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < Cfg::BARRIERS; ++i) mbar_inval(sh.full_bar + 8 * i);
+      sh.init_barriers();
+    }
+    __syncthreads();
+    run_tiles<BN, EPI, true>(tmap_x, tmap_w, tmap_c, tmap_r, p, sh, tmem_base, warp, lane);
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+  }
+  if (*sh.abort_flag != 0) {
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
-  }
-  if (*again != 0 && *abort_flag == 0) {
+  if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  if (sh.again[1] != 0 && *sh.abort_flag == 0) {
     asm volatile("fence.proxy.async;" ::: "memory");  // (the results were written by TMA stores, which have completed)
-    for (FTileIter it(p); it.valid(p); it.next(p)) tile_again(p, it.tm * FBM, it.tn * BN, BN, it.b);
+    for (FTileIter it(p, sh.marks + MARKS); it.valid(p); it.next(p)) tile_again(p, it.tm * FBM, it.tn * BN, BN, it.b);
   }
 }
 

@@ -182,6 +182,61 @@ def test_gemm_f32_pairs_spread(ctx, M, spread):
     assert np.linalg.norm(got - exact) <= 1.05 * np.linalg.norm(plain - exact)
 
 
+def _within_reach(x):
+    return np.copysign(np.clip(np.abs(x), 2.0 ** -5, 4), x).astype(np.float32)
+
+
+@pytest.mark.parametrize("shape,power", [((30, 40, 1280, 132), -14), ((30, 130, 1280, 132), -14), ((30, 130, 1280, 132), -18),
+                                         ((38000, 8, 132, 36), -14)])
+def test_gemm_f32_pairs_grows(ctx, shape, power):
+    """Rows of X whose first step is far smaller than the later ones, for which the weights make up, in some of a CTA's tiles (up to
+    514 of them, the last of which share marks with the first): the same results, bit for bit, and so none of them is worked out
+    again by FMAs."""
+    batch, M, N, K = shape
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = _within_reach(rng.standard_normal((batch, M, K), dtype=np.float32))
+    B = _within_reach(rng.standard_normal((batch, K, N), dtype=np.float32))
+    plain = _matmul(ctx, A, B)
+    for b in (0, 3, 10, 17, 18, batch - 1):
+        A[b, :, :32] *= np.float32(2.0) ** -power
+        B[b, :32] *= np.float32(2.0) ** power
+    B[1, K // 2, 5] = B[-1, K - 1, N - 1] = np.inf
+    got = _matmul(ctx, A, B)
+    assert not np.isfinite(got[1, :, 5]).any() and not np.isfinite(got[-1, :, N - 1]).any()
+    plain[1, :, 5], plain[-1, :, N - 1] = got[1, :, 5], got[-1, :, N - 1]
+    assert np.array_equal(got, plain, equal_nan=True)
+
+
+@pytest.mark.parametrize("act", [0, 6])
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("O", [40, 130])
+def test_conv1x1_f32_pairs_grows(ctx, O, residual, act):
+    """... with the residual, which is read once more."""
+    N, C, HW = 70, 68, 400
+    rng = np.random.Generator(np.random.PCG64(O))
+    x, f = _within_reach(rng.standard_normal((N, C, HW))), _within_reach(rng.standard_normal((O, C)))
+    bias = rng.standard_normal(O).astype(np.float32)
+    r = rng.standard_normal((N, O, HW)).astype(np.float32)
+    got = []
+    for grown in (False, True):
+        if grown:
+            x[:, :32] *= np.float32(2.0 ** -14)
+            f[:, :32] *= np.float32(2.0 ** 14)
+        dx, df, db, dr, do = (ctx.upload(v) for v in (x, f, bias, r, np.zeros((N, O, HW), np.float32)))
+        for name, value in (("f32_gather", 1), ("f32_pairs", 2)):
+            ctx.set_option(name, value)
+        if residual:
+            ctx.conv2d_f32_residual(dx, df, db, dr, do, N, C, HW // 4, 4, O, 1, 1, (1, 1), (1, 1), (0, 0), (HW // 4, 4), act, 0.6, 0.25)
+        else:
+            ctx.conv2d_f32(dx, df, db, do, N, C, HW // 4, 4, O, 1, 1, (1, 1), (1, 1), (0, 0), (HW // 4, 4), act, 0.6, 0.25)
+        for name in ("f32_gather", "f32_pairs"):
+            ctx.set_option(name, 0)
+        got.append(ctx.download(do, (N, O, HW), np.float32))
+        for b in (dx, df, db, dr, do):
+            b.free()
+    assert np.array_equal(*got)
+
+
 @pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
 @pytest.mark.parametrize("M", [40, 150])
 def test_gemm_f32_pairs_scales(ctx, M, powers):
