@@ -17,8 +17,8 @@
 // 220 -> 226 (394 -> 346), 256 -> 64 214 -> 180, 512 -> 128 at 28 x 28 148 -> 128, 128 -> 512 170 -> 148 (258 -> 206), 256 -> 1024 at
 // 14 x 14 156 -> 139 (194 -> 154), 1024 -> 256 147 -> 123, 1024 -> 512 282 -> 227.
 //
-// A row of X has the scale of its first step that has a value.  Where a later one is beyond 2^11 times that the row's results are no
-// finite numbers; the tiles that have some are marked, and a second pass over them has scales from all of a row.  512 -> 128 at
+// A row of X has the scale of its first step that has a value.  Where a later one is beyond 2^11 (with wide ranges 2^3) times that the
+// row's results are no finite numbers; the tiles that have some are marked, and a second pass over them has scales from all of a row.  512 -> 128 at
 // 28 x 28 with channels 2^14 times larger from the 32nd on: in all pixels 497 us (7170 by FMAs), in one of 1000 233 (1863).
 //
 // Structure (one persistent CTA per SM):
@@ -468,10 +468,22 @@ __device__ __forceinline__ void run_tiles(const CUtensorMap &tmap_x, const CUten
         if (!known) {
           // (both warps of a pixel look at all 32 values, and so come to the same scale)
           const float *other = landed(stage) + (half ^ 1) * 16 * FBM;
-          float most = 0.f;
+          // The largest value goes to 2^4 .. 2^5, room for larger ones and smaller ones to come.  Where it stands out, the largest of
+          // another eight does, if it can: small values beside a large one keep their bits.
+          float most = 0.f, group[4] = {};
 #pragma unroll
-          for (int k = 0; k < 16; ++k) most = fmaxf(most, fmaxf(fabsf(v[k]), fabsf(other[k * FBM])));
-          if (scale == 0.f && most > 0.f) scale = f32_row_scale<4>(most);
+          for (int k = 0; k < 16; ++k) {
+            group[k >> 3] = fmaxf(group[k >> 3], fabsf(v[k]));
+            group[2 + (k >> 3)] = fmaxf(group[2 + (k >> 3)], fabsf(other[k * FBM]));
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) most = fmaxf(most, group[g]);
+          if (scale == 0.f && most > 0.f) {
+            scale = f32_row_scale<4>(most);
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              if (group[g] > 0.f) scale = fmaxf(scale, fminf(f32_row_scale<4>(group[g]), f32_row_scale<12>(most)));
+          }
           if (half == 0) x_unscale[(tile % F_SCALE_SLOTS) * FBM + quarter * 32 + lane] = f32_row_unscale(scale);
           known = __all_sync(0xffffffffu, scale != 0.f || !inside);
         }

@@ -237,6 +237,23 @@ def test_conv1x1_f32_pairs_grows(ctx, O, residual, act):
     assert np.array_equal(*got)
 
 
+@pytest.mark.parametrize("M", [40, 150])
+@pytest.mark.parametrize("columns", [(0,), (5, 22), (20, 100), (259,)])
+def test_gemm_f32_pairs_outliers(ctx, M, columns):
+    """Columns of X 1e8 times larger than the others, which meet zeros or weights as much smaller: the others keep their bits."""
+    rng = np.random.Generator(np.random.PCG64(M))
+    A = rng.standard_normal((2, M, 260)).astype(np.float32)
+    B = rng.standard_normal((2, 260, 300)).astype(np.float32)
+    plain, exact = _matmul(ctx, A, B), A.astype(np.float64) @ B.astype(np.float64)
+    plain = np.linalg.norm(plain - exact) / np.linalg.norm(exact)
+    B[:, columns] *= np.float32(1e8)
+    A[:, :, columns] *= np.float32(1e-8)
+    A[:, ::2, columns] = 0
+    exact = A.astype(np.float64) @ B.astype(np.float64)
+    got = _matmul(ctx, A, B)
+    assert np.linalg.norm(got - exact) / np.linalg.norm(exact) <= 1.2 * plain
+
+
 @pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
 @pytest.mark.parametrize("M", [40, 150])
 def test_gemm_f32_pairs_scales(ctx, M, powers):
