@@ -368,10 +368,18 @@ int mb_dwconv_f32_nchw(mb_context *ctx, const float *in, const float *filter,
  * F(2x2,3x3); tile_override 2 or 6 forces a size.  transformed_filter may be
  * NULL (the filter is transformed into scratch on every call) or a buffer of
  * (tile+2)^2 * O * C floats that mb_winograd_transform_filter_f32 filled, the
- * way the CPU delegator caches it for weights (:120-145). */
+ * way the CPU delegator caches it for weights (:120-145).  With both forms at
+ * hand the call takes a direct convolution where that costs less;
+ * mb_conv3x3_winograd_f32_reads_transformed is 0 where it does, and a caller
+ * that has not made the transformed form then passes filter_oihw in its place
+ * (and 1 where it does not). */
 int mb_winograd_transform_filter_f32(mb_context *ctx, const float *filter_oihw,
                                      float *transformed, int64_t C, int64_t O,
                                      int tile);
+int mb_conv3x3_winograd_f32_reads_transformed(
+    mb_context *ctx, const float *in, const float *filter_oihw, int64_t N,
+    int64_t C, int64_t H, int64_t W, int64_t O, int pad_top, int pad_left,
+    int64_t Ho, int64_t Wo, int tile_override);
 int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in,
                                  const float *filter_oihw,
                                  const float *transformed_filter,

@@ -87,6 +87,7 @@ PROTOTYPES = {
     "mb_conv2d_f32_nchw_residual": (_int, [_vp] * 6 + [_i64] * 7 + [_int] * 6 + [_i64] * 2 + [_int, _f32, _f32]),
     "mb_dwconv_f32_nchw": (_int, [_vp] * 5 + [_i64] * 7 + [_int] * 6 + [_i64] * 2 + [_int, _f32, _f32]),
     "mb_winograd_transform_filter_f32": (_int, [_vp] * 3 + [_i64] * 2 + [_int]),
+    "mb_conv3x3_winograd_f32_reads_transformed": (_int, [_vp] * 3 + [_i64] * 5 + [_int] * 2 + [_i64] * 2 + [_int]),
     "mb_conv3x3_winograd_f32_nchw": (_int, [_vp] * 6 + [_i64] * 5 + [_int] * 2 + [_i64] * 2 +
                                      [_int, _f32, _f32, _int]),
     "mb_pooling_f32_nchw": (_int, [_vp] * 3 + [_i64] * 6 + [_int] * 6 + [_i64] * 2 + [_int]),

@@ -387,6 +387,44 @@ static int64_t winograd_cost(const mb_context *ctx, int64_t N, int64_t C, int64_
   return 23000 + bytes / 5000 + rounds * std::max<int64_t>(ceil_div64(C, 32) * 1150, 4500) + (cols % 4 != 0 ? 6000 : 0);
 }
 
+// What a 3x3 convolution with both forms of its filter at hand takes: a direct convolution where the three launches cost more.
+struct Conv3x3Route {
+  mb_f32_gemm g;
+  mb_f32_conv d;
+  bool gather = false, direct = false;  // (direct first, where there is room for it)
+};
+static Conv3x3Route pick_route(mb_context *ctx, const float *in, const float *filter, const float *bias, float *out, int64_t N,
+                               int64_t C, int64_t H, int64_t W, int64_t O, int pad_top, int pad_left, int64_t Ho, int64_t Wo,
+                               int activation, float max_limit, float coefficient, int tile_override) {
+  Conv3x3Route r;
+  const int tile = pick_tile(H, W, tile_override);
+  int64_t best = winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override);
+  mb_f32_gemm &g = r.g;
+  g.X = in; g.W = filter; g.bias = bias; g.C = out;
+  g.M = N * Ho * Wo; g.N = O; g.K = C * 9;
+  g.act = activation; g.max_limit = max_limit; g.coef = coefficient;
+  g.conv = true;
+  g.C_in = static_cast<int>(C); g.H = static_cast<int>(H); g.Wd = static_cast<int>(W);
+  g.KH = 3; g.KW = 3; g.pad_t = pad_top; g.pad_l = pad_left;
+  g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
+  // no larger an error than that of the Winograd kernels: 3.1e-8 times the root of C with F(2,3), 2e-6 and more with F(6,3)
+  g.run = tile == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : C < 200 ? 4 : 6;
+  if (ctx->f32_gather != 1 && mb_gemm_f32_gather_supported(ctx, g)) {
+    const int64_t cost = mb_gemm_f32_gather_cost(ctx, g);
+    r.gather = ctx->f32_gather == 2 || cost < best;
+    if (r.gather) best = cost;
+  }
+  // (errors of 1.3e-7 and 3.5e-7 with runs of one and three filter rows)
+  mb_f32_conv &d = r.d;
+  d.X = in; d.filter = filter; d.bias = bias; d.out = out;
+  d.N = N; d.C = C; d.H = H; d.W = W; d.O = O;
+  d.act = activation; d.max_limit = max_limit; d.coef = coefficient;
+  d.run = r.gather || (tile == 2 && C <= 128) ? 1 : 3;
+  r.direct = Ho == H && Wo == W && pad_top == 1 && pad_left == 1 && ctx->f32_direct != 1 && mb_conv_f32_direct_supported(ctx, d) &&
+             (ctx->f32_direct == 2 || (ctx->f32_gather == 0 && mb_conv_f32_direct_cost(ctx, d) < best));
+  return r;
+}
+
 extern "C" {
 
 int mb_winograd_transform_filter_f32(mb_context *ctx, const float *filter, float *transformed,
@@ -409,6 +447,15 @@ int mb_winograd_transform_filter_f32(mb_context *ctx, const float *filter, float
   return MB_SUCCESS;
 }
 
+int mb_conv3x3_winograd_f32_reads_transformed(mb_context *ctx, const float *in, const float *filter, int64_t N, int64_t C, int64_t H,
+                                              int64_t W, int64_t O, int pad_top, int pad_left, int64_t Ho, int64_t Wo,
+                                              int tile_override) {
+  if (ctx == nullptr || in == nullptr || filter == nullptr || N < 1 || C < 1 || H < 1 || W < 1 || O < 1 || Ho < 1 || Wo < 1) return 1;
+  const Conv3x3Route r = pick_route(ctx, in, filter, nullptr, nullptr, N, C, H, W, O, pad_top, pad_left, Ho, Wo, 0, 0.f, 0.f,
+                                    tile_override);
+  return r.direct || r.gather ? 0 : 1;
+}
+
 int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *filter,
                                  const float *transformed_filter, const float *bias, float *out,
                                  int64_t N, int64_t C, int64_t H, int64_t W, int64_t O, int pad_top,
@@ -425,42 +472,19 @@ int mb_conv3x3_winograd_f32_nchw(mb_context *ctx, const float *in, const float *
   if (Ho > H + 2 * 2 || Wo > W + 2 * 2)
     return mb_fail(ctx, MB_INVALID_ARGS, "mb_conv3x3_winograd_f32_nchw: output larger than a 3x3 stride-1 conv gives");
   MB_CUDA(ctx, cudaSetDevice(ctx->device));
-  // A direct convolution where the three launches cost more.  Only with both forms of the filter at hand: a call with one of
-  // them gives bit for bit what a call with the other does.
+  // Another kernel only with both forms of the filter at hand: a call with one of them gives bit for bit what a call with the other
+  // does.
   if (filter != nullptr && transformed_filter != nullptr) {
-    const int tile = pick_tile(H, W, tile_override);
-    int64_t best = winograd_cost(ctx, N, C, H, W, O, Ho, Wo, tile_override);
-    mb_f32_gemm g;
-    g.X = in; g.W = filter; g.bias = bias; g.C = out;
-    g.M = N * Ho * Wo; g.N = O; g.K = C * 9;
-    g.act = activation; g.max_limit = max_limit; g.coef = coefficient;
-    g.conv = true;
-    g.C_in = static_cast<int>(C); g.H = static_cast<int>(H); g.Wd = static_cast<int>(W);
-    g.KH = 3; g.KW = 3; g.pad_t = pad_top; g.pad_l = pad_left;
-    g.Ho = static_cast<int>(Ho); g.Wo = static_cast<int>(Wo);
-    // no larger an error than that of the Winograd kernels: 3.1e-8 times the root of C with F(2,3), 2e-6 and more with F(6,3)
-    g.run = tile == 6 ? 16 : C < 48 ? 1 : C < 128 ? 2 : C < 200 ? 4 : 6;
-    bool gather = false;
-    if (ctx->f32_gather != 1 && mb_gemm_f32_gather_supported(ctx, g)) {
-      const int64_t cost = mb_gemm_f32_gather_cost(ctx, g);
-      gather = ctx->f32_gather == 2 || cost < best;
-      if (gather) best = cost;
-    }
-    // (errors of 1.3e-7 and 3.5e-7 with runs of one and three filter rows)
-    mb_f32_conv d;
-    d.X = in; d.filter = filter; d.bias = bias; d.out = out;
-    d.N = N; d.C = C; d.H = H; d.W = W; d.O = O;
-    d.act = activation; d.max_limit = max_limit; d.coef = coefficient;
-    d.run = gather || (tile == 2 && C <= 128) ? 1 : 3;
-    if (Ho == H && Wo == W && pad_top == 1 && pad_left == 1 && ctx->f32_direct != 1 && mb_conv_f32_direct_supported(ctx, d) &&
-        (ctx->f32_direct == 2 ||
-         (ctx->f32_gather == 0 && mb_conv_f32_direct_cost(ctx, d) < best))) {
+    const Conv3x3Route r = pick_route(ctx, in, filter, bias, out, N, C, H, W, O, pad_top, pad_left, Ho, Wo, activation, max_limit,
+                                      coefficient, tile_override);
+    if (r.direct) {
       bool done = false;
-      MB_RETURN_IF_ERROR(mb_conv_f32_direct_launch(ctx, d, &done));
+      MB_RETURN_IF_ERROR(mb_conv_f32_direct_launch(ctx, r.d, &done));
       if (done) return MB_SUCCESS;
     }
-    if (gather) return mb_gemm_f32_gather_launch(ctx, g);
+    if (r.gather) return mb_gemm_f32_gather_launch(ctx, r.g);
   }
+  if (transformed_filter == filter) transformed_filter = nullptr;
   const int tile = pick_tile(H, W, tile_override);
   const int T = (tile + 2) * (tile + 2);
   const int64_t th = ceil_div64(Ho, tile), tw = ceil_div64(Wo, tile), tiles = th * tw;

@@ -391,7 +391,7 @@ class Conv2d : public delegator::Conv2d {
   const Tensor *residual_ = nullptr;
 };
 
-// 3x3 stride-1 Winograd; the transformed filter is cached while the filter is a
+// 3x3 stride-1 Winograd; the transformed filter, where it is read, is cached while the filter is a
 // weight, as the CPU delegator does (conv_2d_3x3_winograd.cc:120-145).
 class Conv2dK3x3Winograd : public delegator::Conv2d {
  public:
@@ -406,7 +406,13 @@ class Conv2dK3x3Winograd : public delegator::Conv2d {
     MACE_RETURN_IF_ERROR(output->Resize({input->dim(0), filter->dim(0), g.out_h, g.out_w}));
     const int tile = (input->dim(2) > 16 && input->dim(3) > 16) ? 6 : 2;
     const float *transformed = nullptr;
-    if (filter->is_weight()) {
+    if (filter->is_weight() &&
+        mb_conv3x3_winograd_f32_reads_transformed(
+            rt->ctx(), input->memory<float>(), filter->memory<float>(), input->dim(0), input->dim(1),
+            input->dim(2), input->dim(3), filter->dim(0), g.pad_top, g.pad_left, g.out_h, g.out_w,
+            tile) == 0) {
+      transformed = filter->memory<float>();
+    } else if (filter->is_weight()) {
       if (transformed_filter_ == nullptr || tile != out_tile_size_ || src_ != filter) {
         const index_t t = (tile + 2) * (tile + 2);
         transformed_filter_ = std::make_unique<Tensor>(

@@ -435,6 +435,42 @@ def test_conv3x3_f32_is_as_accurate_as_winograd(ctx, orc, shape):
         b.free()
 
 
+@pytest.mark.parametrize("shape", [(32, 64, 56, 64), (1, 64, 14, 64)])
+def test_conv3x3_f32_without_the_transformed_filter(shape):
+    """Where the transformed filter is not read it need not be made; where it is read the call makes it."""
+    import mace_b200
+    L = mace_b200.lib()
+    N, C, HW, O = shape
+    rng = np.random.Generator(np.random.PCG64(C))
+    c = mace_b200.Context(0)
+    dx, do = c.upload(rng.standard_normal((N, C, HW, HW)).astype(np.float32)), c.alloc(N * O * HW * HW * 4)
+    df = c.upload((rng.standard_normal((O, C, 3, 3)) * np.sqrt(2.0 / (9 * C))).astype(np.float32))
+    tile = 6 if HW > 16 else 2
+    dt = c.alloc((tile + 2) ** 2 * O * C * 4)
+    c.winograd_transform_filter(df, dt, C, O, tile)
+
+    def asked():
+        return L.mb_conv3x3_winograd_f32_reads_transformed(c.h, dx.ptr, df.ptr, N, C, HW, HW, O, 1, 1, HW, HW, tile)
+
+    def run(transformed):
+        c.winograd_f32(dx, df, None, do, N, C, HW, HW, O, (1, 1), (HW, HW), tile=tile, transformed=transformed)
+        return c.download(do, (N, O, HW, HW), np.float32)
+
+    try:
+        assert asked() == 0
+        assert np.array_equal(run(df), run(dt))
+        c.set_option("f32_gather", 1)
+        c.set_option("f32_direct", 1)
+        assert asked() == 1
+        assert np.array_equal(run(df), run(dt))
+        c.set_option("f32_direct", 2)
+        assert asked() == 0
+        assert np.array_equal(run(df), run(dt))
+    finally:
+        L.mb_set_runtime_failure_ratio(0.0)
+        c.close()
+
+
 @pytest.mark.parametrize("maj", [(0, 0), (0, 1), (1, 0), (1, 1)])
 @pytest.mark.parametrize("c_col", [False, True])
 @pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 63, 65, 31), (1, 64, 64, 32), (3, 65, 130, 33), (1, 130, 61, 65), (70000, 2, 3, 5)])
