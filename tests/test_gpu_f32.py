@@ -435,6 +435,46 @@ def test_conv3x3_f32_is_as_accurate_as_winograd(ctx, orc, shape):
         b.free()
 
 
+@pytest.mark.parametrize("what", ["large product", "transposed", "direct", "stem", "small product", "small convolution"])
+def test_f32_results_do_not_depend_on_a_rows_range(ctx, what):
+    """By rule, whatever kernel: a column (channel) 1e6 times larger, whose weights are as much smaller or zero."""
+    rng = np.random.Generator(np.random.PCG64(4))
+    if what in ("large product", "transposed", "small product"):
+        M, N, K = {"large product": (256, 76800, 512), "transposed": (1024, 1024, 1024), "small product": (64, 192, 320)}[what]
+        a, b = rng.standard_normal((1, M, K)).astype(np.float32), rng.standard_normal((1, K, N)).astype(np.float32)
+
+        def run():
+            col = what == "transposed"
+            da, db, dc = ctx.upload(a), ctx.upload(b.transpose(0, 2, 1) if col else b), ctx.alloc(M * N * 4)
+            ctx.gemm_f32(da, db, dc, 1, M, N, K, b_col_major=col)
+            got = ctx.download(dc, (M, N), np.float32)[:, :2000]
+            for d in (da, db, dc):
+                d.free()
+            return _norm_err(got, a[0].astype(np.float64) @ b[0, :, :2000].astype(np.float64))
+    else:
+        n, C, HW, O, k, st = {"direct": (16, 64, 28, 64, 3, 1), "stem": (24, 3, 224, 64, 7, 2), "small convolution": (1, 40, 9, 30, 3, 1)}[what]
+        b, a = rng.standard_normal((n, C, HW, HW)).astype(np.float32), rng.standard_normal((O, C, k, k)).astype(np.float32)
+        ho = HW // st
+
+        def run():
+            db, da, dc = ctx.upload(b), ctx.upload(a), ctx.alloc(n * O * ho * ho * 4)
+            ctx.conv2d_f32(db, da, None, dc, n, C, HW, HW, O, k, k, (st, st), (1, 1), (k // 2, k // 2), (ho, ho))
+            got = ctx.download(dc, (n, O, ho, ho), np.float32)[:1]
+            for d in (da, db, dc):
+                d.free()
+            padded = np.pad(b[:1].astype(np.float64), ((0, 0), (0, 0), (k // 2,) * 2, (k // 2,) * 2))
+            exact = sum(np.einsum("ncyx,oc->noyx", padded[:, :, i:i + st * ho:st, j:j + st * ho:st], a[:, :, i, j].astype(np.float64),
+                                  optimize=True) for i in range(k) for j in range(k))
+            return _norm_err(got, exact)
+
+    plain = run()
+    b[:, 1] *= np.float32(1e6)
+    a[(np.s_[:], np.s_[:], 1) if a.ndim == 3 else (np.s_[:], 1)] *= np.float32(1e-6)
+    assert run() <= 1.1 * plain
+    a[(np.s_[:], np.s_[:], 1) if a.ndim == 3 else (np.s_[:], 1)] = 0
+    assert run() <= 1.1 * plain
+
+
 @pytest.mark.parametrize("shape", [(32, 64, 56, 64), (1, 64, 14, 64)])
 def test_conv3x3_f32_without_the_transformed_filter(shape):
     """Where the transformed filter is not read it need not be made; where it is read the call makes it."""

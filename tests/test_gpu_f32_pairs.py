@@ -19,7 +19,7 @@ def _bound(A, B):
     per 16 of the depth."""
     A, B = np.abs(A), np.abs(B)
     K = A.shape[-1]
-    return (A @ B) * (2.0 ** -21 + (3 * K / 16 + 4) * 2.0 ** -23) + 1e-30
+    return (A @ B) * (2.0 ** -21 + (3 * K / 16 + 4) * 2.0 ** -23) + 1e-37
 
 
 def _matmul(ctx, A, B, pairs=2):

@@ -35,7 +35,7 @@ def _bound(A, B):
     at most 2^-23 of it), and the sums of the runs round once each."""
     A, B = np.abs(A), np.swapaxes(np.abs(B), -1, -2)
     K = A.shape[-1]
-    return (A @ B) * (2.0 ** -21 + (6 + K / 32 + 4) * 2.0 ** -23) + 1e-30
+    return (A @ B) * (2.0 ** -21 + (6 + K / 32 + 4) * 2.0 ** -23) + 1e-37
 
 
 @pytest.mark.parametrize("bn", [64, 128])

@@ -42,7 +42,7 @@ def _bound(x, f, bias, sh, pad, out_hw, ref):
     """hi + lo of a value is within 2^-22 of it; an accumulator holds at most six MMAs per filter row, each of which cuts off at most
     2^-23 of it; the bias and the sum of the two accumulators round once."""
     size = _exact(np.abs(x), np.abs(f), sh, pad, out_hw)
-    return size * (2.0 ** -21 + (6 * f.shape[2] + 2) * 2.0 ** -23) + (np.abs(ref) + np.abs(bias)[None, :, None, None]) * 2.0 ** -23 + 1e-30
+    return size * (2.0 ** -21 + (6 * f.shape[2] + 2) * 2.0 ** -23) + (np.abs(ref) + np.abs(bias)[None, :, None, None]) * 2.0 ** -23 + 1e-37
 
 
 @pytest.mark.parametrize("shape", [
