@@ -83,14 +83,15 @@ __device__ __forceinline__ int64_t value_at(const Params &p, int64_t f) {
   return static_cast<int64_t>(img) * p.C_in * p.H * p.W + y * p.W + x;
 }
 
-// A result by fp32 FMAs.
+// A result by fp32 FMAs, by a warp.
 __device__ __noinline__ void store_exact(const Params &p, int64_t f, int o) {
   const uint32_t img = fast_div(static_cast<uint32_t>(f), p.image_mul, p.image_shift);
   const uint32_t in = static_cast<uint32_t>(f) - img * p.image;
   const int y = static_cast<int>(fast_div(in, p.pitch_mul, p.pitch_shift)), x = static_cast<int>(in) - y * p.pitch;
   const int64_t hw = static_cast<int64_t>(p.H) * p.W;
-  float sum = f32_chain_window(p.X + static_cast<int64_t>(img) * p.C_in * hw, p.filter + static_cast<int64_t>(o) * p.C_in * p.taps,
+  float sum = f32_warp_window(p.X + static_cast<int64_t>(img) * p.C_in * hw, p.filter + static_cast<int64_t>(o) * p.C_in * p.taps,
                                p.C_in, p.H, p.W, p.KH, p.KW, y - p.ph, x - p.pw);
+  if ((threadIdx.x & 31) != 0) return;
   if (p.bias != nullptr) sum += p.bias[o];
   p.C[(static_cast<int64_t>(img) * p.O + o) * hw + static_cast<int64_t>(y) * p.W + x] = mb_activate(sum, p.act, p.max_limit, p.coef);
 }
@@ -476,14 +477,14 @@ conv_f32_direct_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   if (*again == 0 || *abort_flag != 0) return;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x)
     for (int i = threadIdx.x; i < BM * BN; i += blockDim.x) {
-      const int64_t f = static_cast<int64_t>(t / p.tiles_n) * BM + (i & (BM - 1));
+      // (a warp: one channel, 32 places)
+      const int64_t first = static_cast<int64_t>(t / p.tiles_n) * BM + (i & (BM - 32));
       const int o = t % p.tiles_n * BN + i / BM;
-      if (o >= p.O) continue;
       // (the place's result lies where its input does, with O channels instead of C_in)
-      const int64_t at = value_at(p, f);
-      if (at < 0) continue;
+      const int64_t at = o < p.O ? value_at(p, first + lane) : -1;
       const int64_t hw = static_cast<int64_t>(p.H) * p.W, img = at / (p.C_in * hw), pix = at - img * p.C_in * hw;
-      if (__float_as_uint(p.C[(img * p.O + o) * hw + pix]) == F32_AGAIN) store_exact(p, f, o);
+      f32_each_again(at >= 0 && __float_as_uint(p.C[(img * p.O + o) * hw + pix]) == F32_AGAIN,
+                     [&](int of) { store_exact(p, first + of, o); });
     }
 }
 

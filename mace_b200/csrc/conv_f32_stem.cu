@@ -72,11 +72,12 @@ struct Unit {
   }
 };
 
-// A result by fp32 FMAs.
+// A result by fp32 FMAs, by a warp.
 __device__ __noinline__ void store_exact(const Params &p, int channels, float *dst, int img, int o, int y, int x) {
   const int64_t hw = static_cast<int64_t>(p.H) * p.W;
-  float sum = f32_chain_window(p.X + img * channels * hw, p.filter + o * channels * p.KH * p.KW, channels, p.H, p.W, p.KH, p.KW,
+  float sum = f32_warp_window(p.X + img * channels * hw, p.filter + o * channels * p.KH * p.KW, channels, p.H, p.W, p.KH, p.KW,
                                y * p.sh - p.pt, x * 2 - p.pl);
+  if ((threadIdx.x & 31) != 0) return;
   if (p.bias != nullptr) sum += p.bias[o];
   *dst = mb_activate(sum, p.act, p.max_limit, p.coef);
 }
@@ -461,11 +462,22 @@ __global__ void __launch_bounds__(THREADS, 1) conv_f32_stem_kernel(const __grid_
   if (*again == 0 || *abort_flag != 0) return;
   for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
     const Unit t(p, u);
-    const int width = min(p.tile, p.Wo - t.x0);
-    for (int i = threadIdx.x; i < p.O * t.rows * width; i += THREADS) {
-      const int o = i / (t.rows * width), in = i - o * t.rows * width, y = t.y0 + in / width, x = t.x0 + in % width;
-      float *dst = p.C + ((static_cast<int64_t>(t.img) * p.O + o) * p.Ho + y) * p.Wo + x;
-      if (__float_as_uint(*reinterpret_cast<volatile float *>(dst)) == F32_AGAIN) store_exact(p, CI, dst, t.img, o, y, x);
+    const int width = min(p.tile, p.Wo - t.x0), count = p.O * t.rows * width;
+    for (int first = warp * 32; first < count; first += THREADS) {
+      auto place = [&](int i, int &o, int &y, int &x) {
+        const int in = i % (t.rows * width);
+        o = i / (t.rows * width);
+        y = t.y0 + in / width;
+        x = t.x0 + in % width;
+        return p.C + ((static_cast<int64_t>(t.img) * p.O + o) * p.Ho + y) * p.Wo + x;
+      };
+      int o, y, x;
+      const bool mine = first + lane < count &&
+                        __float_as_uint(*reinterpret_cast<volatile float *>(place(first + lane, o, y, x))) == F32_AGAIN;
+      f32_each_again(mine, [&](int of) {
+        float *dst = place(first + of, o, y, x);
+        store_exact(p, CI, dst, t.img, o, y, x);
+      });
     }
   }
 }

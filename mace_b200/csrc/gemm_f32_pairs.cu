@@ -132,18 +132,22 @@ struct FTileIter {
 };
 
 // A result that the second pass has as no finite number either is stored as F32_AGAIN; when its tiles are done a CTA that stored
-// one works those out again, by fp32 FMAs in the order of k.
+// one works those out again, by fp32 FMAs.
 __device__ __noinline__ void tile_again(const F32TcParams &p, int m0, int n0, int bn, int b) {
   for (int i = threadIdx.x; i < FBM * bn; i += blockDim.x) {
-    const int64_t m = m0 + (i & (FBM - 1)), n = n0 + i / FBM;
-    if (m >= p.Mdim || n >= p.Ndim) continue;
-    const int64_t at = b * p.c_batch_stride + n * p.c_row_stride + m;
-    if (__float_as_uint(*reinterpret_cast<volatile float *>(p.C + at)) != F32_AGAIN) continue;
-    const float *x = p.X + b * p.x_bs + m, *w = p.W + b * p.w_bs + n * p.w_rs;
-    float sum = f32_chain(x, p.x_rs, w, p.K);
-    if (p.bias != nullptr) sum += p.bias[n];
-    if (p.residual != nullptr) sum += p.residual[at];
-    p.C[at] = mb_activate(sum, p.act, p.max_limit, p.coef);
+    // (a warp: one channel, 32 pixels)
+    const int64_t m_first = m0 + (i & (FBM - 32)), n = n0 + i / FBM, m = m_first + (i & 31);
+    const int64_t at_first = b * p.c_batch_stride + n * p.c_row_stride + m_first;
+    const bool mine = m < p.Mdim && n < p.Ndim &&
+                      __float_as_uint(*reinterpret_cast<volatile float *>(p.C + at_first + (i & 31))) == F32_AGAIN;
+    f32_each_again(mine, [&](int lane) {
+      float sum = f32_warp_dot(p.X + b * p.x_bs + m_first + lane, p.x_rs, p.W + b * p.w_bs + n * p.w_rs, p.K);
+      if ((i & 31) != lane) return;
+      const int64_t at = at_first + lane;
+      if (p.bias != nullptr) sum += p.bias[n];
+      if (p.residual != nullptr) sum += p.residual[at];
+      p.C[at] = mb_activate(sum, p.act, p.max_limit, p.coef);
+    });
   }
 }
 

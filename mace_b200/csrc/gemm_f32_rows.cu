@@ -64,17 +64,18 @@ struct Cfg {
   static_assert(8 * (3 * STAGES + 2 * ACCS) + 16 <= 256 && SMEM_BYTES <= 227 * 1024, "shared memory");
 };
 
-// Results of a tile that are not finite, by fp32 FMAs in the order of k.
+// Results of a tile that are not finite, by fp32 FMAs.
 __device__ __noinline__ void tile_again(const Params &p, int m0, int n0, int bn, int b) {
   for (int i = threadIdx.x; i < BM * bn; i += blockDim.x) {
-    const int m = m0 + (i & (BM - 1)), n = n0 + i / BM;
-    if (m >= p.M || n >= p.N) continue;
+    // (a warp: one n, 32 of m)
+    const int m_first = m0 + (i & (BM - 32)), n = n0 + i / BM, m = m_first + (i & 31);
     float *c = p.C + b * p.c_bs + n * p.c_ns + m;
-    if (__float_as_uint(*c) != F32_AGAIN) continue;
-    const float *x = p.X + b * p.x_bs + m * p.x_ms, *w = p.W + b * p.w_bs + n * p.w_ns;
-    float sum = f32_chain(x, 1, w, p.K);
-    if (p.bias != nullptr) sum += p.bias[n];
-    *c = mb_activate(sum, p.act, p.max_limit, p.coef);
+    f32_each_again(m < p.M && n < p.N && __float_as_uint(*c) == F32_AGAIN, [&](int lane) {
+      float sum = f32_warp_dot(p.X + b * p.x_bs + (m_first + lane) * p.x_ms, 1, p.W + b * p.w_bs + n * p.w_ns, p.K);
+      if ((i & 31) != lane) return;
+      if (p.bias != nullptr) sum += p.bias[n];
+      *c = mb_activate(sum, p.act, p.max_limit, p.coef);
+    });
   }
 }
 
