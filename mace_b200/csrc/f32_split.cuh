@@ -81,8 +81,9 @@ __device__ __forceinline__ float f32_finite_abs(float v) {
 // The scale of values that share one although they belong to several rows (the places of a convolution's patch or strip), from the
 // largest finite ones that the warps which looked at them found (all zero: 0).  It brings the largest to 2^12 .. 2^13, and is fair
 // for others whose largest comes to F32_LOW at least and stays below F32_HIGH.  A value of 2^-14 and more is then held to 22 bits,
-// 2^-22 of the largest or less.  What does not fit (values that are not finite, and those beyond 2^13 times all that the other
-// warps have) is left out: its results come out as NaN and are worked out again, and the others keep their bits.
+// 2^-22 of the largest or less.  What does not fit (values that are not finite, and those beyond 2^20 times all that the other
+// warps have, whose largest would be held to less than 2^-29 of it) is left out: its results come out as NaN and are worked out
+// again, and the others keep their bits.
 constexpr float F32_LOW = 256.f;
 template <int WARPS>
 __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
@@ -93,7 +94,7 @@ __device__ __forceinline__ float f32_shared_scale(const volatile float *most) {
     second = fmaxf(second, fminf(first, m));
     first = fmaxf(first, m);
   }
-  if (second > 0.f && first * (1.f / 8192.f) > second) first = second;
+  if (second > 0.f && first * (1.f / 1048576.f) > second) first = second;
   return first > 0.f ? f32_row_scale<12>(first) : 0.f;
 }
 

@@ -138,6 +138,23 @@ def test_direct_conv2d_f32_spread(ctx, O, spread):
     assert error(x, f, np.s_[:]) <= 1.05 * plain
 
 
+@pytest.mark.parametrize("O", [20, 100])
+def test_direct_conv2d_f32_beside_an_outlier(ctx, O):
+    """One value up to 1e6 times larger than its tile's others, which is held with them: they keep their bits, and so do its results."""
+    rng = np.random.Generator(np.random.PCG64(O))
+    x = rng.standard_normal((1, 70, 15, 15)).astype(np.float32)
+    f = (rng.standard_normal((O, 70, 3, 3)) * 0.1).astype(np.float32)
+    far = np.ones((15, 15), bool)
+    far[6:9, 4:7] = False
+    plain, exact = _run(ctx, x, f, None), _exact(x.astype(np.float64), f.astype(np.float64))
+    error = np.linalg.norm((plain - exact)[:, :, far]) / np.linalg.norm(exact[:, :, far])
+    for value in (3e4, 1e6):
+        x[0, 40, 7, 5] = value
+        got, exact = _run(ctx, x, f, None), _exact(x.astype(np.float64), f.astype(np.float64))
+        assert (np.abs(got - exact) <= _bound(x, f)).all()
+        assert np.linalg.norm((got - exact)[:, :, far]) / np.linalg.norm(exact[:, :, far]) <= 1.05 * error
+
+
 @pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
 @pytest.mark.parametrize("O", [20, 100])
 def test_direct_conv2d_f32_scales(ctx, O, powers):

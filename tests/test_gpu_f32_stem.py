@@ -136,6 +136,23 @@ def test_conv_f32_stem_spread(ctx, spread):
     assert error(x, f, np.s_[:]) <= 1.05 * all_of_it
 
 
+def test_conv_f32_stem_beside_an_outlier(ctx):
+    """One value up to 1e6 times larger than its strip's others, which is held with them: they keep their bits, and so do its results."""
+    rng = np.random.Generator(np.random.PCG64(8))
+    x = rng.standard_normal((1, 3, 60, 60)).astype(np.float32)
+    f = rng.standard_normal((40, 3, 7, 7)).astype(np.float32)
+    args = (np.zeros(40, np.float32), 2, (3, 3), (30, 30))
+    far = np.ones((30, 30), bool)
+    far[12:18, 12:18] = False
+    plain, exact = _conv(ctx, x, f, *args), _exact(x, f, *args[1:])
+    error = np.linalg.norm((plain - exact)[:, :, far]) / np.linalg.norm(exact[:, :, far])
+    for value in (3e4, 1e6):
+        x[0, 1, 30, 30] = value
+        got, exact = _conv(ctx, x, f, *args), _exact(x, f, *args[1:])
+        assert (np.abs(got - exact) <= _bound(x, f, *args, exact)).all()
+        assert np.linalg.norm((got - exact)[:, :, far]) / np.linalg.norm(exact[:, :, far]) <= 1.05 * error
+
+
 @pytest.mark.parametrize("powers", [(-100, 0), (0, -100), (-70, -40), (60, -110), (-110, 60), (90, -60)])
 def test_conv_f32_stem_scales(ctx, powers):
     """Results are those of operands of ordinary size, bit for bit: nothing is worked out again because a row is small or large."""
