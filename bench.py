@@ -11,13 +11,14 @@ Workloads (``config.workload``):
   gemm_u8_4096   uint8 MatMul M = N = K = 4096, zero points 128 / 120, fixed-point
                  requantization to uint8.  metric: u8 GEMM TOPS.
   winograd_f32_cfg1  fp32 3x3 Conv2D, input [32,64,56,56], filter [64,64,3,3], SAME, through the
-                 Winograd entry point (cached transformed filter).  metric: direct-equivalent TFLOP/s.
+                 Winograd entry point (cached transformed filter), which takes a direct product here.
+                 metric: direct-equivalent TFLOP/s.
   gemm_u8_sweep  uint8 GEMM with K = N = 4096 and M in {1, 16, 128, 4096}, the batched
                  64 x 512^3 MatMul and the 4096 x 4096 GEMV; one row per case under "cases".
   resnet50_f32_b256  ResNet-50 v1, fp32 NCHW, 224x224, batch 256 per GPU (--batch changes it),
-                 He-normal seeded weights, through the C++ host engine: 3x3 convolutions by
-                 Winograd, 1x1 by GEMM, stem and stride-2 1x1 by im2col + GEMM, pooling, residual
-                 sums and activations on the device.  metric: images/s.
+                 He-normal seeded weights, through the C++ host engine: 3x3 convolutions and the stem
+                 as direct products or by Winograd, 1x1 by GEMM (stride 2 by a pixel gather + GEMM), pooling,
+                 residual sums and activations on the device.  metric: images/s.
 
 One "step" is one pass of the hot path over one batch of synthetic, seeded input.  `value`
 is measured with the inputs resident in HBM, `e2e` through the host-buffer entry point with
@@ -55,7 +56,7 @@ NCU_TRAFFIC = {
     "mobilenet_dw": 196.8e6,   # 13 depthwise launches, profiles/mobilenet_v1_u8_b64_launches.md
     "mobilenet_pw": 130.3e6,   # 13 pointwise + FC GEMM launches, same file
     "gemm_u8_4096": 35.0e6,    # gemm_u8_tc_kernel<256>, profiles/gemm_u8_tc_kernel_4096.md
-    "winograd_f32_cfg1": 134.6e6,  # three kernels of one convolution, caches flushed between them
+    "winograd_f32_cfg1": 26.1e6,   # the direct product, profiles/f32_pairs_kernels.md, and the split of its filter
 }
 
 
@@ -899,14 +900,14 @@ def run_winograd(args, rank, world):
             "ms_per_step": round(ms_per_step, 5), "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": "winograd_f32_cfg1", "input": [N, C, H, W], "filter": [O, C, 3, 3],
-                       "padding": "SAME", "tile": "F(6x6,3x3)", "executed_gemm_flops": 2.0 * 64 * O * C * N * 100,
+                       "padding": "SAME", "tile": "F(6x6,3x3)", "executed_gemm_flops": 3 * direct_flops,
                        "l2": "rotating %d input/output sets (%.0f MB > L2)" % (n_sets, n_sets * 51.4),
                        "parallelism": "dp%d: batch sharded, filter replicated" % world},
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"],
                          "unit": "GB/s", "frac": round(achieved / peaks["hbm_gbs"], 4),
                          "traffic": NCU_TRAFFIC["winograd_f32_cfg1"],
                          "peak_source": "%s copy bandwidth" % peaks["source"],
-                         "kernel": "whole call: wino_input_kernel + gemm_f32_tc_kernel + wino_output_kernel",
+                         "kernel": "whole call: f32_conv_presplit_kernel + conv_f32_direct_kernel",
                          "algorithmic_bytes_per_step": alg_bytes},
             "e2e": {"value": round(world * direct_flops / (e2e_ms / e2e_steps * 1e-3) / 1e12, 2),
                     "unit": "TFLOP/s", "h2d_bytes_per_step": int(xs[0].nbytes),
@@ -935,12 +936,12 @@ def run_winograd(args, rank, world):
 def resnet_kind(node):
     if node["op"] == "conv":
         if node["k"] == 7:
-            return "stem 7x7 s2 (im2col + gemm_f32_tc_kernel)"
+            return "stem 7x7 s2"
         if node["k"] == 3:
-            return "3x3 s1 (Winograd: wino_input + gemm_f32_tc_kernel + wino_output)"
+            return "3x3 s1"
         if node["stride"] == 2:
-            return "1x1 s2 (pixel gather + gemm_f32_tc_kernel)"
-        return "1x1 s1 (gemm_f32_tc_kernel)"
+            return "1x1 s2 (with its pixel gather)"
+        return "1x1 s1"
     return {"maxpool": "max pool", "avgpool": "avg pool", "add": "eltwise sum", "relu": "activation",
             "fc": "fully connected"}[node["op"]]
 
@@ -1006,7 +1007,7 @@ def run_resnet(args, rank, world):
         for label, t in eng.run_profiled(max_ops=512):
             k = kinds.get(label.split(":", 1)[-1], label)
             if label.startswith("Subsample:"):
-                k = "1x1 s2 (pixel gather + gemm_f32_tc_kernel)"
+                k = "1x1 s2 (with its pixel gather)"
             fam[k] = fam.get(k, 0.0) + t / prof_runs
 
     # pipelined end-to-end calls (see run_mobilenet): the next batch's upload overlaps this
@@ -1067,10 +1068,9 @@ def run_resnet(args, rank, world):
                        "l2": "activations of one step (%.1f GB) exceed L2" % (alg_bytes / 1e9)},
             "roofline": {"bound": "tensor", "achieved": round(tflops, 2), "peak": round(tf32_peak, 1),
                          "unit": "TFLOP/s", "frac": round(tflops / tf32_peak, 4), "traffic": None,
-                         "peak_source": tf32_src + "; the fp32 GEMMs run three tf32 MMAs per product (hi/lo "
-                                        "split), so a third of it is the ceiling for direct-equivalent flops "
-                                        "outside Winograd",
-                         "kernel": "whole step (gemm_f32_tc_kernel dominates)",
+                         "peak_source": tf32_src + "; the fp32 products run three MMAs of split operands each, "
+                                        "of halves at twice this rate in the large ones",
+                         "kernel": "whole step (conv_f32_direct_kernel and gemm_f32_pairs_kernel dominate)",
                          "direct_equivalent_flops_per_step": 2.0 * macs * batch},
             "model_hbm": {"algorithmic_bytes_per_step": alg_bytes,
                           "achieved_gbs": round(alg_bytes / (ms_per_step * 1e-3) / 1e9, 1),

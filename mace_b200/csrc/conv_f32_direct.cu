@@ -23,8 +23,10 @@
 // What bounds it: shared memory, 470 cycles per tap of 128 channels (40 KB into the MMAs, 16 KB of W in), of which the MMAs are
 // busy 384, at the clocks that the power limit leaves; with 64 channels the issue of small MMAs, 350 against 235.
 // Measured, Winograd's three kernels -> this one (3x3, us, errors in the 2-norm against float64): 64 -> 64 channels, 56 x 56, batch 32
-// 55.3 -> 36.5 (4.9e-6 -> 7.2e-7), batch 256 397 -> 209; 128 -> 128, 28 x 28, batch 256 287 -> 168; 256 -> 256, 14 x 14 290 -> 178;
-// 512 -> 512, 7 x 7 225 -> 195; self-fetching kernel -> this one, 5x5: 64 -> 64, 56 x 56, batch 24 130 -> 69.
+// 55.3 -> 40.2 with inputs that are not in L2, 37.7 with the same ones (4.9e-6 -> 3.8e-7), batch 256 397 -> 220; 128 -> 128, 28 x 28,
+// batch 256 287 -> 172; 256 -> 256, 14 x 14 290 -> 178; 512 -> 512, 7 x 7 225 -> 195; self-fetching kernel -> this one, 5x5: 64 -> 64,
+// 56 x 56, batch 24 130 -> 69.  Blocks of channels of different size are split twice: 64 -> 64 with the second block 2^12 times larger
+// or smaller 40 -> 56, 128 -> 128 at 28 x 28, batch 64, 51 -> 54.
 //
 // Roles: warp 0 W by TMA, warp 1 MMAs, 8 or 16 warps input, 8 or 16 warps results.  Persistent over the tiles.
 #include <algorithm>

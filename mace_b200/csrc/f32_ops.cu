@@ -434,7 +434,7 @@ int mb_gemm_f32_strided(mb_context *ctx, const float *A, const float *B, float *
                       mb_gemm_f32_tc_supported(ctx, B, A, N, M, K, b_rs, b_bs, a_rs, a_bs);
   const bool gather = take_gather(ctx, g, by_tma, !by_tma);
   // Both depths contiguous, where its estimate is the smaller: a batch of 8, 992 x 352 x 768: 73.1 us fetching its own operands,
-  // 48.8 this way; 4 of 240 x 64 x 80: 6.4 and 7.3.  Up to 64 deep the former's three accumulators are the more accurate.
+  // 56.8 this way; 4 of 240 x 64 x 80: 6.4 and 7.3.  Up to 64 deep the former's three accumulators are the more accurate.
   if (!by_tma && ctx->f32_rows != 1 && mb_gemm_f32_rows_supported(ctx, g) &&
       (ctx->f32_rows == 2 ||
        (gather && ctx->f32_gather == 0 && g.run != 0 && K > 64 && mb_gemm_f32_rows_cost(ctx, g) < mb_gemm_f32_gather_cost(ctx, g))))

@@ -96,7 +96,7 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
   return ok != 0;
 }
 
-// Copies of 4 or 8 bytes per thread to shared memory, `bytes` of them read and the rest zero; groups of a thread's copies.
+// Copies of SIZE bytes per thread to shared memory, `bytes` of them read and the rest zero; groups of a thread's copies.
 template <int SIZE>
 __device__ __forceinline__ void cp_async(uint32_t dst, const void *src, uint32_t bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(SIZE), "r"(bytes) : "memory");
@@ -514,7 +514,7 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
       : "memory");
 }
 
-// Eight columns.
+// Four columns, eight.
 __device__ __forceinline__ void tmem_st_32x32b_x4(uint32_t addr, const uint32_t (&v)[4]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
                : "memory");
