@@ -339,9 +339,7 @@ int mb_conv2d_f32_nchw(mb_context *ctx, const float *in, const float *filter_oih
  * convolution and then one sum + activation pass in place.  The values are
  * those of the separate operators: (acc + bias) + residual, then the
  * activation.  residual == NULL is mb_conv2d_f32_nchw.  residual may be out
- * itself where one kernel does it all (every shape but those beyond the limits
- * of the tensor-core kernels, which answer MB_UNSUPPORTED then); a sum that is
- * infinite may come out as NaN in that case. */
+ * itself; a sum that is infinite may come out as NaN then. */
 int mb_conv2d_f32_nchw_residual(mb_context *ctx, const float *in,
                                 const float *filter_oihw, const float *bias,
                                 const float *residual, float *out, int64_t N,

@@ -719,12 +719,20 @@ int mb_conv2d_f32_nchw_residual(mb_context *ctx, const float *in, const float *f
                                  activation, max_limit, coefficient, residual);
   }
   // every other shape: the convolution without activation, then sum + activation in place
-  if (mb_ranges_meet(residual, out, N * O * Ho * Wo * 4))
-    return mb_fail(ctx, MB_UNSUPPORTED, "mb_conv2d_f32_nchw_residual: the residual lies in the output, which is written before the sum");
-  MB_RETURN_IF_ERROR(mb_conv2d_f32_nchw(ctx, in, filter, bias, out, N, C, H, W, O, KH, KW, stride_h, stride_w,
-                                        dil_h, dil_w, pad_top, pad_left, Ho, Wo, 0, 0.f, 0.f));
-  return mb_eltwise_act_f32(ctx, out, residual, out, N * O * Ho * Wo, 0, 0.f, 0, 0.f, 0.f, 0, activation,
-                            max_limit, coefficient);
+  // (of a copy of the residual where it lies in the output)
+  const int64_t count = N * O * Ho * Wo;
+  float *copy = nullptr;
+  if (mb_ranges_meet(residual, out, count * 4)) {
+    MB_CUDA(ctx, cudaMallocAsync(reinterpret_cast<void **>(&copy), count * 4, ctx->stream));
+    MB_CUDA(ctx, cudaMemcpyAsync(copy, residual, count * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    residual = copy;
+  }
+  int status = mb_conv2d_f32_nchw(ctx, in, filter, bias, out, N, C, H, W, O, KH, KW, stride_h, stride_w, dil_h, dil_w, pad_top,
+                                  pad_left, Ho, Wo, 0, 0.f, 0.f);
+  if (status == MB_SUCCESS)
+    status = mb_eltwise_act_f32(ctx, out, residual, out, count, 0, 0.f, 0, 0.f, 0.f, 0, activation, max_limit, coefficient);
+  if (copy != nullptr) MB_CUDA(ctx, cudaFreeAsync(copy, ctx->stream));
+  return status;
 }
 
 int mb_dwconv_f32_nchw(mb_context *ctx, const float *in, const float *filter, const float *bias,

@@ -1,5 +1,7 @@
 """The fp32 GEMM on pairs of halves (gemm_f32_pairs.cu) against float64, with bounds derived from its arithmetic, at the edges of
 its tiles, and where its split of a value into two halves does not reach."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -86,10 +88,13 @@ def test_conv1x1_f32_pairs(ctx, shape, act, residual):
         b.free()
 
 
+@pytest.mark.parametrize("captured", [False, True])
 @pytest.mark.parametrize("where", ["pairs", "gather", "neither"])
-def test_conv1x1_f32_residual_in_place(ctx, where):
+def test_conv1x1_f32_residual_in_place(where, captured):
     """A residual that is the output itself: nothing is read where a result already stands."""
     import mace_b200
+    ctx = mace_b200.Context(0)
+    L = mace_b200.lib()
     N, C, HW, O = 2, 132, 144, 48
     rng = np.random.Generator(np.random.PCG64(O))
     x = rng.standard_normal((N, C, HW)).astype(np.float32)
@@ -97,33 +102,34 @@ def test_conv1x1_f32_residual_in_place(ctx, where):
     r = rng.standard_normal((N, O, HW)).astype(np.float32)
     x[:, 96:, ::3] *= np.float32(2.0 ** 20)
     x[1, 50, 9], f[21, 100] = np.inf, -np.inf
-    dx, df, do = ctx.upload(x), ctx.upload(f), ctx.upload(r)
-    options = {"pairs": {"f32_gather": 1, "f32_pairs": 2}, "gather": {"f32_gather": 2}, "neither": {"tensor_cores": 0}}[where]
-    for name, value in options.items():
+    dx, df, do, dr = ctx.upload(x), ctx.upload(f), ctx.upload(r), ctx.upload(r)
+    for name, value in {"pairs": {"f32_gather": 1, "f32_pairs": 2}, "gather": {"f32_gather": 2}, "neither": {"tensor_cores": 0}}[where].items():
         ctx.set_option(name, value)
-    try:
-        if where == "neither":
-            with pytest.raises(mace_b200.MaceB200Error):
-                ctx.conv2d_f32_residual(dx, df, None, do, do, N, C, 36, 4, O, 1, 1, (1, 1), (1, 1), (0, 0), (36, 4))
-        else:
-            ctx.conv2d_f32_residual(dx, df, None, do, do, N, C, 36, 4, O, 1, 1, (1, 1), (1, 1), (0, 0), (36, 4))
-    finally:
-        for name in options:
-            ctx.set_option(name, int(name == "tensor_cores"))
+
+    def call(out):
+        ctx.conv2d_f32_residual(dx, df, None, out, out, N, C, 36, 4, O, 1, 1, (1, 1), (1, 1), (0, 0), (36, 4))
+
+    if captured:
+        call(dr)
+        g = ctypes.c_void_p()
+        ctx._check(L.mb_graph_begin(ctx.h))
+        call(do)
+        ctx._check(L.mb_graph_end(ctx.h, ctypes.byref(g)))
+        ctx._check(L.mb_graph_launch(ctx.h, g))
+    else:
+        call(do)
     got = ctx.download(do, (N, O, HW), np.float32)
-    for b in (dx, df, do):
-        b.free()
-    if where == "neither":
-        assert np.array_equal(got, r)
-        return
+    if captured:
+        ctx._check(L.mb_graph_destroy(ctx.h, g))
+    ctx.close()
     x, f = x.astype(np.float64), np.broadcast_to(f.astype(np.float64), (N, O, C))
     with np.errstate(all="ignore"):
         ref = f @ x + r
         finite = np.isfinite(ref)
     x, f = np.where(np.isfinite(x), x, 0), np.where(np.isfinite(f), f, 0)
     assert finite.mean() > 0.9 and np.array_equal(np.isfinite(got), finite)
-    # (tf32 pairs: 22 bits, an accumulator cut off after each of twelve MMAs per 32 of k)
-    bound = (np.abs(f) @ np.abs(x)) * (2.0 ** -20 + (12 * C / 32 + 4) * 2.0 ** -23) + 1e-6
+    # (tf32 pairs: 22 bits, an accumulator cut off after each of twelve MMAs per 32 of k; fp32 FMAs: a rounding for each of k)
+    bound = (np.abs(f) @ np.abs(x)) * (2.0 ** -20 + (12 * C / 32 + C + 4) * 2.0 ** -23) + 1e-6
     assert (np.abs(got[finite] - ref[finite]) <= bound[finite]).all()
 
 
